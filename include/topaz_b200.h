@@ -73,7 +73,7 @@ TPZ_API int tpz_matrix(const char *name, int8_t *out625);
  * (query, subject) pairs with exactly the results of
  *   ssw_init(query, qlen, mat, 25, 2) + ssw_align(prof, subject, slen,
  *   gap_open, gap_extend, 0, 0, 0, 15)            (src/ssw.c:799-897)
- * i.e. the u8 pass, its i16 rerun on saturation, and the drop at 32767.
+ * i.e. of the u8 pass, its i16 rerun on saturation, and the drop at 32767.
  * Replaces the per-hit calls in perform_alignment_with_profile
  * (src/query.c:304-340) / align_using_ssw_profile (src/ssw_wrapper.c:157-245).
  *
@@ -116,10 +116,9 @@ TPZ_API int tpz_sw_align_one(const int8_t *q, int32_t qlen, const int8_t *s, int
  * tpz_sw_batch_device; at most TPZ_SW_NOALLOC_MAX_PAIRS pairs per call
  * (TPZ_E_RANGE beyond), queries of at most TPZ_SW_NOALLOC_MAX_QLEN
  * residues (longer ones get status TPZ_SW_INVALID) and matrices whose
- * largest entry is at most TPZ_SW_NOALLOC_MAX_ENTRY (TPZ_E_ARG beyond: such
- * scores can pass the 16-bit range, and the allocating call's 32-bit rerun
- * needs scratch of its own).  Scratch is one static device array per device
- * (about 0.6 MB, held until the process exits) shared by all calls: calls
+ * largest entry is at most TPZ_SW_NOALLOC_MAX_ENTRY (TPZ_E_ARG beyond, so
+ * that no score reaches 32767).  Scratch is one static device array per
+ * device (about 0.4 MB, held until the process exits) shared by all calls: calls
  * whose work overlaps on the GPU (other streams or threads) race on it, so
  * order them on one stream.  All work goes to `stream`; nothing is
  * allocated or freed.  The first call on a device does a one-time set-up

@@ -1084,7 +1084,7 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
             rc = tpz::sw::batch_device_grouped(npairs, (const int8_t *)dq, pq_off, pq_len,
                                                (const int8_t *)ix->d.T, ps_off, ps_len, o->mat625,
                                                o->gap_open, o->gap_extend, sc, re, rd, st, 0, xmap,
-                                               xmap, report ? 1 : 0, nq, dpoff, poff.data(),
+                                               xmap, report ? 1 : 0, nq, poff.data(),
                                                qlen_eff.data());
             if (rc) return bail(rc);
             scatter_sw_kernel<<<(unsigned)std::min<int64_t>((npairs + 255) / 256, 4096), 256>>>(

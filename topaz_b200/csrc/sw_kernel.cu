@@ -1,58 +1,38 @@
 // sw_kernel.cu -- batched Smith-Waterman (scores + end coordinates) for sm_100a.
 //
-// Result semantics: exactly those of TOPAZ's striped SSW calls
-//   ssw_init(q, qlen, mat, 25, 2); ssw_align(prof, s, slen, go, ge, 0, 0, 0, 15)
-// (src/ssw.c:799-897): the u8 pass, the i16 pass when the u8 pass saturates
-// (max + bias >= 255), and the drop when the i16 pass reaches 32767.
+// The recurrence, its arithmetic and why one pass gives the results of SSW's
+// u8 and i16 passes stand in sw_core.cuh.  Here: how alignments are laid on
+// warps, binned and launched.
 //
-// The striped u8/i16 passes split the query into 16 (u8) or 8 (i16) SSW
-// "lanes" of seg = ceil(qlen/lanes) consecutive rows.  What they compute is
-// the recurrence below (pinned against src/ssw.c by the oracle tests):
-//   Hp(r,c) = max(0, H(r-1,c-1) + M[s_c][q_r], E(r,c), Fm(r,c))
-//   H(r,c)  = max(Hp(r,c), F(r,c))
-//   E(r,c+1)= max(E(r,c) - ge, Hp(r,c) - go)
-//   Fm(r+1) = (r+1) % seg == 0 ? 0 : max(Fm(r) - ge, Hp(r) - go)
-//   F(r+1)  = max(F(r) - ge, H(r) - go)
-// With X = max(0, H(r-1,c-1) + M, E) and Xg = X - go, and gap_open >
-// gap_extend, this is the same as
-//   H = max(X, F);  Gp = max(Fm - go, Xg);  E' = max(E - ge, Gp)
-//   F' = max(F - ge, Xg);  Fm' = max(Fm - ge, Xg)  (Fm cleared at SSW lane starts)
-// in which the only serial dependences from row to row are the F and Fm
-// chains, one DPX op each.  ref_end is the first column holding the maximum,
-// read_end the smallest row holding it there (src/ssw.c:264-297).
+// Throughput form (queries of one stripe, <= 1024 residues).  One warp per
+// task; a group of G = 4, 8, 16 or 32 lanes holds two pairs in the halves of
+// its u16x2 words, lane t owning query rows [t*R, t*R + R) of both.  Subject
+// columns stream through a group's lanes as a wavefront, lane t working on
+// column k - t at step k, with H and F of a lane's last row handed to lane
+// t + 1 by __shfl_up_sync.  G is the smallest group that keeps R <= 32, so R
+// is 17..32 for every query above 64 residues: the wavefront's fill (G - 1
+// steps) and the per-step work outside the rows (shuffles, letters, maximum
+// test) shrink against the rows, and a query pads to G*R rows, at most G - 1
+// more than it has.  Groups of a warp take pairs of neighbouring subject
+// lengths.
 //
-// Kernel layout (B200): one warp per task of two pairs packed as int16x2
-// (pair A in the low half, pair B in the high half).  Lane t owns query rows
-// [t*R, t*R+R) of both pairs; subject columns stream through the lanes as a
-// wavefront, lane t working on column k-t at step k, with H/F/Fm of a lane's
-// last row and the subject letters handed to lane t+1 by __shfl_up_sync.
-// Every cell update is a DPX instruction (__viaddmax_s16x2[_relu],
-// __vimax_s16x2_relu, __vimax3_s16x2).  The int8 query profile of both pairs
-// sits in shared memory in a lane-blocked layout with an odd word stride per
-// lane, so the 32 per-lane loads of a step never share a bank; prmt with the
-// sign-replicate selector widens two profile bytes into one int16x2 operand.
+// Query-major form (the hits of one search query): the same, with a block of
+// 8 warps sharing one profile.
 //
-// End coordinates: each lane keeps the running maximum of its rows and the
-// column/row where it last rose.  A rise is only looked at when it reaches
-// the warp maximum of the last refresh (every 32 steps; a lower value cannot
-// be the alignment's maximum), and then the whole warp finds the first row
-// holding the new value with packed DPX ops, so the common case costs one
-// vote per step.  Steps run two at a time, the profile words ping-ponging
-// between two register sets.
+// Stripe form (queries longer than 1024, and batches too small to fill the
+// GPU with warps): W warps per pair; the halves of a warp's words are two row
+// ranges of one alignment, so a warp covers 64*R rows, and the warps of a
+// pair follow each other three blocks of 32 columns apart, passing the last
+// row of one to the first of the next through a ring in shared memory.
 //
-// Pairs are binned on the device by R = ceil(qlen/32) and by subject length
-// (counting sort), paired two per task within a bin, and drained by one
-// persistent kernel per R from an atomic task counter.  Pairs whose u8-pass
-// maximum saturates are appended to their bin's rerun list and re-run with
-// the i16 lane length (seg = ceil(qlen/8)) by a second kernel of the bin on
-// the same stream.  With qlen <= 1024 and |M| <= 127 no score can reach
-// 32767, so 16-bit arithmetic is exact.
+// The int8 query profile sits in shared memory, one column per lane, so the
+// 32 loads of a step never share a bank; PRMT with the sign-replicate
+// selector widens two profile bytes into one operand.  Subject letters sit
+// in rings of 128 columns as profile offsets, refilled 32 columns at a time.
 //
-// Every lane computes every step, also before its first column and past
-// the subject's end (pad letters there), so the step body has no per-lane
-// column test; the refresh every 32 steps and the row search of a risen
-// column (one step late, between the next column's two phases) are the
-// only branches.
+// Pairs are binned on the device by query length class and subject length
+// (counting sort), longest subjects first, and each R has one persistent
+// kernel that drains its bins from an atomic task counter.
 
 #include <stdio.h>
 #include <string.h>
@@ -60,651 +40,469 @@
 #include <algorithm>
 #include <mutex>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "search_internal.cuh"
+#include "sw_core.cuh"
 #include "tpz_common.cuh"
 
 namespace tpz {
 namespace sw {
 
-constexpr int kMaxR = 32;           // rows per lane; one stripe = 32 lanes x R rows
-constexpr int kStripeRows = 32 * kMaxR;
-constexpr int kMaxStripes = (TPZ_SW_MAX_QLEN + kStripeRows - 1) / kStripeRows;
-// row bins: b < 32 -> R = b+1, one stripe; b = 32..38 -> R = 32, b-30 stripes
-constexpr int kRBins = 40;
-constexpr int kSBins = 256;         // subject-length buckets (32 residues each)
-constexpr int kBins = kRBins * kSBins;
-constexpr int kPadLetter = 25;      // subject column past a pair's end
-constexpr int kPadScore = -64;      // profile value of pad rows / pad columns
-constexpr int kMatStride = 32;      // shared matrix row stride (bytes)
-constexpr int kSmatBytes = 26 * kMatStride;
-
-// profile words per lane and pair: 4 rows per word
-__host__ __device__ constexpr int words_for(int R) { return (R + 3) / 4; }
-__host__ __device__ constexpr int profile_bytes(int R) { return 26 * 32 * 4 * words_for(R); }
-constexpr int kRing = 128;          // subject-letter ring per warp (uint16 letter pairs)
-__host__ __device__ constexpr int smem_bytes(int R) {
-    return kSmatBytes + 2 * profile_bytes(R) + 2 * kRing;
-}
-// Fm "cleared" at an SSW lane start: any value <= 0 acts like the cleared
-// one there, so the start row adds -kBig instead of masking (exact while
-// every score stays below kBig; larger scores take the 32-bit rerun).
+constexpr int kStripeRows = 32 * kMaxR;     // longest query of the throughput form
+// scores of tpz_sw_align_one and the allocation-free call stay below this
 constexpr int kBig = 32512;
 
-struct Args {
-    const int8_t *q;
-    const int64_t *qoff;
-    const int32_t *qlen;
-    const int8_t *s;
-    const int64_t *soff;
-    const int32_t *slen;
-    int32_t *score, *ref_end, *read_end, *status;
-    const int32_t *sorted;   // pair ids sorted by bin
-    const int32_t *rinfo;    // per R bin: [start, count]
-    int32_t *next_task;      // per R bin task counter
-    int32_t *rerun;          // pairs that need the i16 lane length
-    int32_t *rerun_count;
-    // per row bin (null: one list for all bins): the u8 pass of bin b appends
-    // its saturated pairs at rerun + rinfo[2b] and counts them here, so the
-    // i16 pass of the bin can follow it on the same stream
-    int32_t *rerun_bin_count;
-    // null: a bin's pairs are sorted[rinfo[2b] ..] and number rinfo[2b + 1];
-    // else the count is task_count[b] (the i16 pass over a bin's rerun list)
-    const int32_t *task_count;
-    int ssw_lanes;           // 16 (u8 pass) or 8 (i16 pass)
-    int gap_open, gap_extend, bias;
-    int translate;           // 1: q/s bytes go through xq/xs first
-    int score_only;          // 1: scores only, no end coordinates (ref_end = read_end = -2)
-    uint32_t *bnd;           // stripe boundary rows, bnd_words per block (multi-stripe bins)
-    int64_t bnd_words;
-    int32_t *exact_list;     // i16-pass pairs near 32767: re-run in 32-bit arithmetic
-    int32_t *exact_count;
-    int exact_threshold;
-    int8_t mat[625];
-    int8_t xq[128], xs[128]; // byte -> matrix index (internal alphabet inputs)
-};
+// row counts per lane with a kernel: 4, 8 and 9..32
+constexpr int kRs = 26;
+__host__ __device__ constexpr int rows_of(int i) { return i < 2 ? 4 * (i + 1) : 7 + i; }
+__host__ __device__ constexpr int rows_index(int R) { return R <= 8 ? (R + 3) / 4 - 1 : R - 7; }
 
-__device__ __forceinline__ uint32_t pack2(int lo, int hi) {
-    return (uint32_t)(uint16_t)(int16_t)lo | ((uint32_t)(uint16_t)(int16_t)hi << 16);
-}
-__device__ __forceinline__ int lo16(uint32_t x) { return (int)(int16_t)(x & 0xFFFFu); }
-__device__ __forceinline__ int hi16(uint32_t x) { return (int)(int16_t)(x >> 16); }
+// Row bins.  Throughput form: queries above 32 residues with G = 32 lanes
+// and R = 9..32 in bins R - 9, with G = 16, 8, 4 and R = 9..16 in bins 24,
+// 32, 40 + R - 9, shorter ones with G = 4 and R = 4, 8 in bins 48, 49.
+// Stripe form: 50..52 for queries up to 2048, 4096 and 8192, and 53, 54 for
+// the short queries of small batches, up to 512 and 1024.
+constexpr int kRBins = 56;
+constexpr int kTinyBin = 48;
+constexpr int kLongBin = 50;
+constexpr int kSmallBin = 53;
+constexpr int kSBins = 256;                 // subject-length buckets (32 residues each)
+constexpr int kBins = kRBins * kSBins;
+static_assert(kBins % 1024 == 0, "the scan gives each of 1024 threads an equal share");
 
-__device__ __forceinline__ uint64_t best_key(int v, int col, int row) {
-    return v > 0 ? ((uint64_t)v << 40) | ((uint64_t)(0xFFFFFF - col) << 16) |
-                       (uint64_t)(0xFFFF - row)
-                 : 0ull;
+// lanes of a group for a query of one stripe
+__host__ __device__ __forceinline__ int group_lanes(int ql) {
+    return ql <= 64 ? 4 : ql <= 128 ? 8 : ql <= 256 ? 16 : 32;
 }
 
-// letter pair (A low byte, B high byte) of subject column c; past a
-// subject's end, and for bytes outside the alphabet, the pad letter
-__device__ __forceinline__ uint32_t letter_pair(const Args &a, const int8_t *sA, int slA,
-                                                const int8_t *sB, int slB, int c) {
-    int la = kPadLetter, lb = kPadLetter;
-    if (c < slA) {
-        la = sA[c];
-        if (a.translate) la = a.xs[la & 127];
-        if ((unsigned)la >= 25u) la = kPadLetter;
-    }
-    if (c < slB) {
-        lb = sB[c];
-        if (a.translate) lb = a.xs[lb & 127];
-        if ((unsigned)lb >= 25u) lb = kPadLetter;
-    }
-    return (uint32_t)la | ((uint32_t)lb << 8);
+__device__ __forceinline__ int row_bin(int ql, int small_batch) {
+    if (ql > kStripeRows) return kLongBin + (ql <= 2048 ? 0 : ql <= 4096 ? 1 : 2);
+    if (small_batch) return kSmallBin + (ql <= 512 ? 0 : 1);
+    if (ql <= 32) return kTinyBin + (ql - 1) / 16;
+    const int G = group_lanes(ql);
+    return (G == 32 ? 0 : G == 16 ? 24 : G == 8 ? 32 : 40) + (ql + G - 1) / G - 9;
 }
 
-// One task: pairs pA and pB (pB < 0: none) in the halves of the int16x2
-// lanes.  The pass (16 SSW lanes = u8, 8 = i16) comes from `a` (QM = false)
-// or, for the query-major kernel, from qm_lanes; saturated u8 results go to
-// qm_rerun / qm_rerun_count when given, else to a.rerun / a.rerun_count.
-// QM = true also means that profA/profB already hold the query profile
-// (both pairs share it).
-template <int R, bool MULTI, bool QM = false, bool SCORE = false>
-__device__ __forceinline__ void run_task(const Args &a, int pA, int pB, const int8_t *smat,
-                                         uint32_t *profA, uint32_t *profB, uint16_t *ring,
-                                         int stripes, uint32_t *bnd, int qm_lanes = 0,
-                                         int32_t *qm_rerun = nullptr,
-                                         int32_t *qm_rerun_count = nullptr) {
-    constexpr bool BUILD = !QM;
-#define TPZ_LANES (QM ? qm_lanes : a.ssw_lanes)
-    constexpr int W = words_for(R);
+// ---------------------------------------------------------- one warp's task
+
+// bytes of a group's letter rings, low and high half
+constexpr int kPairRing = 2 * kRingCols * 2;
+
+// Up to 64 / G pairs, two per group of G lanes: pair_at(first), ..., below
+// `count`.  prof: this warp's two profiles (BUILD), or the block's one
+// profile of the query they share; rings: 32 / G pairs of letter rings.
+template <int R, bool ENDS, bool BUILD, class PairAt>
+__device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int first, int count, int G,
+                                          const uint8_t *matT, uint8_t *prof, uint8_t *rings) {
     const int lane = threadIdx.x & 31;
-
-    const int qlA = a.qlen[pA];
-    const int slA = a.slen[pA];
-    const int8_t *qA = a.q + a.qoff[pA];
-    const int8_t *sA = a.s + a.soff[pA];
-    const int qlB = pB >= 0 ? a.qlen[pB] : 0;
-    const int slB = pB >= 0 ? a.slen[pB] : 0;
-    const int8_t *qB = pB >= 0 ? a.q + a.qoff[pB] : qA;
-    const int8_t *sB = pB >= 0 ? a.s + a.soff[pB] : sA;
-    const int N = max(slA, slB);
-    const int segA = max(1, (qlA + TPZ_LANES - 1) / TPZ_LANES);
-    const int segB = max(1, (qlB + TPZ_LANES - 1) / TPZ_LANES);
-    const uint32_t NGO = pack2(-a.gap_open, -a.gap_open);
-    const uint32_t NGE = pack2(-a.gap_extend, -a.gap_extend);
-    const uint32_t NEGINF = 0x80008000u;
-    // sign-extend byte r%4 of the A word into the low half, of the B word
-    // into the high half
-    constexpr uint32_t SEL[4] = {0xC480u, 0xD591u, 0xE6A2u, 0xF7B3u};
-    uint64_t kA = 0, kB = 0;
-    bool decided = false;      // u8 pass: both pairs already go to the i16 pass
-
-    // Queries longer than one stripe (32 lanes x R rows) run stripe after
-    // stripe; the last row of a stripe (H, F, Fm per column) goes to `bnd`
-    // and enters the next stripe at lane 0.  Lane 0 reads column k at step k
-    // and lane 31 writes column k-31 at step k, so one buffer serves as both.
-    const int nstripes = MULTI ? stripes : 1;
-    for (int st = 0; st < nstripes; ++st) {
-    const int i0 = (st * 32 + lane) * R;
-
-    // ---- profile of this lane's rows for all 26 letters (25 + pad column),
-    // word w of letter l at [(l * W + w) * 32 + lane]: conflict-free per lane
-    if constexpr (BUILD) {
-    int qa[R], qb[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        qa[r] = (i0 + r < qlA) ? qA[i0 + r] : -1;
-        qb[r] = (i0 + r < qlB) ? qB[i0 + r] : -1;
-        if (a.translate) {
-            if (qa[r] >= 0) qa[r] = a.xq[qa[r] & 127];
-            if (qb[r] >= 0) qb[r] = a.xq[qb[r] & 127];
-        }
-        if (qa[r] >= 25) qa[r] = -1;
-        if (qb[r] >= 25) qb[r] = -1;
+    const int lg = 31 - __clz(G), grp = lane >> lg, gl = lane & (G - 1);
+    const int iA = first + 2 * grp, iB = iA + 1;
+    const int pA = iA < count ? pair_at(iA) : -1, pB = iB < count ? pair_at(iB) : -1;
+    const int slA = pA >= 0 ? a.slen[pA] : 0, slB = pB >= 0 ? a.slen[pB] : 0;
+    const int8_t *sA = a.s + (pA >= 0 ? a.soff[pA] : 0), *sB = a.s + (pB >= 0 ? a.soff[pB] : 0);
+    const int N = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)max(slA, slB));
+    uint16_t *ringA = reinterpret_cast<uint16_t *>(rings + grp * kPairRing), *ringB = ringA + kRingCols;
+    Flow f;
+    f.profA = prof + lane * 4;
+    f.profB = f.profA + (BUILD ? profile_bytes(R) : 0);
+    if (BUILD) {
+        build_profile<R>(a, a.q + (pA >= 0 ? a.qoff[pA] : 0), pA >= 0 ? a.qlen[pA] : 0, gl * R, matT,
+                         prof + lane * 4);
+        build_profile<R>(a, a.q + (pB >= 0 ? a.qoff[pB] : 0), pB >= 0 ? a.qlen[pB] : 0, gl * R, matT,
+                         prof + profile_bytes(R) + lane * 4);
+    }
+    f.ringA = ringA; f.ringB = ringB;
+    f.lag = gl; f.lagB = 0; f.width = G;
+    f.mul = gl == 0 ? 0u : 1u;
+    f.add = gl == 0 ? both((uint32_t)a.floor) : 0u;
+    f.bnd = nullptr; f.bnd_end = 0;
+    // columns 0..63, and pad letters where the columns before 0 are read
+#pragma unroll 4
+    for (int c = gl; c < 64; c += G) {
+        ringA[c] = letter_offset<R>(a, sA, slA, c);
+        ringB[c] = letter_offset<R>(a, sB, slB, c);
+        ringA[64 + c] = ringB[64 + c] = kPadLetter * words_for(R) * 128;
     }
     __syncwarp();
-    for (int let = 0; let < 26; ++let) {
-        const int8_t *mrow = smat + let * kMatStride;
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            uint32_t wa = 0, wb = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int r = 4 * w + k;
-                int va = kPadScore, vb = kPadScore;
-                if (r < R) {
-                    if (qa[r] >= 0) va = mrow[qa[r]];
-                    if (qb[r] >= 0) vb = mrow[qb[r]];
-                }
-                wa |= (uint32_t)(uint8_t)(int8_t)va << (8 * k);
-                wb |= (uint32_t)(uint8_t)(int8_t)vb << (8 * k);
-            }
-            profA[(let * W + w) * 32 + lane] = wa;
-            profB[(let * W + w) * 32 + lane] = wb;
-        }
-    }
-    }   // BUILD
-    // ---- subject letters: columns 0..63 in the ring, 64..95 in flight;
-    // every 32 steps the lanes store the next 32 columns and fetch 32 more
-    ring[lane] = (uint16_t)letter_pair(a, sA, slA, sB, slB, lane);
-    ring[32 + lane] = (uint16_t)letter_pair(a, sA, slA, sB, slB, 32 + lane);
-    ring[64 + lane] = (uint16_t)(kPadLetter | (kPadLetter << 8));
-    ring[96 + lane] = (uint16_t)(kPadLetter | (kPadLetter << 8));
-    uint32_t pre = letter_pair(a, sA, slA, sB, slB, 64 + lane);
-    __syncwarp();
-
-    // ---- SSW lane starts: the Fm terms of a start row add -kBig
-    uint32_t ngo[R], nge[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const bool sa = (i0 + r) % segA == 0, sb = (i0 + r) % segB == 0;
-        ngo[r] = pack2(sa ? -kBig : -a.gap_open, sb ? -kBig : -a.gap_open);
-        nge[r] = pack2(sa ? -kBig : -a.gap_extend, sb ? -kBig : -a.gap_extend);
-    }
-
-    uint32_t E[R], H[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) { E[r] = 0u; H[r] = 0u; }
-
-    uint32_t outH = 0u, outF = 0u, outFm = 0u;
-    uint32_t diag = 0u;
-    uint32_t runmax = 0u, wmax = 0u;
-    int colA = -1, rowA = 0, colB = -1, rowB = 0;
-
-    // profile words of this step's column (j = k - lane), fetched one step
-    // ahead; the letter pair of the column after it
-    uint32_t wa[W], wb[W];
-    {
-        const uint32_t l = ring[(-lane) & (kRing - 1)];
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            wa[w] = profA[((l & 0xFFu) * W + w) * 32 + lane];
-            wb[w] = profB[((l >> 8) * W + w) * 32 + lane];
-        }
-    }
-    uint32_t let1 = ring[(1 - lane) & (kRing - 1)];
-
-    // The row search of a column whose maximum rose runs one step late,
-    // between the next column's diagonal terms and its F / Fm chains: H still
-    // holds the risen column there, and the vote that guards the search then
-    // waits on nothing, so no step stalls on the one before it.
-    bool pend = false;                   // the previous column needs its row found
-    uint32_t pcm = 0u, pthr = 0u;        // its column maximum and threshold
-    int pj = 0;                          // its column
-    auto search = [&]() {
-        if (!a.score_only && __any_sync(0xFFFFFFFFu, pend)) {
-            // smallest row holding the column maximum, both halves at once:
-            // max(H - cm, -1) is 0 on rows holding it and -1 elsewhere; those
-            // rows contribute R - r and the largest contribution wins
-            const uint32_t negv = __viaddmax_s16x2(~pcm, 0x00010001u, NEGINF);
-            uint32_t acc = 0u;
-#pragma unroll
-            for (int r = 0; r < R; r += 2) {
-                const uint32_t g0 =
-                    ~__viaddmax_s16x2(H[r], negv, 0xFFFFFFFFu) & pack2(R - r, R - r);
-                if (r + 1 < R) {
-                    const uint32_t g1 = ~__viaddmax_s16x2(H[r + 1], negv, 0xFFFFFFFFu) &
-                                        pack2(R - r - 1, R - r - 1);
-                    acc = __vimax3_s16x2(acc, g0, g1);
-                } else {
-                    acc = __vimax_s16x2_relu(acc, g0);
-                }
-            }
-            if (pend) {
-                if (lo16(pcm) > lo16(pthr)) { colA = pj; rowA = i0 + R - lo16(acc); }
-                if (hi16(pcm) > hi16(pthr)) { colB = pj; rowB = i0 + R - hi16(acc); }
-            }
-        }
-        pend = false;
-    };
-
-    auto step = [&](const int k, const uint32_t (&cwa)[W], const uint32_t (&cwb)[W],
-                    uint32_t (&nwa)[W], uint32_t (&nwb)[W]) {
-        const int j = k - lane;
-        uint32_t inH = __shfl_up_sync(0xFFFFFFFFu, outH, 1);
-        uint32_t inF = __shfl_up_sync(0xFFFFFFFFu, outF, 1);
-        uint32_t inFm = __shfl_up_sync(0xFFFFFFFFu, outFm, 1);
-        if (lane == 0) {
-            if (MULTI && st > 0 && k < N) {
-                const uint32_t *b = bnd + 3 * (size_t)k;
-                inH = b[0]; inF = b[1]; inFm = b[2];
-            } else {
-                inH = 0u; inF = 0u; inFm = 0u;
-            }
-        }
-        // next step's profile words
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            nwa[w] = profA[((let1 & 0xFFu) * W + w) * 32 + lane];
-            nwb[w] = profB[((let1 >> 8) * W + w) * 32 + lane];
-        }
-        let1 = ring[(j + 2) & (kRing - 1)];
-        // every lane computes every step: a lane before its first column
-        // (j < 0) sees pad letters and zero inputs, so its H stays 0 and its
-        // E only goes negative, which no later cell can see through the
-        // relu; past the subject's end (j >= N) the pad columns only hold
-        // values below a real cell's, which can never be the maximum
-        uint32_t F = inF, Fm = inFm, D = diag;
-        // first every row's diagonal term and its gap-open candidate (they
-        // depend only on the previous column), then the F / Fm chains, the
-        // only row-to-row dependences, with E and H hanging off them
-        uint32_t Xa[R], Xga[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const uint32_t sc = prmt(cwa[r >> 2], cwb[r >> 2], SEL[r & 3]);
-            Xa[r] = __viaddmax_s16x2_relu(r == 0 ? D : H[r - 1], sc, E[r]);
-            Xga[r] = __viaddmax_s16x2(Xa[r], NGO, NEGINF);
-        }
-        if constexpr (!SCORE) search();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const uint32_t Hn = __vimax_s16x2_relu(Xa[r], F);
-            const uint32_t Gp = __viaddmax_s16x2(Fm, ngo[r], Xga[r]);
-            E[r] = __viaddmax_s16x2(E[r], NGE, Gp);
-            F = __viaddmax_s16x2(F, NGE, Xga[r]);
-            Fm = __viaddmax_s16x2(Fm, nge[r], Xga[r]);
-            H[r] = Hn;
-        }
-        // column maximum of the lane's rows, floored at the search threshold
-        // max(running max, warp maximum - 1): a half needs its row found when
-        // it rises above the threshold, i.e. above the lane's running max and
-        // not below the warp maximum of the last refresh (anything lower
-        // cannot be the alignment maximum).  The running max may so take the
-        // value warp maximum - 1 without a cell holding it; such a lane can
-        // never hold the final maximum.
-        const uint32_t thr = __viaddmax_s16x2(wmax, 0xFFFFFFFFu, runmax);
-        uint32_t cm = thr;
-#pragma unroll
-        for (int r = 0; r + 1 < R; r += 2) cm = __vimax3_s16x2(cm, H[r], H[r + 1]);
-        if (R & 1) cm = __vimax_s16x2_relu(cm, H[R - 1]);
-        outH = H[R - 1];
-        outF = F;
-        outFm = Fm;
-        if (MULTI && lane == 31 && st + 1 < stripes && j >= 0 && j < N) {
-            uint32_t *b = bnd + 3 * (size_t)j;
-            b[0] = outH; b[1] = outF; b[2] = outFm;
-        }
-        if constexpr (!SCORE) {
-            pend = cm != thr;
-            pcm = cm;
-            pthr = thr;
-            pj = j;
-        }
-        runmax = cm;
-        diag = inH;
-    };
-    uint32_t wa2[W], wb2[W];
-    // an even step count; a step past N + 30 finds every lane past the end
-    const int steps = (N + 32) & ~1;
-    for (int k0 = 0; k0 < steps; k0 += 32) {
+    Lane<R> L;
+    L.start(a, f);
+    // the last lane ends its last column at step N + G - 2
+    const int nsteps = (N + G) & ~1;
+    // a read of the letters that the next refill wants, so that it finds them
+    // in L1
+    int touched = 0;
+    for (int k0 = 0; k0 < nsteps; k0 += 32) {
         if (k0 > 0) {
-            // every 32 steps the lanes store the next 32 columns' letters and
-            // fetch 32 more
-            ring[(k0 + 32 + lane) & (kRing - 1)] = (uint16_t)pre;
-            pre = letter_pair(a, sA, slA, sB, slB, k0 + 64 + lane);
-            // warp maximum so far: a lane's rise below it cannot end up as
-            // the alignment's maximum, so it needs no row search
-            uint32_t wm = runmax;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                wm = __vimax_s16x2_relu(wm, __shfl_xor_sync(0xFFFFFFFFu, wm, o));
-            if (TPZ_LANES == 16) {
-                // u8 pass: a pair whose maximum reached 255 - bias is decided
-                // (the i16 pass reruns it), so it needs no more row searches,
-                // and a task whose pairs are both decided stops here
-                const bool da = lo16(wm) + a.bias >= 255, db = hi16(wm) + a.bias >= 255;
-                if (da) wm = (wm & 0xFFFF0000u) | 0x7FFFu;
-                if (db) wm = (wm & 0x0000FFFFu) | 0x7FFF0000u;
-                if (da && (db || pB < 0)) decided = true;
+            asm volatile("" ::"r"(touched));
+            for (int i = 0; i < 32; i += G) {
+                const int c = k0 + 32 + i + gl;
+                ringA[c & (kRingCols - 1)] = letter_offset<R>(a, sA, slA, c);
+                ringB[c & (kRingCols - 1)] = letter_offset<R>(a, sB, slB, c);
             }
-            wmax = wm;
-            __syncwarp();
-            if (decided) break;
         }
-        const int kend = min(k0 + 32, steps);
-        for (int k = k0; k < kend; k += 2) {
-            step(k, wa, wb, wa2, wb2);
-            step(k + 1, wa2, wb2, wa, wb);
+        {
+            const int c = k0 + 64 + (gl << (5 - lg));
+            touched = (c < slA ? sA[c] : 0) + (c < slB ? sB[c] : 0);
         }
+        if (ENDS) refresh<R, false>(L, G, 0u);
+        __syncwarp();
+        steps<R, ENDS, false>(L, a, f, k0, min(k0 + 32, nsteps), nullptr);
     }
-    if constexpr (!SCORE) search();     // the last column's, if it rose
-
-    if (a.score_only || decided) { colA = colB = 0; rowA = rowB = 0; }
-    kA = max(kA, best_key(lo16(runmax), colA, rowA));
-    kB = max(kB, best_key(hi16(runmax), colB, rowB));
-    __syncwarp();
-    if (decided) break;
-    }   // stripes
-
-    // ---- warp reduction: max value, then first column, then smallest row
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    if (ENDS && L.rose) L.find_row(a, f, nsteps - 1 - gl, L.run, lo16(L.rose), hi16(L.rose));
+    uint64_t kA = lane_key(L, a, false, gl * R), kB = lane_key(L, a, true, gl * R);
+    for (int o = G >> 1; o > 0; o >>= 1) {
         kA = max(kA, __shfl_xor_sync(0xFFFFFFFFu, kA, o));
         kB = max(kB, __shfl_xor_sync(0xFFFFFFFFu, kB, o));
     }
-    if (lane < 2) {
-        const int p = lane == 0 ? pA : pB;
-        const uint64_t key = lane == 0 ? kA : kB;
-        if (p >= 0) {
-            const int v = (int)(key >> 40);
-            const int col = key ? 0xFFFFFF - (int)((key >> 16) & 0xFFFFFF) : -1;
-            const int row = key ? 0xFFFF - (int)(key & 0xFFFF) : 0;
-            if (TPZ_LANES == 16 && v + a.bias >= 255) {
-                // u8 pass saturated: the i16 pass decides (src/ssw.c:863-865)
-                int32_t *rr = qm_rerun ? qm_rerun : a.rerun;
-                const int slot = atomicAdd(qm_rerun ? qm_rerun_count : a.rerun_count, 1);
-                rr[slot] = p;
-            } else if (TPZ_LANES == 8 && a.exact_list && v >= a.exact_threshold) {
-                // near the i16 limit: 16-bit lanes may wrap, redo in 32 bits
-                const int slot = atomicAdd(a.exact_count, 1);
-                a.exact_list[slot] = p;
-            } else {
-                a.score[p] = v;
-                a.ref_end[p] = a.score_only ? -2 : col;
-                a.read_end[p] = a.score_only ? -2 : row;
-                a.status[p] = TPZ_SW_OK;
-            }
-        }
-    }
+    if (gl == 0 && pA >= 0) write_result(a, pA, kA, ENDS);
+    if (gl == 1 && pB >= 0) write_result(a, pB, kB, ENDS);
+    __syncwarp();
 }
 
-#undef TPZ_LANES
+// The bins of one R, with the lanes per group of each; their tasks are taken
+// in this order from the first bin's counter.
+struct BinSet {
+    int n;
+    int bin[4], lanes[4];
+};
 
+// letter rings: one group above 16 rows, up to 8 below
 template <int R>
-__global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args a, int bin,
-                                                    int stripes) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    int8_t *smat = reinterpret_cast<int8_t *>(smem);
-    uint32_t *profA = reinterpret_cast<uint32_t *>(smem + kSmatBytes);
-    uint32_t *profB = profA + profile_bytes(R) / 4;
-    uint16_t *ring = reinterpret_cast<uint16_t *>(profB + profile_bytes(R) / 4);
-    const int lane = threadIdx.x;
-    const int start = a.rinfo[2 * bin];
-    const int count = a.task_count ? a.task_count[bin] : a.rinfo[2 * bin + 1];
-    const int ntask = (count + 1) / 2;
-    if (ntask == 0) return;
-    int32_t *rr_list = a.rerun_bin_count ? a.rerun + start : nullptr;
-    int32_t *rr_count = a.rerun_bin_count ? a.rerun_bin_count + bin : nullptr;
+__host__ __device__ constexpr int bin_smem() {
+    return kMatBytes + 2 * profile_bytes(R) + (R > 16 ? 1 : 8) * kPairRing;
+}
 
-    for (int i = lane; i < 26 * kMatStride; i += 32) {
-        const int r = i / kMatStride, c = i % kMatStride;
-        smat[i] = (r < 25 && c < 25) ? a.mat[r * 25 + c] : (int8_t)kPadScore;
+// A block is one warp: tasks differ in length, and nothing is shared but the
+// matrix.  Shared memory (two profiles, 26 bytes per row and pair) holds the
+// warps per SM down to 4 (R = 32) .. 8 (R = 16); one warp keeps a scheduler's
+// ALU pipe busy because a step's rows hang together only through F.
+template <int R, bool ENDS>
+__global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args a,
+                                                    const __grid_constant__ BinSet b) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint8_t *prof = smem + kMatBytes, *rings = prof + 2 * profile_bytes(R);
+    int total = 0;
+    for (int i = 0; i < b.n; ++i) {
+        const int per = 64 / b.lanes[i];
+        total += (a.rinfo[2 * b.bin[i] + 1] + per - 1) / per;
     }
+    if (total == 0) return;
+    load_matrix(a, smem);
     __syncwarp();
     for (;;) {
         int t = 0;
-        if (lane == 0) t = atomicAdd(&a.next_task[bin], 1);
+        if (threadIdx.x == 0) t = atomicAdd(&a.next_task[b.bin[0]], 1);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
-        if (t >= ntask) break;
-        const int pA = a.sorted[start + 2 * t];
-        const int pB = 2 * t + 1 < count ? a.sorted[start + 2 * t + 1] : -1;
-        if constexpr (R == kMaxR) {
-            if (stripes > 1) {
-                run_task<R, true>(a, pA, pB, smat, profA, profB, ring, stripes,
-                                  a.bnd + (size_t)blockIdx.x * a.bnd_words, 0, rr_list,
-                                  rr_count);
-                continue;
-            }
+        if (t >= total) break;
+        int i = 0, per = 64 / b.lanes[0], count = a.rinfo[2 * b.bin[0] + 1];
+        while (t >= (count + per - 1) / per) {
+            t -= (count + per - 1) / per;
+            ++i;
+            per = 64 / b.lanes[i];
+            count = a.rinfo[2 * b.bin[i] + 1];
         }
-        run_task<R, false>(a, pA, pB, smat, profA, profB, ring, 1, nullptr, 0, rr_list, rr_count);
-    }
-}
-
-// One pair per launch (the per-pair form of ssw_init + ssw_align): the u8
-// lane pass and, when it saturates, the i16 lane pass in the same launch.
-// Pair lengths and the rerun flag live in shared memory.
-template <int R>
-__global__ void __launch_bounds__(32) sw_one_kernel(const __grid_constant__ Args a, int qlen,
-                                                    int slen) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ int64_t s_off;
-    __shared__ int32_t s_ql, s_sl, s_rr[2];
-    int8_t *smat = reinterpret_cast<int8_t *>(smem);
-    uint32_t *profA = reinterpret_cast<uint32_t *>(smem + kSmatBytes);
-    uint32_t *profB = profA + profile_bytes(R) / 4;
-    uint16_t *ring = reinterpret_cast<uint16_t *>(profB + profile_bytes(R) / 4);
-    const int lane = threadIdx.x;
-    for (int i = lane; i < 26 * kMatStride; i += 32) {
-        const int r = i / kMatStride, c = i % kMatStride;
-        smat[i] = (r < 25 && c < 25) ? a.mat[r * 25 + c] : (int8_t)kPadScore;
-    }
-    if (lane == 0) { s_off = 0; s_ql = qlen; s_sl = slen; s_rr[0] = 0; s_rr[1] = 0; }
-    __syncwarp();
-    Args b = a;
-    b.qoff = &s_off; b.soff = &s_off; b.qlen = &s_ql; b.slen = &s_sl;
-    b.rerun_count = &s_rr[0]; b.rerun = &s_rr[1];
-    b.ssw_lanes = 16;
-    run_task<R, false>(b, 0, -1, smat, profA, profB, ring, 1, nullptr);
-    __syncwarp();
-    if (s_rr[0]) {
-        // the u8 pass saturated: the i16 pass decides (src/ssw.c:863-865)
-        b.ssw_lanes = 8;
-        run_task<R, false>(b, 0, -1, smat, profA, profB, ring, 1, nullptr);
+        const int32_t *ids = a.sorted + a.rinfo[2 * b.bin[i]];
+        pair_task<R, ENDS, true>(a, [&](int x) { return ids[x]; }, t * per, count, b.lanes[i], smem,
+                                 prof, rings);
     }
 }
 
 // ------------------------------------------------------------- query-major
 
 // Pairs that share their query (the hits of one search query): a block of
-// kQmWarps warps per query keeps ONE profile of the query in shared memory
-// for all of them, so a warp costs the SM a fraction of the shared memory
-// of the pair-per-task kernel and more warps hide the DPX latency.  The
-// block sorts the query's pairs by subject length (longest first, two per
-// task), runs the u8 pass over all of them and then, with the profile
-// still resident, the i16 pass over those that saturated.
+// kQmWarps warps keeps ONE profile of the query in shared memory for all of
+// them, so registers, not shared memory, bound the warps per SM.  The block
+// sorts the chunk's pairs by subject length, longest first.
 constexpr int kQmWarps = 8;
 constexpr int kQmMaxPairs = 256;      // pairs per chunk: longer pair lists of a query are cut
 constexpr int kQmMinPairs = 2 * kQmWarps;
 constexpr int kQmStreams = 8;
 
-__host__ __device__ constexpr int qm_smem_bytes(int R) {
-    return kSmatBytes + profile_bytes(R) + kQmWarps * 2 * kRing + 8 * kQmMaxPairs +
-           4 * kQmMaxPairs;
-}
-
 struct QmArgs {
-    const int64_t *chunks;    // [first pair, end) per chunk; the pairs of a chunk share the query
-    const int32_t *bin_info;  // per row bin R-1: [first chunk, count]
-    int32_t *next;            // per row bin: chunk counter
+    const int64_t *chunks;    // [first pair, end, lanes per group] per chunk
+    const int32_t *bin_info;  // per row count (rows_index): [first chunk, count]
+    int32_t *next;            // per row count: chunk counter
+    int ring_bytes;           // letter rings of one warp
 };
 
-// profile words of letters warp, warp + kQmWarps, ... for lane's rows of the
-// query of pair p
+__host__ __device__ constexpr int qm_smem_bytes(int R, int ring_bytes) {
+    return kMatBytes + profile_bytes(R) + kQmWarps * ring_bytes + 4 * kQmMaxPairs;
+}
+
+// profile words of a query for the lanes of every group, one word column per
+// warp at a time
 template <int R>
-__device__ __forceinline__ void qm_build_profile(const Args &a, int64_t p, const int8_t *smat,
-                                                 uint32_t *prof, int warp, int lane) {
+__device__ __forceinline__ void qm_build_profile(const Args &a, int64_t p, int G, const uint8_t *matT,
+                                                 uint8_t *prof) {
     constexpr int W = words_for(R);
-    const int ql = a.qlen[p];
-    const int8_t *qp = a.q + a.qoff[p];
-    const int i0 = lane * R;
-    int qv[R];
+    const int lane = threadIdx.x & 31;
+    const int ql = a.qlen[p], i0 = (lane & (G - 1)) * R;
+    const int8_t *q = a.q + a.qoff[p];
+    for (int w = threadIdx.x >> 5; w < W; w += kQmWarps) {
+        int x[4];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        int x = (i0 + r < ql) ? qp[i0 + r] : -1;
-        if (a.translate && x >= 0) x = a.xq[x & 127];
-        qv[r] = (x >= 25) ? -1 : x;
-    }
-    for (int let = warp; let < 26; let += kQmWarps) {
-        const int8_t *mrow = smat + let * kMatStride;
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            uint32_t word = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int r = 4 * w + k;
-                int v = kPadScore;
-                if (r < R && qv[r] >= 0) v = mrow[qv[r]];
-                word |= (uint32_t)(uint8_t)(int8_t)v << (8 * k);
-            }
-            prof[(let * W + w) * 32 + lane] = word;
+        for (int k = 0; k < 4; ++k) {
+            const int r = 4 * w + k;
+            x[k] = query_letter(a, (r < R && i0 + r < ql) ? (int)q[i0 + r] : -1);
         }
+        build_word<W>(matT, x[0], x[1], x[2], x[3], prof + w * 128 + lane * 4);
     }
 }
 
-// SCORE: scores only (report-mode search), with the end-coordinate row
-// search compiled out rather than skipped at run time
-template <int R, bool SCORE>
+template <int R, bool ENDS>
 __global__ void __launch_bounds__(kQmWarps * 32) sw_query_kernel(const __grid_constant__ Args a,
                                                                  QmArgs g, int bin) {
     extern __shared__ __align__(16) uint8_t smem[];
-    int8_t *smat = reinterpret_cast<int8_t *>(smem);
-    uint32_t *prof = reinterpret_cast<uint32_t *>(smem + kSmatBytes);
-    uint16_t *rings = reinterpret_cast<uint16_t *>(prof + profile_bytes(R) / 4);
-    uint64_t *keys = reinterpret_cast<uint64_t *>(rings + kQmWarps * kRing);
-    int32_t *sat = reinterpret_cast<int32_t *>(keys + kQmMaxPairs);
-    __shared__ int s_group, s_next, s_nsat;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint16_t *ring = rings + warp * kRing;
+    uint8_t *prof = smem + kMatBytes;
+    uint8_t *rings = prof + profile_bytes(R) + (threadIdx.x >> 5) * g.ring_bytes;
+    uint32_t *keys = reinterpret_cast<uint32_t *>(prof + profile_bytes(R) + kQmWarps * g.ring_bytes);
+    __shared__ int s_group, s_next;
+    const int lane = threadIdx.x & 31;
     const int gb = g.bin_info[2 * bin], gc = g.bin_info[2 * bin + 1];
     if (gc == 0) return;
-    for (int i = threadIdx.x; i < 26 * kMatStride; i += blockDim.x) {
-        const int r = i / kMatStride, c = i % kMatStride;
-        smat[i] = (r < 25 && c < 25) ? a.mat[r * 25 + c] : (int8_t)kPadScore;
-    }
+    load_matrix(a, smem);
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) {
             s_group = atomicAdd(&g.next[bin], 1);
             s_next = 0;
-            s_nsat = 0;
         }
         __syncthreads();
         if (s_group >= gc) break;
-        const int64_t p0 = g.chunks[2 * (gb + s_group)];
-        const int n = (int)(g.chunks[2 * (gb + s_group) + 1] - p0);
+        const int64_t *ch = g.chunks + 3 * (gb + s_group);
+        const int64_t p0 = ch[0];
+        const int n = (int)(ch[1] - p0), G = (int)ch[2];
         int np = 1;
         while (np < n) np <<= 1;
-        // keys: subject length + 1 (descending), pair id; padding 0 sorts last
+        // keys: subject length (descending; < 2^24), place in the chunk
         for (int i = threadIdx.x; i < np; i += blockDim.x)
-            keys[i] = i < n ? ((uint64_t)(uint32_t)(a.slen[p0 + i] + 1) << 32) | (uint32_t)(p0 + i)
-                            : 0ull;
-        qm_build_profile<R>(a, p0, smat, prof, warp, lane);
+            keys[i] = i < n ? ((uint32_t)a.slen[p0 + i] << 8) | (uint32_t)(255 - i) : 0u;
+        qm_build_profile<R>(a, p0, G, smem, prof);
         __syncthreads();
         for (int k = 2; k <= np; k <<= 1) {
             for (int j = k >> 1; j > 0; j >>= 1) {
                 for (int i = threadIdx.x; i < np; i += blockDim.x) {
                     const int l = i ^ j;
                     if (l > i) {
-                        const uint64_t x = keys[i], y = keys[l];
+                        const uint32_t x = keys[i], y = keys[l];
                         if (((i & k) == 0) ? (x < y) : (x > y)) { keys[i] = y; keys[l] = x; }
                     }
                 }
                 __syncthreads();
             }
         }
-        // u8 pass over every pair of the query
+        const int per = 64 / G;
         for (;;) {
             int t = 0;
             if (lane == 0) t = atomicAdd(&s_next, 1);
             t = __shfl_sync(0xFFFFFFFFu, t, 0);
-            if (2 * t >= n) break;
-            const int pA = (int)(uint32_t)keys[2 * t];
-            const int pB = 2 * t + 1 < n ? (int)(uint32_t)keys[2 * t + 1] : -1;
-            run_task<R, false, true, SCORE>(a, pA, pB, smat, prof, prof, ring, 1, nullptr, 16, sat,
-                                     &s_nsat);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) s_next = 0;
-        __syncthreads();
-        // i16 pass over the pairs that saturated (src/ssw.c:863-865)
-        const int ns = s_nsat;
-        for (;;) {
-            int t = 0;
-            if (lane == 0) t = atomicAdd(&s_next, 1);
-            t = __shfl_sync(0xFFFFFFFFu, t, 0);
-            if (2 * t >= ns) break;
-            const int pA = sat[2 * t];
-            const int pB = 2 * t + 1 < ns ? sat[2 * t + 1] : -1;
-            run_task<R, false, true, SCORE>(a, pA, pB, smat, prof, prof, ring, 1, nullptr, 8, nullptr,
-                                     nullptr);
+            if (t * per >= n) break;
+            pair_task<R, ENDS, false>(a, [&](int x) { return (int)p0 + 255 - (int)(keys[x] & 255u); },
+                                      t * per, n, G, nullptr, prof, rings);
         }
     }
+}
+
+// ------------------------------------------------------------ stripe form
+
+constexpr int kLongWarps = 4;
+constexpr int kStripeLag = 3;      // blocks of 32 columns between two warps of a pair
+
+// W warps of one pair: a block's barrier 1 + group
+__device__ __forceinline__ void group_sync(int group, int W) {
+    if (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(32 * W) : "memory");
+}
+
+// Warp `wg` of the W warps of one pair: rows [wg*64*R, (wg+1)*64*R), the low
+// halves the first 32*R of them.  prof: this warp's two profiles; ring: its
+// letters; above / below: the boundary rings of kRingCols words to the
+// neighbouring warps (null: none).  Lane 31's high half ends column k - 63
+// at step k, so a block of 32 columns is complete in the ring two blocks
+// later, and the warp below takes it in the block after that.  Returns the
+// warp's best key in every lane.
+template <int R, bool ENDS>
+__device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, int ql, const int8_t *s,
+                                                int sl, int group, int W, int wg, const uint8_t *matT,
+                                                uint8_t *prof, uint16_t *ring, const uint32_t *above,
+                                                uint32_t *below) {
+    const int lane = threadIdx.x & 31;
+    const int i0 = (wg * 64 + lane) * R, i1 = i0 + 32 * R;
+    build_profile<R>(a, q, ql, i0, matT, prof + lane * 4);
+    build_profile<R>(a, q, ql, i1, matT, prof + profile_bytes(R) + lane * 4);
+    Flow f;
+    f.profA = prof + lane * 4;
+    f.profB = f.profA + profile_bytes(R);
+    f.ringA = f.ringB = ring;
+    f.lag = lane; f.lagB = 32; f.width = 32;
+    f.mul = lane == 0 ? 65536u : 1u;
+    f.add = lane == 0 ? (uint32_t)a.floor : 0u;
+    f.bnd = lane == 0 ? above : nullptr;
+    f.bnd_end = sl;
+#pragma unroll
+    for (int c = lane; c < 64; c += 32) {
+        ring[c] = letter_offset<R>(a, s, sl, c);
+        ring[64 + c] = kPadLetter * words_for(R) * 128;
+    }
+    __syncwarp();
+    Lane<R> L;
+    L.start(a, f);
+    const int nblk = (sl + 63 + 31) >> 5;
+    int touched = 0;
+    for (int p = 0; p < nblk + kStripeLag * (W - 1); ++p) {
+        const int b = p - kStripeLag * wg, k0 = 32 * b;
+        if (b >= 0 && b < nblk) {
+            if (b > 0) {
+                asm volatile("" ::"r"(touched));
+                ring[(k0 + 32 + lane) & (kRingCols - 1)] = letter_offset<R>(a, s, sl, k0 + 32 + lane);
+            }
+            touched = k0 + 64 + lane < sl ? s[k0 + 64 + lane] : 0;
+            uint32_t in = 0;
+            if (above && k0 + lane < sl) in = lo16(above[(k0 + lane) & (kRingCols - 1)]);
+            if (ENDS) refresh<R, true>(L, 32, in);
+            __syncwarp();
+            steps<R, ENDS, true>(L, a, f, k0, k0 + 32, lane == 31 ? below : nullptr);
+        }
+        group_sync(group, W);
+    }
+    if (ENDS && L.rose) L.find_row(a, f, 32 * nblk - 1 - lane, L.run, lo16(L.rose), hi16(L.rose));
+    uint64_t key = max(lane_key(L, a, false, i0), lane_key(L, a, true, i1));
+    for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, o));
+    return key;
+}
+
+template <bool ENDS, int RMAX>
+__device__ __forceinline__ uint64_t stripe_rows(int R, const Args &a, const int8_t *q, int ql,
+                                                const int8_t *s, int sl, int group, int W, int wg,
+                                                const uint8_t *matT, uint8_t *prof, uint16_t *ring,
+                                                const uint32_t *above, uint32_t *below) {
+#define TPZ_STRIPE(r) \
+    stripe_task<r, ENDS>(a, q, ql, s, sl, group, W, wg, matT, prof, ring, above, below)
+    if (R <= 4) return TPZ_STRIPE(4);
+    if (RMAX == 8 || R <= 8) return TPZ_STRIPE(8);
+    if constexpr (RMAX > 8) {
+        if (R <= 16) return TPZ_STRIPE(16);
+        if (R <= 20) return TPZ_STRIPE(20);
+        if (R <= 24) return TPZ_STRIPE(24);
+        if (R <= 28) return TPZ_STRIPE(28);
+        return TPZ_STRIPE(32);
+    }
+#undef TPZ_STRIPE
+}
+
+// one warp's shared memory: two profiles, the letter ring, the boundary ring
+__host__ __device__ constexpr int stripe_warp_bytes(int RMAX) {
+    return 2 * profile_bytes(RMAX) + 2 * kRingCols + 4 * kRingCols;
+}
+__host__ __device__ constexpr int stripe_smem(int RMAX, int warps) {
+    return kMatBytes + warps * stripe_warp_bytes(RMAX);
+}
+
+// Bins of the stripe form in one launch, and the fewest and most warps that
+// may share a pair of each.
+struct StripeSet {
+    int n;
+    int bin[3], wmin[3], wmax[3];
+};
+
+// Blocks of 4 warps; a pair takes wmin warps, more of them while the bin has
+// fewer pairs than would fill the grid's warps.
+template <bool ENDS, int RMAX>
+__global__ void __launch_bounds__(32 * kLongWarps) sw_stripe_kernel(const __grid_constant__ Args a,
+                                                                    const __grid_constant__ StripeSet b) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint64_t s_key[kLongWarps];
+    __shared__ int s_task[kLongWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint8_t *prof = smem + kMatBytes + warp * stripe_warp_bytes(RMAX);
+    uint16_t *ring = reinterpret_cast<uint16_t *>(prof + 2 * profile_bytes(RMAX));
+    uint32_t *below = reinterpret_cast<uint32_t *>(ring + kRingCols);
+    const uint32_t *above = reinterpret_cast<const uint32_t *>(
+        reinterpret_cast<const uint8_t *>(below) - stripe_warp_bytes(RMAX));
+    bool ready = false;
+    for (int i = 0; i < b.n; ++i) {
+        const int start = a.rinfo[2 * b.bin[i]], count = a.rinfo[2 * b.bin[i] + 1];
+        if (count == 0) continue;
+        if (!ready) load_matrix(a, smem);
+        ready = true;
+        __syncthreads();
+        int W = b.wmin[i];
+        while (W < b.wmax[i] && (int64_t)count * W < (int64_t)gridDim.x * kLongWarps) W *= 2;
+        const int group = warp / W, wg = warp % W;
+        for (;;) {
+            if (wg == 0 && lane == 0) s_task[group] = atomicAdd(&a.next_task[b.bin[i]], 1);
+            group_sync(group, W);
+            const int t = s_task[group];
+            if (t >= count) break;
+            const int p = a.sorted[start + t];
+            const int ql = a.qlen[p];
+            const uint64_t key = stripe_rows<ENDS, RMAX>(
+                (ql + 64 * W - 1) / (64 * W), a, a.q + a.qoff[p], ql, a.s + a.soff[p], a.slen[p], group,
+                W, wg, smem, prof, ring, wg > 0 ? above : nullptr, wg + 1 < W ? below : nullptr);
+            if (lane == 0) s_key[warp] = key;
+            group_sync(group, W);
+            if (wg == 0 && lane == 0) {
+                uint64_t best = key;
+                for (int w = 1; w < W; ++w) best = max(best, s_key[warp + w]);
+                write_result(a, p, best, ENDS);
+            }
+        }
+    }
+}
+
+// One pair per launch (the per-pair form of ssw_init + ssw_align): `W` warps
+// of the stripe form with at most 8 rows per lane, lengths from the host.
+constexpr int kOneMaxQlen = kStripeRows;
+__global__ void __launch_bounds__(64) sw_one_kernel(const __grid_constant__ Args a, int qlen, int slen) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint64_t s_key[2];
+    const int warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+    uint8_t *prof = smem + kMatBytes + warp * stripe_warp_bytes(8);
+    uint16_t *ring = reinterpret_cast<uint16_t *>(prof + 2 * profile_bytes(8));
+    uint32_t *below = reinterpret_cast<uint32_t *>(ring + kRingCols);
+    const uint32_t *above = reinterpret_cast<const uint32_t *>(
+        reinterpret_cast<const uint8_t *>(below) - stripe_warp_bytes(8));
+    load_matrix(a, smem);
+    __syncthreads();
+    const uint64_t key = stripe_rows<true, 8>((qlen + 64 * W - 1) / (64 * W), a, a.q, qlen, a.s, slen, 0, W,
+                                              warp, smem, prof, ring, warp > 0 ? above : nullptr,
+                                              warp + 1 < W ? below : nullptr);
+    if ((threadIdx.x & 31) == 0) s_key[warp] = key;
+    __syncthreads();
+    if (threadIdx.x == 0) write_result(a, 0, W > 1 ? max(s_key[0], s_key[1]) : s_key[0], true);
 }
 
 // ---------------------------------------------------------------- binning
 
-__device__ __forceinline__ int pair_bin(int ql, int sl) {
-    const int rb = ql <= kStripeRows ? (ql + 31) / 32 - 1                 // 0..31
-                                     : 30 + (ql + kStripeRows - 1) / kStripeRows;  // 32..38
+__device__ __forceinline__ int pair_bin(int ql, int sl, int small_batch) {
     const int sb = min(sl >> 5, kSBins - 1);
-    return rb * kSBins + (kSBins - 1 - sb);             // long subjects first
+    return row_bin(ql, small_batch) * kSBins + (kSBins - 1 - sb);      // long subjects first
 }
 
-// list == nullptr: pairs 0..n-1; else list[0 .. *list_n)
-__global__ void bin_count_kernel(int64_t n, const int32_t *list, const int32_t *list_n,
-                                 const int32_t *qlen, const int32_t *slen, int32_t *counts,
-                                 int32_t *status, int max_qlen, int32_t *multi_maxn) {
-    const int64_t limit = list ? (int64_t)*list_n : n;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < limit;
+struct BinArgs {
+    int64_t n;               // pairs 0..n-1, or list[0..n)
+    const int32_t *list;
+    const int32_t *qlen, *slen;
+    int max_qlen, small_batch;
+};
+
+__global__ void bin_count_kernel(BinArgs b, int32_t *counts, int32_t *status) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < b.n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int p = list ? list[i] : (int)i;
-        const int ql = qlen[p], sl = slen[p];
-        if (ql < 1 || ql > max_qlen || sl < 0 || sl >= TPZ_SW_MAX_SLEN) {
+        const int p = b.list ? b.list[i] : (int)i;
+        const int ql = b.qlen[p], sl = b.slen[p];
+        if (ql < 1 || ql > b.max_qlen || sl < 0 || sl >= TPZ_SW_MAX_SLEN) {
             status[p] = TPZ_SW_INVALID;
             continue;
         }
-        atomicAdd(&counts[pair_bin(ql, sl)], 1);
-        if (ql > kStripeRows && multi_maxn) atomicMax(multi_maxn, sl);
+        atomicAdd(&counts[pair_bin(ql, sl, b.small_batch)], 1);
     }
 }
 
-__global__ void set_i32_kernel(int32_t *p, int32_t v) { *p = v; }
-
 // one block of 1024 threads: exclusive scan of kBins counts -> cursor; the
-// per-R-bin [start, count] pairs -> rinfo; task counters cleared.
+// per-row-bin [start, count] pairs -> rinfo; task counters cleared.
 __global__ void bin_scan_kernel(const int32_t *counts, int32_t *cursor, int32_t *rinfo,
                                 int32_t *next_task) {
     constexpr int PER = kBins / 1024;
@@ -736,17 +534,13 @@ __global__ void bin_scan_kernel(const int32_t *counts, int32_t *cursor, int32_t 
     }
 }
 
-__global__ void bin_scatter_kernel(int64_t n, const int32_t *list, const int32_t *list_n,
-                                   const int32_t *qlen, const int32_t *slen, int32_t *cursor,
-                                   int32_t *sorted, int max_qlen) {
-    const int64_t limit = list ? (int64_t)*list_n : n;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < limit;
+__global__ void bin_scatter_kernel(BinArgs b, int32_t *cursor, int32_t *sorted) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < b.n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int p = list ? list[i] : (int)i;
-        const int ql = qlen[p], sl = slen[p];
-        if (ql < 1 || ql > max_qlen || sl < 0 || sl >= TPZ_SW_MAX_SLEN) continue;
-        const int pos = atomicAdd(&cursor[pair_bin(ql, sl)], 1);
-        sorted[pos] = p;
+        const int p = b.list ? b.list[i] : (int)i;
+        const int ql = b.qlen[p], sl = b.slen[p];
+        if (ql < 1 || ql > b.max_qlen || sl < 0 || sl >= TPZ_SW_MAX_SLEN) continue;
+        sorted[atomicAdd(&cursor[pair_bin(ql, sl, b.small_batch)], 1)] = p;
     }
 }
 
@@ -773,239 +567,218 @@ __global__ void __launch_bounds__(256) dpx_probe_kernel(int iters, uint32_t inc,
 
 // ------------------------------------------------------------ host driver
 
-typedef void (*KernelFn)(const Args, int, int);
+// Kernels of one device with their launch attributes, set once.
+struct Kernels {
+    typedef void (*BinFn)(const Args, const BinSet);
+    typedef void (*QmFn)(const Args, QmArgs, int);
+    typedef void (*StripeFn)(const Args, const StripeSet);
+    BinFn bin[2][kRs];                       // [ends][rows_index]
+    QmFn qm[2][kRs];
+    StripeFn stripe8[2], stripe32[2];        // [ends]
+    int bin_smem[kRs], bin_blocks[2][kRs];   // blocks per SM
+    int stripe8_blocks[2], stripe32_blocks[2];
+};
 
-template <int R>
-struct Table {
-    static void fill(KernelFn *k) {
-        k[R - 1] = sw_bin_kernel<R>;
-        Table<R - 1>::fill(k);
+template <int... I>
+static void fill_kernels(Kernels &k, std::integer_sequence<int, I...>) {
+    ((k.bin[0][I] = sw_bin_kernel<rows_of(I), false>), ...);
+    ((k.bin[1][I] = sw_bin_kernel<rows_of(I), true>), ...);
+    ((k.qm[0][I] = sw_query_kernel<rows_of(I), false>), ...);
+    ((k.qm[1][I] = sw_query_kernel<rows_of(I), true>), ...);
+    ((k.bin_smem[I] = bin_smem<rows_of(I)>()), ...);
+}
+
+// dynamic shared memory of a kernel, the whole carveout (so blocks of
+// kernels running side by side share an SM), and its blocks per SM
+static int set_up(const void *f, int smem, int threads, int *blocks) {
+    TPZ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    TPZ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)cudaSharedmemCarveoutMaxShared));
+    if (blocks) {
+        int nb = 0;
+        TPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, threads, smem));
+        *blocks = std::max(1, nb);
     }
-};
-template <>
-struct Table<0> {
-    static void fill(KernelFn *) {}
-};
+    return TPZ_OK;
+}
+
+static int kernels(const Kernels **out) {
+    static std::mutex mu;
+    static std::vector<Kernels *> per_dev;
+    int dev = 0;
+    TPZ_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if ((int)per_dev.size() <= dev) per_dev.resize(dev + 1, nullptr);
+    if (!per_dev[dev]) {
+        Kernels *k = new Kernels();
+        fill_kernels(*k, std::make_integer_sequence<int, kRs>());
+        int rc = TPZ_OK;
+        k->stripe8[0] = sw_stripe_kernel<false, 8>;
+        k->stripe8[1] = sw_stripe_kernel<true, 8>;
+        k->stripe32[0] = sw_stripe_kernel<false, 32>;
+        k->stripe32[1] = sw_stripe_kernel<true, 32>;
+        for (int e = 0; rc == TPZ_OK && e < 2; ++e) {
+            for (int i = 0; rc == TPZ_OK && i < kRs; ++i) {
+                rc = set_up((const void *)k->bin[e][i], k->bin_smem[i], 32, &k->bin_blocks[e][i]);
+                if (rc == TPZ_OK)
+                    rc = set_up((const void *)k->qm[e][i], qm_smem_bytes(rows_of(i), 8 * kPairRing),
+                                kQmWarps * 32, nullptr);
+            }
+            if (rc == TPZ_OK)
+                rc = set_up((const void *)k->stripe8[e], stripe_smem(8, kLongWarps), 32 * kLongWarps,
+                            &k->stripe8_blocks[e]);
+            if (rc == TPZ_OK)
+                rc = set_up((const void *)k->stripe32[e], stripe_smem(32, kLongWarps), 32 * kLongWarps,
+                            &k->stripe32_blocks[e]);
+        }
+        if (rc == TPZ_OK) rc = set_up((const void *)sw_one_kernel, stripe_smem(8, 2), 64, nullptr);
+        if (rc) { delete k; return rc; }
+        per_dev[dev] = k;
+    }
+    *out = per_dev[dev];
+    return TPZ_OK;
+}
 
 constexpr int kAuxStreams = 8;
 
-struct LaunchCfg {
-    KernelFn fn[kMaxR];
-    int smem[kMaxR];
-    int blocks_per_sm[kMaxR];
-    cudaStream_t aux[kAuxStreams];       // bin kernels overlap their tails here
-    cudaEvent_t fork, join[kAuxStreams];
-    int32_t *maxn_pin;                   // pinned copy of a call's multi-stripe maximum
-    cudaEvent_t maxn_ready;
-};
-
 // Per host thread and device: the auxiliary streams and fork/join events of
 // one call must not be shared with a call running in another thread.
-struct LaunchCfgs {
-    std::vector<LaunchCfg *> per_dev;
-    ~LaunchCfgs() {
-        for (LaunchCfg *c : per_dev) {
+struct Streams {
+    cudaStream_t aux[kAuxStreams];       // bin kernels overlap their tails here
+    cudaEvent_t fork, join[kAuxStreams];
+};
+
+struct StreamSets {
+    std::vector<Streams *> per_dev;
+    ~StreamSets() {
+        for (Streams *c : per_dev) {
             if (!c) continue;
             for (int i = 0; i < kAuxStreams; ++i) {
                 cudaStreamDestroy(c->aux[i]);
                 cudaEventDestroy(c->join[i]);
             }
             cudaEventDestroy(c->fork);
-            cudaEventDestroy(c->maxn_ready);
-            cudaFreeHost(c->maxn_pin);
             delete c;
         }
     }
 };
 
 // lane: calls of one thread that run at the same time (the chunks of the
-// host entry point) take different lanes, so they get separate streams
-static int launch_cfg(const LaunchCfg **out, int lane = 0) {
-    static thread_local LaunchCfgs cfgs;
-    std::vector<LaunchCfg *> &per_dev = cfgs.per_dev;
+// host entry point; a search's query-major kernels beside its other pairs)
+// take different lanes, so they get separate streams
+static int streams(Streams **out, int lane) {
+    static thread_local StreamSets sets;
     int dev = 0;
     TPZ_CUDA(cudaGetDevice(&dev));
-    dev = 2 * dev + (lane & 1);
-    if ((int)per_dev.size() <= dev) per_dev.resize(dev + 1, nullptr);
-    if (!per_dev[dev]) {
-        LaunchCfg *c = new LaunchCfg();
-        Table<kMaxR>::fill(c->fn);
-        for (int r = 1; r <= kMaxR; ++r) {
-            c->smem[r - 1] = smem_bytes(r);
-            TPZ_CUDA(cudaFuncSetAttribute((const void *)c->fn[r - 1],
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          c->smem[r - 1]));
-            // one carveout for every bin kernel, so blocks of concurrently
-            // running bins can share an SM
-            TPZ_CUDA(cudaFuncSetAttribute((const void *)c->fn[r - 1],
-                                          cudaFuncAttributePreferredSharedMemoryCarveout,
-                                          (int)cudaSharedmemCarveoutMaxShared));
-            int nb = 0;
-            TPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)c->fn[r - 1],
-                                                                   32, c->smem[r - 1]));
-            c->blocks_per_sm[r - 1] = std::max(1, nb);
-        }
+    const size_t at = 3 * (size_t)dev + lane;
+    if (sets.per_dev.size() <= at) sets.per_dev.resize(at + 1, nullptr);
+    if (!sets.per_dev[at]) {
+        Streams *c = new Streams();
         for (int i = 0; i < kAuxStreams; ++i) {
             TPZ_CUDA(cudaStreamCreateWithFlags(&c->aux[i], cudaStreamNonBlocking));
             TPZ_CUDA(cudaEventCreateWithFlags(&c->join[i], cudaEventDisableTiming));
         }
         TPZ_CUDA(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-        TPZ_CUDA(cudaEventCreateWithFlags(&c->maxn_ready, cudaEventDisableTiming));
-        TPZ_CUDA(cudaHostAlloc((void **)&c->maxn_pin, sizeof(int32_t), cudaHostAllocDefault));
-        per_dev[dev] = c;
+        sets.per_dev[at] = c;
     }
-    *out = per_dev[dev];
+    *out = sets.per_dev[at];
+    return TPZ_OK;
+}
+
+static int fork(Streams *x, cudaStream_t st) {
+    TPZ_CUDA(cudaEventRecord(x->fork, st));
+    for (int i = 0; i < kAuxStreams; ++i) TPZ_CUDA(cudaStreamWaitEvent(x->aux[i], x->fork, 0));
+    return TPZ_OK;
+}
+
+static int join(Streams *x, cudaStream_t st) {
+    for (int i = 0; i < kAuxStreams; ++i) {
+        TPZ_CUDA(cudaEventRecord(x->join[i], x->aux[i]));
+        TPZ_CUDA(cudaStreamWaitEvent(st, x->join[i], 0));
+    }
     return TPZ_OK;
 }
 
 static thread_local int64_t g_last_launches = 0;
 
-// R and stripe count of a row bin
-__host__ __device__ constexpr int bin_rows(int b) { return b < kMaxR ? b + 1 : kMaxR; }
-__host__ __device__ constexpr int bin_stripes(int b) { return b < kMaxR ? 1 : b - 30; }
-constexpr int kUsedRBins = kMaxR + kMaxStripes - 1;     // 39
+// A batch of up to this many pairs takes the stripe form for every query: it
+// would leave most warps idle with two pairs and more per warp, and its time
+// is that of its longest pair.
+constexpr int64_t kSmallBatch = 1024;
 
-// One pass over the pairs (all of them, or list[0 .. *list_n)): counting sort
-// into row bins, then one persistent kernel per bin.  With a16, each bin's
-// kernel is followed on its stream by the i16 pass over the pairs of that bin
-// that saturated, so no pass waits for the whole batch.
-static int launch_round(const LaunchCfg *cfg, Args &a, int64_t n, const int32_t *list,
-                        const int32_t *list_n, int32_t *counts, int32_t *cursor, int32_t *sorted,
-                        int32_t *multi_maxn, cudaStream_t st, int64_t &launches,
-                        int *host_maxn, int known_maxn = -1, Args *a16 = nullptr) {
+// scratch words of one call: counts and cursor per bin, [start, count] and a
+// task counter per row bin, then the sorted pair ids
+constexpr size_t kBinWords = 2 * (size_t)kBins + 3 * kRBins;
+
+// Bins the pairs (all of them, or the n ids of `list`) in ws and launches the
+// kernels that align them, over the auxiliary streams x so that each
+// kernel's tail overlaps the next one (null: all on st).
+static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const int32_t *list,
+                        int32_t *ws, int max_qlen, bool ends, cudaStream_t st, int64_t &launches) {
     const int nsm = sm_count();
+    int32_t *counts = ws, *cursor = counts + kBins, *rinfo = cursor + kBins;
+    int32_t *next_task = rinfo + 2 * kRBins, *sorted = ws + kBinWords;
+    a.sorted = sorted; a.rinfo = rinfo; a.next_task = next_task;
+    const bool small_batch = n <= kSmallBatch;
+    BinArgs b{n, list, a.qlen, a.slen, max_qlen, small_batch ? 1 : 0};
     TPZ_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * kBins, st));
-    const int gb = (int)std::min<int64_t>((n + 255) / 256, (int64_t)nsm * 8);
-    bin_count_kernel<<<std::max(gb, 1), 256, 0, st>>>(n, list, list_n, a.qlen, a.slen, counts,
-                                                      a.status, TPZ_SW_MAX_QLEN, multi_maxn);
-    bin_scan_kernel<<<1, 1024, 0, st>>>(counts, cursor, const_cast<int32_t *>(a.rinfo),
-                                        a.next_task);
-    bin_scatter_kernel<<<std::max(gb, 1), 256, 0, st>>>(n, list, list_n, a.qlen, a.slen, cursor,
-                                                        sorted, TPZ_SW_MAX_QLEN);
+    const int gb = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)nsm * 8));
+    bin_count_kernel<<<gb, 256, 0, st>>>(b, counts, a.status);
+    bin_scan_kernel<<<1, 1024, 0, st>>>(counts, cursor, rinfo, next_task);
+    bin_scatter_kernel<<<gb, 256, 0, st>>>(b, cursor, sorted);
     launches += 4;
-    // The boundary buffer of multi-stripe bins is sized by the longest subject
-    // among queries longer than one stripe.  When the caller does not know it,
-    // the device's count comes back while the single-stripe bins already run,
-    // and the multi-stripe bins are launched after them.
-    const bool defer = host_maxn && known_maxn < 0;
-    auto alloc_bnd = [&](int maxn, cudaStream_t s) -> int {
-        a.bnd_words = 3 * ((int64_t)maxn + 1);
-        const size_t bytes = sizeof(uint32_t) * (size_t)a.bnd_words * nsm *
-                             cfg->blocks_per_sm[kMaxR - 1];
-        TPZ_CUDA(cudaMallocAsync((void **)&a.bnd, bytes, s));
-        if (a16) { a16->bnd = a.bnd; a16->bnd_words = a.bnd_words; }
-        return TPZ_OK;
-    };
-    if (host_maxn && !defer) {
-        *host_maxn = known_maxn;
-        if (known_maxn > 0) {
-            const int rc = alloc_bnd(known_maxn, st);
-            if (rc) return rc;
-        }
+    const int e = ends ? 1 : 0;
+    if (x) {
+        const int rc = fork(x, st);
+        if (rc) return rc;
     }
-    if (defer) {
-        TPZ_CUDA(cudaMemcpyAsync(cfg->maxn_pin, multi_maxn, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        TPZ_CUDA(cudaEventRecord(cfg->maxn_ready, st));
-    }
-    // one persistent kernel per row bin, longest rows first, spread over the
-    // auxiliary streams so that each kernel's tail overlaps the next one;
-    // the multi-stripe bins share one boundary buffer and stay on aux[0]
-    TPZ_CUDA(cudaEventRecord(cfg->fork, st));
-    for (int i = 0; i < kAuxStreams; ++i) TPZ_CUDA(cudaStreamWaitEvent(cfg->aux[i], cfg->fork, 0));
-    int rr = 0;
-    auto launch_bin = [&](int b) {
-        const int R = bin_rows(b), S = bin_stripes(b);
-        const int grid = nsm * cfg->blocks_per_sm[R - 1];
-        cudaStream_t xs = S > 1 ? cfg->aux[0] : cfg->aux[rr++ % kAuxStreams];
-        cfg->fn[R - 1]<<<grid, 32, cfg->smem[R - 1], xs>>>(a, b, S);
+    int at = 0;
+    auto next_stream = [&]() { return x ? x->aux[at++ % kAuxStreams] : st; };
+    // no launch wants more blocks than pairs
+    auto grid = [&](int blocks) { return (unsigned)std::min<int64_t>((int64_t)nsm * blocks, std::max<int64_t>(n, 1)); };
+    if (max_qlen > kStripeRows) {
+        const StripeSet s{3, {kLongBin + 2, kLongBin + 1, kLongBin}, {4, 2, 1}, {4, 4, 4}};
+        k->stripe32[e]<<<grid(k->stripe32_blocks[e]), 32 * kLongWarps, stripe_smem(32, kLongWarps),
+                         next_stream()>>>(a, s);
         ++launches;
-        if (a16) {
-            cfg->fn[R - 1]<<<grid, 32, cfg->smem[R - 1], xs>>>(*a16, b, S);
+    }
+    if (small_batch) {
+        const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {2, 2, 0}};
+        k->stripe8[e]<<<grid(k->stripe8_blocks[e]), 32 * kLongWarps, stripe_smem(8, kLongWarps),
+                        next_stream()>>>(a, s);
+        ++launches;
+    } else {
+        for (int i = kRs - 1; i >= 0; --i) {
+            const int R = rows_of(i);
+            BinSet s{R > 16 ? 1 : 4, {R - 9, 24 + R - 9, 32 + R - 9, 40 + R - 9}, {32, 16, 8, 4}};
+            if (R <= 8) s = BinSet{1, {kTinyBin + i, 0, 0, 0}, {4, 0, 0, 0}};
+            k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, s);
             ++launches;
         }
-    };
-    for (int b = kUsedRBins - 1; b >= 0; --b) {
-        if (bin_stripes(b) > 1 && (defer || !a.bnd)) continue;
-        launch_bin(b);
     }
-    int rc = TPZ_OK;
-    if (defer) {
-        const cudaError_t e = cudaEventSynchronize(cfg->maxn_ready);
-        if (e != cudaSuccess) {
-            rc = cuda_fail(e, "multi-stripe maximum");
-        } else {
-            *host_maxn = *cfg->maxn_pin;
-            if (*host_maxn > 0 && (rc = alloc_bnd(*host_maxn, cfg->aux[0])) == TPZ_OK)
-                for (int b = kUsedRBins - 1; b >= kMaxR; --b) launch_bin(b);
-        }
-    }
-    // the join comes after every launch, also on an error above, so that the
+    // the join comes after every launch, also on an error, so that the
     // caller's stream waits for all kernels before it frees their buffers
-    for (int i = 0; i < kAuxStreams; ++i) {
-        TPZ_CUDA(cudaEventRecord(cfg->join[i], cfg->aux[i]));
-        TPZ_CUDA(cudaStreamWaitEvent(st, cfg->join[i], 0));
+    const cudaError_t err = cudaGetLastError();
+    if (x) {
+        const int rc = join(x, st);
+        if (rc) return rc;
     }
-    if (rc) return rc;
-    TPZ_CUDA(cudaGetLastError());
-    return TPZ_OK;
+    return err == cudaSuccess ? TPZ_OK : cuda_fail(err, "Smith-Waterman launches");
 }
 
-// 32-bit re-run of i16-pass pairs whose maximum came near 32767 (16-bit
-// lanes could wrap there): the same recurrence with the i16 lane length,
-// one thread per pair, rows and columns in a plain loop.  Only pairs whose
-// score can pass 32767 - 2*max(M) get here -- query and subject both longer
-// than ~1900 residues of near-identity.
-constexpr int kExactThreads = 128;
-
-__global__ void __launch_bounds__(kExactThreads) sw_exact_kernel(const __grid_constant__ Args a,
-                                                                 int32_t *scratch) {
-    const int n = *a.exact_count;
-    int32_t *E = scratch + (size_t)threadIdx.x * 2 * TPZ_SW_MAX_QLEN;
-    int32_t *Hc = E + TPZ_SW_MAX_QLEN;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int p = a.exact_list[i];
-        const int ql = a.qlen[p], sl = a.slen[p];
-        const int8_t *qp = a.q + a.qoff[p];
-        const int8_t *sp = a.s + a.soff[p];
-        const int seg = max(1, (ql + 7) / 8);
-        for (int r = 0; r < ql; ++r) { E[r] = 0; Hc[r] = 0; }
-        int best = 0, bc = -1, br = 0;
-        for (int c = 0; c < sl; ++c) {
-            int sc = sp[c];
-            if (a.translate) sc = a.xs[sc & 127];
-            const int8_t *mrow = a.mat + 25 * sc;
-            int F = 0, Fm = 0, D = 0;
-            for (int r = 0; r < ql; ++r) {
-                if (r % seg == 0) Fm = 0;
-                int qc = qp[r];
-                if (a.translate) qc = a.xq[qc & 127];
-                const int X = max(max(0, D + mrow[qc]), E[r]);
-                const int h = max(X, F);
-                const int Xg = X - a.gap_open;
-                const int Gp = max(Fm - a.gap_open, Xg);
-                E[r] = max(E[r] - a.gap_extend, Gp);
-                F = max(F - a.gap_extend, Xg);
-                Fm = max(Fm - a.gap_extend, Xg);
-                D = Hc[r];
-                Hc[r] = h;
-                if (h > best) { best = h; bc = c; br = r; }
-            }
-        }
-        if (best >= 32767) {
-            a.score[p] = 32767; a.ref_end[p] = -1; a.read_end[p] = -1; a.status[p] = TPZ_SW_DROPPED;
-        } else {
-            a.score[p] = best; a.ref_end[p] = bc; a.read_end[p] = best > 0 ? br : 0;
-            a.status[p] = TPZ_SW_OK;
-        }
-    }
+static void pair_args(Args &a, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
+                      const int8_t *s, const int64_t *soff, const int32_t *slen, int32_t *score,
+                      int32_t *ref_end, int32_t *read_end, int32_t *status) {
+    memset(&a, 0, sizeof a);
+    a.q = q; a.qoff = qoff; a.qlen = qlen; a.s = s; a.soff = soff; a.slen = slen;
+    a.score = score; a.ref_end = ref_end; a.read_end = read_end; a.status = status;
 }
 
 int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
                    const int8_t *s, const int64_t *soff, const int32_t *slen, const int8_t *mat,
                    int go, int ge, int32_t *score, int32_t *ref_end, int32_t *read_end,
                    int32_t *status, cudaStream_t st, const int8_t *xq, const int8_t *xs,
-                   int score_only, const int32_t *subset, int64_t nsub, int known_multi_maxn,
-                   int lane) {
+                   int score_only, const int32_t *subset, int64_t nsub, int lane) {
     g_last_launches = 0;
     if (subset && nsub == 0) return TPZ_OK;
     if (n < 0 || n > INT32_MAX / 3 || !mat) { set_error("tpz_sw_batch: bad n or matrix"); return TPZ_E_ARG; }
@@ -1018,163 +791,27 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
         set_error("tpz_sw_batch: NULL buffer");
         return TPZ_E_ARG;
     }
-    const LaunchCfg *cfg = nullptr;
-    int rc = launch_cfg(&cfg, lane);
-    if (rc) return rc;
+    const Kernels *k = nullptr;
+    Streams *x = nullptr;
+    int rc = kernels(&k);
+    if (rc || (rc = streams(&x, lane))) return rc;
     keep_pool_memory();
-
-    // workspace: counts, cursor, rinfo, next_task, rerun_count, multi_maxn,
-    // exact_count, (n_sub), per-bin rerun counts, i16 task counters | sorted,
-    // rerun, exact_list
-    const size_t small = sizeof(int32_t) * (2 * kBins + 2 * kRBins + kRBins + 8 + 2 * kRBins);
-    const size_t bytes = small + sizeof(int32_t) * 3 * (size_t)n;
-    char *ws = nullptr;
-    TPZ_CUDA(cudaMallocAsync((void **)&ws, bytes, st));
-    int32_t *counts = (int32_t *)ws;
-    int32_t *cursor = counts + kBins;
-    int32_t *rinfo = cursor + kBins;
-    int32_t *next_task = rinfo + 2 * kRBins;
-    int32_t *rerun_count = next_task + kRBins;
-    int32_t *multi_maxn = rerun_count + 1;
-    int32_t *exact_count = rerun_count + 2;
-    int32_t *rerun_bin_count = rerun_count + 8;
-    int32_t *next_task16 = rerun_bin_count + kRBins;
-    int32_t *sorted = (int32_t *)(ws + small);
-    int32_t *rerun = sorted + n;
-    int32_t *exact_list = rerun + n;
-
+    if (subset) n = nsub;
+    int32_t *ws = nullptr;
+    TPZ_CUDA(cudaMallocAsync((void **)&ws, sizeof(int32_t) * (kBinWords + (size_t)n), st));
     Args a;
-    a.q = q; a.qoff = qoff; a.qlen = qlen; a.s = s; a.soff = soff; a.slen = slen;
-    a.score = score; a.ref_end = ref_end; a.read_end = read_end; a.status = status;
-    a.sorted = sorted; a.rinfo = rinfo; a.next_task = next_task;
-    a.rerun = rerun; a.rerun_count = rerun_count;
-    a.gap_open = go; a.gap_extend = ge;
-    int mn = 0, mx = 0;
-    for (int i = 0; i < 625; ++i) { mn = std::min<int>(mn, mat[i]); mx = std::max<int>(mx, mat[i]); }
-    a.bias = -mn;
-    memcpy(a.mat, mat, 625);
+    pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
+    set_scoring(a, mat, go, ge);
     a.translate = (xq && xs) ? 1 : 0;
-    a.score_only = score_only;
-    memset(a.xq, 0, sizeof a.xq);
-    memset(a.xs, 0, sizeof a.xs);
     if (a.translate) {
         memcpy(a.xq, xq, 128);
         memcpy(a.xs, xs, 128);
     }
-    a.bnd = nullptr;
-    a.bnd_words = 0;
-    a.exact_list = exact_list;
-    a.exact_count = exact_count;
-    a.exact_threshold = std::min(32767 - 2 * std::max(mx, 1), kBig);
-    a.rerun_bin_count = rerun_bin_count;
-    a.task_count = nullptr;
-    // the i16 pass of a bin: its saturated pairs, in the bin's slice of rerun
-    Args a16 = a;
-    a16.ssw_lanes = 8;
-    a16.sorted = rerun;
-    a16.task_count = rerun_bin_count;
-    a16.next_task = next_task16;
-    a16.rerun_bin_count = nullptr;
-
     int64_t launches = 0;
-    int host_maxn = 0;
-    TPZ_CUDA(cudaMemsetAsync(rerun_count, 0, (8 + 2 * kRBins) * sizeof(int32_t), st));
-    a.ssw_lanes = 16;
-    if (subset) {
-        // the first round over the given pair ids only
-        int32_t *d_nsub = rerun_count + 3;
-        set_i32_kernel<<<1, 1, 0, st>>>(d_nsub, (int32_t)nsub);
-        rc = launch_round(cfg, a, nsub, subset, d_nsub, counts, cursor, sorted, multi_maxn, st,
-                          launches, &host_maxn, -1, &a16);
-    } else {
-        rc = launch_round(cfg, a, n, nullptr, nullptr, counts, cursor, sorted, multi_maxn, st,
-                          launches, &host_maxn, known_multi_maxn, &a16);
-    }
-    if (rc == TPZ_OK && (host_maxn > 0 || (int64_t)kStripeRows * mx >= a.exact_threshold)) {
-        // only queries longer than one stripe, or matrices with large
-        // entries, can come near the 16-bit limit
-        int32_t *scratch = nullptr;
-        rc = cudaMallocAsync((void **)&scratch,
-                             sizeof(int32_t) * 2 * (size_t)TPZ_SW_MAX_QLEN * kExactThreads, st)
-                 == cudaSuccess ? TPZ_OK : cuda_fail(cudaGetLastError(), "exact scratch");
-        if (rc == TPZ_OK) {
-            sw_exact_kernel<<<1, kExactThreads, 0, st>>>(a, scratch);
-            ++launches;
-            cudaFreeAsync(scratch, st);
-        }
-    }
-    if (a.bnd) cudaFreeAsync(a.bnd, st);
-    if (rc) { cudaFreeAsync(ws, st); return rc; }
+    rc = launch_batch(k, x, a, n, subset, ws, TPZ_SW_MAX_QLEN, !score_only, st, launches);
     TPZ_CUDA(cudaFreeAsync(ws, st));
-    TPZ_CUDA(cudaGetLastError());
+    if (rc) return rc;
     g_last_launches = launches;
-    return TPZ_OK;
-}
-
-// Per host thread and device: launch attributes of the query-major kernels
-// and two streams of their own, so that they run beside the pair-per-task
-// kernels of the same call.
-struct QmCfg {
-    typedef void (*Fn)(const Args, QmArgs, int);
-    Fn fn[2][kMaxR];                    // [score only][R - 1]
-    int blocks_per_sm[2][kMaxR];
-    cudaStream_t aux[kQmStreams];
-    cudaEvent_t fork, join[kQmStreams];
-};
-
-template <int R>
-struct QmTable {
-    static void fill(QmCfg::Fn (*k)[kMaxR]) {
-        k[0][R - 1] = sw_query_kernel<R, false>;
-        k[1][R - 1] = sw_query_kernel<R, true>;
-        QmTable<R - 1>::fill(k);
-    }
-};
-template <>
-struct QmTable<0> {
-    static void fill(QmCfg::Fn (*)[kMaxR]) {}
-};
-
-struct QmCfgs {
-    std::vector<QmCfg *> per_dev;
-    ~QmCfgs() {
-        for (QmCfg *c : per_dev) {
-            if (!c) continue;
-            for (int i = 0; i < kQmStreams; ++i) { cudaStreamDestroy(c->aux[i]); cudaEventDestroy(c->join[i]); }
-            cudaEventDestroy(c->fork);
-            delete c;
-        }
-    }
-};
-
-static int qm_cfg(const QmCfg **out) {
-    static thread_local QmCfgs cfgs;
-    int dev = 0;
-    TPZ_CUDA(cudaGetDevice(&dev));
-    if ((int)cfgs.per_dev.size() <= dev) cfgs.per_dev.resize(dev + 1, nullptr);
-    if (!cfgs.per_dev[dev]) {
-        QmCfg *c = new QmCfg();
-        QmTable<kMaxR>::fill(c->fn);
-        for (int so = 0; so < 2; ++so)
-            for (int r = 1; r <= kMaxR; ++r) {
-                const void *f = (const void *)c->fn[so][r - 1];
-                TPZ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              qm_smem_bytes(r)));
-                TPZ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                              (int)cudaSharedmemCarveoutMaxShared));
-                int nb = 0;
-                TPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, kQmWarps * 32,
-                                                                       qm_smem_bytes(r)));
-                c->blocks_per_sm[so][r - 1] = std::max(1, nb);
-            }
-        for (int i = 0; i < kQmStreams; ++i) {
-            TPZ_CUDA(cudaStreamCreateWithFlags(&c->aux[i], cudaStreamNonBlocking));
-            TPZ_CUDA(cudaEventCreateWithFlags(&c->join[i], cudaEventDisableTiming));
-        }
-        TPZ_CUDA(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-        cfgs.per_dev[dev] = c;
-    }
-    *out = cfgs.per_dev[dev];
     return TPZ_OK;
 }
 
@@ -1183,8 +820,7 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
                          const int8_t *mat, int go, int ge, int32_t *score, int32_t *ref_end,
                          int32_t *read_end, int32_t *status, cudaStream_t st, const int8_t *xq,
                          const int8_t *xs, int score_only, int64_t ngroups,
-                         const int64_t *gstart_dev, const int64_t *gstart_host,
-                         const int32_t *gqlen_host) {
+                         const int64_t *gstart_host, const int32_t *gqlen_host) {
     if (n <= 0) return TPZ_OK;
     if (!(go > ge && ge >= 0 && go <= 255) || !mat) {
         set_error("tpz_sw_batch: requires 255 >= gap_open > gap_extend >= 0");
@@ -1193,8 +829,8 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
     // chunks of at most kQmMaxPairs pairs of one query for the query-major
     // kernels (queries with enough pairs and one stripe); every other pair
     // goes by pair
-    std::vector<std::vector<int64_t>> per_r(kMaxR);
-    std::vector<int64_t> work(kMaxR, 0);
+    struct Row { std::vector<int64_t> chunks; int64_t work = 0; int min_lanes = 32; };
+    std::vector<Row> rows(kRs);
     std::vector<int32_t> rest;
     for (int64_t g = 0; g < ngroups; ++g) {
         const int64_t c = gstart_host[g + 1] - gstart_host[g];
@@ -1202,122 +838,88 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         const int ql = gqlen_host[g];
         if (ql >= 1 && ql <= kStripeRows && c >= kQmMinPairs) {
             const int64_t nch = (c + kQmMaxPairs - 1) / kQmMaxPairs;
+            // more lanes per pair (fewer rows each) while a chunk would leave
+            // warps of its block without a task
+            int G = group_lanes(ql);
+            while (G < 32 && c / nch < kQmWarps * (64 / G)) G *= 2;
+            Row &r = rows[rows_index((ql + G - 1) / G)];
             for (int64_t i = 0; i < nch; ++i) {
                 // equal cuts so that no chunk is much smaller than the others
-                per_r[(ql + 31) / 32 - 1].push_back(gstart_host[g] + c * i / nch);
-                per_r[(ql + 31) / 32 - 1].push_back(gstart_host[g] + c * (i + 1) / nch);
+                r.chunks.push_back(gstart_host[g] + c * i / nch);
+                r.chunks.push_back(gstart_host[g] + c * (i + 1) / nch);
+                r.chunks.push_back(G);
             }
-            work[(ql + 31) / 32 - 1] += c * ql;
+            r.work += c * ql;
+            r.min_lanes = std::min(r.min_lanes, G);
         } else {
             for (int64_t k = gstart_host[g]; k < gstart_host[g + 1]; ++k) rest.push_back((int32_t)k);
         }
     }
+    // one upload: chunks, then [first chunk, count] and a zero counter per
+    // row count, then the other pairs
     std::vector<int64_t> chunks;
-    std::vector<int32_t> bin_info(2 * kMaxR, 0);
-    for (int r = 0; r < kMaxR; ++r) {
-        bin_info[2 * r] = (int32_t)(chunks.size() / 2);
-        bin_info[2 * r + 1] = (int32_t)(per_r[r].size() / 2);
-        chunks.insert(chunks.end(), per_r[r].begin(), per_r[r].end());
+    std::vector<int32_t> tail(3 * kRs, 0);
+    std::vector<int> order;
+    for (int i = 0; i < kRs; ++i) {
+        tail[2 * i] = (int32_t)(chunks.size() / 3);
+        tail[2 * i + 1] = (int32_t)(rows[i].chunks.size() / 3);
+        chunks.insert(chunks.end(), rows[i].chunks.begin(), rows[i].chunks.end());
+        if (!rows[i].chunks.empty()) order.push_back(i);
     }
-    const QmCfg *qc = nullptr;
-    int rc = qm_cfg(&qc);
-    if (rc) return rc;
+    tail.insert(tail.end(), rest.begin(), rest.end());
+    const Kernels *k = nullptr;
+    Streams *x = nullptr;
+    int rc = kernels(&k);
+    if (rc || (rc = streams(&x, 2))) return rc;
     int64_t *dchunks = nullptr;
-    int32_t *dbin = nullptr, *dnext = nullptr, *drest = nullptr, *dexact = nullptr,
-            *dexact_n = nullptr;
-    auto cleanup = [&]() {
-        for (void *p : {(void *)dchunks, (void *)dbin, (void *)dnext, (void *)drest, (void *)dexact,
-                        (void *)dexact_n})
-            if (p) cudaFreeAsync(p, st);
-    };
-    if (cudaMallocAsync((void **)&dchunks, 8 * std::max<size_t>(chunks.size(), 1), st) ||
-        cudaMallocAsync((void **)&dbin, 4 * 2 * kMaxR, st) ||
-        cudaMallocAsync((void **)&dnext, 4 * kMaxR, st) ||
-        cudaMallocAsync((void **)&drest, 4 * std::max<size_t>(rest.size(), 1), st) ||
-        cudaMallocAsync((void **)&dexact, 4 * std::max<int64_t>(n, 1), st) ||
-        cudaMallocAsync((void **)&dexact_n, 4, st)) {
-        cleanup();
-        return cuda_fail(cudaGetLastError(), "batch_device_grouped");
-    }
-    if (cudaMemcpyAsync(dchunks, chunks.data(), 8 * chunks.size(), cudaMemcpyHostToDevice, st) ||
-        cudaMemcpyAsync(dbin, bin_info.data(), 4 * 2 * kMaxR, cudaMemcpyHostToDevice, st) ||
-        cudaMemsetAsync(dnext, 0, 4 * kMaxR, st) || cudaMemsetAsync(dexact_n, 0, 4, st) ||
-        (rest.size() && cudaMemcpyAsync(drest, rest.data(), 4 * rest.size(), cudaMemcpyHostToDevice, st))) {
-        cleanup();
+    const size_t cbytes = 8 * chunks.size(), tbytes = 4 * tail.size();
+    TPZ_CUDA(cudaMallocAsync((void **)&dchunks, cbytes + tbytes, st));
+    int32_t *dtail = (int32_t *)((char *)dchunks + cbytes);
+    if ((cbytes && cudaMemcpyAsync(dchunks, chunks.data(), cbytes, cudaMemcpyHostToDevice, st)) ||
+        cudaMemcpyAsync(dtail, tail.data(), tbytes, cudaMemcpyHostToDevice, st)) {
+        cudaFreeAsync(dchunks, st);
         return cuda_fail(cudaGetLastError(), "batch_device_grouped copies");
     }
     Args a;
-    a.rerun_bin_count = nullptr;
-    a.task_count = nullptr;
-    memset(&a, 0, sizeof a);
-    a.q = q; a.qoff = qoff; a.qlen = qlen; a.s = s; a.soff = soff; a.slen = slen;
-    a.score = score; a.ref_end = ref_end; a.read_end = read_end; a.status = status;
-    a.gap_open = go; a.gap_extend = ge;
-    int mn = 0, mx = 0;
-    for (int i = 0; i < 625; ++i) { mn = std::min<int>(mn, mat[i]); mx = std::max<int>(mx, mat[i]); }
-    a.bias = -mn;
-    memcpy(a.mat, mat, 625);
+    pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
+    set_scoring(a, mat, go, ge);
     a.translate = (xq && xs) ? 1 : 0;
     if (a.translate) { memcpy(a.xq, xq, 128); memcpy(a.xs, xs, 128); }
-    a.score_only = score_only;
-    a.exact_list = dexact;
-    a.exact_count = dexact_n;
-    a.exact_threshold = std::min(32767 - 2 * std::max(mx, 1), kBig);
     QmArgs g;
-    g.chunks = dchunks; g.bin_info = dbin; g.next = dnext;
-    const int nsm = sm_count();
+    g.chunks = dchunks; g.bin_info = dtail; g.next = dtail + 2 * kRs;
+    const int nsm = sm_count(), e = score_only ? 0 : 1;
     int64_t launches = 0;
-    if (!chunks.empty()) {
-        // one persistent kernel per row bin, the bins with the most work
-        // first, over kQmStreams streams so that bins share the SMs
-        TPZ_CUDA(cudaEventRecord(qc->fork, st));
-        for (int i = 0; i < kQmStreams; ++i) TPZ_CUDA(cudaStreamWaitEvent(qc->aux[i], qc->fork, 0));
-        std::vector<int> order;
-        for (int r = 1; r <= kMaxR; ++r) if (!per_r[r - 1].empty()) order.push_back(r);
-        std::sort(order.begin(), order.end(), [&](int x, int y) { return work[x - 1] > work[y - 1]; });
-        int k = 0;
-        const int so = a.score_only ? 1 : 0;
-        for (int r : order) {
-            const int grid = (int)std::min<int64_t>((int64_t)nsm * qc->blocks_per_sm[so][r - 1],
-                                                    (int64_t)per_r[r - 1].size() / 2);
-            qc->fn[so][r - 1]<<<grid, kQmWarps * 32, qm_smem_bytes(r), qc->aux[k++ % kQmStreams]>>>(
-                a, g, r - 1);
+    if (!order.empty()) {
+        // one persistent kernel per row count, those with the most work
+        // first, over the streams so that they share the SMs
+        if ((rc = fork(x, st))) { cudaFreeAsync(dchunks, st); return rc; }
+        std::sort(order.begin(), order.end(), [&](int l, int r) { return rows[l].work > rows[r].work; });
+        int at = 0;
+        for (int i : order) {
+            g.ring_bytes = (32 / rows[i].min_lanes) * kPairRing;
+            const int smem = qm_smem_bytes(rows_of(i), g.ring_bytes);
+            int nb = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k->qm[e][i], kQmWarps * 32,
+                                                              smem) != cudaSuccess || nb < 1)
+                nb = 1;
+            const unsigned grid = (unsigned)std::min<int64_t>((int64_t)nsm * nb,
+                                                              (int64_t)rows[i].chunks.size() / 3);
+            k->qm[e][i]<<<grid, kQmWarps * 32, smem, x->aux[at++ % kAuxStreams]>>>(a, g, i);
             ++launches;
         }
     }
     rc = batch_device_x(n, q, qoff, qlen, s, soff, slen, mat, go, ge, score, ref_end, read_end,
-                        status, st, xq, xs, score_only, drest, (int64_t)rest.size());
+                        status, st, xq, xs, score_only, dtail + 3 * kRs, (int64_t)rest.size());
     launches += g_last_launches;
-    if (!chunks.empty()) {
-        for (int i = 0; i < kQmStreams; ++i) {
-            TPZ_CUDA(cudaEventRecord(qc->join[i], qc->aux[i]));
-            TPZ_CUDA(cudaStreamWaitEvent(st, qc->join[i], 0));
-        }
-        if (rc == TPZ_OK && (int64_t)kStripeRows * mx >= a.exact_threshold) {
-            int32_t *scratch = nullptr;
-            rc = cudaMallocAsync((void **)&scratch,
-                                 sizeof(int32_t) * 2 * (size_t)TPZ_SW_MAX_QLEN * kExactThreads, st)
-                     == cudaSuccess ? TPZ_OK : cuda_fail(cudaGetLastError(), "exact scratch");
-            if (rc == TPZ_OK) {
-                sw_exact_kernel<<<1, kExactThreads, 0, st>>>(a, scratch);
-                ++launches;
-                cudaFreeAsync(scratch, st);
-            }
-        }
+    if (!order.empty()) {
+        const int rj = join(x, st);
+        if (rc == TPZ_OK) rc = rj;
     }
-    cleanup();
+    cudaFreeAsync(dchunks, st);
     if (rc) return rc;
     TPZ_CUDA(cudaGetLastError());
     g_last_launches = launches;
     return TPZ_OK;
-}
-
-int batch_device(int64_t n, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
-                 const int8_t *s, const int64_t *soff, const int32_t *slen, const int8_t *mat,
-                 int go, int ge, int32_t *score, int32_t *ref_end, int32_t *read_end,
-                 int32_t *status, cudaStream_t st) {
-    return batch_device_x(n, q, qoff, qlen, s, soff, slen, mat, go, ge, score, ref_end, read_end,
-                          status, st, nullptr, nullptr, 0, nullptr, 0);
 }
 
 }  // namespace sw
@@ -1373,19 +975,17 @@ int ensure(size_t bytes) {
 // the first pair outside the limits (-1: none).
 struct Span {
     int64_t qlo, qhi, slo, shi, bad;
-    int multi_maxn;     // longest subject of a pair whose query spans several stripes
 };
 
 Span scan_pairs(int64_t i0, int64_t i1, const int64_t *qoff, const int32_t *qlen,
                 const int64_t *soff, const int32_t *slen) {
-    Span r{INT64_MAX, 0, INT64_MAX, 0, -1, 0};
+    Span r{INT64_MAX, 0, INT64_MAX, 0, -1};
     for (int64_t i = i0; i < i1; ++i) {
         if (qlen[i] < 1 || qlen[i] > TPZ_SW_MAX_QLEN || slen[i] < 0 || slen[i] >= TPZ_SW_MAX_SLEN ||
             qoff[i] < 0 || soff[i] < 0) {
             r.bad = i;
             return r;
         }
-        if (qlen[i] > tpz::sw::kStripeRows) r.multi_maxn = std::max(r.multi_maxn, slen[i]);
         r.qlo = std::min(r.qlo, qoff[i]);
         r.qhi = std::max(r.qhi, qoff[i] + qlen[i]);
         if (slen[i] > 0) {
@@ -1399,52 +999,6 @@ Span scan_pairs(int64_t i0, int64_t i1, const int64_t *qoff, const int32_t *qlen
 
 }  // namespace
 
-namespace tpz {
-namespace sw {
-
-constexpr int kOneMaxQlen = kStripeRows;
-
-typedef void (*OneFn)(const Args, int, int);
-
-template <int R>
-struct OneTable {
-    static void fill(OneFn *k) {
-        k[R - 1] = sw_one_kernel<R>;
-        OneTable<R - 1>::fill(k);
-    }
-};
-template <>
-struct OneTable<0> {
-    static void fill(OneFn *) {}
-};
-
-struct OneCfg {
-    OneFn fn[kMaxR];
-};
-
-static int one_cfg(const OneCfg **out) {
-    static std::mutex mu;
-    static std::vector<OneCfg *> per_dev;
-    int dev = 0;
-    TPZ_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    if ((int)per_dev.size() <= dev) per_dev.resize(dev + 1, nullptr);
-    if (!per_dev[dev]) {
-        OneCfg *c = new OneCfg();
-        OneTable<kMaxR>::fill(c->fn);
-        for (int r = 1; r <= kMaxR; ++r)
-            TPZ_CUDA(cudaFuncSetAttribute((const void *)c->fn[r - 1],
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          smem_bytes(r)));
-        per_dev[dev] = c;
-    }
-    *out = per_dev[dev];
-    return TPZ_OK;
-}
-
-}  // namespace sw
-}  // namespace tpz
-
 extern "C" {
 
 int tpz_sw_batch_device(int64_t n, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
@@ -1452,9 +1006,9 @@ int tpz_sw_batch_device(int64_t n, const int8_t *q, const int64_t *qoff, const i
                         const int8_t *mat625_host, int gap_open, int gap_extend,
                         int32_t *score, int32_t *ref_end, int32_t *read_end, int32_t *status,
                         void *stream) {
-    return tpz::sw::batch_device(n, q, qoff, qlen, s, soff, slen, mat625_host, gap_open,
-                                 gap_extend, score, ref_end, read_end, status,
-                                 (cudaStream_t)stream);
+    return tpz::sw::batch_device_x(n, q, qoff, qlen, s, soff, slen, mat625_host, gap_open,
+                                   gap_extend, score, ref_end, read_end, status,
+                                   (cudaStream_t)stream, nullptr, nullptr, 0);
 }
 
 int tpz_sw_batch_host(int64_t n, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
@@ -1504,12 +1058,11 @@ int tpz_sw_batch_host(int64_t n, const int8_t *q, const int64_t *qoff, const int
             });
         pieces[0].r = scan_pairs(pieces[0].i0, pieces[0].i1, qoff, qlen, soff, slen);
         for (auto &t : th) t.join();
-        for (int c = 0; c < nch; ++c) sp[c] = Span{INT64_MAX, 0, INT64_MAX, 0, -1, 0};
+        for (int c = 0; c < nch; ++c) sp[c] = Span{INT64_MAX, 0, INT64_MAX, 0, -1};
         for (const Piece &p : pieces) {
             Span &d = sp[p.c];
             const Span &r = p.r;
             if (r.bad >= 0 && (d.bad < 0 || r.bad < d.bad)) d.bad = r.bad;
-            d.multi_maxn = std::max(d.multi_maxn, r.multi_maxn);
             if (p.i1 > p.i0) {
                 d.qlo = std::min(d.qlo, r.qlo);
                 d.qhi = std::max(d.qhi, r.qhi);
@@ -1593,8 +1146,7 @@ int tpz_sw_batch_host(int64_t n, const int8_t *q, const int64_t *qoff, const int
         TPZ_CUDA(cudaStreamWaitEvent(cs, in_ready[c], 0));
         rc = tpz::sw::batch_device_x(m, dq, dqoff + a, dqlen + a, ds, dsoff + a, dslen + a,
                                      mat625, gap_open, gap_extend, dsc + a, dre + a, drd + a,
-                                     dst + a, cs, nullptr, nullptr, 0, nullptr, 0,
-                                     sp[c].multi_maxn, c & 1);
+                                     dst + a, cs, nullptr, nullptr, 0, nullptr, 0, c & 1);
         if (rc) {
             cudaStreamSynchronize(hs);
             cudaStreamSynchronize(cst[0]);
@@ -1629,26 +1181,20 @@ int tpz_sw_align_one(const int8_t *q, int32_t qlen, const int8_t *s, int32_t sle
         tpz::set_error("tpz_sw_align_one: requires 255 >= gap_open > gap_extend >= 0");
         return TPZ_E_ARG;
     }
-    const OneCfg *cfg = nullptr;
-    int rc = one_cfg(&cfg);
+    const Kernels *k = nullptr;
+    int rc = kernels(&k);
     if (rc) return rc;
-    int mn = 0, mx = 0;
-    for (int i = 0; i < 625; ++i) { mn = std::min<int>(mn, mat625_host[i]); mx = std::max<int>(mx, mat625_host[i]); }
+    int mx = 0;
+    for (int i = 0; i < 625; ++i) mx = std::max<int>(mx, mat625_host[i]);
     if ((int64_t)qlen * mx >= kBig) {
         tpz::set_error("tpz_sw_align_one: matrix entries too large for 16-bit scores at this length");
         return TPZ_E_ARG;
     }
     Args a;
-    a.rerun_bin_count = nullptr;
-    a.task_count = nullptr;
-    memset(&a, 0, sizeof a);
-    a.q = q; a.s = s;
-    a.score = out4; a.ref_end = out4 + 1; a.read_end = out4 + 2; a.status = out4 + 3;
-    a.gap_open = gap_open; a.gap_extend = gap_extend; a.bias = -mn;
-    memcpy(a.mat, mat625_host, 625);
-    a.exact_threshold = 32767;
-    const int R = (qlen + 31) / 32;
-    cfg->fn[R - 1]<<<1, 32, smem_bytes(R), (cudaStream_t)stream>>>(a, qlen, slen);
+    pair_args(a, q, nullptr, nullptr, s, nullptr, nullptr, out4, out4 + 1, out4 + 2, out4 + 3);
+    set_scoring(a, mat625_host, gap_open, gap_extend);
+    const int W = qlen <= 512 ? 1 : 2;
+    sw_one_kernel<<<1, 32 * W, stripe_smem(8, W), (cudaStream_t)stream>>>(a, qlen, slen);
     TPZ_CUDA(cudaGetLastError());
     return TPZ_OK;
 }
@@ -1672,82 +1218,34 @@ int tpz_dpx_probe(int64_t blocks, int iters, uint32_t *out, void *stream, int64_
 // memory pressure halfway through a request), or a host loop that must not
 // stall on the allocator -- cudaMalloc/cudaFree synchronize the device and
 // would serialize every concurrent stream.  For them the batched SW below
-// keeps its scratch (bin counts, bin cursors, the sorted pair list and the
-// rerun list) in one statically sized device array instead of a per-call
-// allocation, and enqueues everything on the caller's stream only.
+// keeps its scratch (bin counts, bin cursors and the sorted pair list) in one
+// statically sized device array instead of a per-call allocation, and
+// enqueues everything on the caller's stream only.
 
 namespace tpz {
 namespace sw {
 
 constexpr int64_t kNoAllocMaxPairs = TPZ_SW_NOALLOC_MAX_PAIRS;
 constexpr int kNoAllocMaxQlen = TPZ_SW_NOALLOC_MAX_QLEN;   // one stripe
-// the stated entry limit is the largest one the 16-bit lanes hold exactly
+// the stated entry limit keeps every score below kBig
 static_assert((int64_t)kNoAllocMaxQlen * TPZ_SW_NOALLOC_MAX_ENTRY < kBig &&
                   (int64_t)kNoAllocMaxQlen * (TPZ_SW_NOALLOC_MAX_ENTRY + 1) >= kBig,
               "TPZ_SW_NOALLOC_MAX_ENTRY");
-constexpr size_t kNoAllocWords = 2 * (size_t)kBins + 2 * kRBins + kRBins + 4 + 2 * (size_t)kNoAllocMaxPairs;
 
 // One copy per device that loads the library, kept until the process exits.
-static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocWords];
+static __device__ __align__(256) int32_t g_noalloc_scratch[kBinWords + (size_t)kNoAllocMaxPairs];
 
-struct NoAllocDev {
-    int32_t *scratch = nullptr;      // device address of g_noalloc_scratch
-    KernelFn fn[kMaxR];
-    int blocks_per_sm[kMaxR];
-};
-
-// Per-device set-up, done by the first call on each device with that device
-// current: the device address of the static scratch array (host code cannot
-// use the array's name as a device pointer) and the bin kernels' launch
-// attributes.
-static int noalloc_setup(const NoAllocDev **out) {
+// Device address of the static scratch array of the current device (host
+// code cannot use the array's name as a device pointer).
+static int noalloc_scratch(int32_t **out) {
     static std::mutex mu;
-    static std::vector<NoAllocDev *> per_dev;
+    static std::vector<int32_t *> per_dev;
     int dev = 0;
     TPZ_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(mu);
     if ((int)per_dev.size() <= dev) per_dev.resize(dev + 1, nullptr);
-    if (!per_dev[dev]) {
-        NoAllocDev *d = new NoAllocDev();
-        cudaError_t e = cudaGetSymbolAddress((void **)&d->scratch, g_noalloc_scratch);
-        if (e != cudaSuccess) {
-            delete d;
-            return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-        }
-        Table<kMaxR>::fill(d->fn);
-        for (int r = 1; r <= kMaxR; ++r) {
-            e = cudaFuncSetAttribute((const void *)d->fn[r - 1],
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(r));
-            int nb = 0;
-            if (e == cudaSuccess)
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)d->fn[r - 1], 32,
-                                                                  smem_bytes(r));
-            if (e != cudaSuccess) {
-                delete d;
-                return cuda_fail(e, "allocation-free SW set-up");
-            }
-            d->blocks_per_sm[r - 1] = std::max(1, nb);
-        }
-        per_dev[dev] = d;
-    }
+    if (!per_dev[dev]) TPZ_CUDA(cudaGetSymbolAddress((void **)&per_dev[dev], g_noalloc_scratch));
     *out = per_dev[dev];
-    return TPZ_OK;
-}
-
-static int noalloc_round(const NoAllocDev *d, Args &a, int64_t n, const int32_t *list,
-                         const int32_t *list_n, int32_t *counts, int32_t *cursor, int32_t *sorted,
-                         cudaStream_t st) {
-    const int nsm = sm_count();
-    TPZ_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * kBins, st));
-    const int gb = (int)std::min<int64_t>((n + 255) / 256, (int64_t)nsm * 8);
-    bin_count_kernel<<<std::max(gb, 1), 256, 0, st>>>(n, list, list_n, a.qlen, a.slen, counts,
-                                                      a.status, kNoAllocMaxQlen, nullptr);
-    bin_scan_kernel<<<1, 1024, 0, st>>>(counts, cursor, const_cast<int32_t *>(a.rinfo), a.next_task);
-    bin_scatter_kernel<<<std::max(gb, 1), 256, 0, st>>>(n, list, list_n, a.qlen, a.slen, cursor,
-                                                        sorted, kNoAllocMaxQlen);
-    for (int r = kMaxR; r >= 1; --r)
-        d->fn[r - 1]<<<nsm * d->blocks_per_sm[r - 1], 32, smem_bytes(r), st>>>(a, r - 1, 1);
-    TPZ_CUDA(cudaGetLastError());
     return TPZ_OK;
 }
 
@@ -1783,16 +1281,9 @@ extern "C" int tpz_sw_batch_device_noalloc(int64_t n, const int8_t *q, const int
         tpz::set_error("tpz_sw_batch_device_noalloc: NULL buffer");
         return TPZ_E_ARG;
     }
-    // 16-bit lanes are exact only while every score stays below the Fm
-    // reset addend and clear of the int16 limit; a query of up to
-    // kNoAllocMaxQlen rows can score at most kNoAllocMaxQlen * (largest
-    // entry).  The allocating call re-runs such pairs in 32 bits with
-    // scratch of its own; this one has none, so it refuses the matrix.
-    int mn = 0, mx = 0;
-    for (int i = 0; i < 625; ++i) {
-        mn = std::min<int>(mn, mat625_host[i]);
-        mx = std::max<int>(mx, mat625_host[i]);
-    }
+    // the stated matrix limit of this call
+    int mx = 0;
+    for (int i = 0; i < 625; ++i) mx = std::max<int>(mx, mat625_host[i]);
     if ((int64_t)kNoAllocMaxQlen * mx >= std::min(32767 - 2 * std::max(mx, 1), kBig)) {
         char buf[200];
         snprintf(buf, sizeof buf,
@@ -1802,43 +1293,13 @@ extern "C" int tpz_sw_batch_device_noalloc(int64_t n, const int8_t *q, const int
         tpz::set_error(buf);
         return TPZ_E_ARG;
     }
-    const NoAllocDev *d = nullptr;
-    int rc = noalloc_setup(&d);
-    if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    int32_t *counts = d->scratch;
-    int32_t *cursor = counts + kBins;
-    int32_t *rinfo = cursor + kBins;
-    int32_t *next_task = rinfo + 2 * kRBins;
-    int32_t *rerun_count = next_task + kRBins;
-    int32_t *sorted = rerun_count + 4;
-    int32_t *rerun = sorted + kNoAllocMaxPairs;
-
+    const Kernels *k = nullptr;
+    int32_t *ws = nullptr;
+    int rc = kernels(&k);
+    if (rc || (rc = noalloc_scratch(&ws))) return rc;
     Args a;
-    a.rerun_bin_count = nullptr;
-    a.task_count = nullptr;
-    a.q = q; a.qoff = qoff; a.qlen = qlen; a.s = s; a.soff = soff; a.slen = slen;
-    a.score = score; a.ref_end = ref_end; a.read_end = read_end; a.status = status;
-    a.sorted = sorted; a.rinfo = rinfo; a.next_task = next_task;
-    a.rerun = rerun; a.rerun_count = rerun_count;
-    a.gap_open = gap_open; a.gap_extend = gap_extend;
-    a.bias = -mn;
-    memcpy(a.mat, mat625_host, 625);
-    a.translate = 0;
-    a.score_only = 0;
-    memset(a.xq, 0, sizeof a.xq);
-    memset(a.xs, 0, sizeof a.xs);
-    a.bnd = nullptr;
-    a.bnd_words = 0;
-    a.exact_list = nullptr;
-    a.exact_count = nullptr;
-    a.exact_threshold = 32767;
-
-    // the rerun counter carries the previous call's value: clear it
-    TPZ_CUDA(cudaMemsetAsync(rerun_count, 0, sizeof(int32_t), st));
-    a.ssw_lanes = 16;
-    rc = noalloc_round(d, a, n, nullptr, nullptr, counts, cursor, sorted, st);
-    if (rc) return rc;
-    a.ssw_lanes = 8;
-    return noalloc_round(d, a, n, rerun, rerun_count, counts, cursor, sorted, st);
+    pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
+    set_scoring(a, mat625_host, gap_open, gap_extend);
+    int64_t launches = 0;
+    return launch_batch(k, nullptr, a, n, nullptr, ws, kNoAllocMaxQlen, true, (cudaStream_t)stream, launches);
 }
