@@ -1,0 +1,67 @@
+"""The walk and the hitlist where their parallel forms have edges: runs of
+pops that cross blocks of chain elements (rows 8, 32, 64, ... on), rises of
+hits already listed, capacities around a batch of 32 pops, evictions at one
+and over several scores, stops at -S inside a batch, and cursor counts of
+every shared-memory class up to the one that spills -- pop by pop against
+the oracle, on a database of protein families (long runs of similar rows)."""
+import numpy as np
+import pytest
+
+import oracle
+from sa_util import make_db
+from topaz_b200 import alphabet as ab, native, synth
+
+pytestmark = pytest.mark.gpu
+
+BLOSUM62 = synth.matrix("BLOSUM62")
+
+
+@pytest.fixture(scope="module")
+def family_db():
+    rng = np.random.Generator(np.random.PCG64(71))
+    prot = synth.protein_db(1200, seed=70)
+    seqs = list(prot.seqs)
+    members = []
+    for f in range(12):
+        base = synth.random_residues(rng, int(rng.integers(60, 500)))
+        for identity in rng.uniform(0.5, 1.0, 90):
+            members.append(synth.mutate(rng, base, float(identity), indel_rate=0.01))
+        # proteins that repeat a piece of the family: one protein, many rows
+        members += [np.concatenate([synth.mutate(rng, base[:60], 0.8) for _ in range(6)]) for _ in range(20)]
+    seqs += members
+    order = rng.permutation(len(seqs))
+    db = make_db(synth.Proteins(["p%d" % i for i in range(len(seqs))], [seqs[i] for i in order]))
+    qs = [members[i] for i in rng.choice(len(members), 10, replace=False)]
+    qs += [synth.random_residues(rng, n) for n in (5, 6, 7, 37, 260, 261, 600)]
+    # capacity 1.5 * num_hits above 3000 residues; cursors in global memory
+    # above 4505
+    qs += [np.concatenate([members[3], synth.random_residues(rng, 1700)]),
+           np.concatenate([synth.random_residues(rng, 3000), members[40]]),
+           np.concatenate([synth.random_residues(rng, 4500), members[200]])]
+    return db, [ab.aa_to_internal(s).tobytes() for s in qs]
+
+
+@pytest.mark.parametrize("seeds,aligns,num_hits", [(300000, 5000, 100), (300000, 300, 40), (300000, 33, 1),
+                                                   (300000, 32, 21), (300000, 31, 2), (300000, 1, 3),
+                                                   (1, 5000, 100), (33, 5, 100), (777, 64, 10)])
+def test_every_pop_and_hit(cuda, family_db, seeds, aligns, num_hits):
+    db, qs = family_db
+    ix = native.Index(db)
+    cap = 1 << 17
+    r = ix.search(qs, BLOSUM62, num_hits=num_hits, seeds=seeds, alignments=aligns, trace_pops=cap)
+    opts = oracle.Opts(num_hits, 1e-3, 11, 1, 0.267, 0.041, 0.14, 5, seeds, aligns)
+    longest = 0
+    for q, qi in enumerate(qs):
+        P, hits, npops, ncnt, nh = oracle.oracle_query(db, qi, BLOSUM62, opts)
+        assert nh >= 0 and npops <= cap
+        assert (r["npops"][q], r["ncounted"][q]) == (npops, ncnt), q
+        for name in ("row", "off", "score", "len", "counted"):
+            assert (r["trace_" + name][q, :npops] == P[name][:npops]).all(), (q, name)
+        a, b = r["hit_off"][q], r["hit_off"][q + 1]
+        assert list(r["protein"][a:b]) == [h.db_index for h in hits]
+        assert list(r["gapless_score"][a:b]) == [h.gapless_score for h in hits]
+        assert list(r["gapless_length"][a:b]) == [h.gapless_length for h in hits]
+        assert list(r["suffix_offset"][a:b]) == [h.suffix_offset for h in hits]
+        longest = max(longest, npops)
+    if seeds == 300000:
+        assert r["refill_elems"] > 0 and longest > 2000

@@ -464,6 +464,105 @@ int32_t rank_min_for(const RankTables &t, const tpz_search_opts *o, int32_t qlen
     return lo < (int64_t)t.reps.size() ? t.reps[lo] : INT32_MAX;
 }
 
+// The walk's launches: queries by how many cursors their block keeps in
+// shared memory (a block of the largest class would leave a tenth of the
+// blocks of the smallest on an SM), the longest first in each; past the last
+// class the cursors live in global memory.
+constexpr int kWalkClasses = 5;
+constexpr int kWalkCursors[kWalkClasses] = {512, 1024, 2048, 4096, 9000};
+
+struct WalkPlan {
+    std::vector<int32_t> order;            // queries by class, most cursors first
+    int count[kWalkClasses + 1] = {};      // per class; the last one spills
+    std::vector<int64_t> spill_off;
+    size_t spill_bytes = 0;
+};
+
+WalkPlan walk_plan(const std::vector<int64_t> &cur_base, int64_t nq) {
+    WalkPlan p;
+    p.order.resize(nq);
+    for (int64_t q = 0; q < nq; ++q) p.order[q] = (int32_t)q;
+    auto cursors = [&](int32_t q) { return cur_base[q + 1] - cur_base[q]; };
+    std::sort(p.order.begin(), p.order.end(), [&](int32_t x, int32_t y) {
+        return cursors(x) != cursors(y) ? cursors(x) > cursors(y) : x < y;
+    });
+    for (int32_t q : p.order) {
+        int c = 0;
+        while (c < kWalkClasses && cursors(q) > kWalkCursors[c]) ++c;
+        p.count[c]++;
+        if (c == kWalkClasses) {
+            p.spill_off.push_back((int64_t)p.spill_bytes);
+            p.spill_bytes += (tpz::search::walk_state_bytes((int)cursors(q)) + 255) & ~(size_t)255;
+        }
+    }
+    return p;
+}
+
+// Streams of a host thread's walk launches.
+struct WalkStreams {
+    int dev = -1;
+    cudaStream_t aux[kWalkClasses] = {};
+    cudaEvent_t fork = nullptr, join[kWalkClasses] = {};
+    int init() {
+        int d = 0;
+        TPZ_CUDA(cudaGetDevice(&d));
+        if (d == dev) return TPZ_OK;
+        drop();
+        TPZ_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        for (int i = 0; i < kWalkClasses; ++i) {
+            TPZ_CUDA(cudaStreamCreateWithFlags(&aux[i], cudaStreamNonBlocking));
+            TPZ_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
+        }
+        TPZ_CUDA(cudaFuncSetAttribute((const void *)tpz::search::walk_kernel<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)tpz::search::walk_smem(kWalkCursors[kWalkClasses - 1])));
+        dev = d;
+        return TPZ_OK;
+    }
+    void drop() {
+        if (fork) cudaEventDestroy(fork);
+        fork = nullptr;
+        for (int i = 0; i < kWalkClasses; ++i) {
+            if (aux[i]) cudaStreamDestroy(aux[i]);
+            if (join[i]) cudaEventDestroy(join[i]);
+            aux[i] = nullptr;
+            join[i] = nullptr;
+        }
+        dev = -1;
+    }
+    ~WalkStreams() { drop(); }
+};
+
+int launch_walk(const DevIndex &ix, tpz::search::WalkArgs wa, const WalkPlan &p, cudaStream_t st) {
+    using namespace tpz::search;
+    static thread_local WalkStreams ws;
+    int rc = ws.init();
+    if (rc) return rc;
+    // the classes run side by side: the first on st, the others beside it
+    TPZ_CUDA(cudaEventRecord(ws.fork, st));
+    int used = 0;
+    cudaError_t err = cudaSuccess;
+    for (int c = kWalkClasses; c >= 0 && err == cudaSuccess; --c) {
+        if (p.count[c] == 0) continue;
+        cudaStream_t s = st;
+        if (used > 0) {
+            s = ws.aux[used - 1];
+            if ((err = cudaStreamWaitEvent(s, ws.fork, 0)) != cudaSuccess) break;
+        }
+        ++used;
+        if (c == kWalkClasses) walk_kernel<true><<<p.count[c], 32, walk_smem(0), s>>>(ix, wa);
+        else walk_kernel<false><<<p.count[c], 32, walk_smem(kWalkCursors[c]), s>>>(ix, wa);
+        err = cudaGetLastError();
+        wa.order += p.count[c];
+    }
+    for (int i = 1; i < used; ++i) {
+        if (cudaEventRecord(ws.join[i - 1], ws.aux[i - 1]) != cudaSuccess ||
+            cudaStreamWaitEvent(st, ws.join[i - 1], 0) != cudaSuccess)
+            err = cudaGetLastError();
+    }
+    return err == cudaSuccess ? TPZ_OK : tpz::cuda_fail(err, "walk launches");
+}
+
 bool letters_ok(const char *s, int64_t n) {
     for (int64_t i = 0; i < n; ++i)
         if (s[i] < 'A' || s[i] > 'Y') return false;
@@ -836,20 +935,19 @@ int64_t tpz_search_query_device_bytes(int32_t qlen, const tpz_search_opts *o) {
     using namespace tpz::search;
     if (!o || qlen < 0) return -1;
     // the per-query share of tpz_search_batch's device buffers, with the
-    // capacities it sizes them by: cursors with their chain caches, protein
-    // caches and queue links per searched position; the hitlist scratch
-    // (score-bucket lists, hit slots, the protein hash); the hit records;
-    // and, per hit, the Smith-Waterman pair and result arrays
+    // capacities it sizes them by: cursors with their chain and protein
+    // caches per searched position; the hitlist scratch (hit slots, event
+    // log, the protein table); the hit records; and, per hit, the
+    // Smith-Waterman pair and result arrays
     const int64_t ql = qlen > TPZ_SEARCH_MAX_QLEN ? 0 : qlen;
     const int cap = qlen > 3000 ? (int)(1.5 * o->num_hits) : o->alignments;
     const int64_t npos = std::max<int64_t>(0, ql - o->min_hit_length);
     int hash_size = 16;
     while (hash_size < 2 * (cap + 1)) hash_size <<= 1;
-    auto al = [](size_t x) { return (int64_t)((x + 15) & ~(size_t)15); };
-    const size_t ns = (size_t)cap + 1;
-    const int64_t per_q = 7 * al(4 * ns) + 2 * al(4 * (size_t)kSMax) + al(8 * (kSMax / 64)) +
-                          2 * al(4 * (size_t)hash_size);
-    const int64_t per_pos = 2 * ((int64_t)sizeof(Cursor) + 4 + 2 * 4 * kChain);
+    const int64_t per_q = (int64_t)walk_scratch_bytes(cap) + 8 * (int64_t)hash_size + 16;
+    // (walk_state_bytes: a query with too many cursors for shared memory)
+    const int64_t per_pos = 2 * ((int64_t)sizeof(Cursor) + 2 * 4 * kChainSlots +
+                                 (int64_t)walk_state_bytes(1));
     const int64_t per_hit = (int64_t)sizeof(Hit) + 2 * 8 + 18 * 4;
     return (int64_t)qlen + per_q + npos * per_pos + (int64_t)cap * per_hit + 256;
 }
@@ -887,7 +985,7 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
     std::vector<int64_t> pos_base(nq + 1, 0), cur_base(nq + 1, 0);
     std::vector<int32_t> qstatus(nq, 0), qlen_eff(nq);
     int64_t bytes = 0;
-    int max_cap = 1, max_cursors = 1;
+    int max_cap = 1;
     if (o->ingest < 0 || o->ingest > 2) {
         tpz::set_error("tpz_search_batch: ingest must be 0, 1 or 2");
         return TPZ_E_ARG;
@@ -927,17 +1025,14 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
         const int64_t np = std::max(0, qlen_eff[q] - o->min_hit_length);
         pos_base[q + 1] = pos_base[q] + np;
         cur_base[q + 1] = 2 * pos_base[q + 1];
-        max_cursors = std::max<int>(max_cursors, (int)(2 * np));
         const int cap = qlen[q] > 3000 ? (int)(1.5 * o->num_hits) : o->alignments;
         max_cap = std::max(max_cap, cap);
     }
     const int64_t npos = pos_base[nq];
     int hash_size = 16;
     while (hash_size < 2 * (max_cap + 1)) hash_size <<= 1;
-    auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-    const size_t ns = (size_t)max_cap + 1;
-    const size_t per_q = 7 * al(4 * ns) + 2 * al(4 * (size_t)kSMax) + al(8 * (kSMax / 64)) +
-                         2 * al(4 * (size_t)hash_size);
+    const size_t per_q = walk_scratch_bytes(max_cap);
+    const WalkPlan plan = walk_plan(cur_base, nq);
 
     int8_t sub[625], xmap[128];
     internal_sub(o->mat625, sub);
@@ -946,7 +1041,8 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
     DevBuf b;
     uint8_t *dq, *dscratch; int64_t *dqo, *dpb, *dcb; int32_t *dql, *dqs; int8_t *dsub;
     Cursor *dcur; Hit *dhits; QueryOut *dqout; PopRec *dtrace = nullptr;
-    int32_t *dqnext, *dcprot; uint32_t *dcache;
+    int32_t *dcprot, *dorder; uint32_t *dcache; uint64_t *dtable; uint8_t *dspill = nullptr;
+    int64_t *dspill_off = nullptr;
     int rc;
     // 64 readable bytes in front of the queries and behind them: hsp_at's
     // windows read a little past both ends
@@ -954,10 +1050,18 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
         (rc = b.alloc(&dpb, nq + 1)) || (rc = b.alloc(&dcb, nq + 1)) || (rc = b.alloc(&dqs, nq)) ||
         (rc = b.alloc(&dsub, 625)) || (rc = b.alloc(&dcur, 2 * npos + 1)) ||
         (rc = b.alloc(&dscratch, per_q * nq)) || (rc = b.alloc(&dhits, (size_t)nq * max_cap)) ||
-        (rc = b.alloc(&dqout, nq)) || (rc = b.alloc(&dqnext, 2 * npos + 1)) ||
-        (rc = b.alloc(&dcache, (size_t)kChain * (2 * npos + 1))) ||
-        (rc = b.alloc(&dcprot, (size_t)kChain * (2 * npos + 1))))
+        (rc = b.alloc(&dqout, nq)) || (rc = b.alloc(&dorder, nq)) ||
+        (rc = b.alloc(&dtable, (size_t)nq * hash_size)) ||
+        (rc = b.alloc(&dcache, (size_t)kChainSlots * (2 * npos + 1))) ||
+        (rc = b.alloc(&dcprot, (size_t)kChainSlots * (2 * npos + 1))))
         return rc;
+    if (plan.spill_bytes > 0) {
+        if ((rc = b.alloc(&dspill, plan.spill_bytes)) || (rc = b.alloc(&dspill_off, plan.spill_off.size())))
+            return rc;
+        TPZ_CUDA(cudaMemcpy(dspill_off, plan.spill_off.data(), 8 * plan.spill_off.size(), cudaMemcpyHostToDevice));
+    }
+    TPZ_CUDA(cudaMemcpy(dorder, plan.order.data(), 4 * nq, cudaMemcpyHostToDevice));
+    TPZ_CUDA(cudaMemsetAsync(dtable, 0xFF, 8 * (size_t)nq * hash_size, cudaStreamPerThread));
     dq += 64;
     if (o->trace_pops > 0 && (rc = b.alloc(&dtrace, (size_t)nq * o->trace_pops))) return rc;
     unsigned long long *dqueued;
@@ -988,7 +1092,6 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
         SeedArgs sa;
         sa.qcat = dq; sa.qoff = dqo; sa.qlen = dql; sa.pos_base = dpb; sa.nq = (int)nq;
         sa.npos = npos; sa.sub = dsub; sa.cursors = dcur; sa.lb_out = nullptr; sa.qstatus = dqs;
-        sa.chain = kChain;
         seed_kernel<<<(unsigned)std::min<int64_t>((npos + 127) / 128, (int64_t)nsm * 16), 128>>>(ix->d, sa);
         TPZ_CUDA(cudaEventRecord(ev[4], 0));
         chain_kernel<<<(unsigned)std::min<int64_t>((2 * npos * kChain + 255) / 256, (int64_t)nsm * 64),
@@ -1000,13 +1103,13 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
     wa.qcat = dq; wa.qoff = dqo; wa.qlen = dql; wa.nq = (int)nq; wa.cursor_base = dcb;
     wa.cursors = dcur; wa.sub = dsub; wa.min_hit_length = o->min_hit_length;
     wa.seeds = o->seeds; wa.alignments = o->alignments; wa.num_hits = o->num_hits;
-    wa.max_cap = max_cap; wa.hash_size = hash_size; wa.max_cursors = max_cursors;
+    wa.max_cap = max_cap; wa.hash_size = hash_size; wa.order = dorder; wa.table = dtable;
+    wa.spill = dspill; wa.spill_off = dspill_off;
     wa.scratch = dscratch; wa.scratch_per_query = per_q; wa.hits = dhits; wa.qout = dqout;
     wa.qstatus = dqs; wa.trace = dtrace; wa.trace_cap = o->trace_pops;
-    wa.qnext = dqnext; wa.ccache = dcache; wa.cprot = dcprot;
+    wa.ccache = dcache; wa.cprot = dcprot;
     TPZ_CUDA(cudaEventRecord(ev[1], 0));
-    walk_kernel<<<(unsigned)((nq + kWalkWarps - 1) / kWalkWarps), kWalkWarps * 32>>>(ix->d, wa);
-    TPZ_CUDA(cudaGetLastError());
+    if ((rc = launch_walk(ix->d, wa, plan, cudaStreamPerThread))) return rc;
     TPZ_CUDA(cudaEventRecord(ev[2], 0));
 
     ResultHolder *R = new ResultHolder();

@@ -23,14 +23,12 @@ struct Cursor {
     int64_t row;
     int32_t off;
     int16_t dir;
-    uint8_t cpos, cn;    // next unused / valid entries of the cursor's element cache
     int32_t score, len;
     int32_t prot;        // protein of the current row
 };
 
-constexpr int kWalkWarps = 4;            // queries (warps) per walk block
-constexpr int kChain = 64;               // chain elements cached per cursor
-static_assert(kChain >= 32, "a walk refill stores 32 chain elements in a cursor's cache slot");
+constexpr int kChain = 32;               // chain elements precomputed per cursor
+constexpr int kChainSlots = 64;          // and room for 32 more, which the walk computes
 
 struct Hit {
     int32_t protein, gapless_score, gapless_length, suffix_offset;
@@ -44,7 +42,7 @@ struct PopRec {
 struct QueryOut {
     int64_t npops, ncounted;
     int32_t nhits, status;
-    int64_t refills;              // chain caches the walk refilled (32 elements each)
+    int64_t refills;              // blocks of 32 chain elements the walk computed
 };
 
 struct SeedArgs {
@@ -58,7 +56,6 @@ struct SeedArgs {
     Cursor *cursors;           // 2 per position
     int64_t *lb_out;           // optional: bound per position (-2 skipped)
     int32_t *qstatus;          // per query status bits
-    int chain;                 // chain elements precomputed per cursor (0 or kChain)
 };
 
 struct WalkArgs {
@@ -70,11 +67,14 @@ struct WalkArgs {
     Cursor *cursors;
     const int8_t *sub;
     int min_hit_length, seeds, alignments, num_hits;
-    int max_cap, hash_size, max_cursors;
-    uint8_t *scratch;             // per query: hitlist structures
+    int max_cap, hash_size;
+    const int32_t *order;         // the launch's queries, one block each
+    uint64_t *table;              // per query: hash_size entries, all ones at the start
+    uint8_t *scratch;             // per query: walk_scratch_bytes(max_cap)
     size_t scratch_per_query;
-    int32_t *qnext;               // per cursor (global cursor index)
-    uint32_t *ccache;             // 32 packed chain elements per cursor
+    uint8_t *spill;               // cursor state of the launch's blocks (SPILL launches)
+    const int64_t *spill_off;
+    uint32_t *ccache;             // kChainSlots packed chain elements per cursor
     int32_t *cprot;               // the protein of each chain element's row
     Hit *hits;                    // nq * max_cap
     QueryOut *qout;
@@ -86,7 +86,13 @@ struct WalkArgs {
 __global__ void nl_block_count_kernel(const uint8_t *T, int64_t Tsize, int64_t nblocks, uint32_t *cnt);
 __global__ void lb_build_kernel(const uint8_t *T, int64_t Tsize, const int64_t *SA, int64_t *lb);
 __global__ void seed_kernel(DevIndex ix, SeedArgs a);
-__global__ void walk_kernel(DevIndex ix, WalkArgs a);
+template <bool SPILL>
+__global__ void walk_kernel(DevIndex ix, const __grid_constant__ WalkArgs a);
+// shared memory of a walk block with that many cursors, their part of it,
+// and the scratch of a query with that hitlist capacity
+size_t walk_smem(int cursors);
+size_t walk_state_bytes(int cursors);
+size_t walk_scratch_bytes(int cap);
 __global__ void chain_kernel(DevIndex ix, SeedArgs a, int min_hit_length, uint32_t *cache,
                              int32_t *cprot);
 __global__ void hsp_batch_kernel(DevIndex ix, const uint8_t *qcat, const int64_t *qoff,

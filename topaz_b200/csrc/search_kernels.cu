@@ -25,14 +25,13 @@
 //            because '\n' sorts below every letter, so a lower bound needs a
 //            binary search only inside one bucket, starting 5 symbols in.
 //
-// Walk state per query (one thread, exact sequential semantics):
+// Walk state per query (one warp, exact sequential semantics):
 //   the priority queue of suffix cursors is an array of per-score stacks:
 //   among equal scores the newest insert pops first, as with rb_popmax on a
 //   tree where equal keys go right (rbtree.c:70-78, :410-427);
-//   the hitlist keeps per-score FIFO lists (rb_popmin/rb_getmin take the
-//   oldest of the smallest score, rbtree.c:429-457; rb_reput re-inserts as
-//   newest, :496-505) plus an open-addressing protein -> hit table with
-//   backward-shift deletion.
+//   the hitlist is a protein -> slot table and a log of insertions and score
+//   rises, from which each score's list (oldest first, rbtree.c:429-457) is
+//   read when something is evicted and at the end.
 
 #include <stdio.h>
 #include <string.h>
@@ -250,8 +249,8 @@ __global__ void seed_kernel(DevIndex ix, SeedArgs a) {
         const uint8_t *Q = a.qcat + a.qoff[q];
         const int qlen = a.qlen[q];
         Cursor c0, c1;
-        c0.row = -1; c0.off = i; c0.dir = 1; c0.cpos = 0; c0.cn = a.chain; c0.prot = -1; c0.score = 0; c0.len = -1;
-        c1.row = -1; c1.off = i; c1.dir = -1; c1.cpos = 0; c1.cn = a.chain; c1.prot = -1; c1.score = 0; c1.len = -1;
+        c0.row = -1; c0.off = i; c0.dir = 1; c0.prot = -1; c0.score = 0; c0.len = -1;
+        c1.row = -1; c1.off = i; c1.dir = -1; c1.prot = -1; c1.score = 0; c1.len = -1;
         if (Q[i] != 'V') {                     // _bad_prefix: internal 'V' = X
             const int64_t pos = lower_bound(ix, Q + i, qlen - i);
             if (a.lb_out) a.lb_out[g] = pos;
@@ -397,18 +396,6 @@ __device__ __forceinline__ int bits_max_le(const uint64_t *bits, int from) {
     }
 }
 
-// lowest set bit index >= from, or -1
-__device__ __forceinline__ int bits_min_ge(const uint64_t *bits, int from, int nwords) {
-    int w = from >> 6;
-    if (w >= nwords) return -1;
-    uint64_t m = bits[w] & (~0ull << (from & 63));
-    for (;;) {
-        if (m) return (w << 6) + __ffsll(m) - 1;
-        if (++w >= nwords) return -1;
-        m = bits[w];
-    }
-}
-
 // packed chain element: score in the low half, length in the high half
 constexpr int kLenEnd = -1000;      // row outside [0, 8*Tsize): the cursor is freed
 constexpr int kLenFault = -2000;    // row past the zero-filled SA page
@@ -454,278 +441,653 @@ __global__ void chain_kernel(DevIndex ix, SeedArgs a, int min_hit_length, uint32
             if (a.pos_base[mid] <= g) lo = mid; else hi = mid - 1;
         }
         int32_t pr;
-        cache[x] = chain_elem(ix, cu.row, cu.dir, e + 1, a.qcat + a.qoff[lo], a.qlen[lo], cu.off,
-                              a.sub, &pr);
-        cprot[x] = pr;
+        cache[c * kChainSlots + e] = chain_elem(ix, cu.row, cu.dir, e + 1, a.qcat + a.qoff[lo],
+                                                a.qlen[lo], cu.off, a.sub, &pr);
+        cprot[c * kChainSlots + e] = pr;
     }
 }
 
-struct HitView {
-    int32_t *hprot, *hscore, *hlen, *hoff, *hprev, *hnext, *hfree;   // cap+1 slots
-    int32_t *bhead, *btail;      // kSMax per-score lists (head = oldest)
-    uint64_t *bbits;
-    int32_t *hkey, *hval;        // protein -> slot, open addressing
+// ------------------------------------------------------------------ hitlist
+//
+// hitlist_add (hit.c:126-193) for a warp.  A query's hits sit in slots found
+// through an open-addressing protein table; every insertion and every rise
+// of a hit's score is an event in a log, and a hit's place in its score's
+// list (rb_reput re-inserts as newest, rbtree.c:496-505) is its last event.
+// While the list is below its capacity, a batch of up to 32 pops is added at
+// once, one per lane.  At capacity, pops that do not beat the worst hit are
+// counted without a lookup (also many at once), and the others evict the
+// oldest hit of the smallest score (rb_popmin, rbtree.c:429-457), found by
+// walking the log: hits of the smallest score are never added while it is
+// the smallest, so one pass over the log serves all evictions at a score.
+struct HitState {
+    uint64_t *table;        // protein (low half, all ones: free) and slot
+    uint32_t hmask;
+    int4 *slot;             // protein, score, length, query offset
+    int32_t *last;          // last event of each slot
+    int32_t *log;           // slot of each event
+    int32_t *hist;          // hits per score, kept while the list is full
+    int cap, logcap;
+    int size, nev, smax;    // hits, events, largest score seen
+    // full: smallest score, hits that hold it; how far the log has been read
+    // for them, and which of the last 32 events are theirs (cslot: a lane's)
+    int hmin, cmin, scan;
+    unsigned cand;
+    int cslot;
 };
 
-__device__ __forceinline__ HitView hit_view(const WalkArgs &a, int q) {
-    uint8_t *base = a.scratch + (size_t)q * a.scratch_per_query;
-    HitView v;
-    size_t o = 0;
-    auto take = [&](size_t bytes) { uint8_t *p = base + o; o += (bytes + 15) & ~(size_t)15; return p; };
-    const size_t ns = (size_t)a.max_cap + 1;
-    v.hprot = (int32_t *)take(4 * ns);
-    v.hscore = (int32_t *)take(4 * ns);
-    v.hlen = (int32_t *)take(4 * ns);
-    v.hoff = (int32_t *)take(4 * ns);
-    v.hprev = (int32_t *)take(4 * ns);
-    v.hnext = (int32_t *)take(4 * ns);
-    v.hfree = (int32_t *)take(4 * ns);
-    v.bhead = (int32_t *)take(4 * (size_t)kSMax);
-    v.btail = (int32_t *)take(4 * (size_t)kSMax);
-    v.bbits = (uint64_t *)take(8 * (size_t)(kSMax / 64));
-    v.hkey = (int32_t *)take(4 * (size_t)a.hash_size);
-    v.hval = (int32_t *)take(4 * (size_t)a.hash_size);
-    return v;
+constexpr uint64_t kFree = ~0ull;
+
+__device__ __forceinline__ uint64_t table_entry(int32_t p, int32_t s) {
+    return (uint64_t)(uint32_t)p | ((uint64_t)(uint32_t)s << 32);
 }
 
-// One warp per query.  Lane 0 runs the pop loop of
+// everything below reads mutable memory past L1 (other lanes write it)
+__device__ __forceinline__ int4 load_slot(const HitState &h, int s) { return __ldcg(h.slot + s); }
+
+// events in order, the outdated ones dropped
+__device__ void compact_log(HitState &h, int lane) {
+    int n = 0;
+    for (int base = 0; base < h.nev; base += 32) {
+        const int e = base + lane;
+        const int s = e < h.nev ? __ldcg(h.log + e) : -1;
+        const bool live = s >= 0 && __ldcg(h.last + s) == e;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, live);
+        if (live) {
+            const int i = n + __popc(m & ((1u << lane) - 1u));
+            h.log[i] = s;
+            h.last[s] = i;
+        }
+        n += __popc(m);
+        __syncwarp();
+    }
+    h.nev = n;
+    h.scan = 0;
+    h.cand = 0;
+}
+
+// hits per score into hist[0 .. top]
+__device__ void count_scores(HitState &h, int lane, int top) {
+    for (int s = lane; s <= top; s += 32) h.hist[s] = 0;
+    __syncwarp();
+    for (int base = 0; base < h.nev; base += 32) {
+        const int e = base + lane;
+        const int s = e < h.nev ? __ldcg(h.log + e) : -1;
+        if (s >= 0 && __ldcg(h.last + s) == e) atomicAdd(&h.hist[load_slot(h, s).y], 1);
+    }
+    __syncwarp();
+}
+
+// the smallest score >= from that a hit holds
+__device__ int next_score(const HitState &h, int from, int lane) {
+    for (int b = from; b <= h.smax; b += 32) {
+        const unsigned m =
+            __ballot_sync(0xFFFFFFFFu, b + lane <= h.smax && __ldcg(h.hist + b + lane) > 0);
+        if (m) return b + __ffs(m) - 1;
+    }
+    return kSMax;
+}
+
+// Where protein p is in the table, 32 entries per read: its slot, or -1 and
+// the free entry that ends its probe sequence.
+__device__ int find(const HitState &h, int lane, int p, uint32_t *at) {
+    for (uint32_t b = hash32((uint32_t)p);; b += 32) {
+        const uint32_t i = (b + lane) & h.hmask;
+        const uint64_t e = __ldcg(h.table + i);
+        const unsigned hit = __ballot_sync(0xFFFFFFFFu, e != kFree && (int32_t)(uint32_t)e == p);
+        const unsigned end = __ballot_sync(0xFFFFFFFFu, e == kFree);
+        if (!hit && !end) continue;
+        const int l = __ffs(hit ? hit : end) - 1;
+        *at = (b + l) & h.hmask;
+        return hit ? (int)__shfl_sync(0xFFFFFFFFu, (uint32_t)(e >> 32), l) : -1;
+    }
+}
+
+// deletes protein p from the table (backward shift)
+__device__ void erase(HitState &h, int lane, int p) {
+    uint32_t hole;
+    find(h, lane, p, &hole);
+    for (uint32_t b = hole + 1;; b += 32) {
+        const uint64_t mine = __ldcg(h.table + ((b + lane) & h.hmask));
+        for (int l = 0; l < 32; ++l) {
+            const uint64_t e = __shfl_sync(0xFFFFFFFFu, mine, l);
+            if (e == kFree) {
+                if (lane == 0) h.table[hole] = kFree;
+                __syncwarp();
+                return;
+            }
+            const uint32_t j = (b + l) & h.hmask, k = hash32((uint32_t)e) & h.hmask;
+            // move j into the hole when its home k is not in (hole, j]
+            const bool keep = (hole <= j) ? (hole < k && k <= j) : (hole < k || k <= j);
+            if (!keep) {
+                if (lane == 0) h.table[hole] = e;
+                hole = j;
+            }
+        }
+    }
+}
+
+// the oldest hit of the smallest score: its slot (h.cmin > 0)
+__device__ int oldest_of_min(HitState &h, int lane) {
+    for (;;) {
+        while (h.cand) {
+            // what the last read of the log found, unless it rose since
+            const int l = __ffs(h.cand) - 1;
+            h.cand &= h.cand - 1;
+            const int s = __shfl_sync(0xFFFFFFFFu, h.cslot, l);
+            if (__ldcg(h.last + s) == h.scan - 32 + l) return s;
+        }
+        const int e = h.scan + lane;
+        const int s = e < h.nev ? __ldcg(h.log + e) : -1;
+        const bool hit = s >= 0 && __ldcg(h.last + s) == e && load_slot(h, s).y == h.hmin;
+        h.cslot = s;
+        h.cand = __ballot_sync(0xFFFFFFFFu, hit);
+        h.scan += 32;
+    }
+}
+
+// full list: the smallest score and how many hold it
+__device__ void set_min(HitState &h, int lane, int from) {
+    h.hmin = next_score(h, from, lane);
+    h.cmin = h.hmin < kSMax ? __ldcg(h.hist + h.hmin) : 0;
+    h.scan = 0;
+    h.cand = 0;
+}
+
+__device__ void now_full(HitState &h, int lane) {
+    count_scores(h, lane, kSMax - 1);
+    set_min(h, lane, 0);
+}
+
+// one pop (the same in every lane), which beats the worst hit of a full
+// list; true when it is counted
+__device__ bool add_one(HitState &h, int lane, int p, int gs, int gl, int off) {
+    uint32_t at;
+    int s = find(h, lane, p, &at);
+    const bool fresh = s < 0, full = h.size >= h.cap;
+    int left = -1;                       // score that loses a hit
+    if (fresh) {
+        s = h.size;
+        if (full) {
+            s = oldest_of_min(h, lane);
+            left = h.hmin;
+            const int wp = load_slot(h, s).x;
+            // p first: erase then moves it along if the hole is on its way
+            if (lane == 0) h.table[at] = table_entry(p, s);
+            __syncwarp();
+            erase(h, lane, wp);
+        } else {
+            if (lane == 0) h.table[at] = table_entry(p, s);
+            h.size++;
+        }
+    } else {
+        const int4 x = load_slot(h, s);
+        if (x.y >= gs) return false;
+        left = x.y;
+        off = x.w;                       // the offset stays the first one's
+    }
+    h.smax = max(h.smax, gs);
+    if (lane == 0) {
+        h.slot[s] = make_int4(p, gs, gl, off);
+        h.log[h.nev] = s;
+        h.last[s] = h.nev;
+        if (full) {
+            atomicAdd(&h.hist[gs], 1);
+            atomicSub(&h.hist[left], 1);
+        }
+    }
+    h.nev++;
+    __syncwarp();
+    if (full) {
+        if (left == h.hmin && --h.cmin == 0) set_min(h, lane, h.hmin + 1);
+    } else if (h.size >= h.cap) {
+        now_full(h, lane);
+    }
+    return fresh;
+}
+
+// Adds the pops of lanes 0 .. n-1 in lane order; bit l of the result: pop l
+// is counted.  Stops after the pop that brings the counted ones to `room`:
+// *n is how many were added.
+__device__ unsigned add_pops(HitState &h, int lane, int *n, int64_t room, int p, int gs, int gl, int off) {
+    if (h.nev + 32 > h.logcap) compact_log(h, lane);
+    const int cnt = *n;
+    const bool valid = lane < cnt;
+    const unsigned lt = (1u << lane) - 1u;
+    const unsigned same =
+        __match_any_sync(0xFFFFFFFFu, valid ? (uint64_t)(uint32_t)p : kFree - (uint64_t)lane);
+    if (h.size < h.cap && h.size + cnt <= h.cap && cnt < room) {
+        // pops of one protein one after the other, the rest together
+        unsigned todo = cnt == 32 ? 0xFFFFFFFFu : (1u << cnt) - 1u;
+        unsigned fresh_all = 0, event_all = 0;
+        int s = -1;
+        while (todo) {
+            const bool mine = (todo >> lane & 1) && !(same & todo & lt);
+            uint32_t i = 0;
+            bool fresh = false;
+            if (mine) {
+                i = hash32((uint32_t)p) & h.hmask;
+                for (;;) {
+                    uint64_t e = __ldcg(h.table + i);
+                    if (e == kFree) {
+                        // claim it; the slot number follows below
+                        e = atomicCAS((unsigned long long *)h.table + i, kFree, table_entry(p, -1));
+                        if (e == kFree) { fresh = true; break; }
+                    }
+                    if ((int32_t)(uint32_t)e == p) { s = (int)(e >> 32); break; }
+                    i = (i + 1) & h.hmask;
+                }
+            }
+            const unsigned nf = __ballot_sync(0xFFFFFFFFu, fresh);
+            bool event = fresh;
+            if (fresh) {
+                s = h.size + __popc(nf & lt);
+                h.table[i] = table_entry(p, s);
+                h.slot[s] = make_int4(p, gs, gl, off);
+            } else if (mine) {
+                const int4 x = load_slot(h, s);
+                if (x.y < gs) {
+                    h.slot[s] = make_int4(p, gs, gl, x.w);
+                    event = true;
+                }
+            }
+            h.size += __popc(nf);
+            fresh_all |= nf;
+            event_all |= __ballot_sync(0xFFFFFFFFu, event);
+            todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+            __syncwarp();
+        }
+        // events in pop order; a slot keeps its last one
+        if (event_all >> lane & 1) {
+            const int e = h.nev + __popc(event_all & lt);
+            h.log[e] = s;
+            if (!(same & event_all & ~lt & ~(1u << lane))) h.last[s] = e;
+        }
+        h.nev += __popc(event_all);
+        h.smax = max(h.smax, (int)__reduce_max_sync(0xFFFFFFFFu, valid ? (unsigned)gs : 0u));
+        __syncwarp();
+        if (h.size >= h.cap) now_full(h, lane);
+        return fresh_all;
+    }
+    // At or near capacity.  Every pop that beats the worst hit looks its
+    // protein up (together); what an earlier pop of the batch may change of
+    // that is only a protein it added or raised itself, and a hit it evicted.
+    unsigned counted = 0, stale = 0;
+    int os = -1;                         // score of the pop's protein, -1: not in the list
+    if (valid && (h.size < h.cap || gs > h.hmin)) {
+        for (uint32_t i = hash32((uint32_t)p) & h.hmask;; i = (i + 1) & h.hmask) {
+            const uint64_t e = __ldcg(h.table + i);
+            if (e == kFree) break;
+            if ((int32_t)(uint32_t)e == p) { os = load_slot(h, (int)(e >> 32)).y; break; }
+        }
+    }
+    for (int l = 0; l < cnt;) {
+        const bool full = h.size >= h.cap;
+        // the next pop that may change the list; those before it are counted
+        // when they do not beat the worst hit, and otherwise hold a protein
+        // with a score at least theirs -- above the worst, so not evicted
+        const bool acts = valid && lane >= l && !(full && gs <= h.hmin) && (os < gs || (stale >> lane & 1));
+        const unsigned below = __ballot_sync(0xFFFFFFFFu, valid && full && gs <= h.hmin);
+        const unsigned next = __ballot_sync(0xFFFFFFFFu, acts);
+        const int to = next ? __ffs(next) - 1 : cnt;
+        unsigned run = below & ~((1u << l) - 1u) & (to == 32 ? 0xFFFFFFFFu : (1u << to) - 1u);
+        if (__popc(run) >= room) {
+            // the stop at -S is among them: the room-th set bit
+            while (--room > 0) run &= run - 1;
+            const int at = __ffs(run) - 1;
+            *n = at + 1;
+            return counted | (below & ~((1u << l) - 1u) & ((2u << at) - 1u));
+        }
+        room -= __popc(run);
+        counted |= run;
+        l = to;
+        if (l >= cnt) break;
+        const int bp = __shfl_sync(0xFFFFFFFFu, p, l), bs = __shfl_sync(0xFFFFFFFFu, gs, l);
+        const int bl = __shfl_sync(0xFFFFFFFFu, gl, l), bo = __shfl_sync(0xFFFFFFFFu, off, l);
+        if (add_one(h, lane, bp, bs, bl, bo)) {
+            counted |= 1u << l;
+            if (--room == 0) { *n = l + 1; return counted; }
+        }
+        stale |= __shfl_sync(0xFFFFFFFFu, same, l);
+        ++l;
+    }
+    return counted;
+}
+
+// The hitlist in traversal order (score descending, newest first): a
+// counting sort of the live events from the newest to the oldest.
+__device__ void write_hits(HitState &h, int lane, Hit *out) {
+    count_scores(h, lane, h.smax);
+    int run = 0;
+    for (int top = h.smax; top >= 0; top -= 32) {
+        const int s = top - lane;
+        const int c = s >= 0 ? __ldcg(h.hist + s) : 0;
+        int x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (s >= 0) h.hist[s] = run + x - c;
+        run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+    __syncwarp();
+    for (int base = h.nev - 1; base >= 0; base -= 32) {
+        const int e = base - lane;
+        const int s = e >= 0 ? __ldcg(h.log + e) : -1;
+        const bool live = s >= 0 && __ldcg(h.last + s) == e;
+        int4 x = make_int4(0, -1 - lane, 0, 0);
+        if (live) x = load_slot(h, s);
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, x.y);
+        if (live) {
+            const int rank = __popc(same & ((1u << lane) - 1u));
+            const int at = __ldcg(h.hist + x.y) + rank;
+            Hit o;
+            o.protein = x.x; o.gapless_score = x.y; o.gapless_length = x.z; o.suffix_offset = x.w;
+            out[at] = o;
+        }
+        __syncwarp();
+        if (live && !(same & ((1u << lane) - 1u))) h.hist[x.y] += __popc(same);
+        __syncwarp();
+    }
+}
+
+// --------------------------------------------------------------------- walk
+//
 // query_fetch_alignment_batch (src/query.c:151-157) over pqueue_next
-// (priority_queue.c:36-56) and hitlist_add (hit.c:126-193) exactly, with the
-// per-score cursor stacks in shared memory.  A cursor's next chain elements
-// (sa_hsp at rows row+dir, row+2dir, ...) come from a 32-entry per-cursor
-// cache that all 32 lanes refill in one go whenever lane 0 pops a cursor
-// whose cache is used up, so consecutive pops of a cursor cost no sa_hsp.
-// Elements past the end of a chain are computed and never used.
-__global__ void __launch_bounds__(kWalkWarps * 32) walk_kernel(DevIndex ix, WalkArgs a) {
-    constexpr int NW = kSMax / 64;
-    __shared__ int16_t s_qhead[kWalkWarps][kSMax];
-    __shared__ uint64_t s_qbits[kWalkWarps][NW];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int q = blockIdx.x * kWalkWarps + wib;
-    if (q >= a.nq) return;
-    int16_t *qhead = s_qhead[wib];
-    uint64_t *qbits = s_qbits[wib];
+// (priority_queue.c:36-56): pop the newest cursor of the highest score, move
+// it one row on and push it again, add the popped row to the hitlist.  One
+// warp per query.
+//
+// The order of pops has runs that do not depend on each other.  Let s be the
+// highest score.  The top cursor of its stack pops, and while its next row
+// scores s or more it pops again at once (it is then alone above s, or the
+// newest at s); when it falls below s, or out of the queue, the cursor under
+// it follows.  So up to 32 cursors of the stack take their runs together, a
+// lane each, and their pushes below s are made in stack order.  Nothing in
+// the queue depends on the hitlist, whose only way back is the stop at -S
+// counted pops, so the popped rows are collected and added 32 at a time.
+// All queue state is in shared memory: per cursor the rows advanced, the
+// link to the next in its stack and the scores of its next rows.
+// Bound: latency of dependent shared-memory and L2 reads, now per group of
+// pops: about 40 cycles per cursor to read a stack's links, some 1,000 per
+// group for the rest.  (One lane popping one cursor after the other through
+// global memory took 1.15 us per pop; the same in shared memory 0.45 us.)
+
+// a cursor's state: rows advanced, and the next cursor in its score's stack
+struct CurState {
+    uint32_t k;
+    int32_t link;
+};
+
+constexpr int kBuf = 8;                 // chain elements staged per cursor
+constexpr int kHeadSmem = 1024;         // scores whose stack head is in shared memory
+constexpr int kScoreWords = kSMax / 64;
+// codes of a staged element besides a score >= 0
+constexpr int16_t kNotQueued = -1;      // too short, or past the array: the cursor is not pushed
+constexpr int16_t kFault = -2;          // row past the zero-filled SA page
+static_assert(kChain == 32 && kChainSlots == 64, "blocks of 32 elements in two halves");
+// bitmap, stack heads and pops of a batch in front of the cursors
+constexpr int kPops = 128;              // ring of popped rows
+constexpr int kWalkFixed = 8 * kScoreWords + 2 * kHeadSmem + kPops * (int)sizeof(CurState);
+static_assert(kWalkFixed % 16 == 0, "cursor state alignment");
+
+__device__ __forceinline__ int16_t push_code(uint32_t elem, int minlen) {
+    const int ln = elem_len(elem);
+    if (ln == kLenFault) return kFault;
+    return ln >= minlen ? (int16_t)elem_score(elem) : kNotQueued;
+}
+
+// A query's cursors in shared memory, or (SPILL: queries with too many) in
+// global memory.
+template <bool SPILL>
+__global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_constant__ WalkArgs a) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int lane = threadIdx.x;
+    const int q = a.order[blockIdx.x];
     const uint8_t *Q = a.qcat + a.qoff[q];
     const int qlen = a.qlen[q];
     const int minlen = a.min_hit_length;
     const int64_t cbase = a.cursor_base[q];
     const int ncur = (int)(a.cursor_base[q + 1] - cbase);
-    Cursor *cur = a.cursors + cbase;
-    int32_t *qnext = a.qnext + cbase;
-    uint32_t *cache = a.ccache + cbase * kChain;
-    int32_t *cprot = a.cprot + cbase * kChain;
-    HitView v = hit_view(a, q);
-    const int cap = qlen > 3000 ? (int)(1.5 * a.num_hits) : a.alignments;   // hit.c:106-109
+    const Cursor *cur = a.cursors + cbase;
+    uint32_t *cache = a.ccache + cbase * kChainSlots;
+    int32_t *cprot = a.cprot + cbase * kChainSlots;
 
-    // ---- cooperative initialisation
-    for (int i = lane; i < kSMax; i += 32) {
-        qhead[i] = -1;
-        v.bhead[i] = -1;
-        v.btail[i] = -1;
+    uint64_t *bits = reinterpret_cast<uint64_t *>(smem);
+    int16_t *head_low = reinterpret_cast<int16_t *>(bits + kScoreWords);
+    CurState *pops = reinterpret_cast<CurState *>(head_low + kHeadSmem);     // rows on, cursor
+    int16_t *buf = reinterpret_cast<int16_t *>(SPILL ? a.spill + a.spill_off[blockIdx.x] : smem + kWalkFixed);
+    CurState *state = reinterpret_cast<CurState *>(buf + kBuf * (size_t)ncur);
+
+    HitState h;
+    {
+        uint8_t *base = a.scratch + (size_t)q * a.scratch_per_query;
+        const size_t ns = (size_t)a.max_cap;
+        h.table = a.table + (size_t)q * a.hash_size;
+        h.hmask = (uint32_t)a.hash_size - 1;
+        h.slot = (int4 *)base;
+        h.last = (int32_t *)(h.slot + ns);
+        h.log = h.last + ns;
+        h.logcap = 2 * a.max_cap + 64;
+        h.hist = h.log + h.logcap;
+        h.cap = qlen > 3000 ? (int)(1.5 * a.num_hits) : a.alignments;   // hit.c:106-109
+        h.size = h.nev = 0;
+        h.smax = 0;
+        h.hmin = kSMax;
+        h.cmin = h.scan = h.cslot = 0;
+        h.cand = 0;
     }
-    for (int i = lane; i < NW; i += 32) { qbits[i] = 0; v.bbits[i] = 0; }
-    for (int i = lane; i < a.hash_size; i += 32) v.hkey[i] = -1;
-    for (int i = lane; i <= cap; i += 32) v.hfree[i] = cap - i;
+    // stack heads of the scores past shared memory, after this query's histogram
+    int16_t *head_high = reinterpret_cast<int16_t *>(h.hist + kSMax);
+    auto head = [&](int s) -> int16_t & { return s < kHeadSmem ? head_low[s] : head_high[s]; };
+    auto has = [&](int s) { return (bits[s >> 6] >> (s & 63)) & 1; };
+    // blocks of 32 elements take the two halves of a cursor's slots in turn,
+    // so the element before a new block keeps its place
+    auto chain_at = [](int c, uint32_t e) { return (size_t)c * kChainSlots + e % kChainSlots; };
+
+    // ---- the queue in seeding insertion order: a cursor's link is the one
+    // before it with the same score
+    for (int i = lane; i < kScoreWords; i += 32) bits[i] = 0;
     __syncwarp();
-
     int qmax = -1;
-    int64_t qsize = 0;
-    int nfree = cap + 1, hsize = 0, hmin = kSMax;
-    const uint32_t hmask = (uint32_t)a.hash_size - 1;
-    int64_t npops = 0, counter = 0, refills = 0;
-    int status = 0;
-    PopRec *trace = a.trace ? a.trace + (int64_t)q * a.trace_cap : nullptr;
-    if (lane == 0) {
-        // the queue in seeding insertion order
-        for (int c = 0; c < ncur; ++c) {
-            if (cur[c].len >= minlen) {
-                const int sc = cur[c].score;
-                qnext[c] = qhead[sc];
-                qhead[sc] = (int16_t)c;
-                qbits[sc >> 6] |= 1ull << (sc & 63);
-                if (sc > qmax) qmax = sc;
-                ++qsize;
-            }
+    for (int base = 0; base < ncur; base += 32) {
+        const int c = base + lane;
+        int sc = -1;
+        if (c < ncur && cur[c].len >= minlen) {
+            sc = cur[c].score;
+            // the scores of its first rows
+            const uint4 *e = reinterpret_cast<const uint4 *>(cache + (size_t)c * kChainSlots);
+            const uint4 x = e[0], y = e[1];
+            const uint32_t w[kBuf] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int i = 0; i < kBuf; ++i) buf[kBuf * c + i] = push_code(w[i], minlen);
         }
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, sc >= 0 ? sc : -1 - lane);
+        const unsigned below = same & ((1u << lane) - 1u), above = same & ~((2u << lane) - 1u);
+        if (sc >= 0) {
+            CurState st;
+            st.k = 0;
+            st.link = below ? base + 31 - __clz(below) : has(sc) ? head(sc) : -1;
+            state[c] = st;
+        }
+        __syncwarp();
+        if (sc >= 0 && !above) {
+            head(sc) = (int16_t)c;
+            atomicOr((unsigned long long *)&bits[sc >> 6], 1ull << (sc & 63));
+        }
+        qmax = max(qmax, __reduce_max_sync(0xFFFFFFFFu, sc));
+        __syncwarp();
     }
 
+    int64_t npops = 0, counter = 0, refills = 0;
+    PopRec *trace = a.trace ? a.trace + (int64_t)q * a.trace_cap : nullptr;
+    // why a cursor's run stops before its score falls below the stack's
+    enum { kNo, kBlock, kRefill, kPastEnd };
+    bool open = qmax >= 0;               // the queue goes on
+    bool past_end = false;
+    int first = 0, pending = 0;          // popped rows not yet in the hitlist: pops[first ..]
+    int filled = -1;                     // cursor whose next block of elements has been computed
+    int refill = -1;                     // cursor that waits for that
     for (;;) {
-        // ---- lane 0: pop the newest cursor of the highest score
-        int c = -1, need = 0, off = 0, dir = 0;
-        int64_t row = 0;
-        Cursor cc;
-        if (lane == 0 && qsize > 0) {
+        while (open && refill < 0 && pending < 32) {
             const int s = qmax;
-            c = qhead[s];
-            cc = cur[c];
-            const int nx = qnext[c];
-            qhead[s] = (int16_t)nx;
-            if (nx < 0) {
-                qbits[s >> 6] &= ~(1ull << (s & 63));
-                qmax = s > 0 ? bits_max_le(qbits, s - 1) : -1;
+            // ---- the first 32 cursors of the stack
+            int c = -1, held = 0, under = head(s);
+            while (under >= 0 && held < 32) {
+                if (lane == held) c = under;
+                under = state[under].link;
+                ++held;
             }
-            --qsize;
-            row = cc.row; off = cc.off; dir = cc.dir;
-            need = cc.cpos >= cc.cn;
-        }
-        c = __shfl_sync(0xFFFFFFFFu, c, 0);
-        if (c < 0) break;
-        need = __shfl_sync(0xFFFFFFFFu, need, 0);
-        uint32_t elem = 0;
-        int32_t eprot = -1;
-        if (need) {
-            ++refills;
-            // all lanes: the next 32 rows of this cursor
-            row = __shfl_sync(0xFFFFFFFFu, row, 0);
-            off = __shfl_sync(0xFFFFFFFFu, off, 0);
-            dir = __shfl_sync(0xFFFFFFFFu, dir, 0);
-            elem = chain_elem(ix, row, dir, lane + 1, Q, qlen, off, a.sub, &eprot);
-            cache[(int64_t)c * kChain + lane] = elem;
-            cprot[(int64_t)c * kChain + lane] = eprot;
+            // ---- their runs, inside the staged block of elements
+            uint32_t k0 = 0, k = 0;
+            int stop = kNo, sc = kNotQueued;
+            if (c >= 0) {
+                k = k0 = state[c].k;
+                if ((k & (kBuf - 1)) == 0 && k > 0) {
+                    if (k >= kChain && k % 32 == 0 && c != filled) {
+                        stop = kRefill;
+                    } else {
+                        const uint4 *e = reinterpret_cast<const uint4 *>(cache + chain_at(c, k));
+                        const uint4 x = __ldcg(e), y = __ldcg(e + 1);
+                        const uint32_t w[kBuf] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                        for (int i = 0; i < kBuf; ++i) buf[kBuf * c + i] = push_code(w[i], minlen);
+                    }
+                }
+                while (stop == kNo) {
+                    const int x = buf[kBuf * c + (k & (kBuf - 1))];
+                    if (x == kFault) { stop = kPastEnd; break; }
+                    ++k;
+                    sc = x;
+                    if (x < s) break;
+                    if ((k & (kBuf - 1)) == 0) stop = kBlock;
+                }
+            }
+            // ---- those up to the first stopped run, as far as the ring has room
+            const int run = (int)(k - k0);
+            const unsigned stopped = __ballot_sync(0xFFFFFFFFu, stop != kNo);
+            const int end = stopped ? __ffs(stopped) - 1 : 32;
+            int sum = run;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+                if (lane >= o) sum += y;
+            }
+            const bool take = c >= 0 && (lane < end || (lane == end && run > 0)) && sum <= kPops - 32;
+            const int taken = __popc(__ballot_sync(0xFFFFFFFFu, take));
+            if (take) {
+                for (int i = 0; i < run; ++i) {
+                    CurState r;
+                    r.k = k0 + i;
+                    r.link = c;
+                    pops[(first + pending + sum - run + i) & (kPops - 1)] = r;
+                }
+                state[c].k = k;
+            }
+            if (taken > 0) pending += __shfl_sync(0xFFFFFFFFu, sum, taken - 1);
+            if (__any_sync(0xFFFFFFFFu, take && c == filled)) filled = -1;
+            // ---- what is left of the stack, then the pushes in stack order
+            const int top = taken < held ? __shfl_sync(0xFFFFFFFFu, c, taken & 31) : under;
+            if (lane == 0) {
+                if (top >= 0) head(s) = (int16_t)top;
+                else bits[s >> 6] &= ~(1ull << (s & 63));
+            }
+            if (!take) sc = kNotQueued;
+            const unsigned same = __match_any_sync(0xFFFFFFFFu, sc >= 0 ? sc : -1 - lane);
+            const unsigned below = same & ((1u << lane) - 1u), above = same & ~((2u << lane) - 1u);
+            __syncwarp();
+            const int prev = below ? 31 - __clz(below) : lane;
+            const int pc = __shfl_sync(0xFFFFFFFFu, c, prev);
+            if (sc >= 0) state[c].link = below ? pc : has(sc) ? head(sc) : -1;
+            __syncwarp();
+            if (sc >= 0 && !above) {
+                head(sc) = (int16_t)c;
+                atomicOr((unsigned long long *)&bits[sc >> 6], 1ull << (sc & 63));
+            }
+            const int up = __reduce_max_sync(0xFFFFFFFFu, sc);
+            __syncwarp();
+            if (up >= s) qmax = up;
+            else if (top < 0) qmax = s > 0 ? bits_max_le(bits, s - 1) : -1;
+            open = qmax >= 0;
+            // ---- the stopped run's reason, once every run before it is taken
+            const int why = __shfl_sync(0xFFFFFFFFu, stop, end & 31);
+            const int at_end = __shfl_sync(0xFFFFFFFFu, run, end & 31);
+            if (end < 32 && taken == (at_end > 0 ? end + 1 : end)) {
+                if (why == kRefill) refill = __shfl_sync(0xFFFFFFFFu, c, end);
+                if (why == kPastEnd) { past_end = true; open = false; }
+            }
             __syncwarp();
         }
-        int stop = 0;
-        if (lane == 0) {
-            if (need) {
-                cc.cpos = 1;
-                cc.cn = 32;
-            } else {
-                elem = cache[(int64_t)c * kChain + cc.cpos];
-                eprot = cprot[(int64_t)c * kChain + cc.cpos];
-                cc.cpos++;
+        // ---- popped rows into the hitlist
+        int n = min(pending, 32);
+        if (n > 0) {
+            int p = -1, gs = 0, gl = 0, off = 0;
+            int64_t row = 0;
+            if (lane < n) {
+                const CurState r = pops[(first + lane) & (kPops - 1)];
+                const Cursor x = cur[r.link];
+                off = x.off;
+                row = x.row + (int64_t)x.dir * r.k;
+                p = x.prot; gs = x.score; gl = x.len;
+                if (r.k > 0) {
+                    const size_t at = chain_at(r.link, r.k - 1);
+                    const uint32_t w = __ldcg(cache + at);
+                    gs = elem_score(w);
+                    gl = elem_len(w);
+                    p = __ldcg(cprot + at);
+                }
             }
-            const int gs = cc.score, gl = cc.len, gprot = cc.prot;
-            // suffix_increment + suffix_active
-            const int ln = elem_len(elem);
-            if (ln == kLenFault) {
-                status |= TPZ_Q_SA_END;
-                stop = 1;
-            } else {
-                if (ln != kLenEnd) {
-                    cc.row = row + dir;
-                    cc.len = ln;
-                    cc.prot = eprot;
-                    if (ln >= minlen) {
-                        const int sc = elem_score(elem);
-                        cc.score = sc;
-                        qnext[c] = qhead[sc];
-                        qhead[sc] = (int16_t)c;
-                        qbits[sc >> 6] |= 1ull << (sc & 63);
-                        if (sc > qmax) qmax = sc;
-                        ++qsize;
-                    }
-                }
-                cur[c] = cc;
-
-                // ---- hitlist_add (every queued row is below sa_rows: seeding and
-                // the advance above stop at the first row past it)
-                bool counted = false;
-                if (hsize >= cap && hmin >= gs) {
-                    counted = true;            // full and the worst hit is at least as good
-                } else {
-                    const int p = gprot;      // protein_of(ix, ix.SA[row])
-                    uint32_t hh = hash32((uint32_t)p) & hmask;
-                    while (v.hkey[hh] != -1 && v.hkey[hh] != p) hh = (hh + 1) & hmask;
-                    if (v.hkey[hh] == -1) {
-                        // new protein: newest entry of its score list
-                        const int slot = v.hfree[--nfree];
-                        v.hprot[slot] = p; v.hscore[slot] = gs; v.hlen[slot] = gl; v.hoff[slot] = off;
-                        v.hnext[slot] = -1;
-                        v.hprev[slot] = v.btail[gs];
-                        if (v.btail[gs] >= 0) v.hnext[v.btail[gs]] = slot; else v.bhead[gs] = slot;
-                        v.btail[gs] = slot;
-                        v.bbits[gs >> 6] |= 1ull << (gs & 63);
-                        if (gs < hmin) hmin = gs;
-                        v.hkey[hh] = p; v.hval[hh] = slot;
-                        ++hsize;
-                        if (hsize > cap) {
-                            // evict the oldest entry of the smallest score
-                            const int m = hmin;
-                            const int w = v.bhead[m];
-                            v.bhead[m] = v.hnext[w];
-                            if (v.bhead[m] >= 0) v.hprev[v.bhead[m]] = -1; else {
-                                v.btail[m] = -1;
-                                v.bbits[m >> 6] &= ~(1ull << (m & 63));
-                                const int nm = bits_min_ge(v.bbits, m + 1, NW);
-                                hmin = nm < 0 ? kSMax : nm;
-                            }
-                            // delete its protein from the table (backward shift)
-                            const int wp = v.hprot[w];
-                            uint32_t i = hash32((uint32_t)wp) & hmask;
-                            while (v.hkey[i] != wp) i = (i + 1) & hmask;
-                            uint32_t j = i;
-                            for (;;) {
-                                j = (j + 1) & hmask;
-                                if (v.hkey[j] == -1) break;
-                                const uint32_t k = hash32((uint32_t)v.hkey[j]) & hmask;
-                                // move j into the hole at i when its home k is not in (i, j]
-                                const bool keep = (i <= j) ? (i < k && k <= j) : (i < k || k <= j);
-                                if (!keep) {
-                                    v.hkey[i] = v.hkey[j]; v.hval[i] = v.hval[j];
-                                    i = j;
-                                }
-                            }
-                            v.hkey[i] = -1;
-                            v.hfree[nfree++] = w;
-                            --hsize;
-                        }
-                        counted = true;
-                    } else {
-                        const int h = v.hval[hh];
-                        const int os = v.hscore[h];
-                        if (os < gs) {
-                            // rb_reput: unlink, re-key, append as newest
-                            if (v.hprev[h] >= 0) v.hnext[v.hprev[h]] = v.hnext[h]; else v.bhead[os] = v.hnext[h];
-                            if (v.hnext[h] >= 0) v.hprev[v.hnext[h]] = v.hprev[h]; else v.btail[os] = v.hprev[h];
-                            if (v.bhead[os] < 0) {
-                                v.bbits[os >> 6] &= ~(1ull << (os & 63));
-                                if (hmin == os) {
-                                    const int nm = bits_min_ge(v.bbits, os + 1, NW);
-                                    hmin = nm < 0 ? kSMax : nm;
-                                }
-                            }
-                            v.hscore[h] = gs; v.hlen[h] = gl;
-                            v.hnext[h] = -1;
-                            v.hprev[h] = v.btail[gs];
-                            if (v.btail[gs] >= 0) v.hnext[v.btail[gs]] = h; else v.bhead[gs] = h;
-                            v.btail[gs] = h;
-                            v.bbits[gs >> 6] |= 1ull << (gs & 63);
-                            if (gs < hmin) hmin = gs;
-                        }
-                    }
-                }
-                if (trace && npops < a.trace_cap) {
-                    PopRec r; r.row = row; r.off = off; r.score = gs; r.len = gl; r.counted = counted;
-                    trace[npops] = r;
-                }
-                ++npops;
-                if (counted && ++counter == a.seeds) stop = 1;
+            const unsigned counted = add_pops(h, lane, &n, (int64_t)a.seeds - counter, p, gs, gl, off);
+            if (trace && lane < n && npops + lane < a.trace_cap) {
+                PopRec r;
+                r.row = row; r.off = off; r.score = gs; r.len = gl; r.counted = counted >> lane & 1;
+                trace[npops + lane] = r;
             }
+            npops += n;
+            counter += __popc(counted);
+            first += n;
+            pending -= n;
+            if (counter >= a.seeds) break;
+            if (pending > 0) continue;
         }
-        stop = __shfl_sync(0xFFFFFFFFu, stop, 0);
-        if (stop) break;
+        if (refill >= 0) {
+            // past the computed elements: 32 more rows, a lane each, in the
+            // place of older ones (whose pops are all in the hitlist by now)
+            const Cursor x = cur[refill];
+            int32_t pr;
+            const uint32_t k = state[refill].k;
+            const uint32_t w = chain_elem(ix, x.row, x.dir, (int)k + 1 + lane, Q, qlen, x.off, a.sub, &pr);
+            cache[chain_at(refill, k + lane)] = w;
+            cprot[chain_at(refill, k + lane)] = pr;
+            ++refills;
+            filled = refill;
+            refill = -1;
+            __syncwarp();
+        } else if (!open) {
+            break;
+        }
     }
-
+    write_hits(h, lane, a.hits + (int64_t)q * a.max_cap);
     if (lane == 0) {
-        // ---- hitlist in traversal order: score descending, newest first
-        Hit *out = a.hits + (int64_t)q * a.max_cap;
-        int n = 0;
-        for (int sc = bits_max_le(v.bbits, kSMax - 1); sc >= 0;
-             sc = sc > 0 ? bits_max_le(v.bbits, sc - 1) : -1) {
-            for (int h = v.btail[sc]; h >= 0; h = v.hprev[h]) {
-                Hit o;
-                o.protein = v.hprot[h]; o.gapless_score = v.hscore[h]; o.gapless_length = v.hlen[h];
-                o.suffix_offset = v.hoff[h];
-                out[n++] = o;
-            }
-        }
         QueryOut qo;
-        qo.nhits = n; qo.npops = npops; qo.ncounted = counter; qo.status = status | a.qstatus[q];
-        qo.refills = refills;
+        qo.nhits = h.size; qo.npops = npops; qo.ncounted = counter; qo.refills = refills;
+        // a stop at -S comes before a later pop's end of the array
+        qo.status = a.qstatus[q] | (counter < a.seeds && past_end ? TPZ_Q_SA_END : 0);
         a.qout[q] = qo;
     }
 }
+
+size_t walk_smem(int cursors) {
+    return kWalkFixed + (sizeof(int16_t) * kBuf + sizeof(CurState)) * (size_t)cursors;
+}
+size_t walk_state_bytes(int cursors) { return walk_smem(cursors) - kWalkFixed; }
+
+size_t walk_scratch_bytes(int cap) {
+    const size_t n = (size_t)cap;
+    const size_t b = 16 * n + 4 * n + 4 * (2 * n + 64) + 4 * (size_t)kSMax + 2 * (size_t)kSMax;
+    return (b + 15) & ~(size_t)15;
+}
+
+template __global__ void walk_kernel<false>(DevIndex ix, const __grid_constant__ WalkArgs a);
+template __global__ void walk_kernel<true>(DevIndex ix, const __grid_constant__ WalkArgs a);
 
 }  // namespace search
 }  // namespace tpz
