@@ -1,0 +1,66 @@
+"""The warp form of the --blasttab statistics where it has edges: bands wider
+than the 32 rows of a step block and wider than the subject, segments around
+32 rows, bands that double, and inputs no forward pass gives (another score,
+gap costs the batch alignment does not take), against the host restatement."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from test_stats_gpu import FIELDS, St, _device_stats, _same_double
+from topaz_b200 import native, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(torch, ps, mat, go, ge, fwd):
+    got = _device_stats(torch, ps, mat, go, ge, fwd)
+    L = native.lib()
+    L.tpzh_align_stats.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
+                                   ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int32,
+                                   ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(St)]
+    m = np.ascontiguousarray(mat, np.int8)
+    for i in range(ps.n):
+        q = np.ascontiguousarray(ps.q[ps.qoff[i]:ps.qoff[i] + ps.qlen[i]])
+        s = np.ascontiguousarray(ps.s[ps.soff[i]:ps.soff[i] + ps.slen[i]])
+        h = St()
+        L.tpzh_align_stats(q.ctypes.data, len(q), s.ctypes.data, len(s), m.ctypes.data, go, ge,
+                           int(fwd[2][i]), int(fwd[1][i]), int(fwd[0][i]), ctypes.byref(h))
+        assert tuple(int(got[k][i]) for k in FIELDS) == tuple(getattr(h, k) for k in FIELDS), i
+        assert _same_double(got["identity"][i], h.identity), i
+
+
+def _gapped_pairs():
+    """Subjects that are the query with a piece cut out or put in, at sizes
+    around the row blocks."""
+    rng = np.random.default_rng(5)
+    qs, ss = [], []
+    for n in (31, 32, 33, 63, 64, 65, 97, 300, 900):
+        for gap in (0, 1, 2, 5, 31, 33, 120):
+            q = rng.integers(0, 20, n).astype(np.int8)
+            at = n // 2
+            ins = rng.integers(0, 20, gap).astype(np.int8)
+            s = np.concatenate([q[:at], ins, q[at:]])
+            noise = rng.random(len(s)) < 0.15
+            s[noise] = rng.integers(0, 20, int(noise.sum()))
+            qs += [q, s]
+            ss += [s, q]
+    ql = np.array([len(x) for x in qs], np.int32)
+    sl = np.array([len(x) for x in ss], np.int32)
+    return synth.PairSet(np.concatenate(qs), (np.cumsum(ql) - ql).astype(np.int64), ql, np.concatenate(ss),
+                         (np.cumsum(sl) - sl).astype(np.int64), sl, 0)
+
+
+@pytest.mark.parametrize("go,ge", [(11, 1), (2, 1), (1, 0), (30, 0)])
+def test_bands_around_the_row_blocks(cuda, go, ge):
+    ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62")
+    sc, re_, rd, st = native.sw_batch_host(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat, go, ge)
+    assert (st == native.TPZ_SW_OK).all()
+    _check(cuda, ps, mat, go, ge, (sc, re_, rd))
+
+
+@pytest.mark.parametrize("shift,go,ge", [(-1, 11, 1), (0, 2, 2), (0, 1, 3)])
+def test_inputs_no_forward_pass_gives(cuda, shift, go, ge):
+    ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62")
+    sc, re_, rd, _ = native.sw_batch_host(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat, 11, 1)
+    _check(cuda, ps, mat, go, ge, (np.maximum(sc + shift, 1), re_, rd))

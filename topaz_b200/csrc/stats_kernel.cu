@@ -4,23 +4,26 @@
 // hit by stats_using_ssw_profile, src/ssw_wrapper.c:132-155, from
 // query_perform_statistics, src/query.c:250-299).
 //
-// One thread per hit, two launches:
+// Three stages:
 //
-// 1. Start coordinates.  A local-alignment pass from the end cell backwards:
+// 1. Start coordinates: a local alignment from the end cell backwards, the
 //    subject columns ref_end .. 0 against the query prefix read[0 .. read_end]
-//    reversed, with the recurrence of SSW's striped passes (the in-lane F
-//    term reset every `seg` rows, seg = ceil(rows / 16) when bias + score <
-//    255 and ceil(rows / 8) otherwise, and padding rows past the query that
-//    score 0 but still count toward a column's maximum), stopping at the
-//    first column whose maximum equals the forward score.  The column and
-//    row of the best cell give the subject and query starts.
-//    Then the band search: a banded global-style pass over the aligned
-//    segments (H never below 0 through its gap terms, cells outside the
-//    band read as 0), the band starting at |len difference| + 1 and doubling
-//    until the best cell reaches the score; it yields the final band and the
-//    size of its direction table, or the size guard of the reference (a
-//    table of 2^30 bytes or more gives -1 columns).
-// 2. Path.  The band passes again, now writing per cell the step each of the
+//    reversed, up to the first column whose maximum equals the forward score.
+//    That score is the maximum of the reversed problem, so its end cell in
+//    the batch Smith-Waterman (first column, smallest row of the maximum; no
+//    lane length matters, see sw_core.cuh) is the start: the reversed
+//    prefixes are copied out and aligned as a batch.  (One thread per hit
+//    ran it before: 88 ms of a 500-query --blasttab batch with 211 hits, the
+//    time of its longest hit.)  A hit whose reversed maximum is not its
+//    score -- inputs that no forward pass gave -- takes the pass as SSW
+//    writes it, one thread (reverse_pass).
+// 2. Band search: a banded global-style pass over the aligned segments (H
+//    never below 0 through its gap terms, cells outside the band read as 0),
+//    the band starting at |len difference| + 1 and doubling until the best
+//    cell reaches the score; it yields the final band and the size of its
+//    direction table, or the size guard of the reference (a table of 2^30
+//    bytes or more gives -1 columns).
+// 3. Path: the band passes again, now writing per cell the step each of the
 //    three states (vertical gap, horizontal gap, match) came from into a
 //    table laid out row by row (2 * band + 1 cells of 3 bytes per row, the
 //    passes of every band width writing the same table, as the reference's
@@ -28,6 +31,10 @@
 //    columns, mismatches (residues compared after each diagonal step) and
 //    gap opens, until the walk reaches the first query row or leaves its
 //    row's slot.
+//
+// A warp runs a hit's band passes: 32 rows at a time, a lane each, a row one
+// column behind the row above it, so H and E of the row above come by
+// shuffle.  Bound: latency of that chain, (2 * band + 63) steps per 32 rows.
 #include <algorithm>
 #include <vector>
 
@@ -56,6 +63,9 @@ struct PairArgs {
     // per pair work state between the launches
     int32_t *band;                       // final band width, 0 = no banded pass
     int64_t *dir_bytes;                  // direction table size of the final band
+    // the reversed prefixes aligned: null, or per pair score, end column, end
+    // row and status
+    const int32_t *rscore, *rcol, *rrow, *rstatus;
     // scratch
     int32_t *work;                       // int32 arrays, per pair at work_off
     const int64_t *work_off;
@@ -82,140 +92,197 @@ __host__ __device__ inline int64_t band_words_at(int32_t read_end) {
     return 3 * (((n + 15) / 16) * 16 + 1);
 }
 
-// One banded pass over query rows [0, rl) and subject columns [0, fl):
-// H and E of the previous row live in Hc/Ec by column (cells outside the
-// previous row's band read as 0); dir (may be null) receives the steps.
-// Returns the pass's best cell.
-__device__ int band_pass(const PairArgs &a, const int8_t *rd, const int8_t *rf, int rl, int fl,
-                         int w, int32_t *Hc, int32_t *Ec, int8_t *dir) {
-    const int go = a.gap_open, ge = a.gap_extend;
-    const int64_t wd3 = (int64_t)(2 * w + 1) * 3;
-    int best = 0;
-    for (int j = 0; j < fl + 2; ++j) { Hc[j] = 0; Ec[j] = 0; }
-    int prev_end = -1;
-    for (int i = 0; i < rl; ++i) {
-        const int beg = max(0, i - w), end = min(fl - 1, i + w);
-        // the column past the previous row's band reads as 0
-        if (prev_end + 1 < fl) { Hc[prev_end + 1] = 0; Ec[prev_end + 1] = 0; }
-        const int qi = res_at(a, rd, i);
-        int diag = beg > 0 ? Hc[beg - 1] : 0;      // H(i-1, beg-1), 0 outside
-        int hl = 0, f = 0;                          // H(i, j-1), F(i, j-1)
-        int8_t *dl = dir ? dir + (int64_t)i * wd3 : nullptr;
-        for (int j = beg; j <= end; ++j) {
-            const int hu = Hc[j], eu = Ec[j];           // previous row, column j
-            const int eo = hu - go, ee = eu - ge;
-            const int e = eo > ee ? eo : ee;
-            const int fo = hl - go, fe = f - ge;
-            f = fo > fe ? fo : fe;
-            const int e1 = e > 0 ? e : 0, f1 = f > 0 ? f : 0;
-            const int gap = e1 > f1 ? e1 : f1;
-            const int dg = diag + a.mat[res_at(a, rf, j) * 25 + qi];
-            const int h = gap > dg ? gap : dg;
-            if (dl) {
-                const int8_t de = eo > ee ? 3 : 2, df = fo > fe ? 5 : 4;
-                int8_t *c = dl + (int64_t)(j - beg) * 3;
-                c[0] = de;
-                c[1] = df;
-                c[2] = gap <= dg ? 1 : (e1 > f1 ? de : df);
-            }
-            best = h > best ? h : best;
-            diag = hu;
-            Hc[j] = h;
-            Ec[j] = e;
-            hl = h;
+// The reverse pass as SSW runs it (one thread): start row and column of the
+// best cell, -1 where there is none.
+__device__ void reverse_pass(const PairArgs &a, int64_t p, int *row, int *col) {
+    const int re = a.read_end[p], fe = a.ref_end[p], score = a.score[p];
+    const int8_t *q = a.q + a.qoff[p], *s = a.s + a.soff[p];
+    // rows = reversed query prefix, with the padding rows of the striped
+    // layout (they score 0 but count toward a column's maximum)
+    const int n = re + 1;
+    const bool word = !(a.bias + score < 255);
+    const int lanes = word ? 8 : 16;
+    const int seg = (n + lanes - 1) / lanes;
+    const int rows = seg * lanes;
+    const int terminate = word ? (score & 0xFFFF) : (score & 0xFF);
+    int32_t *w = a.work + a.work_off[p];
+    int32_t *E = w, *Hp = w + (rows + 1), *Hn = w + 2 * (rows + 1);
+    for (int r = 0; r <= rows; ++r) { E[r] = 0; Hp[r] = 0; Hn[r] = 0; }
+    const int go = a.gap_open, gx = a.gap_extend;
+    int best = 0, bc = word ? 0 : -1, br = 0;
+    for (int c = fe; c >= 0; --c) {
+        const int8_t *mrow = a.mat + 25 * res_at(a, s, c);
+        int F = 0, Fm = 0, colmax = 0, cbest = 0, crow = 0;
+        for (int r = 0; r < rows; ++r) {
+            if (r % seg == 0) Fm = 0;
+            const int D = r ? Hp[r - 1] : 0;
+            const int sc = r < n ? mrow[res_at(a, q, re - r)] : 0;
+            const int hp = max(max(0, D + sc), max(E[r], Fm));
+            const int h = max(hp, F);
+            E[r] = max(0, max(E[r] - gx, hp - go));
+            Fm = max(0, max(Fm - gx, hp - go));
+            F = max(0, max(F - gx, h - go));
+            Hn[r] = h;
+            colmax = max(colmax, h);
+            if (r < n && h > cbest) { cbest = h; crow = r; }
         }
-        prev_end = end;
+        int32_t *t = Hp; Hp = Hn; Hn = t;
+        if (cbest > best) {
+            best = cbest;
+            if ((!word && best + a.bias >= 255) || (word && best >= 32767)) break;
+            bc = c;
+            br = crow;
+        }
+        if (colmax == terminate) break;
     }
-    return best;
+    *row = best > 0 ? br : 0;
+    *col = bc;
 }
 
+// One thread per hit: where its alignment starts.
 __global__ void stats_start_kernel(const __grid_constant__ PairArgs a) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n;
          p += (int64_t)gridDim.x * blockDim.x) {
         a.band[p] = 0;
         a.dir_bytes[p] = 0;
         if (a.valid && !a.valid[p]) continue;
-        const int re = a.read_end[p], fe = a.ref_end[p], score = a.score[p];
+        const int re = a.read_end[p], fe = a.ref_end[p];
         if (re < 0 || fe < 0) {
-            a.qstart[p] = a.sstart[p] = a.length[p] = a.gapopen[p] = a.mismatch[p] = -1;
-            a.identity[p] = -1.0;
-            continue;
-        }
-        const int8_t *q = a.q + a.qoff[p], *s = a.s + a.soff[p];
-        // ---- reverse pass: rows = reversed query prefix, columns fe .. 0
-        const int n = re + 1;
-        const bool word = !(a.bias + score < 255);
-        const int lanes = word ? 8 : 16;
-        const int seg = (n + lanes - 1) / lanes;
-        const int rows = seg * lanes;
-        const int terminate = word ? (score & 0xFFFF) : (score & 0xFF);
-        int32_t *w = a.work + a.work_off[p];
-        int32_t *E = w, *Hp = w + (rows + 1), *Hn = w + 2 * (rows + 1);
-        for (int r = 0; r <= rows; ++r) { E[r] = 0; Hp[r] = 0; Hn[r] = 0; }
-        const int go = a.gap_open, gx = a.gap_extend;
-        int best = 0, bc = word ? 0 : -1, br = 0;
-        for (int c = fe; c >= 0; --c) {
-            const int8_t *mrow = a.mat + 25 * res_at(a, s, c);
-            int F = 0, Fm = 0, colmax = 0, cbest = 0, crow = 0;
-            for (int r = 0; r < rows; ++r) {
-                if (r % seg == 0) Fm = 0;
-                const int D = r ? Hp[r - 1] : 0;
-                const int sc = r < n ? mrow[res_at(a, q, re - r)] : 0;
-                const int hp = max(max(0, D + sc), max(E[r], Fm));
-                const int h = max(hp, F);
-                E[r] = max(0, max(E[r] - gx, hp - go));
-                Fm = max(0, max(Fm - gx, hp - go));
-                F = max(0, max(F - gx, h - go));
-                Hn[r] = h;
-                colmax = max(colmax, h);
-                if (r < n && h > cbest) { cbest = h; crow = r; }
+            a.qstart[p] = a.sstart[p] = -1;
+        } else {
+            int row, col;
+            if (a.rscore && a.rstatus[p] == TPZ_SW_OK && a.rscore[p] == a.score[p] && a.score[p] > 0) {
+                row = a.rrow[p];
+                col = fe - a.rcol[p];
+            } else {
+                reverse_pass(a, p, &row, &col);
             }
-            int32_t *t = Hp; Hp = Hn; Hn = t;
-            if (cbest > best) {
-                best = cbest;
-                if ((!word && best + a.bias >= 255) || (word && best >= 32767)) break;
-                bc = c;
-                br = crow;
-            }
-            if (colmax == terminate) break;
+            a.qstart[p] = re - row;
+            a.sstart[p] = col;
+            if (col >= 0) { a.band[p] = 1; continue; }      // to the band search
         }
-        const int rread = best > 0 ? br : 0;
-        const int qs = re - rread, ss = bc;
-        a.qstart[p] = qs;
-        a.sstart[p] = ss;
-        if (ss < 0) {
-            a.length[p] = a.gapopen[p] = a.mismatch[p] = -1;
-            a.identity[p] = -1.0;
-            continue;
-        }
-        // ---- band search
-        const int fl = fe - ss + 1, rl = re - qs + 1;
-        int band = abs(fl - rl) + 1;
-        int32_t *Hc = w + band_words_at(re), *Ec = Hc + (fe + 3);
-        int mx = 0;
-        bool guard = false;
-        for (;;) {
-            // the reference sizes its table as the power of two above this
-            // and gives up (-1 columns) at 2^31
-            const int64_t need = (int64_t)(2 * band + 1) * rl * 3;
-            if (need >= ((int64_t)1 << 30)) { guard = true; break; }
-            mx = max(mx, band_pass(a, q + qs, s + ss, rl, fl, band, Hc, Ec, nullptr));
-            if (mx >= score) break;
-            band *= 2;
-        }
-        if (guard) {
-            a.length[p] = a.gapopen[p] = a.mismatch[p] = -1;
-            a.identity[p] = -1.0;
-            continue;
-        }
-        a.band[p] = band;
-        a.dir_bytes[p] = (int64_t)(2 * band + 1) * rl * 3;
+        a.length[p] = a.gapopen[p] = a.mismatch[p] = -1;
+        a.identity[p] = -1.0;
     }
 }
 
-__global__ void stats_path_kernel(const __grid_constant__ PairArgs a) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n;
-         p += (int64_t)gridDim.x * blockDim.x) {
+// One banded pass over query rows [0, rl) and subject columns [0, fl), by a
+// warp; cells outside the previous row's band read as 0.  H and E of the last
+// row of 32 wait in Hc / Ec by column for the next 32; dir (may be null)
+// receives the steps.  Returns the pass's best cell in every lane.
+__device__ int band_pass(const PairArgs &a, const int8_t *smat, const int8_t *rd, const int8_t *rf,
+                         int rl, int fl, int w, int32_t *Hc, int32_t *Ec, int8_t *dir) {
+    const int lane = threadIdx.x & 31;
+    const int go = a.gap_open, ge = a.gap_extend;
+    const int64_t wd3 = (int64_t)(2 * (int64_t)w + 1) * 3;
+    int best = 0;
+    for (int i0 = 0; i0 < rl; i0 += 32) {
+        const int i = i0 + lane, last = min(i0 + 31, rl - 1);
+        const int beg = max(0, i - w), end = min(fl - 1, i + w);
+        const int c0 = max(0, i0 - w);
+        const int prev_end = i > 0 ? min(fl - 1, i - 1 + w) : -1;   // band of the row above
+        const int qi = i < rl ? res_at(a, rd, i) : 0;
+        int8_t *dl = dir && i < rl ? dir + (int64_t)i * wd3 : nullptr;
+        int h = 0, e = 0, f = 0;                    // this row, column j - 1
+        // H(i-1, j-1): what came from above in the step before
+        int diag = lane == 0 && i0 > 0 && c0 > 0 ? __ldcg(Hc + c0 - 1) : 0;
+        int letter = 0, hb = 0, eb = 0, lb = 0;
+        const int nsteps = min(fl - 1, last + w) - c0 + (last - i0) + 1;
+        for (int t = 0; t < nsteps; ++t) {
+            if ((t & 31) == 0) {
+                // the next 32 columns of the row above the block and of the subject
+                const int j = c0 + t + lane;
+                __syncwarp();
+                hb = eb = lb = 0;
+                if (j < fl) {
+                    lb = res_at(a, rf, j);
+                    if (i0 > 0 && j <= min(fl - 1, i0 - 1 + w)) { hb = __ldcg(Hc + j); eb = __ldcg(Ec + j); }
+                }
+            }
+            const int h0 = __shfl_sync(0xFFFFFFFFu, hb, t & 31), e0 = __shfl_sync(0xFFFFFFFFu, eb, t & 31);
+            const int l0 = __shfl_sync(0xFFFFFFFFu, lb, t & 31);
+            int hu = __shfl_up_sync(0xFFFFFFFFu, h, 1), eu = __shfl_up_sync(0xFFFFFFFFu, e, 1);
+            letter = __shfl_up_sync(0xFFFFFFFFu, letter, 1);
+            const int j = c0 + t - lane;
+            if (lane == 0) { hu = h0; eu = e0; letter = l0; }
+            if (j > prev_end || j < 0) { hu = 0; eu = 0; }
+            if (i < rl && j >= beg && j <= end) {
+                if (j == beg) { h = 0; f = 0; }
+                const int eo = hu - go, ee = eu - ge;
+                e = eo > ee ? eo : ee;
+                const int fo = h - go, fe = f - ge;
+                f = fo > fe ? fo : fe;
+                const int e1 = e > 0 ? e : 0, f1 = f > 0 ? f : 0;
+                const int gap = e1 > f1 ? e1 : f1;
+                const int dg = diag + smat[letter * 25 + qi];
+                h = gap > dg ? gap : dg;
+                if (dl) {
+                    const int8_t de = eo > ee ? 3 : 2, df = fo > fe ? 5 : 4;
+                    int8_t *c = dl + (int64_t)(j - beg) * 3;
+                    c[0] = de;
+                    c[1] = df;
+                    c[2] = gap <= dg ? 1 : (e1 > f1 ? de : df);
+                }
+                best = h > best ? h : best;
+                if (lane == 31) { Hc[j] = h; Ec[j] = e; }
+            }
+            diag = hu;
+        }
+        __syncwarp();
+    }
+    return (int)__reduce_max_sync(0xFFFFFFFFu, best);
+}
+
+constexpr int kBandWarps = 4;
+
+__device__ __forceinline__ void load_scores(const PairArgs &a, int8_t *smat) {
+    for (int i = threadIdx.x; i < 625; i += blockDim.x) smat[i] = a.mat[i];
+    __syncthreads();
+}
+
+// A warp per hit: the final band width and its direction table's size.
+__global__ void __launch_bounds__(32 * kBandWarps) stats_band_kernel(const __grid_constant__ PairArgs a) {
+    __shared__ int8_t smat[640];
+    load_scores(a, smat);
+    for (int64_t p = blockIdx.x * (int64_t)kBandWarps + (threadIdx.x >> 5); p < a.n;
+         p += (int64_t)gridDim.x * kBandWarps) {
+        if (a.band[p] <= 0) continue;
+        const int re = a.read_end[p], fe = a.ref_end[p], score = a.score[p];
+        const int qs = a.qstart[p], ss = a.sstart[p];
+        const int fl = fe - ss + 1, rl = re - qs + 1;
+        const int8_t *rd = a.q + a.qoff[p] + qs, *rf = a.s + a.soff[p] + ss;
+        int32_t *Hc = a.work + a.work_off[p] + band_words_at(re), *Ec = Hc + (fe + 3);
+        int band = abs(fl - rl) + 1, mx = 0;
+        int64_t need;
+        for (;;) {
+            // the reference sizes its table as the power of two above this
+            // and gives up (-1 columns) at 2^31
+            need = (int64_t)(2 * band + 1) * rl * 3;
+            if (need >= ((int64_t)1 << 30)) break;
+            mx = max(mx, band_pass(a, smat, rd, rf, rl, fl, band, Hc, Ec, nullptr));
+            if (mx >= score) break;
+            band *= 2;
+        }
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) {
+            if (need >= ((int64_t)1 << 30)) {
+                a.band[p] = 0;
+                a.length[p] = a.gapopen[p] = a.mismatch[p] = -1;
+                a.identity[p] = -1.0;
+            } else {
+                a.band[p] = band;
+                a.dir_bytes[p] = need;
+            }
+        }
+    }
+}
+
+// A warp per hit: the direction table, then lane 0 walks the path back.
+__global__ void __launch_bounds__(32 * kBandWarps) stats_path_kernel(const __grid_constant__ PairArgs a) {
+    __shared__ int8_t smat[640];
+    load_scores(a, smat);
+    for (int64_t p = blockIdx.x * (int64_t)kBandWarps + (threadIdx.x >> 5); p < a.n;
+         p += (int64_t)gridDim.x * kBandWarps) {
         const int wfinal = a.band[p];
         if (wfinal <= 0) continue;
         const int re = a.read_end[p], fe = a.ref_end[p];
@@ -226,9 +293,11 @@ __global__ void stats_path_kernel(const __grid_constant__ PairArgs a) {
         int8_t *dir = a.dir + a.dir_off[p];
         // every band width up to the final one writes the same table
         for (int band = abs(fl - rl) + 1;; band *= 2) {
-            band_pass(a, rd, rf, rl, fl, band, Hc, Ec, dir);
+            band_pass(a, smat, rd, rf, rl, fl, band, Hc, Ec, dir);
             if (band >= wfinal) break;
         }
+        __syncwarp();
+        if ((threadIdx.x & 31) != 0) continue;
         const int64_t wd3 = (int64_t)(2 * wfinal + 1) * 3;
         int i = rl - 1, j = fl - 1, st = 2, len = 0, mism = 0, gaps = 0, same = 0;
         char prev = 'M';
@@ -238,7 +307,7 @@ __global__ void stats_path_kernel(const __grid_constant__ PairArgs a) {
             const int64_t at = (int64_t)(j - x) * 3 + st;
             if (at < 0 || at >= wd3) break;              // left the row's slot
             char op;
-            switch (dir[(int64_t)i * wd3 + at]) {
+            switch (__ldcg(dir + (int64_t)i * wd3 + at)) {
             case 1: --i; --j; st = 2; op = 'M'; break;
             case 2: --i; st = 0; op = 'I'; break;
             case 3: --i; st = 2; op = 'I'; break;
@@ -258,6 +327,37 @@ __global__ void stats_path_kernel(const __grid_constant__ PairArgs a) {
         a.gapopen[p] = gaps;
         a.mismatch[p] = mism;
         a.identity[p] = broken ? 0.0 : same / (double)len;
+    }
+}
+
+// bytes of a pair's reversed prefixes
+__device__ __forceinline__ bool has_prefixes(const PairArgs &a, int64_t p) {
+    return (!a.valid || a.valid[p]) && a.read_end[p] >= 0 && a.ref_end[p] >= 0;
+}
+
+__global__ void prefix_bytes_kernel(const __grid_constant__ PairArgs a, int64_t *bytes) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n;
+         p += (int64_t)gridDim.x * blockDim.x)
+        bytes[p] = has_prefixes(a, p) ? (int64_t)a.read_end[p] + a.ref_end[p] + 2 : 0;
+}
+
+// The reversed prefixes of every pair as matrix indices, the query's at
+// off[p] and the subject's behind it, with the pair list of their alignment
+// (length 0 where there is nothing to align).  A warp per pair.
+__global__ void __launch_bounds__(128) reverse_kernel(const __grid_constant__ PairArgs a, const int64_t *off,
+                                                      int8_t *rev, int64_t *soff, int32_t *qlen, int32_t *slen) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t p = blockIdx.x * (int64_t)4 + (threadIdx.x >> 5); p < a.n; p += (int64_t)gridDim.x * 4) {
+        const int nq = has_prefixes(a, p) ? a.read_end[p] + 1 : 0, ns = nq ? a.ref_end[p] + 1 : 0;
+        const int8_t *q = a.q + a.qoff[p], *s = a.s + a.soff[p];
+        int8_t *d = rev + off[p];
+        for (int i = lane; i < nq; i += 32) d[i] = (int8_t)res_at(a, q, nq - 1 - i);
+        for (int i = lane; i < ns; i += 32) d[nq + i] = (int8_t)res_at(a, s, ns - 1 - i);
+        if (lane == 0) {
+            soff[p] = off[p] + nq;
+            qlen[p] = nq;
+            slen[p] = ns;
+        }
     }
 }
 
@@ -312,8 +412,36 @@ int stats_batch(PairArgs a, cudaStream_t st) {
     int32_t *work;
     if ((rc = alloc((void **)&work, 4 * (size_t)total_words))) { cleanup(); return rc; }
     a.band = band; a.dir_bytes = dbytes; a.work = work; a.work_off = woff;
-    // few hits per batch: small blocks spread them over the SMs
+    // the alignment of the reversed prefixes, for gap costs its batch call
+    // takes; the pairs it does not answer go through reverse_pass
+    const int warps = (int)std::max<int64_t>(1, std::min<int64_t>((a.n + kBandWarps - 1) / kBandWarps, 4096));
+    if (a.gap_open > a.gap_extend && a.gap_extend >= 0 && a.gap_open <= 255 && a.n <= INT32_MAX / 3) {
+        int64_t *bytes = words, *boff, *rsoff, total_rev = 0;    // words: used up by the scan above
+        int32_t *r;
+        int8_t *rev;
+        if ((rc = alloc((void **)&boff, 8 * a.n)) || (rc = alloc((void **)&rsoff, 8 * a.n)) ||
+            (rc = alloc((void **)&r, 6 * 4 * (size_t)a.n))) {
+            cleanup();
+            return rc;
+        }
+        prefix_bytes_kernel<<<grid, 128, 0, st>>>(a, bytes);
+        if ((rc = exclusive_offsets(bytes, a.n, boff, st, mem, &total_rev)) ||
+            (rc = alloc((void **)&rev, (size_t)total_rev))) {
+            cleanup();
+            return rc;
+        }
+        int32_t *rql = r, *rsl = r + a.n, *rs = r + 2 * a.n, *rc_ = r + 3 * a.n, *rr = r + 4 * a.n,
+                *rst = r + 5 * a.n;
+        reverse_kernel<<<warps, 128, 0, st>>>(a, boff, rev, rsoff, rql, rsl);
+        if ((rc = sw::batch_device_x(a.n, rev, boff, rql, rev, rsoff, rsl, a.mat, a.gap_open, a.gap_extend, rs,
+                                     rc_, rr, rst, st, nullptr, nullptr, 0))) {
+            cleanup();
+            return rc;
+        }
+        a.rscore = rs; a.rcol = rc_; a.rrow = rr; a.rstatus = rst;
+    }
     stats_start_kernel<<<grid, 128, 0, st>>>(a);
+    stats_band_kernel<<<warps, 32 * kBandWarps, 0, st>>>(a);
     TPZ_CUDA(cudaGetLastError());
     int64_t total_dir = 0;
     if ((rc = exclusive_offsets(dbytes, a.n, doff, st, mem, &total_dir))) { cleanup(); return rc; }
@@ -322,7 +450,7 @@ int stats_batch(PairArgs a, cudaStream_t st) {
     // never-written table cells read as "no step" (the walk stops there)
     TPZ_CUDA(cudaMemsetAsync(dir, 0, (size_t)total_dir, st));
     a.dir = dir; a.dir_off = doff;
-    stats_path_kernel<<<grid, 128, 0, st>>>(a);
+    stats_path_kernel<<<warps, 32 * kBandWarps, 0, st>>>(a);
     TPZ_CUDA(cudaGetLastError());
     cleanup();
     return TPZ_OK;
