@@ -5,7 +5,7 @@
 // (seq_2internal, src/seq.c:106-117) -- what run_query does to each query
 // before seeding (src/engine.c:250-277).
 //
-// One thread per query.  SEG (Wootton & Federhen 1993) decides with doubles;
+// One warp per query.  SEG (Wootton & Federhen 1993) decides with doubles;
 // for the masks to equal the host's bit for bit, every transcendental value
 // comes from tables the host computes with the C library (the full-window
 // entropy terms, log(x / t) of the partial-window terms, ln n! rounded to 6
@@ -13,13 +13,14 @@
 // in the host's order, rounded to nearest without fused multiply-adds (this
 // file is compiled with -fmad=false).
 //
-// The per-query state: a window's residue counts and the descending
-// multiset of its non-zero counts (the entropy and the probability depend
-// only on that multiset), the entropy of every 12-residue window, and a
-// stack of nested searches (a trigger window lost to a segment's left trim
-// is searched again in the part that was cut, which is at most 100 residues
-// long, so nesting stays shallow).  Segments merge as they are found: an
-// overlapping successor gives its end to the segment before it.
+// What a query's decisions depend on in sequence -- triggers, extension, the
+// nested search of a part cut off by a left trim (at most 100 residues long,
+// so nesting stays shallow), merging -- runs the same in every lane; the work
+// in between is split over them: the entropies of 32 windows at a time, and
+// the trim's sub-windows by length, a length per lane.  An entropy and a
+// probability depend only on the descending multiset of a window's non-zero
+// residue counts.  (With one thread per query a batch took as long as its
+// query with the most low-complexity residues: 5.9 ms for 500 queries.)
 #include <algorithm>
 #include <mutex>
 
@@ -109,20 +110,39 @@ __device__ bool win_shift(const char *s, const Tables &t, int end, Win &w) {
     return true;
 }
 
-__device__ double sv_entropy(const Tables &t, const int *sv) {
-    int total = 0, n = 0;
-    while (sv[n] != 0) total += sv[n++];
-    double ent = 0.0;
-    if (total == kWin) {
-        for (int i = 0; i < n; ++i) ent += t.ent_full[sv[i]];
-        return ent;
+// entropy of the 12 residues from s: the counts of the 20 residue types in 4
+// bits each, then how many types have each count, summed from the largest
+__device__ double window_entropy(const Tables &t, const char *s) {
+    uint64_t lo = 0, hi = 0;                  // types 0..9, 10..19
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < kWin; ++i) {
+        const int k = t.res_index[(uint8_t)s[i]];
+        if (k < 0) continue;
+        ++total;
+        if (k < 10) lo += 1ull << (4 * k);
+        else hi += 1ull << (4 * (k - 10));
     }
     if (total == 0) return 0.;
-    const double rt = 1. / (double)total;
-    for (int i = 0; i < n; ++i) {
-        const double x = sv[i];
-        ent += x * t.logxr[total * (kWin + 1) + sv[i]];
+    uint64_t types = 0;                       // types with count c in bits 4c .. 4c+3
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+        types += 1ull << (4 * (int)(lo >> (4 * k) & 15));
+        types += 1ull << (4 * (int)(hi >> (4 * k) & 15));
+        types &= ~15ull;                      // count 0
     }
+    double ent = 0.0;
+    if (total == kWin) {
+        for (int c = kWin; c >= 1; --c)
+            for (int m = (int)(types >> (4 * c) & 15); m > 0; --m) ent += t.ent_full[c];
+        return ent;
+    }
+    const double rt = 1. / (double)total;
+    for (int c = kWin; c >= 1; --c)
+        for (int m = (int)(types >> (4 * c) & 15); m > 0; --m) {
+            const double x = c;
+            ent += x * t.logxr[total * (kWin + 1) + c];
+        }
     return -ent * rt / kLn2;
 }
 
@@ -157,25 +177,35 @@ __device__ double sv_prob(const double *lnfac, const int *sv, int total) {
 }
 
 // the most improbable sub-window of s[start, start + len) at least
-// len - 100 long: moves *left / *right to its ends
+// len - 100 long: moves *left / *right to its ends.  Lengths go from the
+// longest down, positions from the left, and the first minimum counts; a lane
+// takes every 32nd length.
 __device__ void seg_trim(const char *s, const Tables &t, const double *lnfac, int start, int len,
                          int *left, int *right) {
-    int lend = 0, rend = len - 1, minlen = 1;
+    const int lane = threadIdx.x & 31;
+    int minlen = 1;
     if (len - kMaxTrim > minlen) minlen = len - kMaxTrim;
-    double minprob = 1.;
-    for (int wl = len; wl > minlen; --wl) {
+    double best = 1.;
+    int blen = len, bpos = 0;
+    for (int wl = len - lane; wl > minlen; wl -= 32) {
         Win w;
         win_open(s, t, start, wl, w);
         int i = 0;
         for (;;) {
             const double p = sv_prob(lnfac, w.sv, wl);
-            if (p < minprob) { minprob = p; lend = i; rend = wl + i - 1; }
+            if (p < best) { best = p; blen = wl; bpos = i; }
             if (!win_shift(s, t, start + len, w)) break;
             ++i;
         }
     }
-    *left += lend;
-    *right -= (len - rend - 1);
+    __syncwarp();
+    for (int o = 16; o > 0; o >>= 1) {
+        const double p = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+        const int l = __shfl_xor_sync(0xFFFFFFFFu, blen, o), x = __shfl_xor_sync(0xFFFFFFFFu, bpos, o);
+        if (p < best || (p == best && (l > blen || (l == blen && x < bpos)))) { best = p; blen = l; bpos = x; }
+    }
+    *left += bpos;
+    *right -= len - (bpos + blen);
 }
 
 struct Frame {
@@ -190,7 +220,7 @@ struct Merger {                   // mergesegs, as segments arrive
     int cb = 0, ce = -1;
     bool open = false;
     __device__ void flush(char *o) {
-        if (open) for (int k = cb; k <= ce; ++k) o[k] = 'X';
+        if (open) for (int k = cb + (int)(threadIdx.x & 31); k <= ce; k += 32) o[k] = 'X';
         open = false;
     }
     __device__ void push(char *o, int b, int e) {
@@ -200,15 +230,24 @@ struct Merger {                   // mergesegs, as segments arrive
     }
 };
 
-__global__ void prepare_kernel(const __grid_constant__ Tables t, Args a) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.n;
-         q += (int64_t)gridDim.x * blockDim.x) {
+constexpr int kPrepWarps = 4;
+
+__global__ void __launch_bounds__(32 * kPrepWarps) prepare_kernel(const __grid_constant__ Tables params,
+                                                                  Args a) {
+    __shared__ Tables t;                          // indexed by each lane's own residues
+    for (int i = threadIdx.x; i < (int)(sizeof t / 4); i += blockDim.x)
+        reinterpret_cast<int *>(&t)[i] = reinterpret_cast<const int *>(&params)[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int64_t q = blockIdx.x * (int64_t)kPrepWarps + (threadIdx.x >> 5); q < a.n;
+         q += (int64_t)gridDim.x * kPrepWarps) {
         const char *s = a.in + a.off[q];
         char *o = a.out + a.off[q];
         const int len = a.len[q];
-        for (int i = 0; i < len; ++i) o[i] = s[i];
+        for (int i = lane; i < len; i += 32) o[i] = s[i];
+        __syncwarp();
         if (a.seg && len >= kLnFac) {
-            atomicExch(a.err, 2);                 // beyond the ln n! table
+            if (lane == 0) atomicExch(a.err, 2);  // beyond the ln n! table
         } else if (a.seg && len >= kWin) {
             double *H = a.scratch + a.off[q] + kScratchExtra * q;
             const int cap = len + kScratchExtra;
@@ -220,15 +259,11 @@ __global__ void prepare_kernel(const __grid_constant__ Tables t, Args a) {
                 if (kWin > flen) { f.i = 1; f.last = 0; return true; }
                 if (hoff + flen > cap) return false;
                 double *h = H + hoff;
-                for (int i = 0; i < flen; ++i) h[i] = -1.;
                 const int first = kDown;
                 f.last = flen - kUp;
-                Win w;
-                win_open(s, t, start, kWin, w);
-                for (int i = first; i <= f.last; ++i) {
-                    h[i] = sv_entropy(t, w.sv);
-                    win_shift(s, t, start + flen, w);
-                }
+                for (int i = lane; i < flen; i += 32)
+                    h[i] = i >= first && i <= f.last ? window_entropy(t, s + start + i - first) : -1.;
+                __syncwarp();
                 f.i = first;
                 f.lowlim = first;
                 return true;
@@ -246,9 +281,16 @@ __global__ void prepare_kernel(const __grid_constant__ Tables t, Args a) {
                     f.i = ni + 1;
                 }
                 bool nested = false;
-                for (; f.i <= f.last; ++f.i) {
-                    const int i = f.i;
-                    if (!(h[i] <= kLoCut && h[i] != -1)) continue;
+                for (;;) {
+                    // the next trigger window, 32 at a time
+                    int i = f.last + 1;
+                    for (int b = f.i; b <= f.last; b += 32) {
+                        const double x = b + lane <= f.last ? h[b + lane] : -1.;
+                        const unsigned m = __ballot_sync(0xFFFFFFFFu, x <= kLoCut && x != -1);
+                        if (m) { i = b + __ffs(m) - 1; break; }
+                    }
+                    f.i = i;
+                    if (i > f.last) break;
                     int j;
                     for (j = i; j >= f.lowlim; --j) if (h[j] == -1 || h[j] > kHiCut) break;
                     const int loi = j + 1;
@@ -272,13 +314,15 @@ __global__ void prepare_kernel(const __grid_constant__ Tables t, Args a) {
                     mg.push(o, leftend + f.start, rightend + f.start);
                     f.i = hii < rightend + kDown ? hii : rightend + kDown;
                     f.lowlim = f.i + 1;
+                    ++f.i;
                 }
                 if (!nested && ok) --top;
             }
-            if (!ok) atomicExch(a.err, 1);
+            if (!ok && lane == 0) atomicExch(a.err, 1);
             mg.flush(o);
+            __syncwarp();
         }
-        for (int i = 0; i < len; ++i) o[i] = t.to_internal[(uint8_t)o[i]];
+        for (int i = lane; i < len; i += 32) o[i] = t.to_internal[(uint8_t)o[i]];
     }
 }
 
@@ -329,9 +373,8 @@ int prepare_device(const char *in, char *out, const int64_t *off, const int32_t 
     Args a;
     a.in = in; a.out = out; a.off = off; a.len = len; a.n = n; a.seg = seg;
     a.scratch = scratch; a.lnfac = lnfac; a.err = err;
-    // few long-running threads: small blocks spread them over the SMs
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, 8192));
-    prepare_kernel<<<grid, 32, 0, st>>>(g_tables, a);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kPrepWarps - 1) / kPrepWarps, 8192));
+    prepare_kernel<<<grid, 32 * kPrepWarps, 0, st>>>(g_tables, a);
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st) || cudaStreamSynchronize(st)) {
         cleanup();
