@@ -43,7 +43,7 @@ def family_db():
 
 @pytest.mark.parametrize("seeds,aligns,num_hits", [(300000, 5000, 100), (300000, 300, 40), (300000, 33, 1),
                                                    (300000, 32, 21), (300000, 31, 2), (300000, 1, 3),
-                                                   (1, 5000, 100), (33, 5, 100), (777, 64, 10)])
+                                                   (300000, 64, 10), (1, 5000, 100), (33, 5, 100), (777, 64, 10)])
 def test_every_pop_and_hit(cuda, family_db, seeds, aligns, num_hits):
     db, qs = family_db
     ix = native.Index(db)

@@ -469,7 +469,7 @@ int32_t rank_min_for(const RankTables &t, const tpz_search_opts *o, int32_t qlen
 // blocks of the smallest on an SM), the longest first in each; past the last
 // class the cursors live in global memory.
 constexpr int kWalkClasses = 5;
-constexpr int kWalkCursors[kWalkClasses] = {512, 1024, 2048, 4096, 9000};
+constexpr int kWalkCursors[kWalkClasses] = {512, 1024, 2048, 3072, 5600};
 
 struct WalkPlan {
     std::vector<int32_t> order;            // queries by class, most cursors first
@@ -942,7 +942,7 @@ int64_t tpz_search_query_device_bytes(int32_t qlen, const tpz_search_opts *o) {
     const int64_t ql = qlen > TPZ_SEARCH_MAX_QLEN ? 0 : qlen;
     const int cap = qlen > 3000 ? (int)(1.5 * o->num_hits) : o->alignments;
     const int64_t npos = std::max<int64_t>(0, ql - o->min_hit_length);
-    int hash_size = 16;
+    int hash_size = 256;
     while (hash_size < 2 * (cap + 1)) hash_size <<= 1;
     const int64_t per_q = (int64_t)walk_scratch_bytes(cap) + 8 * (int64_t)hash_size + 16;
     // (walk_state_bytes: a query with too many cursors for shared memory)
@@ -1029,7 +1029,7 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
         max_cap = std::max(max_cap, cap);
     }
     const int64_t npos = pos_base[nq];
-    int hash_size = 16;
+    int hash_size = 256;
     while (hash_size < 2 * (max_cap + 1)) hash_size <<= 1;
     const size_t per_q = walk_scratch_bytes(max_cap);
     const WalkPlan plan = walk_plan(cur_base, nq);

@@ -468,6 +468,7 @@ struct HitState {
     int32_t *hist;          // hits per score, kept while the list is full
     int cap, logcap;
     int size, nev, smax;    // hits, events, largest score seen
+    int used;               // table entries that are not free
     // full: smallest score, hits that hold it; how far the log has been read
     // for them, and which of the last 32 events are theirs (cslot: a lane's)
     int hmin, cmin, scan;
@@ -476,6 +477,7 @@ struct HitState {
 };
 
 constexpr uint64_t kFree = ~0ull;
+constexpr uint64_t kGone = ~0ull - 1;    // an evicted protein's entry: probes go on past it
 
 __device__ __forceinline__ uint64_t table_entry(int32_t p, int32_t s) {
     return (uint64_t)(uint32_t)p | ((uint64_t)(uint32_t)s << 32);
@@ -531,9 +533,8 @@ __device__ int next_score(const HitState &h, int from, int lane) {
 // the free entry that ends its probe sequence.
 __device__ int find(const HitState &h, int lane, int p, uint32_t *at) {
     for (uint32_t b = hash32((uint32_t)p);; b += 32) {
-        const uint32_t i = (b + lane) & h.hmask;
-        const uint64_t e = __ldcg(h.table + i);
-        const unsigned hit = __ballot_sync(0xFFFFFFFFu, e != kFree && (int32_t)(uint32_t)e == p);
+        const uint64_t e = __ldcg(h.table + ((b + lane) & h.hmask));
+        const unsigned hit = __ballot_sync(0xFFFFFFFFu, (int32_t)(uint32_t)e == p);
         const unsigned end = __ballot_sync(0xFFFFFFFFu, e == kFree);
         if (!hit && !end) continue;
         const int l = __ffs(hit ? hit : end) - 1;
@@ -542,47 +543,62 @@ __device__ int find(const HitState &h, int lane, int p, uint32_t *at) {
     }
 }
 
-// deletes protein p from the table (backward shift)
-__device__ void erase(HitState &h, int lane, int p) {
-    uint32_t hole;
-    find(h, lane, p, &hole);
-    for (uint32_t b = hole + 1;; b += 32) {
-        const uint64_t mine = __ldcg(h.table + ((b + lane) & h.hmask));
-        for (int l = 0; l < 32; ++l) {
-            const uint64_t e = __shfl_sync(0xFFFFFFFFu, mine, l);
-            if (e == kFree) {
-                if (lane == 0) h.table[hole] = kFree;
-                __syncwarp();
-                return;
-            }
-            const uint32_t j = (b + l) & h.hmask, k = hash32((uint32_t)e) & h.hmask;
-            // move j into the hole when its home k is not in (hole, j]
-            const bool keep = (hole <= j) ? (hole < k && k <= j) : (hole < k || k <= j);
-            if (!keep) {
-                if (lane == 0) h.table[hole] = e;
-                hole = j;
-            }
+// one lane: protein p's entry (entries are p's, another's, gone or free)
+__device__ __forceinline__ uint32_t probe(const HitState &h, int p, uint64_t *e) {
+    uint32_t i = hash32((uint32_t)p) & h.hmask;
+    while ((*e = __ldcg(h.table + i)) != kFree && (int32_t)(uint32_t)*e != p) i = (i + 1) & h.hmask;
+    return i;
+}
+
+// one lane: claims an entry for protein p with slot s, beside other lanes
+// that add other proteins; or the entry p already has, in *e
+__device__ __forceinline__ bool claim(const HitState &h, int p, int s, uint32_t *at, uint64_t *e) {
+    uint32_t i = hash32((uint32_t)p) & h.hmask;
+    for (;; i = (i + 1) & h.hmask) {
+        *e = __ldcg(h.table + i);
+        if (*e == kFree) {
+            *e = atomicCAS((unsigned long long *)h.table + i, kFree, table_entry(p, s));
+            if (*e == kFree) { *at = i; return true; }
         }
+        if ((int32_t)(uint32_t)*e == p) return false;
     }
 }
 
-// the oldest hit of the smallest score: its slot (h.cmin > 0)
-__device__ int oldest_of_min(HitState &h, int lane) {
-    for (;;) {
-        while (h.cand) {
-            // what the last read of the log found, unless it rose since
-            const int l = __ffs(h.cand) - 1;
-            h.cand &= h.cand - 1;
-            const int s = __shfl_sync(0xFFFFFFFFu, h.cslot, l);
-            if (__ldcg(h.last + s) == h.scan - 32 + l) return s;
+// the table without its gone entries
+__device__ void rebuild(HitState &h, int lane) {
+    for (uint32_t i = lane; i <= h.hmask; i += 32) h.table[i] = kFree;
+    __syncwarp();
+    for (int s = lane; s < h.size; s += 32) {
+        uint32_t at;
+        uint64_t e;
+        claim(h, load_slot(h, s).x, s, &at, &e);
+    }
+    h.used = h.size;
+    __syncwarp();
+}
+
+// The `want` oldest hits of the smallest score (want <= h.cmin): lane i gets
+// the slot of the i-th.
+__device__ int oldest_of_min(HitState &h, int lane, int want) {
+    int mine = -1;
+    for (int got = 0; got < want;) {
+        // what the last read of the log found, without those that rose since
+        unsigned live = __ballot_sync(0xFFFFFFFFu, (h.cand >> lane & 1) &&
+                                                       __ldcg(h.last + max(h.cslot, 0)) == h.scan - 32 + lane);
+        for (; live && got < want; live &= live - 1) {
+            const int s = __shfl_sync(0xFFFFFFFFu, h.cslot, __ffs(live) - 1);
+            if (lane == got) mine = s;
+            ++got;
         }
+        h.cand = live;
+        if (got == want) break;
         const int e = h.scan + lane;
-        const int s = e < h.nev ? __ldcg(h.log + e) : -1;
-        const bool hit = s >= 0 && __ldcg(h.last + s) == e && load_slot(h, s).y == h.hmin;
-        h.cslot = s;
+        h.cslot = e < h.nev ? __ldcg(h.log + e) : -1;
+        const bool hit = h.cslot >= 0 && __ldcg(h.last + h.cslot) == e && load_slot(h, h.cslot).y == h.hmin;
         h.cand = __ballot_sync(0xFFFFFFFFu, hit);
         h.scan += 32;
     }
+    return mine;
 }
 
 // full list: the smallest score and how many hold it
@@ -608,17 +624,16 @@ __device__ bool add_one(HitState &h, int lane, int p, int gs, int gl, int off) {
     if (fresh) {
         s = h.size;
         if (full) {
-            s = oldest_of_min(h, lane);
+            s = __shfl_sync(0xFFFFFFFFu, oldest_of_min(h, lane, 1), 0);
             left = h.hmin;
-            const int wp = load_slot(h, s).x;
-            // p first: erase then moves it along if the hole is on its way
-            if (lane == 0) h.table[at] = table_entry(p, s);
-            __syncwarp();
-            erase(h, lane, wp);
+            uint32_t gone;
+            find(h, lane, load_slot(h, s).x, &gone);
+            if (lane == 0) h.table[gone] = kGone;
         } else {
-            if (lane == 0) h.table[at] = table_entry(p, s);
             h.size++;
         }
+        if (lane == 0) h.table[at] = table_entry(p, s);
+        h.used++;
     } else {
         const int4 x = load_slot(h, s);
         if (x.y >= gs) return false;
@@ -650,6 +665,8 @@ __device__ bool add_one(HitState &h, int lane, int p, int gs, int gl, int off) {
 // *n is how many were added.
 __device__ unsigned add_pops(HitState &h, int lane, int *n, int64_t room, int p, int gs, int gl, int off) {
     if (h.nev + 32 > h.logcap) compact_log(h, lane);
+    // (the table has two entries per hit and 256 at least: a quarter stays free)
+    if (h.used + 32 > (int)(h.hmask - h.hmask / 4)) rebuild(h, lane);
     const int cnt = *n;
     const bool valid = lane < cnt;
     const unsigned lt = (1u << lane) - 1u;
@@ -665,17 +682,9 @@ __device__ unsigned add_pops(HitState &h, int lane, int *n, int64_t room, int p,
             uint32_t i = 0;
             bool fresh = false;
             if (mine) {
-                i = hash32((uint32_t)p) & h.hmask;
-                for (;;) {
-                    uint64_t e = __ldcg(h.table + i);
-                    if (e == kFree) {
-                        // claim it; the slot number follows below
-                        e = atomicCAS((unsigned long long *)h.table + i, kFree, table_entry(p, -1));
-                        if (e == kFree) { fresh = true; break; }
-                    }
-                    if ((int32_t)(uint32_t)e == p) { s = (int)(e >> 32); break; }
-                    i = (i + 1) & h.hmask;
-                }
+                uint64_t e;
+                fresh = claim(h, p, -1, &i, &e);          // the slot number follows below
+                if (!fresh) s = (int)(e >> 32);
             }
             const unsigned nf = __ballot_sync(0xFFFFFFFFu, fresh);
             bool event = fresh;
@@ -691,6 +700,7 @@ __device__ unsigned add_pops(HitState &h, int lane, int *n, int64_t room, int p,
                 }
             }
             h.size += __popc(nf);
+            h.used += __popc(nf);
             fresh_all |= nf;
             event_all |= __ballot_sync(0xFFFFFFFFu, event);
             todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
@@ -709,17 +719,66 @@ __device__ unsigned add_pops(HitState &h, int lane, int *n, int64_t room, int p,
         return fresh_all;
     }
     // At or near capacity.  Every pop that beats the worst hit looks its
-    // protein up (together); what an earlier pop of the batch may change of
-    // that is only a protein it added or raised itself, and a hit it evicted.
-    unsigned counted = 0, stale = 0;
-    int os = -1;                         // score of the pop's protein, -1: not in the list
-    if (valid && (h.size < h.cap || gs > h.hmin)) {
-        for (uint32_t i = hash32((uint32_t)p) & h.hmask;; i = (i + 1) & h.hmask) {
-            const uint64_t e = __ldcg(h.table + i);
-            if (e == kFree) break;
-            if ((int32_t)(uint32_t)e == p) { os = load_slot(h, (int)(e >> 32)).y; break; }
+    // protein up (together).
+    int os = -1, own = -1;               // score and slot of the pop's protein, -1: not in the list
+    int4 x = make_int4(0, 0, 0, 0);
+    const bool looks = valid && (h.size < h.cap || gs > h.hmin);
+    if (looks) {
+        uint64_t e;
+        probe(h, p, &e);
+        if (e != kFree) {
+            own = (int)(e >> 32);
+            x = load_slot(h, own);
+            os = x.y;
         }
     }
+    if (h.size >= h.cap && cnt < room) {
+        // Full: while the smallest score keeps hits, it and so the pops that
+        // change the list are known beforehand, and if none of them is about
+        // a hit of that score or a protein of another of them, they change
+        // different hits: all at once, each new protein in the place of the
+        // next oldest hit of the smallest score.
+        const unsigned news = __ballot_sync(0xFFFFFFFFu, looks && os < 0);
+        const unsigned rise = __ballot_sync(0xFFFFFFFFu, looks && os >= 0 && os < gs);
+        const unsigned acts = news | rise;
+        const bool clash = (acts >> lane & 1) && (os == h.hmin || (same & acts & ~(1u << lane)));
+        if (!__any_sync(0xFFFFFFFFu, clash || (looks && (same & acts & ~(1u << lane)))) && __popc(news) < h.cmin) {
+            if (acts) {
+                const int victim = oldest_of_min(h, lane, __popc(news));
+                const int s = __shfl_sync(0xFFFFFFFFu, victim, __popc(news & lt)) * (int)(news >> lane & 1) +
+                              own * (int)(rise >> lane & 1);
+                const int e = h.nev + __popc(acts & lt);
+                __syncwarp();
+                if (news >> lane & 1) {
+                    uint64_t we, te;
+                    uint32_t at;
+                    const uint32_t gone = probe(h, load_slot(h, s).x, &we);
+                    claim(h, p, s, &at, &te);
+                    h.table[gone] = kGone;
+                    h.slot[s] = make_int4(p, gs, gl, off);
+                    atomicAdd(&h.hist[gs], 1);
+                } else if (rise >> lane & 1) {
+                    h.slot[s] = make_int4(p, gs, gl, x.w);
+                    atomicAdd(&h.hist[gs], 1);
+                    atomicSub(&h.hist[os], 1);
+                }
+                if (acts >> lane & 1) {
+                    h.log[e] = s;
+                    h.last[s] = e;
+                }
+                if (lane == 0 && news) atomicSub(&h.hist[h.hmin], __popc(news));
+                h.cmin -= __popc(news);
+                h.used += __popc(news);
+                h.nev += __popc(acts);
+                h.smax = max(h.smax, (int)__reduce_max_sync(0xFFFFFFFFu, (acts >> lane & 1) ? (unsigned)gs : 0u));
+                __syncwarp();
+            }
+            return news | __ballot_sync(0xFFFFFFFFu, valid && gs <= h.hmin);
+        }
+    }
+    // One by one: what an earlier pop of the batch may change of a lookup is
+    // only a protein it added or raised itself, and a hit it evicted.
+    unsigned counted = 0, stale = 0;
     for (int l = 0; l < cnt;) {
         const bool full = h.size >= h.cap;
         // the next pop that may change the list; those before it are counted
@@ -818,7 +877,7 @@ struct CurState {
     int32_t link;
 };
 
-constexpr int kBuf = 8;                 // chain elements staged per cursor
+constexpr int kBuf = 16;                // chain elements staged per cursor
 constexpr int kHeadSmem = 1024;         // scores whose stack head is in shared memory
 constexpr int kScoreWords = kSMax / 64;
 // codes of a staged element besides a score >= 0
@@ -870,7 +929,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
         h.logcap = 2 * a.max_cap + 64;
         h.hist = h.log + h.logcap;
         h.cap = qlen > 3000 ? (int)(1.5 * a.num_hits) : a.alignments;   // hit.c:106-109
-        h.size = h.nev = 0;
+        h.size = h.nev = h.used = 0;
         h.smax = 0;
         h.hmin = kSMax;
         h.cmin = h.scan = h.cslot = 0;
@@ -883,10 +942,24 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
     // blocks of 32 elements take the two halves of a cursor's slots in turn,
     // so the element before a new block keeps its place
     auto chain_at = [](int c, uint32_t e) { return (size_t)c * kChainSlots + e % kChainSlots; };
+    // the kBuf elements from e on into cursor c's staging
+    auto stage = [&](int c, uint32_t e) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(cache + chain_at(c, e));
+        uint4 x[kBuf / 4];
+#pragma unroll
+        for (int i = 0; i < kBuf / 4; ++i) x[i] = __ldcg(src + i);
+        uint32_t *b = reinterpret_cast<uint32_t *>(buf + kBuf * c);
+#pragma unroll
+        for (int i = 0; i < kBuf / 4; ++i) {
+            b[2 * i] = (uint16_t)push_code(x[i].x, minlen) | ((uint32_t)(uint16_t)push_code(x[i].y, minlen) << 16);
+            b[2 * i + 1] = (uint16_t)push_code(x[i].z, minlen) | ((uint32_t)(uint16_t)push_code(x[i].w, minlen) << 16);
+        }
+    };
 
     // ---- the queue in seeding insertion order: a cursor's link is the one
-    // before it with the same score
+    // before it with the same score, ncur (which links to itself) at the end
     for (int i = lane; i < kScoreWords; i += 32) bits[i] = 0;
+    if (lane == 0) state[ncur].link = ncur;
     __syncwarp();
     int qmax = -1;
     for (int base = 0; base < ncur; base += 32) {
@@ -894,19 +967,16 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
         int sc = -1;
         if (c < ncur && cur[c].len >= minlen) {
             sc = cur[c].score;
-            // the scores of its first rows
-            const uint4 *e = reinterpret_cast<const uint4 *>(cache + (size_t)c * kChainSlots);
-            const uint4 x = e[0], y = e[1];
-            const uint32_t w[kBuf] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-#pragma unroll
-            for (int i = 0; i < kBuf; ++i) buf[kBuf * c + i] = push_code(w[i], minlen);
+            stage(c, 0);
+            // the rest of its elements on the way to L2
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(cache + chain_at(c, kBuf)));
         }
         const unsigned same = __match_any_sync(0xFFFFFFFFu, sc >= 0 ? sc : -1 - lane);
         const unsigned below = same & ((1u << lane) - 1u), above = same & ~((2u << lane) - 1u);
         if (sc >= 0) {
             CurState st;
             st.k = 0;
-            st.link = below ? base + 31 - __clz(below) : has(sc) ? head(sc) : -1;
+            st.link = below ? base + 31 - __clz(below) : has(sc) ? head(sc) : ncur;
             state[c] = st;
         }
         __syncwarp();
@@ -921,7 +991,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
     int64_t npops = 0, counter = 0, refills = 0;
     PopRec *trace = a.trace ? a.trace + (int64_t)q * a.trace_cap : nullptr;
     // why a cursor's run stops before its score falls below the stack's
-    enum { kNo, kBlock, kRefill, kPastEnd };
+    enum { kNo, kLong, kRefill, kPastEnd };
     bool open = qmax >= 0;               // the queue goes on
     bool past_end = false;
     int first = 0, pending = 0;          // popped rows not yet in the hitlist: pops[first ..]
@@ -931,35 +1001,31 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
         while (open && refill < 0 && pending < 32) {
             const int s = qmax;
             // ---- the first 32 cursors of the stack
-            int c = -1, held = 0, under = head(s);
-            while (under >= 0 && held < 32) {
-                if (lane == held) c = under;
-                under = state[under].link;
-                ++held;
+            int c = ncur, under = head(s);
+            for (int i = 0; i < 32 && under != ncur; i += 4) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (lane == i + j) c = under;
+                    under = state[under].link;
+                }
             }
-            // ---- their runs, inside the staged block of elements
+            const int held = __popc(__ballot_sync(0xFFFFFFFFu, c != ncur));
+            // ---- their runs
             uint32_t k0 = 0, k = 0;
             int stop = kNo, sc = kNotQueued;
-            if (c >= 0) {
+            if (c != ncur) {
                 k = k0 = state[c].k;
-                if ((k & (kBuf - 1)) == 0 && k > 0) {
-                    if (k >= kChain && k % 32 == 0 && c != filled) {
-                        stop = kRefill;
-                    } else {
-                        const uint4 *e = reinterpret_cast<const uint4 *>(cache + chain_at(c, k));
-                        const uint4 x = __ldcg(e), y = __ldcg(e + 1);
-                        const uint32_t w[kBuf] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-#pragma unroll
-                        for (int i = 0; i < kBuf; ++i) buf[kBuf * c + i] = push_code(w[i], minlen);
+                for (;;) {
+                    if ((k & (kBuf - 1)) == 0 && k > 0) {
+                        if (k >= kChain && k % 32 == 0 && (c != filled || k != k0)) { stop = kRefill; break; }
+                        stage(c, k);
                     }
-                }
-                while (stop == kNo) {
                     const int x = buf[kBuf * c + (k & (kBuf - 1))];
                     if (x == kFault) { stop = kPastEnd; break; }
                     ++k;
                     sc = x;
                     if (x < s) break;
-                    if ((k & (kBuf - 1)) == 0) stop = kBlock;
+                    if (k - k0 == 32) { stop = kLong; break; }
                 }
             }
             // ---- those up to the first stopped run, as far as the ring has room
@@ -971,7 +1037,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
                 const int y = __shfl_up_sync(0xFFFFFFFFu, sum, o);
                 if (lane >= o) sum += y;
             }
-            const bool take = c >= 0 && (lane < end || (lane == end && run > 0)) && sum <= kPops - 32;
+            const bool take = c != ncur && (lane < end || (lane == end && run > 0)) && sum <= kPops - 32;
             const int taken = __popc(__ballot_sync(0xFFFFFFFFu, take));
             if (take) {
                 for (int i = 0; i < run; ++i) {
@@ -981,13 +1047,15 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
                     pops[(first + pending + sum - run + i) & (kPops - 1)] = r;
                 }
                 state[c].k = k;
+            } else if (c != ncur && (k0 == 0 || (k0 & (kBuf - 1)) != 0) && (k0 ^ k) >= kBuf) {
+                stage(c, k0 & ~(uint32_t)(kBuf - 1));     // its run went on to later elements
             }
             if (taken > 0) pending += __shfl_sync(0xFFFFFFFFu, sum, taken - 1);
             if (__any_sync(0xFFFFFFFFu, take && c == filled)) filled = -1;
             // ---- what is left of the stack, then the pushes in stack order
             const int top = taken < held ? __shfl_sync(0xFFFFFFFFu, c, taken & 31) : under;
             if (lane == 0) {
-                if (top >= 0) head(s) = (int16_t)top;
+                if (top != ncur) head(s) = (int16_t)top;
                 else bits[s >> 6] &= ~(1ull << (s & 63));
             }
             if (!take) sc = kNotQueued;
@@ -996,7 +1064,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
             __syncwarp();
             const int prev = below ? 31 - __clz(below) : lane;
             const int pc = __shfl_sync(0xFFFFFFFFu, c, prev);
-            if (sc >= 0) state[c].link = below ? pc : has(sc) ? head(sc) : -1;
+            if (sc >= 0) state[c].link = below ? pc : has(sc) ? head(sc) : ncur;
             __syncwarp();
             if (sc >= 0 && !above) {
                 head(sc) = (int16_t)c;
@@ -1005,7 +1073,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
             const int up = __reduce_max_sync(0xFFFFFFFFu, sc);
             __syncwarp();
             if (up >= s) qmax = up;
-            else if (top < 0) qmax = s > 0 ? bits_max_le(bits, s - 1) : -1;
+            else if (top == ncur) qmax = s > 0 ? bits_max_le(bits, s - 1) : -1;
             open = qmax >= 0;
             // ---- the stopped run's reason, once every run before it is taken
             const int why = __shfl_sync(0xFFFFFFFFu, stop, end & 31);
@@ -1076,7 +1144,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
 }
 
 size_t walk_smem(int cursors) {
-    return kWalkFixed + (sizeof(int16_t) * kBuf + sizeof(CurState)) * (size_t)cursors;
+    return kWalkFixed + (sizeof(int16_t) * kBuf + sizeof(CurState)) * (size_t)cursors + sizeof(CurState);
 }
 size_t walk_state_bytes(int cursors) { return walk_smem(cursors) - kWalkFixed; }
 
