@@ -24,6 +24,7 @@ struct tpz_index {
     std::vector<void *> mem;
     int64_t bytes = 0;
     std::vector<int64_t> pstart;   // host copy, Psize + 1
+    int32_t max_protein = 0;       // residues of the longest protein
 };
 
 namespace {
@@ -714,6 +715,7 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
     const Rec *rec = (const Rec *)ind;
     std::vector<int64_t> pstart(Psize + 1);
     int64_t run = 0;
+    int32_t longest = 0;
     for (int64_t p = 0; p < Psize; ++p) {
         if ((int64_t)rec[p].ps != run || rec[p].pl < 0 || run + rec[p].pl >= Tsize ||
             T[run + rec[p].pl] != '\n') {
@@ -725,6 +727,7 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
         }
         pstart[p] = run;
         run += rec[p].pl + 1;
+        longest = std::max(longest, rec[p].pl);
     }
     if (run != Tsize) {
         tpz::set_error("tpz_index_create: .ind does not cover the text");
@@ -793,6 +796,7 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
     ix->d.Tsize = Tsize; ix->d.Psize = Psize; ix->d.sa_rows = sa_rows;
     ix->d.T = dT; ix->d.SA = dSA; ix->d.pstart = dps; ix->d.nl = dnl; ix->d.lb = dlb;
     ix->pstart.swap(pstart);
+    ix->max_protein = longest;
     *out = ix;
     return TPZ_OK;
 }
@@ -1188,7 +1192,7 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
                                                (const int8_t *)ix->d.T, ps_off, ps_len, o->mat625,
                                                o->gap_open, o->gap_extend, sc, re, rd, st, 0, xmap,
                                                xmap, report ? 1 : 0, nq, poff.data(),
-                                               qlen_eff.data());
+                                               qlen_eff.data(), ix->max_protein);
             if (rc) return bail(rc);
             scatter_sw_kernel<<<(unsigned)std::min<int64_t>((npairs + 255) / 256, 4096), 256>>>(
                 npairs, p_hit, sc, re, rd, st, raw, send, qend, psw, report ? hit2pair : nullptr);

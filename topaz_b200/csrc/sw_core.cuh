@@ -199,8 +199,11 @@ struct Flow {
     int lagB;                         // the high half's column is that much earlier
     int width;                        // lanes of a group (pair tasks)
     uint32_t mul, add;                // the incoming word is shuffled * mul + add
-    const uint32_t *bnd;              // column boundary words (H | F << 16) or null
-    int bnd_end;                      // columns of the boundary
+    // the row above lane 0's first, by column: null, or (one alignment) a ring
+    // of H | F << 16, or (two) a ring of [H, F]
+    const uint32_t *bnd;
+    const uint2 *bnd2;
+    int bnd_end;                      // its columns
 };
 
 // One lane's state between steps.
@@ -267,7 +270,8 @@ struct Lane {
 // LONG: the halves are rows [0, 32R) and [32R, 64R) of one stripe, the high
 // half 32 columns behind; lane 0 takes the low half from the stripe above
 // (f.bnd) and the high half from lane 31's low half.
-template <int R, bool ENDS, bool LONG>
+// STRIPED: two alignments, lane 0 below another stripe of each (f.bnd2).
+template <int R, bool ENDS, bool LONG, bool STRIPED>
 __device__ __forceinline__ void step(Lane<R> &L, const Args &a, const Flow &f, int j,
                                      const uint32_t (&cwa)[Lane<R>::W],
                                      const uint32_t (&cwb)[Lane<R>::W],
@@ -292,8 +296,14 @@ __device__ __forceinline__ void step(Lane<R> &L, const Args &a, const Flow &f, i
         inH = mad(vH, f.mul, bH);
         inF = mad(vF, f.mul, bF);
     } else {
-        inH = mad(__shfl_up_sync(0xFFFFFFFFu, L.outH, 1, f.width), f.mul, f.add);
-        inF = mad(__shfl_up_sync(0xFFFFFFFFu, L.outF, 1, f.width), f.mul, f.add);
+        uint32_t bH = f.add, bF = f.add;
+        if (STRIPED && f.bnd2 && j < f.bnd_end) {
+            const uint2 b = f.bnd2[j & 63];
+            bH = b.x;
+            bF = b.y;
+        }
+        inH = mad(__shfl_up_sync(0xFFFFFFFFu, L.outH, 1, f.width), f.mul, bH);
+        inF = mad(__shfl_up_sync(0xFFFFFFFFu, L.outF, 1, f.width), f.mul, bF);
     }
     L.load_words(f, nwa, nwb);
     L.load_offsets(f, j + 2);
@@ -327,17 +337,20 @@ __device__ __forceinline__ void step(Lane<R> &L, const Args &a, const Flow &f, i
     L.diag = inH;
 }
 
-// steps [k0, kend), an even number of them
-template <int R, bool ENDS, bool LONG>
+// steps [k0, kend), an even number of them.  bnd_out (LONG) / rows_out
+// (STRIPED): where lane 31 leaves its last row, null in the others.
+template <int R, bool ENDS, bool LONG, bool STRIPED>
 __device__ __forceinline__ void steps(Lane<R> &L, const Args &a, const Flow &f, int k0, int kend,
-                                      uint32_t *bnd_out) {
+                                      uint32_t *bnd_out, uint2 *rows_out) {
     constexpr int W = Lane<R>::W;
     uint32_t wa2[W], wb2[W];
     for (int k = k0; k < kend; k += 2) {
-        step<R, ENDS, LONG>(L, a, f, k - f.lag, L.wa, L.wb, wa2, wb2);
+        step<R, ENDS, LONG, STRIPED>(L, a, f, k - f.lag, L.wa, L.wb, wa2, wb2);
         if (LONG && bnd_out) bnd_out[(k - 63) & (kRingCols - 1)] = prmt(L.outH, L.outF, 0x7632);
-        step<R, ENDS, LONG>(L, a, f, k + 1 - f.lag, wa2, wb2, L.wa, L.wb);
+        if (STRIPED && rows_out && k >= 31 && k - 31 < f.bnd_end) rows_out[k - 31] = make_uint2(L.outH, L.outF);
+        step<R, ENDS, LONG, STRIPED>(L, a, f, k + 1 - f.lag, wa2, wb2, L.wa, L.wb);
         if (LONG && bnd_out) bnd_out[(k - 62) & (kRingCols - 1)] = prmt(L.outH, L.outF, 0x7632);
+        if (STRIPED && rows_out && k >= 30 && k - 30 < f.bnd_end) rows_out[k - 30] = make_uint2(L.outH, L.outF);
     }
 }
 

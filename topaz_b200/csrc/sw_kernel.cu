@@ -17,7 +17,9 @@
 // lengths.
 //
 // Query-major form (the hits of one search query): the same, with a block of
-// 8 warps sharing one profile.
+// 8 warps sharing one profile.  Queries above 1024 residues take the pairs
+// through stripes of 32*R rows, the last row of a stripe going to the next
+// through memory, two words per column.
 //
 // Stripe form (queries longer than 1024, and batches too small to fill the
 // GPU with warps): W warps per pair; the halves of a warp's words are two row
@@ -31,8 +33,9 @@
 // in rings of 128 columns as profile offsets, refilled 32 columns at a time.
 //
 // Pairs are binned on the device by query length class and subject length
-// (counting sort), longest subjects first, and each R has one persistent
-// kernel that drains its bins from an atomic task counter.
+// (counting sort), longest subjects first, and drained by persistent kernels
+// from atomic task counters, one kernel for all R with the same shared
+// memory (4 values of R).
 
 #include <stdio.h>
 #include <string.h>
@@ -53,11 +56,6 @@ namespace sw {
 constexpr int kStripeRows = 32 * kMaxR;     // longest query of the throughput form
 // scores of tpz_sw_align_one and the allocation-free call stay below this
 constexpr int kBig = 32512;
-
-// row counts per lane with a kernel: 4, 8 and 9..32
-constexpr int kRs = 26;
-__host__ __device__ constexpr int rows_of(int i) { return i < 2 ? 4 * (i + 1) : 7 + i; }
-__host__ __device__ constexpr int rows_index(int R) { return R <= 8 ? (R + 3) / 4 - 1 : R - 7; }
 
 // Row bins.  Throughput form: queries above 32 residues with G = 32 lanes
 // and R = 9..32 in bins R - 9, with G = 16, 8, 4 and R = 9..16 in bins 24,
@@ -90,12 +88,35 @@ __device__ __forceinline__ int row_bin(int ql, int small_batch) {
 // bytes of a group's letter rings, low and high half
 constexpr int kPairRing = 2 * kRingCols * 2;
 
+// columns of a stripe's boundary kept in shared memory, [H, F] each
+constexpr int kBndCols = 64;
+
+// A stripe of a query above kStripeRows: which one, of how many, and the
+// boundary rows -- the warp's ring, and one [H, F] per column in memory,
+// read from the stripe above and written for the one below (the same words:
+// lane 0 is past a column when lane 31 ends it).
+struct Stripe {
+    int index, count;
+    uint2 *ring, *rows;
+};
+
+// f(R as a constant) for a run-time R in [R0, R1]
+template <int R0, int R1, class F>
+__device__ __forceinline__ void with_rows(int R, F &&f) {
+    if constexpr (R0 == R1) f(std::integral_constant<int, R0>());
+    else if (R == R0) f(std::integral_constant<int, R0>());
+    else with_rows<R0 + 1, R1>(R, f);
+}
+
 // Up to 64 / G pairs, two per group of G lanes: pair_at(first), ..., below
 // `count`.  prof: this warp's two profiles (BUILD), or the block's one
 // profile of the query they share; rings: 32 / G pairs of letter rings.
-template <int R, bool ENDS, bool BUILD, class PairAt>
+// STRIPED (G = 32): one stripe of the pairs; keyA / keyB carry their best
+// keys from stripe to stripe.
+template <int R, bool ENDS, bool BUILD, bool STRIPED, class PairAt>
 __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int first, int count, int G,
-                                          const uint8_t *matT, uint8_t *prof, uint8_t *rings) {
+                                          const uint8_t *matT, uint8_t *prof, uint8_t *rings,
+                                          const Stripe &sp, uint64_t &keyA, uint64_t &keyB) {
     const int lane = threadIdx.x & 31;
     const int lg = 31 - __clz(G), grp = lane >> lg, gl = lane & (G - 1);
     const int iA = first + 2 * grp, iB = iA + 1;
@@ -103,6 +124,7 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
     const int slA = pA >= 0 ? a.slen[pA] : 0, slB = pB >= 0 ? a.slen[pB] : 0;
     const int8_t *sA = a.s + (pA >= 0 ? a.soff[pA] : 0), *sB = a.s + (pB >= 0 ? a.soff[pB] : 0);
     const int N = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)max(slA, slB));
+    const int i0 = STRIPED ? (sp.index * 32 + lane) * R : gl * R;
     uint16_t *ringA = reinterpret_cast<uint16_t *>(rings + grp * kPairRing), *ringB = ringA + kRingCols;
     Flow f;
     f.profA = prof + lane * 4;
@@ -113,11 +135,14 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
         build_profile<R>(a, a.q + (pB >= 0 ? a.qoff[pB] : 0), pB >= 0 ? a.qlen[pB] : 0, gl * R, matT,
                          prof + profile_bytes(R) + lane * 4);
     }
+    const bool above = STRIPED && sp.index > 0, below = STRIPED && sp.index + 1 < sp.count;
     f.ringA = ringA; f.ringB = ringB;
     f.lag = gl; f.lagB = 0; f.width = G;
     f.mul = gl == 0 ? 0u : 1u;
     f.add = gl == 0 ? both((uint32_t)a.floor) : 0u;
-    f.bnd = nullptr; f.bnd_end = 0;
+    f.bnd = nullptr;
+    f.bnd2 = above && lane == 0 ? sp.ring : nullptr;
+    f.bnd_end = N;
     // columns 0..63, and pad letters where the columns before 0 are read
 #pragma unroll 4
     for (int c = gl; c < 64; c += G) {
@@ -125,6 +150,8 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
         ringB[c] = letter_offset<R>(a, sB, slB, c);
         ringA[64 + c] = ringB[64 + c] = kPadLetter * words_for(R) * 128;
     }
+    uint2 next = make_uint2(0, 0);              // boundary column k0 + lane of the next block
+    if (above && lane < N) next = __ldcg(sp.rows + lane);
     __syncwarp();
     Lane<R> L;
     L.start(a, f);
@@ -146,43 +173,57 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
             const int c = k0 + 64 + (gl << (5 - lg));
             touched = (c < slA ? sA[c] : 0) + (c < slB ? sB[c] : 0);
         }
+        if (above) {
+            sp.ring[(k0 + lane) & (kBndCols - 1)] = next;
+            if (k0 + 32 + lane < N) next = __ldcg(sp.rows + k0 + 32 + lane);
+        }
         if (ENDS) refresh<R, false>(L, G, 0u);
         __syncwarp();
-        steps<R, ENDS, false>(L, a, f, k0, min(k0 + 32, nsteps), nullptr);
+        steps<R, ENDS, false, STRIPED>(L, a, f, k0, min(k0 + 32, nsteps), nullptr,
+                                       below && lane == 31 ? sp.rows : nullptr);
     }
     if (ENDS && L.rose) L.find_row(a, f, nsteps - 1 - gl, L.run, lo16(L.rose), hi16(L.rose));
-    uint64_t kA = lane_key(L, a, false, gl * R), kB = lane_key(L, a, true, gl * R);
+    uint64_t kA = lane_key(L, a, false, i0), kB = lane_key(L, a, true, i0);
     for (int o = G >> 1; o > 0; o >>= 1) {
         kA = max(kA, __shfl_xor_sync(0xFFFFFFFFu, kA, o));
         kB = max(kB, __shfl_xor_sync(0xFFFFFFFFu, kB, o));
     }
-    if (gl == 0 && pA >= 0) write_result(a, pA, kA, ENDS);
-    if (gl == 1 && pB >= 0) write_result(a, pB, kB, ENDS);
+    if (STRIPED) {
+        kA = keyA = max(keyA, kA);
+        kB = keyB = max(keyB, kB);
+    }
+    if (!below) {
+        if (gl == 0 && pA >= 0) write_result(a, pA, kA, ENDS);
+        if (gl == 1 && pB >= 0) write_result(a, pB, kB, ENDS);
+    }
     __syncwarp();
 }
 
-// The bins of one R, with the lanes per group of each; their tasks are taken
-// in this order from the first bin's counter.
+// The bins of one launch, with rows per lane and lanes per group of each;
+// their tasks are taken in this order from the first bin's counter.
+constexpr int kSetBins = 16;
 struct BinSet {
     int n;
-    int bin[4], lanes[4];
+    int bin[kSetBins], rows[kSetBins], lanes[kSetBins];
 };
 
 // letter rings: one group above 16 rows, up to 8 below
-template <int R>
+template <int R1>
 __host__ __device__ constexpr int bin_smem() {
-    return kMatBytes + 2 * profile_bytes(R) + (R > 16 ? 1 : 8) * kPairRing;
+    return kMatBytes + 2 * profile_bytes(R1) + (R1 > 16 ? 1 : 8) * kPairRing;
 }
 
 // A block is one warp: tasks differ in length, and nothing is shared but the
 // matrix.  Shared memory (two profiles, 26 bytes per row and pair) holds the
-// warps per SM down to 4 (R = 32) .. 8 (R = 16); one warp keeps a scheduler's
-// ALU pipe busy because a step's rows hang together only through F.
-template <int R, bool ENDS>
+// warps per SM down to 4 (R = 32) .. 8 (R = 9).  The R of a launch (R0..R1)
+// take the same profile words per lane; with a launch per R (26) instead of
+// one per word count (7) a kernel's last tasks had only 8 streams of others
+// beside them.
+template <int R0, int R1, bool ENDS>
 __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args a,
                                                     const __grid_constant__ BinSet b) {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t *prof = smem + kMatBytes, *rings = prof + 2 * profile_bytes(R);
+    uint8_t *prof = smem + kMatBytes, *rings = prof + 2 * profile_bytes(R1);
     int total = 0;
     for (int i = 0; i < b.n; ++i) {
         const int per = 64 / b.lanes[i];
@@ -191,6 +232,8 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
     if (total == 0) return;
     load_matrix(a, smem);
     __syncwarp();
+    const Stripe none{0, 1, nullptr, nullptr};
+    uint64_t kA = 0, kB = 0;
     for (;;) {
         int t = 0;
         if (threadIdx.x == 0) t = atomicAdd(&a.next_task[b.bin[0]], 1);
@@ -204,8 +247,18 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
             count = a.rinfo[2 * b.bin[i] + 1];
         }
         const int32_t *ids = a.sorted + a.rinfo[2 * b.bin[i]];
-        pair_task<R, ENDS, true>(a, [&](int x) { return ids[x]; }, t * per, count, b.lanes[i], smem,
-                                 prof, rings);
+        auto id = [&](int x) { return ids[x]; };
+        if constexpr (R1 == 8) {
+            if (b.rows[i] == 4)
+                pair_task<4, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, none, kA, kB);
+            else
+                pair_task<8, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, none, kA, kB);
+        } else {
+            with_rows<R0, R1>(b.rows[i], [&](auto r) {
+                pair_task<decltype(r)::value, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof,
+                                                                 rings, none, kA, kB);
+            });
+        }
     }
 }
 
@@ -218,90 +271,134 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
 constexpr int kQmWarps = 8;
 constexpr int kQmMaxPairs = 256;      // pairs per chunk: longer pair lists of a query are cut
 constexpr int kQmMinPairs = 2 * kQmWarps;
-constexpr int kQmStreams = 8;
 
-struct QmArgs {
-    const int64_t *chunks;    // [first pair, end, lanes per group] per chunk
-    const int32_t *bin_info;  // per row count (rows_index): [first chunk, count]
-    int32_t *next;            // per row count: chunk counter
-    int ring_bytes;           // letter rings of one warp
+struct Chunk {
+    int64_t first;            // pairs [first, first + pairs) of one query
+    int32_t pairs, rows, lanes, stripes;
 };
 
-__host__ __device__ constexpr int qm_smem_bytes(int R, int ring_bytes) {
-    return kMatBytes + profile_bytes(R) + kQmWarps * ring_bytes + 4 * kQmMaxPairs;
+struct QmArgs {
+    const Chunk *chunks;
+    int count;
+    int32_t *next;            // chunk counter
+    int profile, ring;        // bytes of the profile, and of one warp's letter rings
+    uint2 *bnd;               // stripe boundary rows, bnd_cols per warp
+    int64_t bnd_cols;
+};
+
+__host__ __device__ constexpr int qm_smem_bytes(int profile, int ring, bool striped) {
+    return kMatBytes + profile + kQmWarps * (ring + (striped ? kBndCols * 8 : 0)) + 4 * kQmMaxPairs;
 }
 
-// profile words of a query for the lanes of every group, one word column per
-// warp at a time
+// profile words of a query for the lanes of every group, one word column of
+// one stripe per warp at a time; the stripes' profiles follow each other
 template <int R>
-__device__ __forceinline__ void qm_build_profile(const Args &a, int64_t p, int G, const uint8_t *matT,
-                                                 uint8_t *prof) {
+__device__ __forceinline__ void qm_build_profile(const Args &a, int64_t p, int G, int stripes,
+                                                 const uint8_t *matT, uint8_t *prof) {
     constexpr int W = words_for(R);
     const int lane = threadIdx.x & 31;
-    const int ql = a.qlen[p], i0 = (lane & (G - 1)) * R;
+    const int ql = a.qlen[p];
     const int8_t *q = a.q + a.qoff[p];
-    for (int w = threadIdx.x >> 5; w < W; w += kQmWarps) {
+    for (int i = threadIdx.x >> 5; i < W * stripes; i += kQmWarps) {
+        const int w = i % W, st = i / W, i0 = (st * 32 + (lane & (G - 1))) * R;
         int x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int r = 4 * w + k;
             x[k] = query_letter(a, (r < R && i0 + r < ql) ? (int)q[i0 + r] : -1);
         }
-        build_word<W>(matT, x[0], x[1], x[2], x[3], prof + w * 128 + lane * 4);
+        build_word<W>(matT, x[0], x[1], x[2], x[3], prof + st * profile_bytes(R) + w * 128 + lane * 4);
     }
 }
 
-template <int R, bool ENDS>
-__global__ void __launch_bounds__(kQmWarps * 32) sw_query_kernel(const __grid_constant__ Args a,
-                                                                 QmArgs g, int bin) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t *prof = smem + kMatBytes;
-    uint8_t *rings = prof + profile_bytes(R) + (threadIdx.x >> 5) * g.ring_bytes;
-    uint32_t *keys = reinterpret_cast<uint32_t *>(prof + profile_bytes(R) + kQmWarps * g.ring_bytes);
-    __shared__ int s_group, s_next;
+// pair i of a chunk in the order of its sorted keys
+struct ChunkPair {
+    const uint32_t *keys;
+    int first;
+    __device__ __forceinline__ int operator()(int i) const { return first + 255 - (int)(keys[i] & 255u); }
+};
+
+// One chunk with R rows per lane: the profile, the keys sorted, the tasks.
+template <int R, bool ENDS, bool STRIPED>
+__device__ __forceinline__ void run_chunk(const Args &a, const Chunk &ch, const uint8_t *matT, uint8_t *prof,
+                                          uint8_t *rings, uint32_t *keys, uint2 *ring, uint2 *rows,
+                                          int *next) {
     const int lane = threadIdx.x & 31;
-    const int gb = g.bin_info[2 * bin], gc = g.bin_info[2 * bin + 1];
-    if (gc == 0) return;
+    const int n = ch.pairs, G = STRIPED ? 32 : ch.lanes, stripes = STRIPED ? ch.stripes : 1;
+    int np = 1;
+    while (np < n) np <<= 1;
+    // keys: subject length (descending; < 2^24), place in the chunk
+    for (int i = threadIdx.x; i < np; i += blockDim.x)
+        keys[i] = i < n ? ((uint32_t)a.slen[ch.first + i] << 8) | (uint32_t)(255 - i) : 0u;
+    qm_build_profile<R>(a, ch.first, G, stripes, matT, prof);
+    __syncthreads();
+    for (int k = 2; k <= np; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < np; i += blockDim.x) {
+                const int l = i ^ j;
+                if (l > i) {
+                    const uint32_t x = keys[i], y = keys[l];
+                    if (((i & k) == 0) ? (x < y) : (x > y)) { keys[i] = y; keys[l] = x; }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    const int per = 64 / G;
+    const ChunkPair id{keys, (int)ch.first};
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(next, 1);
+        t = __shfl_sync(0xFFFFFFFFu, t, 0);
+        if (t * per >= n) break;
+        uint64_t kA = 0, kB = 0;
+        for (int st = 0; st < stripes; ++st) {
+            const Stripe sp{st, stripes, ring, rows};
+            pair_task<R, ENDS, false, STRIPED>(a, id, t * per, n, G, nullptr, prof + st * profile_bytes(R), rings,
+                                               sp, kA, kB);
+        }
+    }
+}
+
+template <int R, bool ENDS, bool STRIPED>
+__device__ __forceinline__ void run_chunk_rows(const Args &a, const Chunk &ch, const uint8_t *matT, uint8_t *prof,
+                                               uint8_t *rings, uint32_t *keys, uint2 *ring, uint2 *rows,
+                                               int *next) {
+    if constexpr (R == kMaxR) {
+        run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
+    } else {
+        if (ch.rows <= R) run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
+        else run_chunk_rows<R < 8 ? 8 : R + 1, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
+    }
+}
+
+// One launch for the chunks of all row counts (the longest chunks first):
+// every R fits the 128 registers of two blocks per SM, so a chunk's end is
+// filled by whatever chunk comes next.  (A launch per R over 8 streams left
+// the SMs of a 1000-query batch half empty at each launch's end.)
+template <bool ENDS, bool STRIPED>
+__global__ void __launch_bounds__(kQmWarps * 32, 2) sw_query_kernel(const __grid_constant__ Args a,
+                                                                    const QmArgs g) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int warp = threadIdx.x >> 5;
+    uint8_t *prof = smem + kMatBytes;
+    uint8_t *rings = prof + g.profile + warp * g.ring;
+    uint2 *bnd = reinterpret_cast<uint2 *>(prof + g.profile + kQmWarps * g.ring) + warp * kBndCols;
+    uint32_t *keys = reinterpret_cast<uint32_t *>(prof + g.profile + kQmWarps * g.ring +
+                                                  (STRIPED ? kQmWarps * kBndCols * 8 : 0));
+    uint2 *rows = g.bnd + (int64_t)(blockIdx.x * kQmWarps + warp) * g.bnd_cols;
+    __shared__ int s_chunk, s_next;
     load_matrix(a, smem);
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            s_group = atomicAdd(&g.next[bin], 1);
+            s_chunk = atomicAdd(g.next, 1);
             s_next = 0;
         }
         __syncthreads();
-        if (s_group >= gc) break;
-        const int64_t *ch = g.chunks + 3 * (gb + s_group);
-        const int64_t p0 = ch[0];
-        const int n = (int)(ch[1] - p0), G = (int)ch[2];
-        int np = 1;
-        while (np < n) np <<= 1;
-        // keys: subject length (descending; < 2^24), place in the chunk
-        for (int i = threadIdx.x; i < np; i += blockDim.x)
-            keys[i] = i < n ? ((uint32_t)a.slen[p0 + i] << 8) | (uint32_t)(255 - i) : 0u;
-        qm_build_profile<R>(a, p0, G, smem, prof);
-        __syncthreads();
-        for (int k = 2; k <= np; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = threadIdx.x; i < np; i += blockDim.x) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const uint32_t x = keys[i], y = keys[l];
-                        if (((i & k) == 0) ? (x < y) : (x > y)) { keys[i] = y; keys[l] = x; }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        const int per = 64 / G;
-        for (;;) {
-            int t = 0;
-            if (lane == 0) t = atomicAdd(&s_next, 1);
-            t = __shfl_sync(0xFFFFFFFFu, t, 0);
-            if (t * per >= n) break;
-            pair_task<R, ENDS, false>(a, [&](int x) { return (int)p0 + 255 - (int)(keys[x] & 255u); },
-                                      t * per, n, G, nullptr, prof, rings);
-        }
+        if (s_chunk >= g.count) break;
+        const Chunk ch = g.chunks[s_chunk];
+        run_chunk_rows<STRIPED ? 17 : 4, ENDS, STRIPED>(a, ch, smem, prof, rings, keys, bnd, rows, &s_next);
     }
 }
 
@@ -340,6 +437,7 @@ __device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, 
     f.mul = lane == 0 ? 65536u : 1u;
     f.add = lane == 0 ? (uint32_t)a.floor : 0u;
     f.bnd = lane == 0 ? above : nullptr;
+    f.bnd2 = nullptr;
     f.bnd_end = sl;
 #pragma unroll
     for (int c = lane; c < 64; c += 32) {
@@ -363,7 +461,7 @@ __device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, 
             if (above && k0 + lane < sl) in = lo16(above[(k0 + lane) & (kRingCols - 1)]);
             if (ENDS) refresh<R, true>(L, 32, in);
             __syncwarp();
-            steps<R, ENDS, true>(L, a, f, k0, k0 + 32, lane == 31 ? below : nullptr);
+            steps<R, ENDS, true, false>(L, a, f, k0, k0 + 32, lane == 31 ? below : nullptr, nullptr);
         }
         group_sync(group, W);
     }
@@ -567,25 +665,40 @@ __global__ void __launch_bounds__(256) dpx_probe_kernel(int iters, uint32_t inc,
 
 // ------------------------------------------------------------ host driver
 
+constexpr int kMaxSmem = 225 * 1024;  // dynamic shared memory of a block, at most
+
 // Kernels of one device with their launch attributes, set once.
+constexpr int kBinKernels = 7;
 struct Kernels {
     typedef void (*BinFn)(const Args, const BinSet);
-    typedef void (*QmFn)(const Args, QmArgs, int);
+    typedef void (*QmFn)(const Args, const QmArgs);
     typedef void (*StripeFn)(const Args, const StripeSet);
-    BinFn bin[2][kRs];                       // [ends][rows_index]
-    QmFn qm[2][kRs];
+    BinFn bin[2][kBinKernels];               // [ends][most rows first]
+    QmFn qm[2][2];                           // [ends][striped]
     StripeFn stripe8[2], stripe32[2];        // [ends]
-    int bin_smem[kRs], bin_blocks[2][kRs];   // blocks per SM
+    BinSet set[kBinKernels];
+    int bin_smem[kBinKernels], bin_blocks[2][kBinKernels];   // blocks per SM
     int stripe8_blocks[2], stripe32_blocks[2];
 };
 
-template <int... I>
-static void fill_kernels(Kernels &k, std::integer_sequence<int, I...>) {
-    ((k.bin[0][I] = sw_bin_kernel<rows_of(I), false>), ...);
-    ((k.bin[1][I] = sw_bin_kernel<rows_of(I), true>), ...);
-    ((k.qm[0][I] = sw_query_kernel<rows_of(I), false>), ...);
-    ((k.qm[1][I] = sw_query_kernel<rows_of(I), true>), ...);
-    ((k.bin_smem[I] = bin_smem<rows_of(I)>()), ...);
+template <int I, int R0, int R1>
+static void fill_bin(Kernels &k) {
+    k.bin[0][I] = sw_bin_kernel<R0, R1, false>;
+    k.bin[1][I] = sw_bin_kernel<R0, R1, true>;
+    k.bin_smem[I] = bin_smem<R1>();
+    BinSet &s = k.set[I];
+    s.n = 0;
+    auto add = [&](int bin, int rows, int lanes) {
+        s.bin[s.n] = bin; s.rows[s.n] = rows; s.lanes[s.n++] = lanes;
+    };
+    if (R1 == 8) {
+        add(kTinyBin + 1, 8, 4);
+        add(kTinyBin, 4, 4);
+        return;
+    }
+    for (int R = R1; R >= R0; --R) add(R - 9, R, 32);
+    for (int g = 0; g < 3 && R1 <= 16; ++g)
+        for (int R = R1; R >= R0; --R) add(24 + 8 * g + R - 9, R, 16 >> g);
 }
 
 // dynamic shared memory of a kernel, the whole carveout (so blocks of
@@ -611,19 +724,27 @@ static int kernels(const Kernels **out) {
     if ((int)per_dev.size() <= dev) per_dev.resize(dev + 1, nullptr);
     if (!per_dev[dev]) {
         Kernels *k = new Kernels();
-        fill_kernels(*k, std::make_integer_sequence<int, kRs>());
+        fill_bin<0, 29, 32>(*k);
+        fill_bin<1, 25, 28>(*k);
+        fill_bin<2, 21, 24>(*k);
+        fill_bin<3, 17, 20>(*k);
+        fill_bin<4, 13, 16>(*k);
+        fill_bin<5, 9, 12>(*k);
+        fill_bin<6, 4, 8>(*k);
         int rc = TPZ_OK;
+        k->qm[0][0] = sw_query_kernel<false, false>;
+        k->qm[0][1] = sw_query_kernel<false, true>;
+        k->qm[1][0] = sw_query_kernel<true, false>;
+        k->qm[1][1] = sw_query_kernel<true, true>;
         k->stripe8[0] = sw_stripe_kernel<false, 8>;
         k->stripe8[1] = sw_stripe_kernel<true, 8>;
         k->stripe32[0] = sw_stripe_kernel<false, 32>;
         k->stripe32[1] = sw_stripe_kernel<true, 32>;
         for (int e = 0; rc == TPZ_OK && e < 2; ++e) {
-            for (int i = 0; rc == TPZ_OK && i < kRs; ++i) {
+            for (int i = 0; rc == TPZ_OK && i < kBinKernels; ++i)
                 rc = set_up((const void *)k->bin[e][i], k->bin_smem[i], 32, &k->bin_blocks[e][i]);
-                if (rc == TPZ_OK)
-                    rc = set_up((const void *)k->qm[e][i], qm_smem_bytes(rows_of(i), 8 * kPairRing),
-                                kQmWarps * 32, nullptr);
-            }
+            for (int x = 0; rc == TPZ_OK && x < 2; ++x)
+                rc = set_up((const void *)k->qm[e][x], kMaxSmem, kQmWarps * 32, nullptr);
             if (rc == TPZ_OK)
                 rc = set_up((const void *)k->stripe8[e], stripe_smem(8, kLongWarps), 32 * kLongWarps,
                             &k->stripe8_blocks[e]);
@@ -639,7 +760,7 @@ static int kernels(const Kernels **out) {
     return TPZ_OK;
 }
 
-constexpr int kAuxStreams = 8;
+constexpr int kAuxStreams = 8;           // a kernel of a batch each
 
 // Per host thread and device: the auxiliary streams and fork/join events of
 // one call must not be shared with a call running in another thread.
@@ -748,11 +869,8 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
                         next_stream()>>>(a, s);
         ++launches;
     } else {
-        for (int i = kRs - 1; i >= 0; --i) {
-            const int R = rows_of(i);
-            BinSet s{R > 16 ? 1 : 4, {R - 9, 24 + R - 9, 32 + R - 9, 40 + R - 9}, {32, 16, 8, 4}};
-            if (R <= 8) s = BinSet{1, {kTinyBin + i, 0, 0, 0}, {4, 0, 0, 0}};
-            k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, s);
+        for (int i = 0; i < kBinKernels; ++i) {
+            k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
             ++launches;
         }
     }
@@ -820,102 +938,159 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
                          const int8_t *mat, int go, int ge, int32_t *score, int32_t *ref_end,
                          int32_t *read_end, int32_t *status, cudaStream_t st, const int8_t *xq,
                          const int8_t *xs, int score_only, int64_t ngroups,
-                         const int64_t *gstart_host, const int32_t *gqlen_host) {
+                         const int64_t *gstart_host, const int32_t *gqlen_host, int max_slen) {
     if (n <= 0) return TPZ_OK;
     if (!(go > ge && ge >= 0 && go <= 255) || !mat) {
         set_error("tpz_sw_batch: requires 255 >= gap_open > gap_extend >= 0");
         return TPZ_E_ARG;
     }
-    // chunks of at most kQmMaxPairs pairs of one query for the query-major
-    // kernels (queries with enough pairs and one stripe); every other pair
-    // goes by pair
-    struct Row { std::vector<int64_t> chunks; int64_t work = 0; int min_lanes = 32; };
-    std::vector<Row> rows(kRs);
+    const int nsm = sm_count();
+    // Chunks of pairs of one query for the query-major kernels (queries with
+    // enough pairs); every other pair goes by pair.  A chunk holds at most
+    // kQmMaxPairs, and fewer while the blocks of the GPU would not get four
+    // each, down to four tasks per warp.
+    int64_t cells = 0;                  // pairs * rows, the measure of a chunk's time
+    for (int64_t g = 0; g < ngroups; ++g)
+        cells += (gstart_host[g + 1] - gstart_host[g]) * gqlen_host[g];
+    const int64_t share = cells / (8 * nsm) + 1;
+    std::vector<Chunk> chunks[5];       // one stripe, and 2, up to 4, 6, 8 of them
+    int min_lanes = 32, max_rows = 1;
+    int striped_profile[5] = {0, 0, 0, 0, 0};
     std::vector<int32_t> rest;
     for (int64_t g = 0; g < ngroups; ++g) {
         const int64_t c = gstart_host[g + 1] - gstart_host[g];
         if (c <= 0) continue;
         const int ql = gqlen_host[g];
-        if (ql >= 1 && ql <= kStripeRows && c >= kQmMinPairs) {
-            const int64_t nch = (c + kQmMaxPairs - 1) / kQmMaxPairs;
-            // more lanes per pair (fewer rows each) while a chunk would leave
-            // warps of its block without a task
-            int G = group_lanes(ql);
-            while (G < 32 && c / nch < kQmWarps * (64 / G)) G *= 2;
-            Row &r = rows[rows_index((ql + G - 1) / G)];
-            for (int64_t i = 0; i < nch; ++i) {
-                // equal cuts so that no chunk is much smaller than the others
-                r.chunks.push_back(gstart_host[g] + c * i / nch);
-                r.chunks.push_back(gstart_host[g] + c * (i + 1) / nch);
-                r.chunks.push_back(G);
-            }
-            r.work += c * ql;
-            r.min_lanes = std::min(r.min_lanes, G);
-        } else {
+        if (ql < 1 || c < kQmMinPairs) {
             for (int64_t k = gstart_host[g]; k < gstart_host[g + 1]; ++k) rest.push_back((int32_t)k);
+            continue;
+        }
+        const int stripes = (ql + kStripeRows - 1) / kStripeRows;
+        const int64_t most = std::min<int64_t>(kQmMaxPairs, std::max<int64_t>(8 * kQmWarps, share / ql));
+        const int64_t nch = (c + most - 1) / most;
+        // more lanes per pair (fewer rows each) while a chunk would leave
+        // warps of its block without a task
+        int G = stripes > 1 ? 32 : group_lanes(ql);
+        while (G < 32 && c / nch < kQmWarps * (64 / G)) G *= 2;
+        const int rows = (ql + G * stripes - 1) / (G * stripes);
+        const int cls = stripes == 1 ? 0 : stripes == 2 ? 1 : (stripes + 1) / 2;
+        for (int64_t i = 0; i < nch; ++i) {
+            // equal cuts so that no chunk is much smaller than the others
+            const int64_t b0 = gstart_host[g] + c * i / nch, b1 = gstart_host[g] + c * (i + 1) / nch;
+            chunks[cls].push_back(Chunk{b0, (int32_t)(b1 - b0), rows, G, stripes});
+        }
+        if (cls == 0) {
+            min_lanes = std::min(min_lanes, G);
+            max_rows = std::max(max_rows, rows);
+        } else {
+            striped_profile[cls] = std::max(striped_profile[cls], stripes * profile_bytes(rows));
         }
     }
-    // one upload: chunks, then [first chunk, count] and a zero counter per
-    // row count, then the other pairs
-    std::vector<int64_t> chunks;
-    std::vector<int32_t> tail(3 * kRs, 0);
-    std::vector<int> order;
-    for (int i = 0; i < kRs; ++i) {
-        tail[2 * i] = (int32_t)(chunks.size() / 3);
-        tail[2 * i + 1] = (int32_t)(rows[i].chunks.size() / 3);
-        chunks.insert(chunks.end(), rows[i].chunks.begin(), rows[i].chunks.end());
-        if (!rows[i].chunks.empty()) order.push_back(i);
+    // one upload: a zero counter per class, the other pairs, the chunks
+    // (longest first)
+    std::vector<int32_t> head(8, 0);
+    head.insert(head.end(), rest.begin(), rest.end());
+    if (head.size() & 1) head.push_back(0);
+    size_t nchunks = 0;
+    for (std::vector<Chunk> &c : chunks) {
+        std::sort(c.begin(), c.end(), [](const Chunk &x, const Chunk &y) {
+            return (int64_t)x.pairs * x.rows * x.stripes * x.lanes > (int64_t)y.pairs * y.rows * y.stripes * y.lanes;
+        });
+        nchunks += c.size();
     }
-    tail.insert(tail.end(), rest.begin(), rest.end());
+    const size_t hbytes = 4 * head.size();
+    std::vector<char> up(hbytes + sizeof(Chunk) * nchunks);
+    memcpy(up.data(), head.data(), hbytes);
+    size_t at = hbytes;
+    for (const std::vector<Chunk> &c : chunks) {
+        if (!c.empty()) memcpy(up.data() + at, c.data(), sizeof(Chunk) * c.size());
+        at += sizeof(Chunk) * c.size();
+    }
     const Kernels *k = nullptr;
     Streams *x = nullptr;
     int rc = kernels(&k);
     if (rc || (rc = streams(&x, 2))) return rc;
-    int64_t *dchunks = nullptr;
-    const size_t cbytes = 8 * chunks.size(), tbytes = 4 * tail.size();
-    TPZ_CUDA(cudaMallocAsync((void **)&dchunks, cbytes + tbytes, st));
-    int32_t *dtail = (int32_t *)((char *)dchunks + cbytes);
-    if ((cbytes && cudaMemcpyAsync(dchunks, chunks.data(), cbytes, cudaMemcpyHostToDevice, st)) ||
-        cudaMemcpyAsync(dtail, tail.data(), tbytes, cudaMemcpyHostToDevice, st)) {
-        cudaFreeAsync(dchunks, st);
+    char *dup = nullptr;
+    uint2 *dbnd = nullptr;
+    auto drop = [&]() {
+        if (dup) cudaFreeAsync(dup, st);
+        if (dbnd) cudaFreeAsync(dbnd, st);
+    };
+    TPZ_CUDA(cudaMallocAsync((void **)&dup, up.size(), st));
+    if (cudaMemcpyAsync(dup, up.data(), up.size(), cudaMemcpyHostToDevice, st)) {
+        drop();
         return cuda_fail(cudaGetLastError(), "batch_device_grouped copies");
     }
+    int32_t *dhead = (int32_t *)dup;
     Args a;
     pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
     set_scoring(a, mat, go, ge);
     a.translate = (xq && xs) ? 1 : 0;
     if (a.translate) { memcpy(a.xq, xq, 128); memcpy(a.xs, xs, 128); }
-    QmArgs g;
-    g.chunks = dchunks; g.bin_info = dtail; g.next = dtail + 2 * kRs;
-    const int nsm = sm_count(), e = score_only ? 0 : 1;
+    const int e = score_only ? 0 : 1;
     int64_t launches = 0;
-    if (!order.empty()) {
-        // one persistent kernel per row count, those with the most work
-        // first, over the streams so that they share the SMs
-        if ((rc = fork(x, st))) { cudaFreeAsync(dchunks, st); return rc; }
-        std::sort(order.begin(), order.end(), [&](int l, int r) { return rows[l].work > rows[r].work; });
-        int at = 0;
-        for (int i : order) {
-            g.ring_bytes = (32 / rows[i].min_lanes) * kPairRing;
-            const int smem = qm_smem_bytes(rows_of(i), g.ring_bytes);
-            int nb = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k->qm[e][i], kQmWarps * 32,
-                                                              smem) != cudaSuccess || nb < 1)
-                nb = 1;
-            const unsigned grid = (unsigned)std::min<int64_t>((int64_t)nsm * nb,
-                                                              (int64_t)rows[i].chunks.size() / 3);
-            k->qm[e][i]<<<grid, kQmWarps * 32, smem, x->aux[at++ % kAuxStreams]>>>(a, g, i);
+    struct Launch { QmArgs g; unsigned grid; int smem, striped; };
+    std::vector<Launch> todo;
+    int64_t bnd_words = 0;
+    at = hbytes;
+    for (int cls = 0; cls < 5; ++cls) {
+        const std::vector<Chunk> &c = chunks[cls];
+        if (c.empty()) continue;
+        Launch l;
+        l.striped = cls > 0;
+        l.g.chunks = (const Chunk *)(dup + at);
+        at += sizeof(Chunk) * c.size();
+        l.g.count = (int)c.size();
+        l.g.next = dhead + cls;
+        l.g.profile = cls ? striped_profile[cls] : profile_bytes(max_rows <= 8 ? 8 : max_rows);
+        l.g.ring = cls ? kPairRing : (32 / min_lanes) * kPairRing;
+        l.smem = qm_smem_bytes(l.g.profile, l.g.ring, l.striped);
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k->qm[e][l.striped], kQmWarps * 32,
+                                                          l.smem) != cudaSuccess || nb < 1)
+            nb = 1;
+        l.grid = (unsigned)std::min<int64_t>((int64_t)nsm * nb, (int64_t)c.size());
+        l.g.bnd = nullptr;
+        l.g.bnd_cols = 0;
+        if (cls) {
+            // (at most 1 GB of boundary rows: fewer blocks where subjects are long)
+            l.g.bnd_cols = std::max(max_slen, 1);
+            const int64_t per_block = kQmWarps * l.g.bnd_cols;
+            l.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(l.grid, ((int64_t)1 << 27) / per_block));
+            bnd_words += per_block * l.grid;
+        }
+        todo.push_back(l);
+    }
+    if (bnd_words > 0) {
+        if (cudaMallocAsync((void **)&dbnd, sizeof(uint2) * (size_t)bnd_words, st)) {
+            drop();
+            return cuda_fail(cudaGetLastError(), "batch_device_grouped boundary rows");
+        }
+        bnd_words = 0;
+        for (Launch &l : todo) {
+            if (!l.striped) continue;
+            l.g.bnd = dbnd + bnd_words;
+            bnd_words += kQmWarps * l.g.bnd_cols * l.grid;
+        }
+    }
+    if (!todo.empty()) {
+        // the classes with most stripes first: their chunks take longest
+        if ((rc = fork(x, st))) { drop(); return rc; }
+        int stream = 0;
+        for (size_t i = todo.size(); i-- > 0;) {
+            const Launch &l = todo[i];
+            k->qm[e][l.striped]<<<l.grid, kQmWarps * 32, l.smem, x->aux[stream++ % kAuxStreams]>>>(a, l.g);
             ++launches;
         }
     }
     rc = batch_device_x(n, q, qoff, qlen, s, soff, slen, mat, go, ge, score, ref_end, read_end,
-                        status, st, xq, xs, score_only, dtail + 3 * kRs, (int64_t)rest.size());
+                        status, st, xq, xs, score_only, dhead + 8, (int64_t)rest.size());
     launches += g_last_launches;
-    if (!order.empty()) {
+    if (!todo.empty()) {
         const int rj = join(x, st);
         if (rc == TPZ_OK) rc = rj;
     }
-    cudaFreeAsync(dchunks, st);
+    drop();
     if (rc) return rc;
     TPZ_CUDA(cudaGetLastError());
     g_last_launches = launches;
