@@ -118,7 +118,7 @@ TPZ_API int tpz_sw_align_one(const int8_t *q, int32_t qlen, const int8_t *s, int
  * residues (longer ones get status TPZ_SW_INVALID) and matrices whose
  * largest entry is at most TPZ_SW_NOALLOC_MAX_ENTRY (TPZ_E_ARG beyond, so
  * that no score reaches 32767).  Scratch is one static device array per
- * device (about 0.4 MB, held until the process exits) shared by all calls: calls
+ * device (about 5 MB, held until the process exits) shared by all calls: calls
  * whose work overlaps on the GPU (other streams or threads) race on it, so
  * order them on one stream.  All work goes to `stream`; nothing is
  * allocated or freed.  The first call on a device does a one-time set-up

@@ -30,10 +30,10 @@
 // Arithmetic: two alignments (or two row ranges of one) ride in the halves
 // of u16x2 words, every value raised by `floor` (= the zero of a score).
 // floor >= go + ge - min(M), so X - go never borrows: it is one 32-bit
-// multiply-add on the FMA pipe, which leaves the ALU pipe -- the bound: its
+// addition, which the compiler may put beside the ALU pipe -- the bound: its
 // packed min/max/add and PRMT issue at 16 lanes a clock and scheduler --
-// with 5.5 operations per cell pair: PRMT (profile bytes), X, H, E, F and
-// half a column maximum.  (With Fm, the lane starts and X - go on the same
+// and leaves that with 5.5 operations per cell pair: PRMT (profile bytes), X,
+// H, E, F and half a column maximum.  (With Fm, the lane starts and X - go on the same
 // pipe it was 8.5, and 1.3 times the cells because saturated pairs ran
 // twice.)  A score that reaches 32767 is final (the pair is dropped) however
 // far its 16 bits run on, so nothing is recomputed in wider arithmetic.
@@ -41,13 +41,14 @@
 // End coordinates: each lane keeps its running maximum of X (the alignment's
 // maximum is an X: F and E only hold less than an X before them).  A rise is
 // looked at only when it reaches the group maximum of the last refresh (every
-// 32 steps; less cannot be the alignment's maximum), and its row is looked up
-// one step later, so a column whose successor rises again is passed over.  H
-// is gone by then, but E tells the row: a column whose maximum m is above
-// every earlier X of the lane leaves E = m - go in exactly the rows that hold
-// m.  (Carrying the row in the low bits of the maximum, one more FMA-pipe
-// operation per cell pair, measured 12.5 against 11.6 cycles per row with
-// four warps per scheduler and 16.3 against 12.8 with one.)
+// 32 steps; less cannot be the alignment's maximum); then the lane stores its
+// column of H, and the row is looked up once, in the last column stored.  A
+// rise so costs R / 4 stores that nothing waits for.  (Of the steps of the
+// 200,000-pair case 31 % have one in some lane of the warp.  Looking the row
+// up at once took 1.5 ALU operations per row and their latency: 11.1 ms
+// against 9.0 ms without ends.  Carrying it in the low bits of the maximum,
+// one more FMA-pipe operation per cell pair, took 12.5 against 11.6 cycles
+// per row with four warps per scheduler and 16.3 against 12.8 with one.)
 #pragma once
 
 #include "tpz_common.cuh"
@@ -83,7 +84,7 @@ struct Args {
     int32_t *next_task;      // per row bin: task counter
     int gap_open, gap_extend;
     int floor;               // the zero of every stored value
-    uint32_t one, sixty4;    // multipliers the compiler must not know (FMA pipe)
+    uint4 *snap;             // columns stored at a rise: snap_words() per warp
     int translate;           // 1: q/s bytes go through xq/xs first
     int8_t mat[625];
     int8_t xq[128], xs[128]; // byte -> matrix index (internal alphabet inputs)
@@ -99,8 +100,6 @@ inline void set_scoring(Args &a, const int8_t *mat, int go, int ge) {
     a.gap_open = go;
     a.gap_extend = ge;
     a.floor = go + ge - mn;                 // <= 255 + 254 + 128
-    a.one = 1;
-    a.sixty4 = 64;
 }
 
 __device__ __forceinline__ uint32_t both(uint32_t x) { return x | (x << 16); }
@@ -204,6 +203,7 @@ struct Flow {
     const uint32_t *bnd;
     const uint2 *bnd2;
     int bnd_end;                      // its columns
+    uint4 *snap;                      // this lane's stored columns
 };
 
 // One lane's state between steps.
@@ -213,8 +213,7 @@ struct Lane {
     uint32_t E[R], H[R];
     uint32_t diag, outH, outF;
     uint32_t run;                 // running maxima of X
-    uint32_t rose;                // halves in which the last column raised run
-    uint32_t atA, atB;            // column << 5 | row where run was first reached
+    int colA, colB;               // the columns that reached them
     uint32_t wa[W], wb[W];        // profile words of the next step's column
     uint32_t nA, nB;              // profile offsets of the column after it
 
@@ -233,35 +232,40 @@ struct Lane {
     __device__ __forceinline__ void start(const Args &a, const Flow &f) {
         const uint32_t z = both((uint32_t)a.floor);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            E[r] = z - both((uint32_t)a.gap_open);       // E never above run - go (find_row)
-            H[r] = z;
-        }
+        for (int r = 0; r < R; ++r) { E[r] = z; H[r] = z; }
         diag = outH = outF = run = z;
-        rose = atA = atB = 0;
+        colA = colB = 0;
         load_offsets(f, -f.lag);
         load_words(f, wa, wb);
         load_offsets(f, 1 - f.lag);
     }
-    // the row of the rises of column j, whose maxima are `top`, in the halves
-    // `lo` / `hi`: E as column j left it
-    __device__ __forceinline__ void find_row(const Args &a, const Flow &f, int j, uint32_t top, bool lo,
-                                             bool hi) {
-        const uint32_t neg = __vsub2(both((uint32_t)a.gap_open), top);       // -(top - go)
-        uint32_t acc = 0x00FF00FFu;
+    // this column of H
+    __device__ __forceinline__ void store(uint4 *snap) const {
 #pragma unroll
-        for (int r = 0; r < R; r += 2) {
-            // 0 in the rows holding the maximum, 1 elsewhere; times 64
-            const uint32_t e0 = mad(__viaddmin_u16x2(E[r], neg, 0x00010001u), a.sixty4, both(r));
-            const uint32_t e1 = r + 1 < R ? mad(__viaddmin_u16x2(E[r + 1 < R ? r + 1 : r], neg, 0x00010001u),
-                                                a.sixty4, both(r + 1))
-                                          : e0;
-            acc = __vimin3_u16x2(acc, e0, e1);
+        for (int w = 0; w < W; ++w)
+            snap[32 * w] = make_uint4(H[4 * w], 4 * w + 1 < R ? H[4 * w + 1 < R ? 4 * w + 1 : 0] : 0u,
+                                      4 * w + 2 < R ? H[4 * w + 2 < R ? 4 * w + 2 : 0] : 0u,
+                                      4 * w + 3 < R ? H[4 * w + 3 < R ? 4 * w + 3 : 0] : 0u);
+    }
+    // the first row of a stored column that holds the running maximum
+    __device__ __forceinline__ int find_row(const uint4 *snap, bool high) const {
+        const uint32_t v = high ? hi16(run) : lo16(run);
+        int row = 0;
+#pragma unroll
+        for (int w = W - 1; w >= 0; --w) {
+            const uint4 x = snap[32 * w];
+            const uint32_t h[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int k = 3; k >= 0; --k)
+                if ((high ? hi16(h[k]) : lo16(h[k])) == v) row = 4 * w + k;
         }
-        if (lo) atA = ((uint32_t)j << 5) + lo16(acc);
-        if (hi) atB = ((uint32_t)(j - f.lagB) << 5) + hi16(acc);
+        return row;
     }
 };
+
+// words of uint4 a warp stores columns in: the low half's, then the high
+// half's, by word and lane
+__host__ __device__ constexpr int snap_words(int R) { return 2 * 32 * words_for(R); }
 
 // Step k of a lane: column j = k - lag.  Every lane computes every step: a
 // lane before its first column sees pad letters and floor inputs, so its H
@@ -314,24 +318,22 @@ __device__ __forceinline__ void step(Lane<R> &L, const Args &a, const Flow &f, i
                                 L.E[r]);
 #pragma unroll
     for (int r = 0; r < R; r += 2) m = __vimax3_u16x2(m, X[r], X[r + 1 < R ? r + 1 : r]);
-    if constexpr (ENDS) {
-        const uint32_t d = m ^ L.run;
-        if (L.rose) {
-            // the previous column's rises that this column does not top
-            const bool lo = lo16(L.rose) && !lo16(d), hi = hi16(L.rose) && !hi16(d);
-            if (lo || hi) L.find_row(a, f, j - 1, L.run, lo, hi);
-        }
-        L.rose = d;
-    }
-    L.run = m;
     uint32_t F = inF;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const uint32_t Xg = mad(X[r], a.one, NGO);
+        const uint32_t Xg = X[r] + NGO;
         L.H[r] = __vimax3_u16x2(X[r], F, Z);
         L.E[r] = __viaddmax_u16x2(L.E[r], NGE, Xg);
         F = __viaddmax_u16x2(F, NGE, Xg);
     }
+    if constexpr (ENDS) {
+        const uint32_t d = m ^ L.run;
+        if (d) {
+            if (lo16(d)) { L.store(f.snap); L.colA = j; }
+            if (hi16(d)) { L.store(f.snap + 32 * words_for(R)); L.colB = j - f.lagB; }
+        }
+    }
+    L.run = m;
     L.outH = L.H[R - 1];
     L.outF = F;
     L.diag = inH;
@@ -365,19 +367,16 @@ __device__ __forceinline__ void refresh(Lane<R> &L, int width, uint32_t above) {
     uint32_t m = LONG ? max2u(L.run, above) : L.run;
     for (int o = width >> 1; o > 0; o >>= 1) m = max2u(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     if (LONG) m = max2u(m, (m << 16) | (m >> 16));
-    m = max2u(L.run, m - 0x00010001u);           // halves are at least the floor: no borrow
-    // the last column's rise is out of the running where that passed it
-    const uint32_t d = m ^ L.run;
-    if (lo16(d)) L.rose &= 0xFFFF0000u;
-    if (hi16(d)) L.rose &= 0x0000FFFFu;
-    L.run = m;
+    L.run = max2u(L.run, m - 0x00010001u);       // halves are at least the floor: no borrow
 }
 
 // the lane's best (score, column, row) of one half, rows from i0
-template <int R>
-__device__ __forceinline__ uint64_t lane_key(const Lane<R> &L, const Args &a, bool high, int i0) {
-    const uint32_t at = high ? L.atB : L.atA;
-    return best_key((int)(high ? hi16(L.run) : lo16(L.run)) - a.floor, at >> 5, i0 + (at & 31));
+template <int R, bool ENDS>
+__device__ __forceinline__ uint64_t lane_key(const Lane<R> &L, const Args &a, const Flow &f, bool high, int i0) {
+    const int v = (int)(high ? hi16(L.run) : lo16(L.run)) - a.floor;
+    if (!ENDS || v <= 0) return best_key(v, 0, 0);
+    return best_key(v, high ? L.colB : L.colA,
+                    i0 + L.find_row(f.snap + (high ? 32 * words_for(R) : 0), high));
 }
 
 // result of pair p from its best key; the 16-bit pass of the reference drops

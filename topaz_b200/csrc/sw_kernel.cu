@@ -116,7 +116,7 @@ __device__ __forceinline__ void with_rows(int R, F &&f) {
 template <int R, bool ENDS, bool BUILD, bool STRIPED, class PairAt>
 __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int first, int count, int G,
                                           const uint8_t *matT, uint8_t *prof, uint8_t *rings,
-                                          const Stripe &sp, uint64_t &keyA, uint64_t &keyB) {
+                                          uint4 *snap, const Stripe &sp, uint64_t &keyA, uint64_t &keyB) {
     const int lane = threadIdx.x & 31;
     const int lg = 31 - __clz(G), grp = lane >> lg, gl = lane & (G - 1);
     const int iA = first + 2 * grp, iB = iA + 1;
@@ -143,6 +143,7 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
     f.bnd = nullptr;
     f.bnd2 = above && lane == 0 ? sp.ring : nullptr;
     f.bnd_end = N;
+    f.snap = ENDS ? snap + lane : nullptr;
     // columns 0..63, and pad letters where the columns before 0 are read
 #pragma unroll 4
     for (int c = gl; c < 64; c += G) {
@@ -182,8 +183,7 @@ __device__ __forceinline__ void pair_task(const Args &a, PairAt pair_at, int fir
         steps<R, ENDS, false, STRIPED>(L, a, f, k0, min(k0 + 32, nsteps), nullptr,
                                        below && lane == 31 ? sp.rows : nullptr);
     }
-    if (ENDS && L.rose) L.find_row(a, f, nsteps - 1 - gl, L.run, lo16(L.rose), hi16(L.rose));
-    uint64_t kA = lane_key(L, a, false, i0), kB = lane_key(L, a, true, i0);
+    uint64_t kA = lane_key<R, ENDS>(L, a, f, false, i0), kB = lane_key<R, ENDS>(L, a, f, true, i0);
     for (int o = G >> 1; o > 0; o >>= 1) {
         kA = max(kA, __shfl_xor_sync(0xFFFFFFFFu, kA, o));
         kB = max(kB, __shfl_xor_sync(0xFFFFFFFFu, kB, o));
@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
     load_matrix(a, smem);
     __syncwarp();
     const Stripe none{0, 1, nullptr, nullptr};
+    uint4 *snap = a.snap + (size_t)blockIdx.x * snap_words(R1);
     uint64_t kA = 0, kB = 0;
     for (;;) {
         int t = 0;
@@ -250,13 +251,15 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
         auto id = [&](int x) { return ids[x]; };
         if constexpr (R1 == 8) {
             if (b.rows[i] == 4)
-                pair_task<4, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, none, kA, kB);
+                pair_task<4, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, snap,
+                                                 none, kA, kB);
             else
-                pair_task<8, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, none, kA, kB);
+                pair_task<8, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof, rings, snap,
+                                                 none, kA, kB);
         } else {
             with_rows<R0, R1>(b.rows[i], [&](auto r) {
                 pair_task<decltype(r)::value, ENDS, true, false>(a, id, t * per, count, b.lanes[i], smem, prof,
-                                                                 rings, none, kA, kB);
+                                                                 rings, snap, none, kA, kB);
             });
         }
     }
@@ -321,8 +324,8 @@ struct ChunkPair {
 // One chunk with R rows per lane: the profile, the keys sorted, the tasks.
 template <int R, bool ENDS, bool STRIPED>
 __device__ __forceinline__ void run_chunk(const Args &a, const Chunk &ch, const uint8_t *matT, uint8_t *prof,
-                                          uint8_t *rings, uint32_t *keys, uint2 *ring, uint2 *rows,
-                                          int *next) {
+                                          uint8_t *rings, uint32_t *keys, uint4 *snap, uint2 *ring,
+                                          uint2 *rows, int *next) {
     const int lane = threadIdx.x & 31;
     const int n = ch.pairs, G = STRIPED ? 32 : ch.lanes, stripes = STRIPED ? ch.stripes : 1;
     int np = 1;
@@ -355,20 +358,20 @@ __device__ __forceinline__ void run_chunk(const Args &a, const Chunk &ch, const 
         for (int st = 0; st < stripes; ++st) {
             const Stripe sp{st, stripes, ring, rows};
             pair_task<R, ENDS, false, STRIPED>(a, id, t * per, n, G, nullptr, prof + st * profile_bytes(R), rings,
-                                               sp, kA, kB);
+                                               snap, sp, kA, kB);
         }
     }
 }
 
 template <int R, bool ENDS, bool STRIPED>
 __device__ __forceinline__ void run_chunk_rows(const Args &a, const Chunk &ch, const uint8_t *matT, uint8_t *prof,
-                                               uint8_t *rings, uint32_t *keys, uint2 *ring, uint2 *rows,
-                                               int *next) {
+                                               uint8_t *rings, uint32_t *keys, uint4 *snap, uint2 *ring,
+                                               uint2 *rows, int *next) {
     if constexpr (R == kMaxR) {
-        run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
+        run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, snap, ring, rows, next);
     } else {
-        if (ch.rows <= R) run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
-        else run_chunk_rows<R < 8 ? 8 : R + 1, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, ring, rows, next);
+        if (ch.rows <= R) run_chunk<R, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, snap, ring, rows, next);
+        else run_chunk_rows<R < 8 ? 8 : R + 1, ENDS, STRIPED>(a, ch, matT, prof, rings, keys, snap, ring, rows, next);
     }
 }
 
@@ -387,6 +390,7 @@ __global__ void __launch_bounds__(kQmWarps * 32, 2) sw_query_kernel(const __grid
     uint32_t *keys = reinterpret_cast<uint32_t *>(prof + g.profile + kQmWarps * g.ring +
                                                   (STRIPED ? kQmWarps * kBndCols * 8 : 0));
     uint2 *rows = g.bnd + (int64_t)(blockIdx.x * kQmWarps + warp) * g.bnd_cols;
+    uint4 *snap = a.snap + (size_t)(blockIdx.x * kQmWarps + warp) * snap_words(kMaxR);
     __shared__ int s_chunk, s_next;
     load_matrix(a, smem);
     for (;;) {
@@ -398,7 +402,7 @@ __global__ void __launch_bounds__(kQmWarps * 32, 2) sw_query_kernel(const __grid
         __syncthreads();
         if (s_chunk >= g.count) break;
         const Chunk ch = g.chunks[s_chunk];
-        run_chunk_rows<STRIPED ? 17 : 4, ENDS, STRIPED>(a, ch, smem, prof, rings, keys, bnd, rows, &s_next);
+        run_chunk_rows<STRIPED ? 17 : 4, ENDS, STRIPED>(a, ch, smem, prof, rings, keys, snap, bnd, rows, &s_next);
     }
 }
 
@@ -424,7 +428,7 @@ template <int R, bool ENDS>
 __device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, int ql, const int8_t *s,
                                                 int sl, int group, int W, int wg, const uint8_t *matT,
                                                 uint8_t *prof, uint16_t *ring, const uint32_t *above,
-                                                uint32_t *below) {
+                                                uint32_t *below, uint4 *snap) {
     const int lane = threadIdx.x & 31;
     const int i0 = (wg * 64 + lane) * R, i1 = i0 + 32 * R;
     build_profile<R>(a, q, ql, i0, matT, prof + lane * 4);
@@ -439,6 +443,7 @@ __device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, 
     f.bnd = lane == 0 ? above : nullptr;
     f.bnd2 = nullptr;
     f.bnd_end = sl;
+    f.snap = ENDS ? snap + lane : nullptr;
 #pragma unroll
     for (int c = lane; c < 64; c += 32) {
         ring[c] = letter_offset<R>(a, s, sl, c);
@@ -465,8 +470,7 @@ __device__ __forceinline__ uint64_t stripe_task(const Args &a, const int8_t *q, 
         }
         group_sync(group, W);
     }
-    if (ENDS && L.rose) L.find_row(a, f, 32 * nblk - 1 - lane, L.run, lo16(L.rose), hi16(L.rose));
-    uint64_t key = max(lane_key(L, a, false, i0), lane_key(L, a, true, i1));
+    uint64_t key = max(lane_key<R, ENDS>(L, a, f, false, i0), lane_key<R, ENDS>(L, a, f, true, i1));
     for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, o));
     return key;
 }
@@ -475,9 +479,9 @@ template <bool ENDS, int RMAX>
 __device__ __forceinline__ uint64_t stripe_rows(int R, const Args &a, const int8_t *q, int ql,
                                                 const int8_t *s, int sl, int group, int W, int wg,
                                                 const uint8_t *matT, uint8_t *prof, uint16_t *ring,
-                                                const uint32_t *above, uint32_t *below) {
+                                                const uint32_t *above, uint32_t *below, uint4 *snap) {
 #define TPZ_STRIPE(r) \
-    stripe_task<r, ENDS>(a, q, ql, s, sl, group, W, wg, matT, prof, ring, above, below)
+    stripe_task<r, ENDS>(a, q, ql, s, sl, group, W, wg, matT, prof, ring, above, below, snap)
     if (R <= 4) return TPZ_STRIPE(4);
     if (RMAX == 8 || R <= 8) return TPZ_STRIPE(8);
     if constexpr (RMAX > 8) {
@@ -490,9 +494,10 @@ __device__ __forceinline__ uint64_t stripe_rows(int R, const Args &a, const int8
 #undef TPZ_STRIPE
 }
 
-// one warp's shared memory: two profiles, the letter ring, the boundary ring
+// one warp's shared memory: two profiles, the letter ring, the boundary ring,
+// and (up to 8 rows: what one pair per launch has) the stored columns
 __host__ __device__ constexpr int stripe_warp_bytes(int RMAX) {
-    return 2 * profile_bytes(RMAX) + 2 * kRingCols + 4 * kRingCols;
+    return 2 * profile_bytes(RMAX) + 2 * kRingCols + 4 * kRingCols + (RMAX <= 8 ? 16 * snap_words(RMAX) : 0);
 }
 __host__ __device__ constexpr int stripe_smem(int RMAX, int warps) {
     return kMatBytes + warps * stripe_warp_bytes(RMAX);
@@ -519,6 +524,8 @@ __global__ void __launch_bounds__(32 * kLongWarps) sw_stripe_kernel(const __grid
     uint32_t *below = reinterpret_cast<uint32_t *>(ring + kRingCols);
     const uint32_t *above = reinterpret_cast<const uint32_t *>(
         reinterpret_cast<const uint8_t *>(below) - stripe_warp_bytes(RMAX));
+    uint4 *snap = RMAX <= 8 ? reinterpret_cast<uint4 *>(below + kRingCols)
+                            : a.snap + (size_t)(blockIdx.x * kLongWarps + warp) * snap_words(RMAX);
     bool ready = false;
     for (int i = 0; i < b.n; ++i) {
         const int start = a.rinfo[2 * b.bin[i]], count = a.rinfo[2 * b.bin[i] + 1];
@@ -538,7 +545,7 @@ __global__ void __launch_bounds__(32 * kLongWarps) sw_stripe_kernel(const __grid
             const int ql = a.qlen[p];
             const uint64_t key = stripe_rows<ENDS, RMAX>(
                 (ql + 64 * W - 1) / (64 * W), a, a.q + a.qoff[p], ql, a.s + a.soff[p], a.slen[p], group,
-                W, wg, smem, prof, ring, wg > 0 ? above : nullptr, wg + 1 < W ? below : nullptr);
+                W, wg, smem, prof, ring, wg > 0 ? above : nullptr, wg + 1 < W ? below : nullptr, snap);
             if (lane == 0) s_key[warp] = key;
             group_sync(group, W);
             if (wg == 0 && lane == 0) {
@@ -566,7 +573,8 @@ __global__ void __launch_bounds__(64) sw_one_kernel(const __grid_constant__ Args
     __syncthreads();
     const uint64_t key = stripe_rows<true, 8>((qlen + 64 * W - 1) / (64 * W), a, a.q, qlen, a.s, slen, 0, W,
                                               warp, smem, prof, ring, warp > 0 ? above : nullptr,
-                                              warp + 1 < W ? below : nullptr);
+                                              warp + 1 < W ? below : nullptr,
+                                              reinterpret_cast<uint4 *>(below + kRingCols));
     if ((threadIdx.x & 31) == 0) s_key[warp] = key;
     __syncthreads();
     if (threadIdx.x == 0) write_result(a, 0, W > 1 ? max(s_key[0], s_key[1]) : s_key[0], true);
@@ -831,11 +839,30 @@ constexpr int64_t kSmallBatch = 1024;
 // task counter per row bin, then the sorted pair ids
 constexpr size_t kBinWords = 2 * (size_t)kBins + 3 * kRBins;
 
+// blocks of a launch: no more than pairs
+static unsigned grid_of(int blocks_per_sm, int64_t n) {
+    return (unsigned)std::min<int64_t>((int64_t)sm_count() * blocks_per_sm, std::max<int64_t>(n, 1));
+}
+
+// uint4 words for the columns that launch_batch's kernels store, for the
+// largest kernel (they follow each other) or all (they run side by side)
+static size_t batch_snap_words(const Kernels *k, int64_t n, int max_qlen, bool side_by_side) {
+    size_t sum = 0, most = 0;
+    auto add = [&](size_t w) { sum += w; most = std::max(most, w); };
+    if (max_qlen > kStripeRows)
+        add((size_t)grid_of(k->stripe32_blocks[1], n) * kLongWarps * snap_words(kMaxR));
+    if (n > kSmallBatch)
+        for (int i = 0; i < kBinKernels; ++i)
+            add((size_t)grid_of(k->bin_blocks[1][i], n) * snap_words(k->set[i].rows[0]));
+    return side_by_side ? sum : most;
+}
+
 // Bins the pairs (all of them, or the n ids of `list`) in ws and launches the
 // kernels that align them, over the auxiliary streams x so that each
 // kernel's tail overlaps the next one (null: all on st).
 static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const int32_t *list,
-                        int32_t *ws, int max_qlen, bool ends, cudaStream_t st, int64_t &launches) {
+                        int32_t *ws, uint4 *snap, int max_qlen, bool ends, cudaStream_t st,
+                        int64_t &launches) {
     const int nsm = sm_count();
     int32_t *counts = ws, *cursor = counts + kBins, *rinfo = cursor + kBins;
     int32_t *next_task = rinfo + 2 * kRBins, *sorted = ws + kBinWords;
@@ -855,13 +882,14 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
     }
     int at = 0;
     auto next_stream = [&]() { return x ? x->aux[at++ % kAuxStreams] : st; };
-    // no launch wants more blocks than pairs
-    auto grid = [&](int blocks) { return (unsigned)std::min<int64_t>((int64_t)nsm * blocks, std::max<int64_t>(n, 1)); };
+    auto grid = [&](int blocks) { return grid_of(blocks, n); };
+    a.snap = ends ? snap : nullptr;
     if (max_qlen > kStripeRows) {
         const StripeSet s{3, {kLongBin + 2, kLongBin + 1, kLongBin}, {4, 2, 1}, {4, 4, 4}};
         k->stripe32[e]<<<grid(k->stripe32_blocks[e]), 32 * kLongWarps, stripe_smem(32, kLongWarps),
                          next_stream()>>>(a, s);
         ++launches;
+        if (ends && x) a.snap += (size_t)grid(k->stripe32_blocks[e]) * kLongWarps * snap_words(kMaxR);
     }
     if (small_batch) {
         const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {2, 2, 0}};
@@ -872,6 +900,7 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
         for (int i = 0; i < kBinKernels; ++i) {
             k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
             ++launches;
+            if (ends && x) a.snap += (size_t)grid(k->bin_blocks[e][i]) * snap_words(k->set[i].rows[0]);
         }
     }
     // the join comes after every launch, also on an error, so that the
@@ -915,8 +944,10 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
     if (rc || (rc = streams(&x, lane))) return rc;
     keep_pool_memory();
     if (subset) n = nsub;
-    int32_t *ws = nullptr;
-    TPZ_CUDA(cudaMallocAsync((void **)&ws, sizeof(int32_t) * (kBinWords + (size_t)n), st));
+    // workspace: the stored columns, then the bins and the sorted ids
+    const size_t snaps = score_only ? 0 : batch_snap_words(k, n, TPZ_SW_MAX_QLEN, true);
+    uint4 *ws = nullptr;
+    TPZ_CUDA(cudaMallocAsync((void **)&ws, sizeof(uint4) * snaps + sizeof(int32_t) * (kBinWords + (size_t)n), st));
     Args a;
     pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
     set_scoring(a, mat, go, ge);
@@ -926,7 +957,7 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
         memcpy(a.xs, xs, 128);
     }
     int64_t launches = 0;
-    rc = launch_batch(k, x, a, n, subset, ws, TPZ_SW_MAX_QLEN, !score_only, st, launches);
+    rc = launch_batch(k, x, a, n, subset, (int32_t *)(ws + snaps), ws, TPZ_SW_MAX_QLEN, !score_only, st, launches);
     TPZ_CUDA(cudaFreeAsync(ws, st));
     if (rc) return rc;
     g_last_launches = launches;
@@ -1031,7 +1062,7 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
     int64_t launches = 0;
     struct Launch { QmArgs g; unsigned grid; int smem, striped; };
     std::vector<Launch> todo;
-    int64_t bnd_words = 0;
+    int64_t bnd_words = 0, snaps = 0;   // uint2 of boundary rows, uint4 of stored columns
     at = hbytes;
     for (int cls = 0; cls < 5; ++cls) {
         const std::vector<Chunk> &c = chunks[cls];
@@ -1057,20 +1088,23 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
             l.g.bnd_cols = std::max(max_slen, 1);
             const int64_t per_block = kQmWarps * l.g.bnd_cols;
             l.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(l.grid, ((int64_t)1 << 27) / per_block));
-            bnd_words += per_block * l.grid;
+            bnd_words += (per_block * l.grid + 1) & ~(int64_t)1;
         }
+        if (e) snaps += (int64_t)l.grid * kQmWarps * snap_words(kMaxR);
         todo.push_back(l);
     }
-    if (bnd_words > 0) {
-        if (cudaMallocAsync((void **)&dbnd, sizeof(uint2) * (size_t)bnd_words, st)) {
+    uint4 *dsnap = nullptr;
+    if (bnd_words + snaps > 0) {
+        if (cudaMallocAsync((void **)&dbnd, sizeof(uint2) * (size_t)bnd_words + sizeof(uint4) * (size_t)snaps, st)) {
             drop();
             return cuda_fail(cudaGetLastError(), "batch_device_grouped boundary rows");
         }
+        dsnap = reinterpret_cast<uint4 *>(dbnd + bnd_words);
         bnd_words = 0;
         for (Launch &l : todo) {
             if (!l.striped) continue;
             l.g.bnd = dbnd + bnd_words;
-            bnd_words += kQmWarps * l.g.bnd_cols * l.grid;
+            bnd_words += (kQmWarps * l.g.bnd_cols * l.grid + 1) & ~(int64_t)1;
         }
     }
     if (!todo.empty()) {
@@ -1079,6 +1113,8 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         int stream = 0;
         for (size_t i = todo.size(); i-- > 0;) {
             const Launch &l = todo[i];
+            a.snap = dsnap;
+            if (e) dsnap += (size_t)l.grid * kQmWarps * snap_words(kMaxR);
             k->qm[e][l.striped]<<<l.grid, kQmWarps * 32, l.smem, x->aux[stream++ % kAuxStreams]>>>(a, l.g);
             ++launches;
         }
@@ -1408,7 +1444,11 @@ static_assert((int64_t)kNoAllocMaxQlen * TPZ_SW_NOALLOC_MAX_ENTRY < kBig &&
               "TPZ_SW_NOALLOC_MAX_ENTRY");
 
 // One copy per device that loads the library, kept until the process exits.
-static __device__ __align__(256) int32_t g_noalloc_scratch[kBinWords + (size_t)kNoAllocMaxPairs];
+// Behind the bins: the columns stored by the largest by-pair kernel, for the
+// SMs and blocks per SM this library is built for.
+constexpr size_t kNoAllocBins = (kBinWords + (size_t)kNoAllocMaxPairs + 3) & ~(size_t)3;
+constexpr size_t kNoAllocSnaps = 148 * 4 * (size_t)snap_words(kMaxR);
+static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocBins + 4 * kNoAllocSnaps];
 
 // Device address of the static scratch array of the current device (host
 // code cannot use the array's name as a device pointer).
@@ -1472,9 +1512,14 @@ extern "C" int tpz_sw_batch_device_noalloc(int64_t n, const int8_t *q, const int
     int32_t *ws = nullptr;
     int rc = kernels(&k);
     if (rc || (rc = noalloc_scratch(&ws))) return rc;
+    if (batch_snap_words(k, n, kNoAllocMaxQlen, false) > kNoAllocSnaps) {
+        tpz::set_error("tpz_sw_batch_device_noalloc: more SMs than the fixed scratch is sized for");
+        return TPZ_E_DEVICE;
+    }
     Args a;
     pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
     set_scoring(a, mat625_host, gap_open, gap_extend);
     int64_t launches = 0;
-    return launch_batch(k, nullptr, a, n, nullptr, ws, kNoAllocMaxQlen, true, (cudaStream_t)stream, launches);
+    return launch_batch(k, nullptr, a, n, nullptr, ws, (uint4 *)(ws + kNoAllocBins), kNoAllocMaxQlen, true,
+                        (cudaStream_t)stream, launches);
 }
