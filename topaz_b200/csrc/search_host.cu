@@ -418,48 +418,62 @@ struct RankTables {
 };
 
 int rank_tables(const tpz_search_opts *o, RankTables *t) {
+    // bits / ln 2 of each score, as tpz_karlin computes it
     std::vector<double> b(kRawRanks);
-    double ev;
+    const double logk = log(o->k);
+    bool rising = true;
     for (int r = 0; r < kRawRanks; ++r) {
-        tpz_karlin(1, 1, 1, o->lambda, o->k, o->H, r, &b[r], &ev);
+        b[r] = (o->lambda * r - logk) / M_LN2;
         if (b[r] != b[r]) { tpz::set_error("tpz_search_batch: bitscores are NaN (check lambda, k)"); return TPZ_E_ARG; }
         // two scores sharing a bitscore must share the E-value too (the cut
         // is taken per rank)
-        if (r > 0 && b[r] == b[r - 1] && o->lambda * r - log(o->k) != o->lambda * (r - 1) - log(o->k)) {
+        if (r > 0 && b[r] == b[r - 1] && o->lambda * r - logk != o->lambda * (r - 1) - logk) {
             tpz::set_error("tpz_search_batch: lambda too small to rank scores by bitscore");
             return TPZ_E_ARG;
         }
+        rising = rising && (r == 0 || b[r] >= b[r - 1]);
     }
+    // the distinct bitscores and 0, ascending
     std::vector<double> u(b);
-    u.push_back(0.0);
-    std::sort(u.begin(), u.end());
+    if (rising) u.insert(std::lower_bound(u.begin(), u.end(), 0.0), 0.0);
+    else {
+        u.push_back(0.0);
+        std::sort(u.begin(), u.end());
+    }
     u.erase(std::unique(u.begin(), u.end()), u.end());
     auto rank = [&](double v) { return (int32_t)(std::lower_bound(u.begin(), u.end(), v) - u.begin()); };
     t->rank_of_raw.resize(kRawRanks);
     std::vector<int32_t> rep(u.size(), -1);
     int32_t minr = INT32_MAX;
+    int32_t k = 0;
     for (int r = 0; r < kRawRanks; ++r) {
-        const int32_t k = rank(b[r]);
+        if (rising) while (u[k] != b[r]) ++k;      // the ranks rise with the scores
+        else k = rank(b[r]);
         t->rank_of_raw[r] = k;
         if (rep[k] < 0) rep[k] = r;
         minr = std::min(minr, k);
     }
-    for (size_t k = 0; k < rep.size(); ++k)
-        if (rep[k] >= 0) { t->reps.push_back((int32_t)k); t->rep_raw.push_back(rep[k]); }
+    for (size_t i = 0; i < rep.size(); ++i)
+        if (rep[i] >= 0) { t->reps.push_back((int32_t)i); t->rep_raw.push_back(rep[i]); }
     t->rank_low = rank(0.0);
     t->low_last = t->rank_low < minr;
     t->low_pass = 1000.0 <= o->max_evalue;
     return TPZ_OK;
 }
 
-// lowest rank whose E-value passes for a query of length qlen (INT32_MAX: none)
+// lowest rank whose E-value passes for a query of length qlen (INT32_MAX:
+// none); tpz_karlin's E-value, its part that the score does not enter once
 int32_t rank_min_for(const RankTables &t, const tpz_search_opts *o, int32_t qlen) {
+    const double logk = log(o->k);
+    const double correction = log(o->k * qlen * o->db_size) / o->H;
+    const double corrected_q = fmax(qlen - correction, 1.0);
+    const double corrected_db = fmax(o->db_size - (correction * o->db_proteins), 1.0);
     int64_t lo = 0, hi = (int64_t)t.reps.size();
     while (lo < hi) {
         const int64_t mid = lo + (hi - lo) / 2;
-        double bits, ev;
-        tpz_karlin(qlen, o->db_size, o->db_proteins, o->lambda, o->k, o->H,
-                   t.rep_raw[mid], &bits, &ev);
+        const double bits = o->lambda * t.rep_raw[mid] - logk;
+        double ev = corrected_q * corrected_db * exp(-bits);
+        ev = ev > 1.0e-180 ? ev : 0.0;
         if (ev <= o->max_evalue) hi = mid; else lo = mid + 1;
     }
     return lo < (int64_t)t.reps.size() ? t.reps[lo] : INT32_MAX;
