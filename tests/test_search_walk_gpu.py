@@ -3,7 +3,8 @@ pops that cross blocks of chain elements (rows 8, 32, 64, ... on), rises of
 hits already listed, capacities around a batch of 32 pops, evictions at one
 and over several scores, stops at -S inside a batch, and cursor counts of
 every shared-memory class up to the one that spills -- pop by pop against
-the oracle, on a database of protein families (long runs of similar rows)."""
+the oracle, on a database of protein families (long runs of similar rows);
+and the extensions they rest on, at every kind of end."""
 import numpy as np
 import pytest
 
@@ -65,3 +66,52 @@ def test_every_pop_and_hit(cuda, family_db, seeds, aligns, num_hits):
         longest = max(longest, npops)
     if seeds == 300000:
         assert r["refill_elems"] > 0 and longest > 2000
+
+
+@pytest.mark.parametrize("name,scale", [("BLOSUM62", 1), ("PAM30", 1), ("BLOSUM62", 11)])
+def test_extensions_at_every_end(cuda, family_db, name, scale):
+    # window ends at the query's start and end, the text's start and end,
+    # protein ends, 32-byte rounds and the 128-residue limit; entries up to 121
+    db, qs = family_db
+    mat = (synth.matrix(name).astype(np.int64) * scale).astype(np.int8)
+    ix, orc = native.Index(db), oracle.liboracle()
+    rng = np.random.default_rng(3)
+    first = [int(np.flatnonzero(db.SA == p)[0]) for p in (0, 1, 31, 32, 33, db.Tsize - 2, db.Tsize - 34)]
+    qof, off, row = [], [], []
+    for qi, q in enumerate(qs):
+        ends = [i for i in (0, 1, 2, 31, 32, 33, 34, 127, 128, 129, len(q) // 2) if i < len(q)]
+        ends += [len(q) - 1 - i for i in (0, 1, 31, 32, 33, 127, 128) if i < len(q)]
+        for i in ends:
+            near = ix.sa_search([q[i:]])[0]
+            rows = first + [min(max(int(near) + d, 0), db.Tsize - 1) for d in (-2, -1, 0, 1)]
+            rows += rng.integers(0, db.Tsize, 3).tolist()
+            for r in rows:
+                qof.append(qi)
+                off.append(i)
+                row.append(r)
+    sc, ln = ix.sa_hsp(qs, qof, off, row, mat)
+    sub = ab.internal_to_index(np.arange(65, 90, dtype=np.uint8)).astype(np.int64)
+    for k in range(len(row)):
+        want = _extension(db.T, int(db.SA[row[k]]), qs[qof[k]], off[k], mat, sub)
+        assert (sc[k], ln[k]) == want, (qof[k], off[k], row[k])
+
+
+def _extension(T, at, q, off, mat, sub):
+    """sa_hsp of one pair of positions, residue by residue."""
+    if T[at] != q[off]:
+        return 0, -1
+
+    def walk(steps, first):
+        run = best = arg = 0
+        for i in range(first, steps):
+            t, c = (T[at + i], q[off + i]) if first == 0 else (T[at - i], q[off - i])
+            if t == 10:
+                break
+            run += int(mat[sub[t - 65], sub[c - 65]])
+            if run >= best:
+                best, arg = run, i
+        return best, arg
+
+    r, i = walk(min(len(T) - at, len(q) - off, 128), 0)
+    l, j = walk(min(at, off, 128), 1)
+    return r + l, i + j

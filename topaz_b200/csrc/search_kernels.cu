@@ -104,18 +104,51 @@ __device__ __forceinline__ void load32(const uint8_t *p, uint32_t (&w)[8]) {
     for (int k = 0; k < 8; ++k) w[k] = __funnelshift_r(r[k], r[k + 1], sh);
 }
 
-// byte k (a compile-time index after unrolling) of a load32 window
-__device__ __forceinline__ uint32_t byte_of(const uint32_t (&w)[8], int k) {
-    return (w[k >> 2] >> (8 * (k & 3))) & 0xFFu;
+// Extension table of a block (shared memory), by query letter and text
+// letter (the low 5 bits of the byte, 1..25): 256 * score + 1, and in row and
+// column 0 a value that no extension makes up for.  A running sum of entries
+// is 256 * score + index, so one addition and one maximum per residue keep
+// the best score with the last index that reached it, and a residue past an
+// end counts as the end.  Lanes that extend one query offset read one row of
+// 32 words: different banks for different text letters.
+constexpr int kExtWords = 32 * 32;
+constexpr int kExtEnd = -(1 << 23);        // 128 entries of 127 * 256 stay below its half
+
+__device__ __forceinline__ void load_ext(int32_t *ext, const int8_t *sub) {
+    for (int i = threadIdx.x; i < kExtWords; i += blockDim.x) {
+        const int q = i >> 5, t = i & 31;
+        const bool in = q >= 1 && q <= 25 && t >= 1 && t <= 25;
+        ext[i] = in ? 256 * sub[(t - 1) * 25 + (q - 1)] + 1 : kExtEnd;
+    }
+}
+
+// bytes of a word below / from `n` (any int)
+__device__ __forceinline__ uint32_t low_bytes(int n) {
+    return n >= 4 ? ~0u : n <= 0 ? 0u : (1u << (8 * n)) - 1u;
+}
+
+// table byte offsets (q * 128 + t * 4) of bytes 0, 2 and 1, 3 of a text and a
+// query word, two to a word; a '\n' (bit 6 clear) has text letter 0
+__device__ __forceinline__ void ext_offsets(uint32_t t, uint32_t q, uint32_t &even, uint32_t &odd) {
+    t &= ((t >> 6) & 0x01010101u) * 0x1Fu;
+    q &= 0x1F1F1F1Fu;
+    even = (q & 0x00FF00FFu) * 128u + (t & 0x00FF00FFu) * 4u;
+    odd = (q >> 8 & 0x00FF00FFu) * 128u + (t >> 8 & 0x00FF00FFu) * 4u;
+}
+
+__device__ __forceinline__ int32_t ext_at(const int32_t *ext, uint32_t off) {
+    return *reinterpret_cast<const int32_t *>(reinterpret_cast<const uint8_t *>(ext) + off);
 }
 
 // sa_hsp (src/search.c:99-190) at text position idx for query offset off.
 // Returns the length (-1 when the first symbols differ; score untouched then).
 // The windows (up to 128 bytes each side) are read 32 bytes per round trip
-// into registers; the running sums walk them in the reference's order and
-// stop at the first '\n' exactly as its byte loop does.
+// into registers and walked in the reference's order; its stops -- a '\n', an
+// end of query or text -- are table entries.  Bound: instruction issue.  (Byte
+// compares, a matrix look-up in global memory and two selects per residue
+// took 4.4 ms for the 20.8 M chain elements of a 1000-query search.)
 __device__ int hsp_at(const DevIndex &ix, int64_t idx, const uint8_t *Q, int qlen, int off,
-                      const int8_t *sub, int *score) {
+                      const int32_t *ext, int *score) {
     const uint8_t *t = ix.T + idx;
     const uint8_t *q = Q + off;
     int64_t mr = ix.Tsize - idx;
@@ -125,48 +158,53 @@ __device__ int hsp_at(const DevIndex &ix, int64_t idx, const uint8_t *Q, int qle
     load32(t, tw);
     load32(q, qw);
     if ((tw[0] & 0xFFu) != (qw[0] & 0xFFu)) return -1;
-    int run = 0, best_r = 0, arg_r = 0;
-    bool stop = false;
-    for (int i0 = 0; i0 < (int)mr && !stop; i0 += 32) {
-        if (i0 > 0) { load32(t + i0, tw); load32(q + i0, qw); }
+    int sum = -1, best_r = 0;
+    for (int i0 = 0; i0 < (int)mr; i0 += 32) {
+        if (i0 > 0) {
+            if (sum < kExtEnd / 2) break;
+            load32(t + i0, tw);
+            load32(q + i0, qw);
+        }
+        if (i0 + 32 > (int)mr) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            const uint32_t c = byte_of(tw, k);
-            if (!stop && i0 + k < (int)mr) {
-                if (c == '\n') {
-                    stop = true;
-                } else {
-                    run += sub[(c - 'A') * 25 + (byte_of(qw, k) - 'A')];
-                    if (run >= best_r) { best_r = run; arg_r = i0 + k; }
-                }
-            }
+            for (int w = 0; w < 8; ++w) qw[w] &= low_bytes((int)mr - i0 - 4 * w);
+        }
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            uint32_t even, odd;
+            ext_offsets(tw[w], qw[w], even, odd);
+            sum += ext_at(ext, even & 0xFFFFu); best_r = max(best_r, sum);
+            sum += ext_at(ext, odd & 0xFFFFu); best_r = max(best_r, sum);
+            sum += ext_at(ext, even >> 16); best_r = max(best_r, sum);
+            sum += ext_at(ext, odd >> 16); best_r = max(best_r, sum);
         }
     }
     int64_t ml = idx < off ? idx : off;
     if (ml > 128) ml = 128;
-    int best_l = 0, arg_l = 0;
-    run = 0;
-    stop = false;
+    int best_l = 0;
+    sum = 0;
     // left: i = 1 .. ml-1 reads t[-i]; a round loads the 32 bytes that end at
     // t[-i0], so t[-(i0 + k)] is byte 31 - k
-    for (int i0 = 1; i0 < (int)ml && !stop; i0 += 32) {
+    for (int i0 = 1; i0 < (int)ml; i0 += 32) {
+        if (sum < kExtEnd / 2) break;
         load32(t - (i0 + 31), tw);
         load32(q - (i0 + 31), qw);
+        if (i0 + 32 > (int)ml) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            const uint32_t c = byte_of(tw, 31 - k);
-            if (!stop && i0 + k < (int)ml) {
-                if (c == '\n') {
-                    stop = true;
-                } else {
-                    run += sub[(c - 'A') * 25 + (byte_of(qw, 31 - k) - 'A')];
-                    if (run >= best_l) { best_l = run; arg_l = i0 + k; }
-                }
-            }
+            for (int w = 0; w < 8; ++w) qw[w] &= ~low_bytes(32 - ((int)ml - i0) - 4 * w);
+        }
+#pragma unroll
+        for (int w = 7; w >= 0; --w) {
+            uint32_t even, odd;
+            ext_offsets(tw[w], qw[w], even, odd);
+            sum += ext_at(ext, odd >> 16); best_l = max(best_l, sum);
+            sum += ext_at(ext, even >> 16); best_l = max(best_l, sum);
+            sum += ext_at(ext, odd & 0xFFFFu); best_l = max(best_l, sum);
+            sum += ext_at(ext, even & 0xFFFFu); best_l = max(best_l, sum);
         }
     }
-    *score = best_l + best_r;
-    return arg_l + arg_r;
+    *score = (best_l >> 8) + (best_r >> 8);
+    return (best_l & 255) + (best_r & 255);
 }
 
 // lower bound of the suffix P[0, m) (letters only) over the whole SA
@@ -236,6 +274,9 @@ __global__ void lb_build_kernel(const uint8_t *T, int64_t Tsize, const int64_t *
 // bound row with direction +1, slot 1 the row before with direction -1
 // (len < min_hit_length marks a slot that is not inserted).
 __global__ void seed_kernel(DevIndex ix, SeedArgs a) {
+    __shared__ int32_t ext[kExtWords];
+    load_ext(ext, a.sub);
+    __syncthreads();
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < a.npos;
          g += (int64_t)gridDim.x * blockDim.x) {
         // query of this position
@@ -259,13 +300,13 @@ __global__ void seed_kernel(DevIndex ix, SeedArgs a) {
             } else {
                 int sc = 0;
                 const int64_t t0 = ix.SA[pos];
-                int ln = hsp_at(ix, t0, Q, qlen, i, a.sub, &sc);
+                int ln = hsp_at(ix, t0, Q, qlen, i, ext, &sc);
                 c0.row = pos; c0.score = sc; c0.len = ln;
                 c0.prot = (int32_t)protein_of(ix, t0);
                 if (pos != 0) {
                     sc = 0;
                     const int64_t t1 = ix.SA[pos - 1];
-                    ln = hsp_at(ix, t1, Q, qlen, i, a.sub, &sc);
+                    ln = hsp_at(ix, t1, Q, qlen, i, ext, &sc);
                     c1.row = pos - 1; c1.score = sc; c1.len = ln;
                     c1.prot = (int32_t)protein_of(ix, t1);
                 }
@@ -367,12 +408,15 @@ __global__ void hsp_batch_kernel(DevIndex ix, const uint8_t *qcat, const int64_t
                                  const int32_t *qlen, const int32_t *query_of, const int32_t *off,
                                  const int64_t *row, int64_t n, const int8_t *sub, int32_t *score,
                                  int32_t *len) {
+    __shared__ int32_t ext[kExtWords];
+    load_ext(ext, sub);
+    __syncthreads();
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n;
          g += (int64_t)gridDim.x * blockDim.x) {
         const int q = query_of[g];
         const int64_t r = row[g];
         int sc = 0, ln = -2;
-        if (r >= 0 && r < ix.sa_rows) ln = hsp_at(ix, ix.SA[r], qcat + qoff[q], qlen[q], off[g], sub, &sc);
+        if (r >= 0 && r < ix.sa_rows) ln = hsp_at(ix, ix.SA[r], qcat + qoff[q], qlen[q], off[g], ext, &sc);
         score[g] = sc;
         len[g] = ln;
     }
@@ -410,14 +454,14 @@ __device__ __forceinline__ int elem_len(uint32_t e) { return (int)(int16_t)(e >>
 // the protein of that row (db_index, the hitlist's key), -1 with a marker.
 __device__ __forceinline__ uint32_t chain_elem(const DevIndex &ix, int64_t row, int dir, int step,
                                                const uint8_t *Q, int qlen, int off,
-                                               const int8_t *sub, int32_t *prot) {
+                                               const int32_t *ext, int32_t *prot) {
     const int64_t nr = row + (int64_t)dir * step;
     *prot = -1;
     if (nr < 0 || nr >= 8 * ix.Tsize) return pack_elem(0, kLenEnd);
     if (nr >= ix.sa_rows) return pack_elem(0, kLenFault);
     int sc = 0;
     const int64_t pos = ix.SA[nr];
-    const int ln = hsp_at(ix, pos, Q, qlen, off, sub, &sc);
+    const int ln = hsp_at(ix, pos, Q, qlen, off, ext, &sc);
     *prot = (int32_t)protein_of(ix, pos);
     return pack_elem(sc, ln);
 }
@@ -427,6 +471,9 @@ __device__ __forceinline__ uint32_t chain_elem(const DevIndex &ix, int64_t row, 
 // them ready.  Elements a cursor never reaches are computed and not used.
 __global__ void chain_kernel(DevIndex ix, SeedArgs a, int min_hit_length, uint32_t *cache,
                              int32_t *cprot) {
+    __shared__ int32_t ext[kExtWords];
+    load_ext(ext, a.sub);
+    __syncthreads();
     const int64_t total = 2 * a.npos * kChain;
     for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
          x += (int64_t)gridDim.x * blockDim.x) {
@@ -442,7 +489,7 @@ __global__ void chain_kernel(DevIndex ix, SeedArgs a, int min_hit_length, uint32
         }
         int32_t pr;
         cache[c * kChainSlots + e] = chain_elem(ix, cu.row, cu.dir, e + 1, a.qcat + a.qoff[lo],
-                                                a.qlen[lo], cu.off, a.sub, &pr);
+                                                a.qlen[lo], cu.off, ext, &pr);
         cprot[c * kChainSlots + e] = pr;
     }
 }
@@ -884,9 +931,9 @@ constexpr int kScoreWords = kSMax / 64;
 constexpr int16_t kNotQueued = -1;      // too short, or past the array: the cursor is not pushed
 constexpr int16_t kFault = -2;          // row past the zero-filled SA page
 static_assert(kChain == 32 && kChainSlots == 64, "blocks of 32 elements in two halves");
-// bitmap, stack heads and pops of a batch in front of the cursors
+// bitmap, stack heads, pops of a batch and extension table in front of the cursors
 constexpr int kPops = 128;              // ring of popped rows
-constexpr int kWalkFixed = 8 * kScoreWords + 2 * kHeadSmem + kPops * (int)sizeof(CurState);
+constexpr int kWalkFixed = 8 * kScoreWords + 2 * kHeadSmem + kPops * (int)sizeof(CurState) + 4 * kExtWords;
 static_assert(kWalkFixed % 16 == 0, "cursor state alignment");
 
 __device__ __forceinline__ int16_t push_code(uint32_t elem, int minlen) {
@@ -914,6 +961,8 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
     uint64_t *bits = reinterpret_cast<uint64_t *>(smem);
     int16_t *head_low = reinterpret_cast<int16_t *>(bits + kScoreWords);
     CurState *pops = reinterpret_cast<CurState *>(head_low + kHeadSmem);     // rows on, cursor
+    int32_t *ext = reinterpret_cast<int32_t *>(pops + kPops);
+    load_ext(ext, a.sub);
     int16_t *buf = reinterpret_cast<int16_t *>(SPILL ? a.spill + a.spill_off[blockIdx.x] : smem + kWalkFixed);
     CurState *state = reinterpret_cast<CurState *>(buf + kBuf * (size_t)ncur);
 
@@ -1122,7 +1171,7 @@ __global__ void __launch_bounds__(32) walk_kernel(DevIndex ix, const __grid_cons
             const Cursor x = cur[refill];
             int32_t pr;
             const uint32_t k = state[refill].k;
-            const uint32_t w = chain_elem(ix, x.row, x.dir, (int)k + 1 + lane, Q, qlen, x.off, a.sub, &pr);
+            const uint32_t w = chain_elem(ix, x.row, x.dir, (int)k + 1 + lane, Q, qlen, x.off, ext, &pr);
             cache[chain_at(refill, k + lane)] = w;
             cprot[chain_at(refill, k + lane)] = pr;
             ++refills;
