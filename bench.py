@@ -35,7 +35,7 @@ METRIC = ("queries/s + SW GCUPS at identical hits; batched vs per-pair GPU; p50/
 WORKLOAD = ("batched Smith-Waterman: 1,000,000 pairs/step, qlen lognormal(350) 30-1000, "
             "slen lognormal(350) 30-5000, 20% homologues 25-60% identity, BLOSUM62 11/1, "
             "scores+ends (ssw_align u8->i16->drop semantics)")
-DPX_OPS_PER_CELL = 4      # 8 DPX instructions per int16x2 cell pair in the inner loop
+DPX_OPS_PER_CELL = 2.75   # 5.5 packed operations and PRMTs of the ALU pipe per cell pair
 
 
 def parse():
@@ -857,7 +857,7 @@ def native_arm(args, rank, local_rank, world):
             "roofline": {"bound": "dpx", "achieved": round(achieved, 2),
                          "peak": round(peak_gcups, 2), "unit": "GCUPS",
                          "frac": round(achieved / peak_gcups, 4),
-                         "peak_source": "measured live: __viaddmax_s16x2 issue rate %.3e op/s / %d DPX ops per cell"
+                         "peak_source": "measured live: __viaddmax_s16x2 issue rate %.3e op/s / %.2f ALU ops per cell"
                                         % (dpx_ops_s, DPX_OPS_PER_CELL),
                          "traffic": (round(traffic_per_cell * cells) if traffic_per_cell else None),
                          "traffic_source": ("not measured in this run: DRAM bytes per cell of the "

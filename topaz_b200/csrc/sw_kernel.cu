@@ -504,7 +504,8 @@ __host__ __device__ constexpr int stripe_smem(int RMAX, int warps) {
 }
 
 // Bins of the stripe form in one launch, and the fewest and most warps that
-// may share a pair of each.
+// may share a pair of each (64 pairs: 0.20 ms with up to 4 warps for queries
+// above 512 residues, 0.21 ms with 2).
 struct StripeSet {
     int n;
     int bin[3], wmin[3], wmax[3];
@@ -892,7 +893,7 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
         if (ends && x) a.snap += (size_t)grid(k->stripe32_blocks[e]) * kLongWarps * snap_words(kMaxR);
     }
     if (small_batch) {
-        const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {2, 2, 0}};
+        const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {4, 2, 0}};
         k->stripe8[e]<<<grid(k->stripe8_blocks[e]), 32 * kLongWarps, stripe_smem(8, kLongWarps),
                         next_stream()>>>(a, s);
         ++launches;
@@ -1232,20 +1233,24 @@ int tpz_sw_batch_host(int64_t n, const int8_t *q, const int64_t *qoff, const int
         return TPZ_E_ARG;
     }
     if (n == 0) return TPZ_OK;
-    // Pairs go in three chunks of 1/16, 3/16 and 12/16 of the batch: the copy
-    // in of the inputs runs about six times faster than the kernels, so each
-    // chunk's inputs arrive while the chunk before it computes and the GPU
-    // waits only for the first sixteenth.  Consecutive chunks run on
-    // alternating streams (lanes), so a chunk's kernels fill the GPU while
-    // the previous chunk's last tasks finish; each chunk's results are
-    // copied out as soon as they are done.  (Four chunks from 1/64 measured
-    // 3 % slower: a small chunk still pays its longest task twice.)
+    // Pairs go in chunks of growing size: the copy in of the inputs runs
+    // several times faster than the kernels, so each chunk's inputs arrive
+    // while the chunk before it computes and the GPU waits only for the first
+    // one's.  Consecutive chunks run on alternating streams (lanes), so a
+    // chunk's kernels fill the GPU while the previous chunk's last tasks
+    // finish; each chunk's results are copied out as soon as they are done.
+    // A chunk also pays its longest task: 1/8 and 7/8 took 6.3 ms at 70,000
+    // pairs against 7.2 ms for 1/16, 3/16 and 12/16, 12.5 against 12.8 ms at
+    // 150,000, and 23.3 against 22.5 ms at 300,000.
     constexpr int kMaxChunks = 4;
     int64_t cut[kMaxChunks + 1] = {0, n};
     int nch = 1;
-    if (n >= 65536) {
+    if (n >= 200000) {
         cut[1] = n / 16; cut[2] = 4 * (n / 16); cut[3] = n;
         nch = 3;
+    } else if (n >= 65536) {
+        cut[1] = n / 8; cut[2] = n;
+        nch = 2;
     }
     // host-side validation and the byte ranges each chunk reads: the chunks
     // cut into pieces in proportion to their size, scanned on up to 16 host
