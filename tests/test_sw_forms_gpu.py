@@ -53,18 +53,18 @@ def test_class_edges(cuda, name, go, ge, small):
     qs, ss = _edge_pairs(np.random.default_rng(go + 7 * small))
     n = len(qs)
     if not small:                                   # past the size where short queries change form
-        fill = synth.sw_pairs(1025, seed=go, q_range=(1, 90), q_median=30, s_range=(0, 200), s_median=60)
+        fill = synth.sw_pairs(4097, seed=go, q_range=(1, 90), q_median=30, s_range=(0, 200), s_median=60)
         qs += [fill.q[o:o + k] for o, k in zip(fill.qoff, fill.qlen)]
         ss += [fill.s[o:o + k] for o, k in zip(fill.soff, fill.slen)]
     ps, mat = _pairs(qs, ss), synth.matrix(name)
-    assert (ps.n > 1024) != small and n <= 1024
+    assert (ps.n > 4096) != small and n <= 4096
     got = _run(cuda, ps, mat, go, ge)
     want = np.stack(oracle.oracle_sw(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat, go, ge))
     bad = np.flatnonzero((got != want).any(axis=0))
     assert bad.size == 0, (bad[:5], got[:, bad[:5]], want[:, bad[:5]], ps.qlen[bad[:5]], ps.slen[bad[:5]])
 
 
-@pytest.mark.parametrize("n", [1, 3, 1023, 1024, 1025])
+@pytest.mark.parametrize("n", [1, 3, 1025, 4095, 4096, 4097])
 def test_batch_size_where_the_form_changes(cuda, n):
     ps = synth.sw_pairs(n, seed=n, s_range=(0, 3000))
     mat = synth.matrix("BLOSUM62")
@@ -85,7 +85,7 @@ def test_drop_at_16_bits_in_every_form(cuda):
             ss.append(np.full(m, 17, np.int8))
             qs.append(np.full(n, 16, np.int8))
             ss.append(np.full(m, 16, np.int8))
-    for copies in (1, 25):                          # stripe form, throughput form
+    for copies in (1, 90):                          # stripe form, throughput form
         ps = _pairs(qs * copies, ss * copies)
         got = _run(cuda, ps, mat, 11, 1)
         want = np.stack(oracle.oracle_sw(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat))

@@ -833,8 +833,10 @@ static thread_local int64_t g_last_launches = 0;
 
 // A batch of up to this many pairs takes the stripe form for every query: it
 // would leave most warps idle with two pairs and more per warp, and its time
-// is that of its longest pair.
-constexpr int64_t kSmallBatch = 1024;
+// is that of its longest pair.  Stripe form against by-pair, pairs of the
+// microbench: 128 pairs 0.28 / 0.41 ms, 1,024 0.32 / 0.54, 2,048 0.45 / 0.55,
+// 4,096 0.51 / 0.63, 8,192 0.80 / 0.81.
+constexpr int64_t kSmallBatch = 4096;
 
 // scratch words of one call: counts and cursor per bin, [start, count] and a
 // task counter per row bin, then the sorted pair ids
