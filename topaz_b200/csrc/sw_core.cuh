@@ -29,14 +29,18 @@
 //
 // Arithmetic: two alignments (or two row ranges of one) ride in the halves
 // of u16x2 words, every value raised by `floor` (= the zero of a score).
-// floor >= go + ge - min(M), so X - go never borrows: it is one 32-bit
-// addition, which the compiler may put beside the ALU pipe -- the bound: its
-// packed min/max/add and PRMT issue at 16 lanes a clock and scheduler --
-// and leaves that with 5.5 operations per cell pair: PRMT (profile bytes), X,
-// H, E, F and half a column maximum.  (With Fm, the lane starts and X - go on the same
-// pipe it was 8.5, and 1.3 times the cells because saturated pairs ran
-// twice.)  A score that reaches 32767 is final (the pair is dropped) however
-// far its 16 bits run on, so nothing is recomputed in wider arithmetic.
+// floor >= go + ge - min(M), so X - go does not borrow while no value passes
+// 65,535: it is one 32-bit addition, which the compiler may put beside the
+// ALU pipe -- the bound: its packed min/max/add and PRMT issue at 16 lanes a
+// clock and scheduler -- and leaves that with 5.5 operations per cell pair:
+// PRMT (profile bytes), X, H, E, F and half a column maximum.  (With Fm, the
+// lane starts and X - go on the same pipe it was 8.5, and 1.3 times the cells
+// because saturated pairs ran twice.)  A score that reaches 32767 is final
+// (the pair is dropped) however far its own 16 bits run on, so nothing is
+// recomputed in wider arithmetic.  But a half that wraps can leave a cell
+// below go, whose subtraction borrows from the other half: a pair that may
+// score past 65,535 - floor (shared_steps in sw_plan.h) takes the stripe
+// form, where both halves are its own.
 //
 // End coordinates: each lane keeps its running maximum of X (the alignment's
 // maximum is an X: F and E only hold less than an X before them).  A rise is
@@ -51,15 +55,14 @@
 // per row with four warps per scheduler and 16.3 against 12.8 with one.)
 #pragma once
 
+#include "sw_plan.h"
 #include "tpz_common.cuh"
 
 namespace tpz {
 namespace sw {
 
-constexpr int kMaxR = 32;           // rows per lane
 constexpr int kLetters = 26;        // 25 matrix columns + the pad letter
 constexpr int kPadLetter = 25;      // subject column past a pair's end
-constexpr int kPadScore = -64;      // profile value of pad rows / pad columns
 // transposed matrix in shared memory: 26 query letters x 26 subject letters,
 // rows of 9 words (an odd stride keeps the lanes' rows on different banks)
 constexpr int kMatWords = 9;
@@ -84,6 +87,7 @@ struct Args {
     int32_t *next_task;      // per row bin: task counter
     int gap_open, gap_extend;
     int floor;               // the zero of every stored value
+    int steps;               // diagonal steps that 16 bits hold (shared_steps)
     uint4 *snap;             // columns stored at a rise: snap_words() per warp
     int translate;           // 1: q/s bytes go through xq/xs first
     int8_t mat[625];
@@ -92,14 +96,16 @@ struct Args {
 
 // gap costs, floor and matrix of a launch
 inline void set_scoring(Args &a, const int8_t *mat, int go, int ge) {
-    int mn = kPadScore;
+    int mn = kPadScore, mx = 0;
     for (int i = 0; i < 625; ++i) {
         mn = mat[i] < mn ? mat[i] : mn;
+        mx = mat[i] > mx ? mat[i] : mx;
         a.mat[i] = mat[i];
     }
     a.gap_open = go;
     a.gap_extend = ge;
     a.floor = go + ge - mn;                 // <= 255 + 254 + 128
+    a.steps = shared_steps(a.floor, mx);
 }
 
 __device__ __forceinline__ uint32_t both(uint32_t x) { return x | (x << 16); }

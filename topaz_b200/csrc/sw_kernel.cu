@@ -53,35 +53,12 @@
 namespace tpz {
 namespace sw {
 
-constexpr int kStripeRows = 32 * kMaxR;     // longest query of the throughput form
 // scores of tpz_sw_align_one and the allocation-free call stay below this
 constexpr int kBig = 32512;
 
-// Row bins.  Throughput form: queries above 32 residues with G = 32 lanes
-// and R = 9..32 in bins R - 9, with G = 16, 8, 4 and R = 9..16 in bins 24,
-// 32, 40 + R - 9, shorter ones with G = 4 and R = 4, 8 in bins 48, 49.
-// Stripe form: 50..52 for queries up to 2048, 4096 and 8192, and 53, 54 for
-// the short queries of small batches, up to 512 and 1024.
-constexpr int kRBins = 56;
-constexpr int kTinyBin = 48;
-constexpr int kLongBin = 50;
-constexpr int kSmallBin = 53;
 constexpr int kSBins = 256;                 // subject-length buckets (32 residues each)
 constexpr int kBins = kRBins * kSBins;
 static_assert(kBins % 1024 == 0, "the scan gives each of 1024 threads an equal share");
-
-// lanes of a group for a query of one stripe
-__host__ __device__ __forceinline__ int group_lanes(int ql) {
-    return ql <= 64 ? 4 : ql <= 128 ? 8 : ql <= 256 ? 16 : 32;
-}
-
-__device__ __forceinline__ int row_bin(int ql, int small_batch) {
-    if (ql > kStripeRows) return kLongBin + (ql <= 2048 ? 0 : ql <= 4096 ? 1 : 2);
-    if (small_batch) return kSmallBin + (ql <= 512 ? 0 : 1);
-    if (ql <= 32) return kTinyBin + (ql - 1) / 16;
-    const int G = group_lanes(ql);
-    return (G == 32 ? 0 : G == 16 ? 24 : G == 8 ? 32 : 40) + (ql + G - 1) / G - 9;
-}
 
 // ---------------------------------------------------------- one warp's task
 
@@ -583,17 +560,18 @@ __global__ void __launch_bounds__(64) sw_one_kernel(const __grid_constant__ Args
 
 // ---------------------------------------------------------------- binning
 
-__device__ __forceinline__ int pair_bin(int ql, int sl, int small_batch) {
-    const int sb = min(sl >> 5, kSBins - 1);
-    return row_bin(ql, small_batch) * kSBins + (kSBins - 1 - sb);      // long subjects first
-}
-
 struct BinArgs {
     int64_t n;               // pairs 0..n-1, or list[0..n)
     const int32_t *list;
     const int32_t *qlen, *slen;
     int max_qlen, small_batch;
+    int steps;               // shared_steps of the scoring
 };
+
+__device__ __forceinline__ int pair_bin(const BinArgs &b, int ql, int sl) {
+    const int sb = min(sl >> 5, kSBins - 1);
+    return row_bin(ql, sl, b.small_batch, b.steps) * kSBins + (kSBins - 1 - sb);      // long subjects first
+}
 
 __global__ void bin_count_kernel(BinArgs b, int32_t *counts, int32_t *status) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < b.n;
@@ -604,7 +582,7 @@ __global__ void bin_count_kernel(BinArgs b, int32_t *counts, int32_t *status) {
             status[p] = TPZ_SW_INVALID;
             continue;
         }
-        atomicAdd(&counts[pair_bin(ql, sl, b.small_batch)], 1);
+        atomicAdd(&counts[pair_bin(b, ql, sl)], 1);
     }
 }
 
@@ -647,7 +625,7 @@ __global__ void bin_scatter_kernel(BinArgs b, int32_t *cursor, int32_t *sorted) 
         const int p = b.list ? b.list[i] : (int)i;
         const int ql = b.qlen[p], sl = b.slen[p];
         if (ql < 1 || ql > b.max_qlen || sl < 0 || sl >= TPZ_SW_MAX_SLEN) continue;
-        sorted[atomicAdd(&cursor[pair_bin(ql, sl, b.small_batch)], 1)] = p;
+        sorted[atomicAdd(&cursor[pair_bin(b, ql, sl)], 1)] = p;
     }
 }
 
@@ -871,7 +849,7 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
     int32_t *next_task = rinfo + 2 * kRBins, *sorted = ws + kBinWords;
     a.sorted = sorted; a.rinfo = rinfo; a.next_task = next_task;
     const bool small_batch = n <= kSmallBatch;
-    BinArgs b{n, list, a.qlen, a.slen, max_qlen, small_batch ? 1 : 0};
+    BinArgs b{n, list, a.qlen, a.slen, max_qlen, small_batch ? 1 : 0, a.steps};
     TPZ_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * kBins, st));
     const int gb = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)nsm * 8));
     bin_count_kernel<<<gb, 256, 0, st>>>(b, counts, a.status);
@@ -894,12 +872,14 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
         ++launches;
         if (ends && x) a.snap += (size_t)grid(k->stripe32_blocks[e]) * kLongWarps * snap_words(kMaxR);
     }
-    if (small_batch) {
+    // (in a large batch: the pairs that have to have their words to themselves)
+    if (small_batch || std::min(max_qlen, kStripeRows) > a.steps) {
         const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {4, 2, 0}};
         k->stripe8[e]<<<grid(k->stripe8_blocks[e]), 32 * kLongWarps, stripe_smem(8, kLongWarps),
                         next_stream()>>>(a, s);
         ++launches;
-    } else {
+    }
+    if (!small_batch) {
         for (int i = 0; i < kBinKernels; ++i) {
             k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
             ++launches;
@@ -979,8 +959,14 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         return TPZ_E_ARG;
     }
     const int nsm = sm_count();
+    Args a;
+    pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
+    set_scoring(a, mat, go, ge);
+    a.translate = (xq && xs) ? 1 : 0;
+    if (a.translate) { memcpy(a.xq, xq, 128); memcpy(a.xs, xs, 128); }
     // Chunks of pairs of one query for the query-major kernels (queries with
-    // enough pairs); every other pair goes by pair.  A chunk holds at most
+    // enough pairs, none of which has to have its words to itself); every
+    // other pair goes by pair.  A chunk holds at most
     // kQmMaxPairs, and fewer while the blocks of the GPU would not get four
     // each, down to four tasks per warp.
     int64_t cells = 0;                  // pairs * rows, the measure of a chunk's time
@@ -995,7 +981,7 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         const int64_t c = gstart_host[g + 1] - gstart_host[g];
         if (c <= 0) continue;
         const int ql = gqlen_host[g];
-        if (ql < 1 || c < kQmMinPairs) {
+        if (ql < 1 || c < kQmMinPairs || std::min(ql, max_slen) > a.steps) {
             for (int64_t k = gstart_host[g]; k < gstart_host[g + 1]; ++k) rest.push_back((int32_t)k);
             continue;
         }
@@ -1056,11 +1042,6 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         return cuda_fail(cudaGetLastError(), "batch_device_grouped copies");
     }
     int32_t *dhead = (int32_t *)dup;
-    Args a;
-    pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
-    set_scoring(a, mat, go, ge);
-    a.translate = (xq && xs) ? 1 : 0;
-    if (a.translate) { memcpy(a.xq, xq, 128); memcpy(a.xs, xs, 128); }
     const int e = score_only ? 0 : 1;
     int64_t launches = 0;
     struct Launch { QmArgs g; unsigned grid; int smem, striped; };

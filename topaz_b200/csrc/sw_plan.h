@@ -1,0 +1,54 @@
+// sw_plan.h -- which form of the batch Smith-Waterman kernels a pair takes
+// (plain C++: the binning kernels and the host share it, tests compile it).
+#pragma once
+
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define TPZ_HD __host__ __device__ __forceinline__
+#else
+#define TPZ_HD inline
+#endif
+
+namespace tpz {
+namespace sw {
+
+constexpr int kMaxR = 32;                   // rows per lane
+constexpr int kStripeRows = 32 * kMaxR;     // longest query of one stripe
+constexpr int kPadScore = -64;              // score of pad rows, pad columns and bytes outside the alphabet
+
+// Row bins.  Throughput form: queries above 32 residues with G = 32 lanes
+// and R = 9..32 in bins R - 9, with G = 16, 8, 4 and R = 9..16 in bins 24,
+// 32, 40 + R - 9, shorter ones with G = 4 and R = 4, 8 in bins 48, 49.
+// Stripe form: 50..52 for queries up to 2048, 4096 and 8192, and 53, 54 for
+// shorter ones, up to 512 and 1024.
+constexpr int kRBins = 56;
+constexpr int kTinyBin = 48;
+constexpr int kLongBin = 50;
+constexpr int kSmallBin = 53;
+
+// lanes of a group for a query of one stripe: the fewest that keep 16 rows
+// per lane, 32 from 257 residues on
+TPZ_HD int group_lanes(int ql) {
+    return ql <= 64 ? 4 : ql <= 128 ? 8 : ql <= 256 ? 16 : 32;
+}
+
+// Words of 16 bits hold an alignment of up to this many diagonal steps, from
+// `floor` (the zero of a score) on in steps of up to `entry`.  A pair that
+// may have more of them is not laid beside another pair (see Arithmetic in
+// sw_core.cuh).
+TPZ_HD int shared_steps(int floor, int entry) {
+    return entry > 0 ? (65535 - floor) / entry : INT32_MAX;
+}
+
+// The bin of a pair; small_batch: the stripe form for every query.
+TPZ_HD int row_bin(int ql, int sl, int small_batch, int steps) {
+    if (ql > kStripeRows) return kLongBin + (ql <= 2048 ? 0 : ql <= 4096 ? 1 : 2);
+    if (small_batch || (ql < sl ? ql : sl) > steps) return kSmallBin + (ql <= 512 ? 0 : 1);
+    if (ql <= 32) return kTinyBin + (ql - 1) / 16;
+    const int G = group_lanes(ql);
+    return (G == 32 ? 0 : G == 16 ? 24 : G == 8 ? 32 : 40) + (ql + G - 1) / G - 9;
+}
+
+}  // namespace sw
+}  // namespace tpz
