@@ -295,6 +295,11 @@ TPZ_API void tpz_search_result_free(tpz_search_result *r);
  * arguments. */
 TPZ_API int64_t tpz_search_query_device_bytes(int32_t qlen, const tpz_search_opts *o);
 
+/* The same for what a batch takes once, however many queries it has, when
+ * its longest one has max_qlen residues: the Smith-Waterman kernels' stored
+ * columns and stripe boundaries.  To be added to the queries' shares. */
+TPZ_API int64_t tpz_search_batch_device_bytes(int32_t max_qlen, const tpz_search_opts *o);
+
 /* Query ingest of a batch, in place (run_seg + seq_2internal,
  * src/engine.c:250-277): query i = cat[off[i] .. off[i]+len[i]) holds
  * upper-case residues (as the FASTA reader gives them); with seg != 0 SEG

@@ -5,6 +5,7 @@ import ctypes
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -15,6 +16,10 @@ using namespace tpz::sw;
 extern "C" {
 int t_row_bin(int ql, int sl, int small, int steps) { return row_bin(ql, sl, small, steps); }
 int t_group_lanes(int ql) { return group_lanes(ql); }
+int64_t t_boundary_blocks(int64_t want, int classes, int64_t cols, int sms) {
+    return boundary_blocks(want, classes, cols, sms);
+}
+int64_t t_boundary_bytes() { return kBoundaryBytes; }
 int t_shared_steps(int floor, int entry) { return shared_steps(floor, entry); }
 }
 """
@@ -27,7 +32,10 @@ def plan(tmp_path_factory):
     so = str(d / "plan.so")
     subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "topaz_b200", "csrc"),
                            str(d / "shim.cpp"), "-o", so])
-    return ctypes.CDLL(so)
+    lib = ctypes.CDLL(so)
+    lib.t_boundary_blocks.restype = lib.t_boundary_bytes.restype = ctypes.c_int64
+    lib.t_boundary_blocks.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
+    return lib
 
 
 def _rows_lanes(b):
@@ -60,3 +68,42 @@ def test_pairs_past_16_bits_have_their_words_to_themselves(plan, floor, entry):
             b = plan.t_row_bin(n, m, 0, steps)
             assert (b >= 50) == (min(n, m) * entry + floor > 65535)
     assert plan.t_shared_steps(floor, 0) == plan.t_shared_steps(floor, -3) == 2 ** 31 - 1
+
+
+def test_boundary_rows_stay_within_their_bytes(plan):
+    total = plan.t_boundary_bytes()
+    for cols in (0, 1, 300, 5000, 36_000, 110_000, 1_000_000, (1 << 24) - 1):
+        for classes in (1, 2, 4):
+            for want in (1, 7, 74, 148, 296):
+                got = plan.t_boundary_blocks(want, classes, cols, 148)
+                assert 0 <= got <= want
+                assert classes * got * 8 * 8 * max(cols, 1) <= total
+                assert got == 0 or 2 * got >= min(want, 148)
+    assert plan.t_boundary_blocks(296, 4, 5000, 148) == 296
+    assert plan.t_boundary_blocks(148, 1, 36_000, 148) == 148
+    assert plan.t_boundary_blocks(1, 1, (1 << 24) - 1, 148) == 0
+
+
+def test_admission_counts_what_a_batch_takes_once(plan):
+    from topaz_b200 import native, serve
+    short, long_ = native.batch_device_bytes(1024), native.batch_device_bytes(1025)
+    assert long_ - short == plan.t_boundary_bytes()
+    assert native.batch_device_bytes(1025, report_hits=0) > long_
+    assert native.batch_device_bytes(9000) == short            # not searched
+
+    taken = []
+
+    class Index:
+        def search(self, queries, mat, report=None, **kw):
+            taken.append([len(q) for q in queries])
+            raise RuntimeError("not searched here")
+
+    # room for the short queries, none for the long one's boundary rows
+    q = [b"A" * 900] * 3 + [b"A" * 1500] + [b"A" * 900] * 2
+    share = [serve.query_device_bytes(len(x)) for x in q]
+    srv = serve.SearchServer(Index(), np.zeros((25, 25), np.int8), workers=1,
+                             mem_budget=short + sum(share[:4]))
+    f = srv.submit(q)
+    assert isinstance(f.exception(timeout=30), RuntimeError)
+    srv.close()
+    assert taken == [[900] * 3, [1500], [900] * 2]

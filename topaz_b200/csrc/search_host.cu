@@ -24,7 +24,6 @@ struct tpz_index {
     std::vector<void *> mem;
     int64_t bytes = 0;
     std::vector<int64_t> pstart;   // host copy, Psize + 1
-    int32_t max_protein = 0;       // residues of the longest protein
 };
 
 namespace {
@@ -209,14 +208,20 @@ __global__ void pack_hits_kernel(PackArgs a) {
 }
 
 // sum of qlen * slen over the SW pairs
+// sum[0]: cells; sum[1]: the longest subject of a query above one stripe
 __global__ void pair_cells_kernel(int64_t n, const int32_t *ql, const int32_t *sl,
-                                  unsigned long long *cells) {
+                                  unsigned long long *sum) {
     unsigned long long c = 0;
+    int longest = 0;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * blockDim.x)
+         k += (int64_t)gridDim.x * blockDim.x) {
         c += (unsigned long long)ql[k] * (unsigned long long)sl[k];
+        if (ql[k] > tpz::sw::kStripeRows) longest = max(longest, sl[k]);
+    }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(cells, c);
+    longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sum[0], c);
+    if ((threadIdx.x & 31) == 0 && longest) atomicMax(&sum[1], (unsigned long long)longest);
 }
 
 // SW results of pair k back to hit p_hit[k]; hit2pair (optional) records k
@@ -729,7 +734,6 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
     const Rec *rec = (const Rec *)ind;
     std::vector<int64_t> pstart(Psize + 1);
     int64_t run = 0;
-    int32_t longest = 0;
     for (int64_t p = 0; p < Psize; ++p) {
         if ((int64_t)rec[p].ps != run || rec[p].pl < 0 || run + rec[p].pl >= Tsize ||
             T[run + rec[p].pl] != '\n') {
@@ -741,7 +745,6 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
         }
         pstart[p] = run;
         run += rec[p].pl + 1;
-        longest = std::max(longest, rec[p].pl);
     }
     if (run != Tsize) {
         tpz::set_error("tpz_index_create: .ind does not cover the text");
@@ -810,7 +813,6 @@ int tpz_index_create(const uint8_t *T, int64_t Tsize, const int64_t *SA, const v
     ix->d.Tsize = Tsize; ix->d.Psize = Psize; ix->d.sa_rows = sa_rows;
     ix->d.T = dT; ix->d.SA = dSA; ix->d.pstart = dps; ix->d.nl = dnl; ix->d.lb = dlb;
     ix->pstart.swap(pstart);
-    ix->max_protein = longest;
     *out = ix;
     return TPZ_OK;
 }
@@ -968,6 +970,11 @@ int64_t tpz_search_query_device_bytes(int32_t qlen, const tpz_search_opts *o) {
                                  (int64_t)walk_state_bytes(1));
     const int64_t per_hit = (int64_t)sizeof(Hit) + 2 * 8 + 18 * 4;
     return (int64_t)qlen + per_q + npos * per_pos + (int64_t)cap * per_hit + 256;
+}
+
+int64_t tpz_search_batch_device_bytes(int32_t max_qlen, const tpz_search_opts *o) {
+    if (!o || max_qlen < 0) return -1;
+    return tpz::sw::search_scratch_bytes(max_qlen > TPZ_SEARCH_MAX_QLEN ? 0 : max_qlen, o->report_hits <= 0);
 }
 
 int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
@@ -1189,15 +1196,17 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
             return bail(tpz::cuda_fail(cudaGetLastError(), "tpz_search_batch pairs"));
         const int64_t npairs = poff[nq];
         R->sw_pairs = npairs;
+        unsigned long long cells[2] = {0, 0};
         if (npairs > 0) {
             unsigned long long *dcells;
-            if ((rc = b.alloc(&dcells, 1))) return bail(rc);
-            TPZ_CUDA(cudaMemset(dcells, 0, 8));
+            if ((rc = b.alloc(&dcells, 2))) return bail(rc);
+            if (cudaMemset(dcells, 0, 16) != cudaSuccess)
+                return bail(tpz::cuda_fail(cudaGetLastError(), "tpz_search_batch cells"));
             pair_cells_kernel<<<(unsigned)std::min<int64_t>((npairs + 255) / 256, 2048), 256>>>(
                 npairs, pq_len, ps_len, dcells);
-            unsigned long long cells = 0;
-            TPZ_CUDA(cudaMemcpy(&cells, dcells, 8, cudaMemcpyDeviceToHost));
-            R->sw_cells = (int64_t)cells;
+            if (cudaMemcpy(cells, dcells, 16, cudaMemcpyDeviceToHost) != cudaSuccess)
+                return bail(tpz::cuda_fail(cudaGetLastError(), "tpz_search_batch cells"));
+            R->sw_cells = (int64_t)cells[0];
         }
         if (npairs > 0) {
             // the pairs of a query share its profile; report mode ranks on
@@ -1206,7 +1215,7 @@ int tpz_search_batch(const tpz_index *ix, const char *qcat, const int64_t *qoff,
                                                (const int8_t *)ix->d.T, ps_off, ps_len, o->mat625,
                                                o->gap_open, o->gap_extend, sc, re, rd, st, 0, xmap,
                                                xmap, report ? 1 : 0, nq, poff.data(),
-                                               qlen_eff.data(), ix->max_protein);
+                                               qlen_eff.data(), (int)cells[1]);
             if (rc) return bail(rc);
             scatter_sw_kernel<<<(unsigned)std::min<int64_t>((npairs + 255) / 256, 4096), 256>>>(
                 npairs, p_hit, sc, re, rd, st, raw, send, qend, psw, report ? hit2pair : nullptr);

@@ -1,6 +1,7 @@
 // search_internal.cuh -- device structures of the search path.
 #pragma once
 
+#include "sw_plan.h"
 #include "tpz_common.cuh"
 
 namespace tpz {
@@ -119,15 +120,19 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
                    int lane = 0);
 // lane 0/1: calls of one host thread that run concurrently use different
 // lanes (own streams).
-// The same, with no subject above max_slen, for pairs grouped by query (group g = pairs [gstart[g],
+// The same for pairs grouped by query (group g = pairs [gstart[g],
 // gstart[g+1]), all with query length gqlen[g]): groups with enough pairs go
 // to the query-major kernels, one shared profile per query; the rest by pair.
+// long_slen: the longest subject of a query above kStripeRows.
 int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const int32_t *qlen,
                          const int8_t *s, const int64_t *soff, const int32_t *slen,
                          const int8_t *mat, int go, int ge, int32_t *score, int32_t *ref_end,
                          int32_t *read_end, int32_t *status, cudaStream_t st, const int8_t *xq,
                          const int8_t *xs, int score_only, int64_t ngroups,
-                         const int64_t *gstart_host, const int32_t *gqlen_host, int max_slen);
+                         const int64_t *gstart_host, const int32_t *gqlen_host, int long_slen);
+// Device memory that the calls of a search batch take beside their pairs:
+// stored columns and boundary rows, at most.
+int64_t search_scratch_bytes(int max_qlen, bool ends);
 }  // namespace sw
 
 namespace stats {

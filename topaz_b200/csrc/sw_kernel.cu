@@ -248,7 +248,6 @@ __global__ void __launch_bounds__(32) sw_bin_kernel(const __grid_constant__ Args
 // kQmWarps warps keeps ONE profile of the query in shared memory for all of
 // them, so registers, not shared memory, bound the warps per SM.  The block
 // sorts the chunk's pairs by subject length, longest first.
-constexpr int kQmWarps = 8;
 constexpr int kQmMaxPairs = 256;      // pairs per chunk: longer pair lists of a query are cut
 constexpr int kQmMinPairs = 2 * kQmWarps;
 
@@ -838,6 +837,20 @@ static size_t batch_snap_words(const Kernels *k, int64_t n, int max_qlen, bool s
     return side_by_side ? sum : most;
 }
 
+// blocks of one SM that shared memory allows (228 KB, 1 KB of it per block)
+constexpr int blocks_by_smem(int smem) { return 228 * 1024 / (smem + 1024); }
+template <int R1>
+constexpr size_t bin_snaps() { return (size_t)blocks_by_smem(bin_smem<R1>()) * snap_words(R1); }
+
+int64_t search_scratch_bytes(int max_qlen, bool ends) {
+    // by pair: the hits that report mode aligns again, or the rest of a batch
+    size_t words = bin_snaps<32>() + bin_snaps<28>() + bin_snaps<24>() + bin_snaps<20>() + bin_snaps<16>() +
+                   bin_snaps<12>() + bin_snaps<8>() + (size_t)kLongWarps * snap_words(kMaxR);
+    // query-major, two blocks of an SM in each class
+    if (ends) words += (max_qlen > kStripeRows ? 5 : 1) * (size_t)(2 * kQmWarps) * snap_words(kMaxR);
+    return (int64_t)(16 * words * sm_count() + 4 * kBinWords) + (max_qlen > kStripeRows ? kBoundaryBytes : 0);
+}
+
 // Bins the pairs (all of them, or the n ids of `list`) in ws and launches the
 // kernels that align them, over the auxiliary streams x so that each
 // kernel's tail overlaps the next one (null: all on st).
@@ -952,13 +965,18 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
                          const int8_t *mat, int go, int ge, int32_t *score, int32_t *ref_end,
                          int32_t *read_end, int32_t *status, cudaStream_t st, const int8_t *xq,
                          const int8_t *xs, int score_only, int64_t ngroups,
-                         const int64_t *gstart_host, const int32_t *gqlen_host, int max_slen) {
+                         const int64_t *gstart_host, const int32_t *gqlen_host, int long_slen) {
     if (n <= 0) return TPZ_OK;
     if (!(go > ge && ge >= 0 && go <= 255) || !mat) {
         set_error("tpz_sw_batch: requires 255 >= gap_open > gap_extend >= 0");
         return TPZ_E_ARG;
     }
+    const Kernels *k = nullptr;
+    Streams *x = nullptr;
+    int rc = kernels(&k);
+    if (rc || (rc = streams(&x, 2))) return rc;
     const int nsm = sm_count();
+    const int e = score_only ? 0 : 1;
     Args a;
     pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
     set_scoring(a, mat, go, ge);
@@ -976,12 +994,16 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
     std::vector<Chunk> chunks[5];       // one stripe, and 2, up to 4, 6, 8 of them
     int min_lanes = 32, max_rows = 1;
     int striped_profile[5] = {0, 0, 0, 0, 0};
+    // shared memory of a class's blocks: profile, a warp's letter rings, all
+    auto profile = [&](int cls) { return cls ? striped_profile[cls] : profile_bytes(max_rows <= 8 ? 8 : max_rows); };
+    auto ring = [&](int cls) { return cls ? kPairRing : (32 / min_lanes) * kPairRing; };
+    auto qm_bytes = [&](int cls) { return qm_smem_bytes(profile(cls), ring(cls), cls > 0); };
     std::vector<int32_t> rest;
     for (int64_t g = 0; g < ngroups; ++g) {
         const int64_t c = gstart_host[g + 1] - gstart_host[g];
         if (c <= 0) continue;
         const int ql = gqlen_host[g];
-        if (ql < 1 || c < kQmMinPairs || std::min(ql, max_slen) > a.steps) {
+        if (ql < 1 || c < kQmMinPairs || (ql <= kStripeRows ? ql : std::min(ql, long_slen)) > a.steps) {
             for (int64_t k = gstart_host[g]; k < gstart_host[g + 1]; ++k) rest.push_back((int32_t)k);
             continue;
         }
@@ -1006,6 +1028,26 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
             striped_profile[cls] = std::max(striped_profile[cls], stripes * profile_bytes(rows));
         }
     }
+    // blocks of each class, and by pair where the boundary rows of its
+    // subjects would take too much
+    int64_t grids[5] = {};
+    int striped = 0;
+    for (int cls = 1; cls < 5; ++cls) striped += !chunks[cls].empty();
+    for (int cls = 0; cls < 5; ++cls) {
+        std::vector<Chunk> &c = chunks[cls];
+        if (c.empty()) continue;
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k->qm[e][cls > 0], kQmWarps * 32,
+                                                          qm_bytes(cls)) != cudaSuccess || nb < 1)
+            nb = 1;
+        grids[cls] = std::min<int64_t>((int64_t)nsm * nb, (int64_t)c.size());
+        if (cls == 0) continue;
+        grids[cls] = boundary_blocks(grids[cls], striped, long_slen, nsm);
+        if (grids[cls] > 0) continue;
+        for (const Chunk &x : c)
+            for (int32_t i = 0; i < x.pairs; ++i) rest.push_back((int32_t)(x.first + i));
+        c.clear();
+    }
     // one upload: a zero counter per class, the other pairs, the chunks
     // (longest first)
     std::vector<int32_t> head(8, 0);
@@ -1026,10 +1068,6 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         if (!c.empty()) memcpy(up.data() + at, c.data(), sizeof(Chunk) * c.size());
         at += sizeof(Chunk) * c.size();
     }
-    const Kernels *k = nullptr;
-    Streams *x = nullptr;
-    int rc = kernels(&k);
-    if (rc || (rc = streams(&x, 2))) return rc;
     char *dup = nullptr;
     uint2 *dbnd = nullptr;
     auto drop = [&]() {
@@ -1042,7 +1080,6 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         return cuda_fail(cudaGetLastError(), "batch_device_grouped copies");
     }
     int32_t *dhead = (int32_t *)dup;
-    const int e = score_only ? 0 : 1;
     int64_t launches = 0;
     struct Launch { QmArgs g; unsigned grid; int smem, striped; };
     std::vector<Launch> todo;
@@ -1057,22 +1094,15 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
         at += sizeof(Chunk) * c.size();
         l.g.count = (int)c.size();
         l.g.next = dhead + cls;
-        l.g.profile = cls ? striped_profile[cls] : profile_bytes(max_rows <= 8 ? 8 : max_rows);
-        l.g.ring = cls ? kPairRing : (32 / min_lanes) * kPairRing;
-        l.smem = qm_smem_bytes(l.g.profile, l.g.ring, l.striped);
-        int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)k->qm[e][l.striped], kQmWarps * 32,
-                                                          l.smem) != cudaSuccess || nb < 1)
-            nb = 1;
-        l.grid = (unsigned)std::min<int64_t>((int64_t)nsm * nb, (int64_t)c.size());
+        l.g.profile = profile(cls);
+        l.g.ring = ring(cls);
+        l.smem = qm_bytes(cls);
+        l.grid = (unsigned)grids[cls];
         l.g.bnd = nullptr;
         l.g.bnd_cols = 0;
         if (cls) {
-            // (at most 1 GB of boundary rows: fewer blocks where subjects are long)
-            l.g.bnd_cols = std::max(max_slen, 1);
-            const int64_t per_block = kQmWarps * l.g.bnd_cols;
-            l.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(l.grid, ((int64_t)1 << 27) / per_block));
-            bnd_words += (per_block * l.grid + 1) & ~(int64_t)1;
+            l.g.bnd_cols = std::max(long_slen, 1);
+            bnd_words += (kQmWarps * l.g.bnd_cols * l.grid + 1) & ~(int64_t)1;
         }
         if (e) snaps += (int64_t)l.grid * kQmWarps * snap_words(kMaxR);
         todo.push_back(l);

@@ -50,5 +50,19 @@ TPZ_HD int row_bin(int ql, int sl, int small_batch, int steps) {
     return (G == 32 ? 0 : G == 16 ? 24 : G == 8 ? 32 : 40) + (ql + G - 1) / G - 9;
 }
 
+// Query-major stripes keep a boundary row of 8 bytes per subject column for
+// each of a block's warps.  `want` blocks of one of `classes` stripe counts,
+// on a GPU of `sms` multiprocessors, may take this many with subjects of
+// `cols`; 0 where the classes' share of kBoundaryBytes holds fewer than half
+// of what would run (those pairs go by pair, whose boundaries are rings in
+// shared memory).
+constexpr int64_t kBoundaryBytes = (int64_t)512 << 20;
+constexpr int kQmWarps = 8;                 // warps of a query-major block
+inline int64_t boundary_blocks(int64_t want, int classes, int64_t cols, int sms) {
+    const int64_t fit = kBoundaryBytes / classes / (8 * kQmWarps * (cols > 1 ? cols : 1));
+    const int64_t need = want < sms ? want : sms;
+    return fit >= want ? want : 2 * fit >= need ? fit : 0;
+}
+
 }  // namespace sw
 }  // namespace tpz

@@ -191,6 +191,8 @@ def _search_sigs(L):
                              ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]
     L.tpz_search_query_device_bytes.argtypes = [ctypes.c_int32, ctypes.POINTER(_SearchOpts)]
     L.tpz_search_query_device_bytes.restype = ctypes.c_int64
+    L.tpz_search_batch_device_bytes.argtypes = [ctypes.c_int32, ctypes.POINTER(_SearchOpts)]
+    L.tpz_search_batch_device_bytes.restype = ctypes.c_int64
     L._search_sigs = True
 
 
@@ -325,6 +327,19 @@ def query_device_bytes(qlen, num_hits=100, alignments=5000, min_hit_length=5,
     _search_sigs(L)
     o = _SearchOpts(num_hits, gap_open, gap_extend, min_hit_length, seeds, alignments, None, 0)
     v = L.tpz_search_query_device_bytes(int(qlen), ctypes.byref(o))
+    if v < 0:
+        raise TopazError(-1, "bad arguments")
+    return int(v)
+
+
+def batch_device_bytes(max_qlen, report_hits=100):
+    """tpz_search_batch_device_bytes: device memory a batch takes once,
+    beside its queries' shares (report_hits 0: all hits come back)."""
+    L = lib()
+    _search_sigs(L)
+    o = _SearchOpts()
+    o.report_hits = int(report_hits)
+    v = L.tpz_search_batch_device_bytes(int(max_qlen), ctypes.byref(o))
     if v < 0:
         raise TopazError(-1, "bad arguments")
     return int(v)

@@ -122,10 +122,12 @@ class SearchServer:
         with self._cv:
             while True:
                 if self._pending:
-                    batch, need = [], 0
+                    batch, need, once = [], 0, 0
                     while self._pending and len(batch) < self.max_batch:
                         req, i = self._pending[0]
-                        b = query_device_bytes(len(req.queries[i]), **self._size_kw())
+                        # the query's share, and by how much it raises the batch's
+                        grown = max(once, native.batch_device_bytes(len(req.queries[i])))
+                        b = query_device_bytes(len(req.queries[i]), **self._size_kw()) + grown - once
                         if batch and self._mem_used + need + b > self.mem_budget:
                             break
                         if not batch and self._mem_used + b > self.mem_budget and self._mem_used:
@@ -133,6 +135,7 @@ class SearchServer:
                         self._pending.popleft()
                         batch.append((req, i))
                         need += b
+                        once = grown
                     if batch:
                         self._mem_used += need
                         return batch, need
