@@ -19,6 +19,9 @@ int t_group_lanes(int ql) { return group_lanes(ql); }
 int64_t t_boundary_blocks(int64_t want, int classes, int64_t cols, int sms) {
     return boundary_blocks(want, classes, cols, sms);
 }
+unsigned t_grid_blocks(int64_t sms, int64_t per_sm, int64_t pairs, int64_t fit) {
+    return grid_blocks(sms, per_sm, pairs, fit);
+}
 int64_t t_boundary_bytes() { return kBoundaryBytes; }
 int t_shared_steps(int floor, int entry) { return shared_steps(floor, entry); }
 }
@@ -35,6 +38,7 @@ def plan(tmp_path_factory):
     lib = ctypes.CDLL(so)
     lib.t_boundary_blocks.restype = lib.t_boundary_bytes.restype = ctypes.c_int64
     lib.t_boundary_blocks.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
+    lib.t_grid_blocks.argtypes = [ctypes.c_int64] * 4
     return lib
 
 
@@ -107,3 +111,11 @@ def test_admission_counts_what_a_batch_takes_once(plan):
     assert isinstance(f.exception(timeout=30), RuntimeError)
     srv.close()
     assert taken == [[900] * 3, [1500], [900] * 2]
+
+
+def test_blocks_of_a_launch(plan):
+    # more SMs than fixed scratch is for: as many blocks as it holds
+    assert plan.t_grid_blocks(148, 4, 1 << 20, 148 * 4) == 148 * 4
+    assert plan.t_grid_blocks(160, 4, 1 << 20, 148 * 4) == 148 * 4
+    assert plan.t_grid_blocks(148, 4, 100, 148 * 4) == 100
+    assert plan.t_grid_blocks(148, 4, 0, 148 * 4) == 1

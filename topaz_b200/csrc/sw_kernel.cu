@@ -819,22 +819,18 @@ constexpr int64_t kSmallBatch = 4096;
 // task counter per row bin, then the sorted pair ids
 constexpr size_t kBinWords = 2 * (size_t)kBins + 3 * kRBins;
 
-// blocks of a launch: no more than pairs
 static unsigned grid_of(int blocks_per_sm, int64_t n) {
-    return (unsigned)std::min<int64_t>((int64_t)sm_count() * blocks_per_sm, std::max<int64_t>(n, 1));
+    return grid_blocks(sm_count(), blocks_per_sm, n, INT64_MAX);
 }
 
-// uint4 words for the columns that launch_batch's kernels store, for the
-// largest kernel (they follow each other) or all (they run side by side)
-static size_t batch_snap_words(const Kernels *k, int64_t n, int max_qlen, bool side_by_side) {
-    size_t sum = 0, most = 0;
-    auto add = [&](size_t w) { sum += w; most = std::max(most, w); };
-    if (max_qlen > kStripeRows)
-        add((size_t)grid_of(k->stripe32_blocks[1], n) * kLongWarps * snap_words(kMaxR));
+// uint4 words for the columns that launch_batch's kernels store
+static size_t batch_snap_words(const Kernels *k, int64_t n, int max_qlen) {
+    size_t sum = 0;
+    if (max_qlen > kStripeRows) sum += (size_t)grid_of(k->stripe32_blocks[1], n) * kLongWarps * snap_words(kMaxR);
     if (n > kSmallBatch)
         for (int i = 0; i < kBinKernels; ++i)
-            add((size_t)grid_of(k->bin_blocks[1][i], n) * snap_words(k->set[i].rows[0]));
-    return side_by_side ? sum : most;
+            sum += (size_t)grid_of(k->bin_blocks[1][i], n) * snap_words(k->set[i].rows[0]);
+    return sum;
 }
 
 // blocks of one SM that shared memory allows (228 KB, 1 KB of it per block)
@@ -853,9 +849,11 @@ int64_t search_scratch_bytes(int max_qlen, bool ends) {
 
 // Bins the pairs (all of them, or the n ids of `list`) in ws and launches the
 // kernels that align them, over the auxiliary streams x so that each
-// kernel's tail overlaps the next one (null: all on st).
+// kernel's tail overlaps the next one.  x null: all on st, so that the kernels
+// share the snap_cap words of stored columns, with no more blocks than those
+// are for (x: batch_snap_words of them).
 static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const int32_t *list,
-                        int32_t *ws, uint4 *snap, int max_qlen, bool ends, cudaStream_t st,
+                        int32_t *ws, uint4 *snap, int64_t snap_cap, int max_qlen, bool ends, cudaStream_t st,
                         int64_t &launches) {
     const int nsm = sm_count();
     int32_t *counts = ws, *cursor = counts + kBins, *rinfo = cursor + kBins;
@@ -876,27 +874,30 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
     }
     int at = 0;
     auto next_stream = [&]() { return x ? x->aux[at++ % kAuxStreams] : st; };
-    auto grid = [&](int blocks) { return grid_of(blocks, n); };
+    auto grid = [&](int blocks, int words) { return grid_blocks(nsm, blocks, n, x ? INT64_MAX : snap_cap / words); };
     a.snap = ends ? snap : nullptr;
     if (max_qlen > kStripeRows) {
         const StripeSet s{3, {kLongBin + 2, kLongBin + 1, kLongBin}, {4, 2, 1}, {4, 4, 4}};
-        k->stripe32[e]<<<grid(k->stripe32_blocks[e]), 32 * kLongWarps, stripe_smem(32, kLongWarps),
-                         next_stream()>>>(a, s);
+        const int words = kLongWarps * snap_words(kMaxR);
+        const unsigned blocks = grid(k->stripe32_blocks[e], words);
+        k->stripe32[e]<<<blocks, 32 * kLongWarps, stripe_smem(32, kLongWarps), next_stream()>>>(a, s);
         ++launches;
-        if (ends && x) a.snap += (size_t)grid(k->stripe32_blocks[e]) * kLongWarps * snap_words(kMaxR);
+        if (ends && x) a.snap += (size_t)blocks * words;
     }
     // (in a large batch: the pairs that have to have their words to themselves)
     if (small_batch || std::min(max_qlen, kStripeRows) > a.steps) {
         const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {4, 2, 0}};
-        k->stripe8[e]<<<grid(k->stripe8_blocks[e]), 32 * kLongWarps, stripe_smem(8, kLongWarps),
+        k->stripe8[e]<<<grid_of(k->stripe8_blocks[e], n), 32 * kLongWarps, stripe_smem(8, kLongWarps),
                         next_stream()>>>(a, s);
         ++launches;
     }
     if (!small_batch) {
         for (int i = 0; i < kBinKernels; ++i) {
-            k->bin[e][i]<<<grid(k->bin_blocks[e][i]), 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
+            const int words = snap_words(k->set[i].rows[0]);
+            const unsigned blocks = grid(k->bin_blocks[e][i], words);
+            k->bin[e][i]<<<blocks, 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
             ++launches;
-            if (ends && x) a.snap += (size_t)grid(k->bin_blocks[e][i]) * snap_words(k->set[i].rows[0]);
+            if (ends && x) a.snap += (size_t)blocks * words;
         }
     }
     // the join comes after every launch, also on an error, so that the
@@ -941,7 +942,7 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
     keep_pool_memory();
     if (subset) n = nsub;
     // workspace: the stored columns, then the bins and the sorted ids
-    const size_t snaps = score_only ? 0 : batch_snap_words(k, n, TPZ_SW_MAX_QLEN, true);
+    const size_t snaps = score_only ? 0 : batch_snap_words(k, n, TPZ_SW_MAX_QLEN);
     uint4 *ws = nullptr;
     TPZ_CUDA(cudaMallocAsync((void **)&ws, sizeof(uint4) * snaps + sizeof(int32_t) * (kBinWords + (size_t)n), st));
     Args a;
@@ -953,7 +954,7 @@ int batch_device_x(int64_t n, const int8_t *q, const int64_t *qoff, const int32_
         memcpy(a.xs, xs, 128);
     }
     int64_t launches = 0;
-    rc = launch_batch(k, x, a, n, subset, (int32_t *)(ws + snaps), ws, TPZ_SW_MAX_QLEN, !score_only, st, launches);
+    rc = launch_batch(k, x, a, n, subset, (int32_t *)(ws + snaps), ws, (int64_t)snaps, TPZ_SW_MAX_QLEN, !score_only, st, launches);
     TPZ_CUDA(cudaFreeAsync(ws, st));
     if (rc) return rc;
     g_last_launches = launches;
@@ -1447,9 +1448,9 @@ int tpz_dpx_probe(int64_t blocks, int iters, uint32_t *out, void *stream, int64_
 // memory pressure halfway through a request), or a host loop that must not
 // stall on the allocator -- cudaMalloc/cudaFree synchronize the device and
 // would serialize every concurrent stream.  For them the batched SW below
-// keeps its scratch (bin counts, bin cursors and the sorted pair list) in one
-// statically sized device array instead of a per-call allocation, and
-// enqueues everything on the caller's stream only.
+// keeps its scratch (bin counts, bin cursors, the sorted pair list and the
+// stored columns) in one statically sized device array instead of a per-call
+// allocation, and enqueues everything on the caller's stream only.
 
 namespace tpz {
 namespace sw {
@@ -1462,8 +1463,8 @@ static_assert((int64_t)kNoAllocMaxQlen * TPZ_SW_NOALLOC_MAX_ENTRY < kBig &&
               "TPZ_SW_NOALLOC_MAX_ENTRY");
 
 // One copy per device that loads the library, kept until the process exits.
-// Behind the bins: the columns stored by the largest by-pair kernel, for the
-// SMs and blocks per SM this library is built for.
+// Behind the bins: the columns stored by the largest by-pair kernel on 148
+// SMs (a kernel launches no more blocks than there is room for).
 constexpr size_t kNoAllocBins = (kBinWords + (size_t)kNoAllocMaxPairs + 3) & ~(size_t)3;
 constexpr size_t kNoAllocSnaps = 148 * 4 * (size_t)snap_words(kMaxR);
 static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocBins + 4 * kNoAllocSnaps];
@@ -1530,14 +1531,10 @@ extern "C" int tpz_sw_batch_device_noalloc(int64_t n, const int8_t *q, const int
     int32_t *ws = nullptr;
     int rc = kernels(&k);
     if (rc || (rc = noalloc_scratch(&ws))) return rc;
-    if (batch_snap_words(k, n, kNoAllocMaxQlen, false) > kNoAllocSnaps) {
-        tpz::set_error("tpz_sw_batch_device_noalloc: more SMs than the fixed scratch is sized for");
-        return TPZ_E_DEVICE;
-    }
     Args a;
     pair_args(a, q, qoff, qlen, s, soff, slen, score, ref_end, read_end, status);
     set_scoring(a, mat625_host, gap_open, gap_extend);
     int64_t launches = 0;
-    return launch_batch(k, nullptr, a, n, nullptr, ws, (uint4 *)(ws + kNoAllocBins), kNoAllocMaxQlen, true,
-                        (cudaStream_t)stream, launches);
+    return launch_batch(k, nullptr, a, n, nullptr, ws, (uint4 *)(ws + kNoAllocBins), (int64_t)kNoAllocSnaps,
+                        kNoAllocMaxQlen, true, (cudaStream_t)stream, launches);
 }

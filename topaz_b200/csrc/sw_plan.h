@@ -50,6 +50,14 @@ TPZ_HD int row_bin(int ql, int sl, int small_batch, int steps) {
     return (G == 32 ? 0 : G == 16 ? 24 : G == 8 ? 32 : 40) + (ql + G - 1) / G - 9;
 }
 
+// Blocks of a launch: no more than pairs, nor than `fit`.
+inline unsigned grid_blocks(int64_t sms, int64_t blocks_per_sm, int64_t pairs, int64_t fit) {
+    int64_t b = sms * blocks_per_sm;
+    b = b < pairs ? b : pairs;
+    b = b < fit ? b : fit;
+    return (unsigned)(b > 1 ? b : 1);
+}
+
 // Query-major stripes keep a boundary row of 8 bytes per subject column for
 // each of a block's warps.  `want` blocks of one of `classes` stripe counts,
 // on a GPU of `sms` multiprocessors, may take this many with subjects of
