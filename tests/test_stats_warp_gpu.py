@@ -64,3 +64,27 @@ def test_inputs_no_forward_pass_gives(cuda, shift, go, ge):
     ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62")
     sc, re_, rd, _ = native.sw_batch_host(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat, 11, 1)
     _check(cuda, ps, mat, go, ge, (np.maximum(sc + shift, 1), re_, rd))
+
+
+@pytest.mark.parametrize("go,ge", [(11, 1), (2, 2)])
+def test_bytes_outside_the_alphabet(cuda, go, ge):
+    # they score -64, as in the forward pass: the same columns as for a letter
+    # whose scores are all -64
+    ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62").copy()
+    mat[24, :] = mat[:, 24] = -64
+    rng = np.random.default_rng(9)
+    known = synth.PairSet(ps.q.copy(), ps.qoff, ps.qlen, ps.s.copy(), ps.soff, ps.slen, 0)
+    for i in range(ps.n):                            # in half of the pairs each
+        buf, off, n = (ps.q, ps.qoff, ps.qlen) if i % 4 < 2 else (ps.s, ps.soff, ps.slen)
+        at = off[i] + rng.integers(0, n[i], 1 + n[i] // 40)
+        buf[at] = rng.choice(np.array([25, 30, 127, -1, -128], np.int8), len(at))
+        (known.q if i % 4 < 2 else known.s)[at] = 24
+    fwd = native.sw_batch_host(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat, 11, 1)
+    same = native.sw_batch_host(known.q, known.qoff, known.qlen, known.s, known.soff, known.slen, mat, 11, 1)
+    assert all((x == y).all() for x, y in zip(fwd, same)) and (fwd[3] == 0).all()
+    got = _device_stats(cuda, ps, mat, go, ge, fwd[:3])
+    want = _device_stats(cuda, known, mat, go, ge, fwd[:3])
+    for k in FIELDS:
+        assert (got[k] == want[k]).all(), k
+    assert got["identity"].tobytes() == want["identity"].tobytes()
+    assert (got["length"] > 0).sum() > ps.n // 2

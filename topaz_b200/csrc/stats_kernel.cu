@@ -79,6 +79,11 @@ __device__ __forceinline__ int res_at(const PairArgs &a, const int8_t *p, int64_
     return v;
 }
 
+// a residue as a row and column of the score table: bytes outside the
+// alphabet share the pad's, as in the forward pass
+__device__ __forceinline__ int letter_of(int residue) { return (unsigned)residue < 25u ? residue : 25; }
+constexpr int kScores = 26;
+
 // scratch words of a pair: reverse pass 3 * (rows + 1), band rows 2 * (cols + 2)
 __host__ __device__ inline int64_t work_words(int32_t read_end, int32_t ref_end) {
     const int64_t n = (int64_t)read_end + 1;
@@ -92,9 +97,18 @@ __host__ __device__ inline int64_t band_words_at(int32_t read_end) {
     return 3 * (((n + 15) / 16) * 16 + 1);
 }
 
+// the score table, every thread of the block
+__device__ __forceinline__ void load_scores(const PairArgs &a, int8_t *smat) {
+    for (int i = threadIdx.x; i < kScores * kScores; i += blockDim.x) {
+        const int s = i / kScores, q = i % kScores;
+        smat[i] = s < 25 && q < 25 ? a.mat[s * 25 + q] : (int8_t)sw::kPadScore;
+    }
+    __syncthreads();
+}
+
 // The reverse pass as SSW runs it (one thread): start row and column of the
 // best cell, -1 where there is none.
-__device__ void reverse_pass(const PairArgs &a, int64_t p, int *row, int *col) {
+__device__ void reverse_pass(const PairArgs &a, const int8_t *smat, int64_t p, int *row, int *col) {
     const int re = a.read_end[p], fe = a.ref_end[p], score = a.score[p];
     const int8_t *q = a.q + a.qoff[p], *s = a.s + a.soff[p];
     // rows = reversed query prefix, with the padding rows of the striped
@@ -111,12 +125,12 @@ __device__ void reverse_pass(const PairArgs &a, int64_t p, int *row, int *col) {
     const int go = a.gap_open, gx = a.gap_extend;
     int best = 0, bc = word ? 0 : -1, br = 0;
     for (int c = fe; c >= 0; --c) {
-        const int8_t *mrow = a.mat + 25 * res_at(a, s, c);
+        const int8_t *mrow = smat + kScores * letter_of(res_at(a, s, c));
         int F = 0, Fm = 0, colmax = 0, cbest = 0, crow = 0;
         for (int r = 0; r < rows; ++r) {
             if (r % seg == 0) Fm = 0;
             const int D = r ? Hp[r - 1] : 0;
-            const int sc = r < n ? mrow[res_at(a, q, re - r)] : 0;
+            const int sc = r < n ? mrow[letter_of(res_at(a, q, re - r))] : 0;
             const int hp = max(max(0, D + sc), max(E[r], Fm));
             const int h = max(hp, F);
             E[r] = max(0, max(E[r] - gx, hp - go));
@@ -141,6 +155,8 @@ __device__ void reverse_pass(const PairArgs &a, int64_t p, int *row, int *col) {
 
 // One thread per hit: where its alignment starts.
 __global__ void stats_start_kernel(const __grid_constant__ PairArgs a) {
+    __shared__ int8_t smat[kScores * kScores];
+    load_scores(a, smat);
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n;
          p += (int64_t)gridDim.x * blockDim.x) {
         a.band[p] = 0;
@@ -155,7 +171,7 @@ __global__ void stats_start_kernel(const __grid_constant__ PairArgs a) {
                 row = a.rrow[p];
                 col = fe - a.rcol[p];
             } else {
-                reverse_pass(a, p, &row, &col);
+                reverse_pass(a, smat, p, &row, &col);
             }
             a.qstart[p] = re - row;
             a.sstart[p] = col;
@@ -181,7 +197,7 @@ __device__ int band_pass(const PairArgs &a, const int8_t *smat, const int8_t *rd
         const int beg = max(0, i - w), end = min(fl - 1, i + w);
         const int c0 = max(0, i0 - w);
         const int prev_end = i > 0 ? min(fl - 1, i - 1 + w) : -1;   // band of the row above
-        const int qi = i < rl ? res_at(a, rd, i) : 0;
+        const int qi = i < rl ? letter_of(res_at(a, rd, i)) : 0;
         int8_t *dl = dir && i < rl ? dir + (int64_t)i * wd3 : nullptr;
         int h = 0, e = 0, f = 0;                    // this row, column j - 1
         // H(i-1, j-1): what came from above in the step before
@@ -195,7 +211,7 @@ __device__ int band_pass(const PairArgs &a, const int8_t *smat, const int8_t *rd
                 __syncwarp();
                 hb = eb = lb = 0;
                 if (j < fl) {
-                    lb = res_at(a, rf, j);
+                    lb = letter_of(res_at(a, rf, j));
                     if (i0 > 0 && j <= min(fl - 1, i0 - 1 + w)) { hb = __ldcg(Hc + j); eb = __ldcg(Ec + j); }
                 }
             }
@@ -214,7 +230,7 @@ __device__ int band_pass(const PairArgs &a, const int8_t *smat, const int8_t *rd
                 f = fo > fe ? fo : fe;
                 const int e1 = e > 0 ? e : 0, f1 = f > 0 ? f : 0;
                 const int gap = e1 > f1 ? e1 : f1;
-                const int dg = diag + smat[letter * 25 + qi];
+                const int dg = diag + smat[letter * kScores + qi];
                 h = gap > dg ? gap : dg;
                 if (dl) {
                     const int8_t de = eo > ee ? 3 : 2, df = fo > fe ? 5 : 4;
@@ -235,14 +251,9 @@ __device__ int band_pass(const PairArgs &a, const int8_t *smat, const int8_t *rd
 
 constexpr int kBandWarps = 4;
 
-__device__ __forceinline__ void load_scores(const PairArgs &a, int8_t *smat) {
-    for (int i = threadIdx.x; i < 625; i += blockDim.x) smat[i] = a.mat[i];
-    __syncthreads();
-}
-
 // A warp per hit: the final band width and its direction table's size.
 __global__ void __launch_bounds__(32 * kBandWarps) stats_band_kernel(const __grid_constant__ PairArgs a) {
-    __shared__ int8_t smat[640];
+    __shared__ int8_t smat[kScores * kScores];
     load_scores(a, smat);
     for (int64_t p = blockIdx.x * (int64_t)kBandWarps + (threadIdx.x >> 5); p < a.n;
          p += (int64_t)gridDim.x * kBandWarps) {
@@ -279,7 +290,7 @@ __global__ void __launch_bounds__(32 * kBandWarps) stats_band_kernel(const __gri
 
 // A warp per hit: the direction table, then lane 0 walks the path back.
 __global__ void __launch_bounds__(32 * kBandWarps) stats_path_kernel(const __grid_constant__ PairArgs a) {
-    __shared__ int8_t smat[640];
+    __shared__ int8_t smat[kScores * kScores];
     load_scores(a, smat);
     for (int64_t p = blockIdx.x * (int64_t)kBandWarps + (threadIdx.x >> 5); p < a.n;
          p += (int64_t)gridDim.x * kBandWarps) {
