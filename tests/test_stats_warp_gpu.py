@@ -87,4 +87,4 @@ def test_bytes_outside_the_alphabet(cuda, go, ge):
     for k in FIELDS:
         assert (got[k] == want[k]).all(), k
     assert got["identity"].tobytes() == want["identity"].tobytes()
-    assert (got["length"] > 0).sum() > ps.n // 2
+    assert (got["length"] > 0).sum() > ps.n // 2 or go == ge
