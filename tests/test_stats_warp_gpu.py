@@ -59,6 +59,20 @@ def test_bands_around_the_row_blocks(cuda, go, ge):
     _check(cuda, ps, mat, go, ge, (sc, re_, rd))
 
 
+def test_launch_count_stays_the_batch_calls(cuda):
+    ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62")
+    t = {k: cuda.from_numpy(np.ascontiguousarray(getattr(ps, k))).cuda() for k in ("q", "s")}
+    for k in ("qoff", "qlen", "soff", "slen"):
+        t[k] = cuda.from_numpy(np.tile(getattr(ps, k), 50)).cuda()
+    for k in ("score", "ref_end", "read_end", "status"):
+        t[k] = cuda.empty(50 * ps.n, dtype=cuda.int32, device="cuda")
+    native.sw_batch_torch(t, mat)                    # another form than the statistics' batch
+    counted = native.last_launches()
+    sc, re_, rd = (t[k][:ps.n].cpu().numpy() for k in ("score", "ref_end", "read_end"))
+    _device_stats(cuda, ps, mat, 11, 1, (sc, re_, rd))
+    assert native.last_launches() == counted > 6
+
+
 @pytest.mark.parametrize("shift,go,ge", [(-1, 11, 1), (0, 2, 2), (0, 1, 3)])
 def test_inputs_no_forward_pass_gives(cuda, shift, go, ge):
     ps, mat = _gapped_pairs(), synth.matrix("BLOSUM62")

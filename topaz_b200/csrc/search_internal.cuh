@@ -130,6 +130,9 @@ int batch_device_grouped(int64_t n, const int8_t *q, const int64_t *qoff, const 
                          int32_t *read_end, int32_t *status, cudaStream_t st, const int8_t *xq,
                          const int8_t *xs, int score_only, int64_t ngroups,
                          const int64_t *gstart_host, const int32_t *gqlen_host, int long_slen);
+// What tpz_sw_last_launches gives: a batch inside another entry point puts it
+// back.
+int64_t &last_launches();
 // Device memory that the calls of a search batch take beside their pairs:
 // stored columns and boundary rows, at most.
 int64_t search_scratch_bytes(int max_qlen, bool ends);

@@ -444,8 +444,11 @@ int stats_batch(PairArgs a, cudaStream_t st) {
         int32_t *rql = r, *rsl = r + a.n, *rs = r + 2 * a.n, *rc_ = r + 3 * a.n, *rr = r + 4 * a.n,
                 *rst = r + 5 * a.n;
         reverse_kernel<<<warps, 128, 0, st>>>(a, boff, rev, rsoff, rql, rsl);
-        if ((rc = sw::batch_device_x(a.n, rev, boff, rql, rev, rsoff, rsl, a.mat, a.gap_open, a.gap_extend, rs,
-                                     rc_, rr, rst, st, nullptr, nullptr, 0))) {
+        const int64_t counted = sw::last_launches();
+        rc = sw::batch_device_x(a.n, rev, boff, rql, rev, rsoff, rsl, a.mat, a.gap_open, a.gap_extend, rs, rc_, rr,
+                                rst, st, nullptr, nullptr, 0);
+        sw::last_launches() = counted;
+        if (rc) {
             cleanup();
             return rc;
         }

@@ -808,6 +808,8 @@ static int join(Streams *x, cudaStream_t st) {
 
 static thread_local int64_t g_last_launches = 0;
 
+int64_t &last_launches() { return g_last_launches; }
+
 // A batch of up to this many pairs takes the stripe form for every query: it
 // would leave most warps idle with two pairs and more per warp, and its time
 // is that of its longest pair.  Stripe form against by-pair, pairs of the
