@@ -56,7 +56,10 @@ def _child():
 
 
 def test_memory_of_a_batch_beside_a_long_protein(cuda):
-    out = subprocess.run([sys.executable, __file__], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    # (in a process of its own: the pool keeps what other batches grew it to)
+    run = "import sys; sys.path[:0] = %r; import test_batch_memory_gpu as t; t._child()" % [
+        ROOT, os.path.join(ROOT, "tests")]
+    out = subprocess.run([sys.executable, "-c", run], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr[-2000:]
     used = json.loads(out.stdout.strip().splitlines()[-1])
     # queries' shares, stored columns, and 60 blocks' boundaries of 1,300 columns
@@ -83,8 +86,3 @@ def test_hits_longer_than_the_boundary_rows(cuda):
     assert on.sum() >= 16
     for got, w in (("rawscore", 0), ("send", 1), ("qend", 2), ("sw_status", 3)):
         assert (r[got][a:b][on] == want[w][on]).all(), got
-
-
-if __name__ == "__main__":
-    sys.path.insert(0, ROOT)
-    _child()
