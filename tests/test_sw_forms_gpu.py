@@ -11,7 +11,7 @@ from topaz_b200 import native, synth
 
 pytestmark = pytest.mark.gpu
 
-EDGES = (1, 2, 16, 17, 32, 33, 36, 64, 65, 72, 128, 129, 144, 256, 257, 288, 289, 511, 512, 513, 992,
+EDGES = (1, 2, 16, 17, 32, 33, 36, 64, 65, 72, 128, 129, 144, 256, 257, 288, 289, 384, 385, 511, 512, 513, 768, 992,
          1023, 1024, 1025, 1280, 2047, 2048, 2049, 4095, 4096, 4097, 6144, 8192)
 
 
@@ -71,6 +71,29 @@ def test_batch_size_where_the_form_changes(cuda, n):
     got = _run(cuda, ps, mat, 11, 1)
     want = np.stack(oracle.oracle_sw(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat))
     assert (got == want).all()
+
+
+@pytest.mark.parametrize("n", [300, 1536, 1537, 4096, 4097, 8192, 8193])
+def test_class_edges_at_every_batch_size(cuda, n):
+    # the ends of the length classes again, in the forms that a batch of n takes
+    qs, ss = _edge_pairs(np.random.default_rng(n))
+    rng = np.random.default_rng(n + 1)
+    for k in (17, 64, 65, 128, 129, 256, 257):      # both sides of the subject length in the rule
+        for m in (3071, 3072):
+            q = rng.integers(0, 25, k).astype(np.int8)
+            s = rng.integers(0, 25, m).astype(np.int8)
+            s[-k:] = q
+            qs.append(q)
+            ss.append(s)
+    fill = synth.sw_pairs(n - len(qs), seed=n, q_range=(1, 300), q_median=60, s_range=(0, 200), s_median=60)
+    qs += [fill.q[o:o + k] for o, k in zip(fill.qoff, fill.qlen)]
+    ss += [fill.s[o:o + k] for o, k in zip(fill.soff, fill.slen)]
+    ps, mat = _pairs(qs, ss), synth.matrix("BLOSUM62")
+    assert ps.n == n
+    got = _run(cuda, ps, mat, 11, 1)
+    want = np.stack(oracle.oracle_sw(ps.q, ps.qoff, ps.qlen, ps.s, ps.soff, ps.slen, mat))
+    bad = np.flatnonzero((got != want).any(axis=0))
+    assert bad.size == 0, (bad[:5], got[:, bad[:5]], want[:, bad[:5]], ps.qlen[bad[:5]], ps.slen[bad[:5]])
 
 
 def test_drop_at_16_bits_in_every_form(cuda):

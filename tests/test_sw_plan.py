@@ -14,7 +14,7 @@ SHIM = """
 #include "sw_plan.h"
 using namespace tpz::sw;
 extern "C" {
-int t_row_bin(int ql, int sl, int small, int steps) { return row_bin(ql, sl, small, steps); }
+int t_row_bin(int ql, int sl, int64_t pairs, int steps) { return row_bin(ql, sl, forms_of(pairs), steps); }
 int t_group_lanes(int ql) { return group_lanes(ql); }
 int64_t t_boundary_blocks(int64_t want, int classes, int64_t cols, int sms) {
     return boundary_blocks(want, classes, cols, sms);
@@ -38,6 +38,7 @@ def plan(tmp_path_factory):
     lib = ctypes.CDLL(so)
     lib.t_boundary_blocks.restype = lib.t_boundary_bytes.restype = ctypes.c_int64
     lib.t_boundary_blocks.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
+    lib.t_row_bin.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
     lib.t_grid_blocks.argtypes = [ctypes.c_int64] * 4
     return lib
 
@@ -47,20 +48,24 @@ def _rows_lanes(b):
         return b + 9, 32
     if b < 48:
         return (b - 24) % 8 + 9, (16, 8, 4)[(b - 24) // 8]
-    return (4, 8)[b - 48], 4
+    return {48: (4, 4), 49: (8, 4), 55: (4, 8), 56: (8, 8), 57: (8, 16), 58: (8, 32)}[b]
 
 
-def test_every_length_has_a_bin_that_holds_it(plan):
-    for ql in range(1, 8193):
-        b = plan.t_row_bin(ql, 100, 0, 1 << 30)
-        if ql <= 1024:
-            R, G = _rows_lanes(b)
-            assert b < 50 and R * G >= ql and (R <= 16 or G == 32)
-            small = plan.t_row_bin(ql, 100, 1, 1 << 30)
-            assert small in (53, 54) and (small == 54) == (ql > 512)
-        else:
-            assert 50 <= b <= 52 and ql <= (2048, 4096, 8192)[b - 50]
-            assert plan.t_row_bin(ql, 100, 1, 1 << 30) == b
+@pytest.mark.parametrize("pairs,stripe,wide,long_slen", [
+    (1, 0, 0, None), (64, 0, 0, None), (65, 64, 64, None), (1536, 64, 64, None), (1537, 64, 64, 3072),
+    (4096, 64, 64, 3072), (4097, 1024, 64, None), (8192, 1024, 64, None), (8193, 1024, 0, None), (1 << 30, 1024, 0, None)])
+def test_every_length_has_a_bin_that_holds_it(plan, pairs, stripe, wide, long_slen):
+    for sl in (0, 100, 3071, 3072, 1 << 23):
+        for ql in range(1, 8193):
+            b = plan.t_row_bin(ql, sl, pairs, 1 << 30)
+            is_wide = 16 < ql <= wide or (64 < ql <= 256 and long_slen is not None and sl >= long_slen)
+            if ql > 1024:
+                assert 50 <= b <= 52 and ql <= (2048, 4096, 8192)[b - 50]
+            elif ql > stripe and not is_wide:
+                assert b == (53 if ql <= 512 else 54)
+            else:
+                R, G = _rows_lanes(b)
+                assert R * G >= ql and (R <= 16 or G == 32) and (b >= 55) == is_wide
 
 
 @pytest.mark.parametrize("floor,entry", [(76, 11), (97, 15), (238, 17), (373, 64), (637, 127), (513, 127), (65, 1)])
@@ -69,8 +74,8 @@ def test_pairs_past_16_bits_have_their_words_to_themselves(plan, floor, entry):
     assert floor + steps * entry <= 65535 < floor + (steps + 1) * entry
     for n in (1, 30, 100, 400, 505, 512, 513, 516, 517, 1000, 1024):
         for m in (0, 100, 505, 513, 517, 1024, 5000):
-            b = plan.t_row_bin(n, m, 0, steps)
-            assert (b >= 50) == (min(n, m) * entry + floor > 65535)
+            b = plan.t_row_bin(n, m, 1 << 20, steps)
+            assert (b in (53, 54)) == (min(n, m) * entry + floor > 65535)
     assert plan.t_shared_steps(floor, 0) == plan.t_shared_steps(floor, -3) == 2 ** 31 - 1
 
 

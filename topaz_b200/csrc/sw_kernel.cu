@@ -9,12 +9,13 @@
 // its u16x2 words, lane t owning query rows [t*R, t*R + R) of both.  Subject
 // columns stream through a group's lanes as a wavefront, lane t working on
 // column k - t at step k, with H and F of a lane's last row handed to lane
-// t + 1 by __shfl_up_sync.  G is the smallest group that keeps R <= 32, so R
-// is 17..32 for every query above 64 residues: the wavefront's fill (G - 1
-// steps) and the per-step work outside the rows (shuffles, letters, maximum
-// test) shrink against the rows, and a query pads to G*R rows, at most G - 1
-// more than it has.  Groups of a warp take pairs of neighbouring subject
-// lengths.
+// t + 1 by __shfl_up_sync.  G is the smallest group that keeps R <= 16 (32
+// above 512 residues; batches of up to 8,192 pairs take more lanes for short
+// queries, see sw_plan.h): the wavefront's fill (G - 1 steps) and the per-step
+// work outside the rows (shuffles, letters, maximum test) shrink against the
+// rows, more rows would leave fewer warps, and a query pads to G*R rows, at
+// most G - 1 more than it has.  Groups of a warp take pairs of neighbouring
+// subject lengths.
 //
 // Query-major form (the hits of one search query): the same, with a block of
 // 8 warps sharing one profile.  Queries above 1024 residues take the pairs
@@ -563,13 +564,14 @@ struct BinArgs {
     int64_t n;               // pairs 0..n-1, or list[0..n)
     const int32_t *list;
     const int32_t *qlen, *slen;
-    int max_qlen, small_batch;
+    int max_qlen;
+    Forms forms;             // of the batch's size
     int steps;               // shared_steps of the scoring
 };
 
 __device__ __forceinline__ int pair_bin(const BinArgs &b, int ql, int sl) {
     const int sb = min(sl >> 5, kSBins - 1);
-    return row_bin(ql, sl, b.small_batch, b.steps) * kSBins + (kSBins - 1 - sb);      // long subjects first
+    return row_bin(ql, sl, b.forms, b.steps) * kSBins + (kSBins - 1 - sb);      // long subjects first
 }
 
 __global__ void bin_count_kernel(BinArgs b, int32_t *counts, int32_t *status) {
@@ -678,6 +680,7 @@ static void fill_bin(Kernels &k) {
         s.bin[s.n] = bin; s.rows[s.n] = rows; s.lanes[s.n++] = lanes;
     };
     if (R1 == 8) {
+        for (int w = 3; w >= 0; --w) add(kWideBin + w, w ? 8 : 4, w ? 4 << w : 8);
         add(kTinyBin + 1, 8, 4);
         add(kTinyBin, 4, 4);
         return;
@@ -810,16 +813,18 @@ static thread_local int64_t g_last_launches = 0;
 
 int64_t &last_launches() { return g_last_launches; }
 
-// A batch of up to this many pairs takes the stripe form for every query: it
-// would leave most warps idle with two pairs and more per warp, and its time
-// is that of its longest pair.  Stripe form against by-pair, pairs of the
-// microbench: 128 pairs 0.28 / 0.41 ms, 1,024 0.32 / 0.54, 2,048 0.45 / 0.55,
-// 4,096 0.51 / 0.63, 8,192 0.80 / 0.81.
-constexpr int64_t kSmallBatch = 4096;
-
 // scratch words of one call: counts and cursor per bin, [start, count] and a
 // task counter per row bin, then the sorted pair ids
 constexpr size_t kBinWords = 2 * (size_t)kBins + 3 * kRBins;
+
+// Blocks per SM of by-pair kernel i, 0 where a batch of these forms has no
+// pairs for it: small batches only for the one of up to 8 rows, and that with
+// 8 blocks, so that some hundred tasks do not end up on a few SMs (3,000
+// pairs of 10 x 5000: 0.70 ms, 0.84 with 12).
+static int bin_blocks(const Kernels *k, int e, int i, Forms f) {
+    if (f.stripe >= kStripeRows) return k->bin_blocks[e][i];
+    return f.wide > 0 && i == kBinKernels - 1 ? std::min(8, k->bin_blocks[e][i]) : 0;
+}
 
 static unsigned grid_of(int blocks_per_sm, int64_t n) {
     return grid_blocks(sm_count(), blocks_per_sm, n, INT64_MAX);
@@ -829,9 +834,9 @@ static unsigned grid_of(int blocks_per_sm, int64_t n) {
 static size_t batch_snap_words(const Kernels *k, int64_t n, int max_qlen) {
     size_t sum = 0;
     if (max_qlen > kStripeRows) sum += (size_t)grid_of(k->stripe32_blocks[1], n) * kLongWarps * snap_words(kMaxR);
-    if (n > kSmallBatch)
-        for (int i = 0; i < kBinKernels; ++i)
-            sum += (size_t)grid_of(k->bin_blocks[1][i], n) * snap_words(k->set[i].rows[0]);
+    for (int i = 0; i < kBinKernels; ++i)
+        if (const int per_sm = bin_blocks(k, 1, i, forms_of(n)))
+            sum += (size_t)grid_of(per_sm, n) * snap_words(k->set[i].rows[0]);
     return sum;
 }
 
@@ -861,8 +866,8 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
     int32_t *counts = ws, *cursor = counts + kBins, *rinfo = cursor + kBins;
     int32_t *next_task = rinfo + 2 * kRBins, *sorted = ws + kBinWords;
     a.sorted = sorted; a.rinfo = rinfo; a.next_task = next_task;
-    const bool small_batch = n <= kSmallBatch;
-    BinArgs b{n, list, a.qlen, a.slen, max_qlen, small_batch ? 1 : 0, a.steps};
+    const Forms f = forms_of(n);
+    BinArgs b{n, list, a.qlen, a.slen, max_qlen, f, a.steps};
     TPZ_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * kBins, st));
     const int gb = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)nsm * 8));
     bin_count_kernel<<<gb, 256, 0, st>>>(b, counts, a.status);
@@ -887,20 +892,20 @@ static int launch_batch(const Kernels *k, Streams *x, Args &a, int64_t n, const 
         if (ends && x) a.snap += (size_t)blocks * words;
     }
     // (in a large batch: the pairs that have to have their words to themselves)
-    if (small_batch || std::min(max_qlen, kStripeRows) > a.steps) {
+    if (f.stripe < kStripeRows || std::min(max_qlen, kStripeRows) > a.steps) {
         const StripeSet s{2, {kSmallBin + 1, kSmallBin, 0}, {2, 1, 0}, {4, 2, 0}};
         k->stripe8[e]<<<grid_of(k->stripe8_blocks[e], n), 32 * kLongWarps, stripe_smem(8, kLongWarps),
                         next_stream()>>>(a, s);
         ++launches;
     }
-    if (!small_batch) {
-        for (int i = 0; i < kBinKernels; ++i) {
-            const int words = snap_words(k->set[i].rows[0]);
-            const unsigned blocks = grid(k->bin_blocks[e][i], words);
-            k->bin[e][i]<<<blocks, 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
-            ++launches;
-            if (ends && x) a.snap += (size_t)blocks * words;
-        }
+    for (int i = 0; i < kBinKernels; ++i) {
+        const int per_sm = bin_blocks(k, e, i, f);
+        if (per_sm == 0) continue;
+        const int words = snap_words(k->set[i].rows[0]);
+        const unsigned blocks = grid(per_sm, words);
+        k->bin[e][i]<<<blocks, 32, k->bin_smem[i], next_stream()>>>(a, k->set[i]);
+        ++launches;
+        if (ends && x) a.snap += (size_t)blocks * words;
     }
     // the join comes after every launch, also on an error, so that the
     // caller's stream waits for all kernels before it frees their buffers
