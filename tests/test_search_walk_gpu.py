@@ -3,8 +3,9 @@ pops that cross blocks of chain elements (rows 8, 32, 64, ... on), rises of
 hits already listed, capacities around a batch of 32 pops, evictions at one
 and over several scores, stops at -S inside a batch, and cursor counts of
 every shared-memory class up to the one that spills -- pop by pop against
-the oracle, on a database of protein families (long runs of similar rows);
-and the extensions they rest on, at every kind of end."""
+the oracle, with the hits' Smith-Waterman columns, on a database of protein
+families (long runs of similar rows); and the extensions they rest on, at
+every kind of end."""
 import numpy as np
 import pytest
 
@@ -34,9 +35,11 @@ def family_db():
     db = make_db(synth.Proteins(["p%d" % i for i in range(len(seqs))], [seqs[i] for i in order]))
     qs = [members[i] for i in rng.choice(len(members), 10, replace=False)]
     qs += [synth.random_residues(rng, n) for n in (5, 6, 7, 37, 260, 261, 600)]
-    # capacity 1.5 * num_hits above 3000 residues; cursors in global memory
-    # above 4505
-    qs += [np.concatenate([members[3], synth.random_residues(rng, 1700)]),
+    # capacity 1.5 * num_hits above 3000 residues; two cursors per searched
+    # position: classes of 512, 1,024, 2,048 (600 residues above), 3,072 (1,300)
+    # and 5,600 (1,700 and more), in global memory above 2,805
+    qs += [synth.random_residues(rng, 1300),
+           np.concatenate([members[3], synth.random_residues(rng, 1700)]),
            np.concatenate([synth.random_residues(rng, 3000), members[40]]),
            np.concatenate([synth.random_residues(rng, 4500), members[200]])]
     return db, [ab.aa_to_internal(s).tobytes() for s in qs]
@@ -63,6 +66,9 @@ def test_every_pop_and_hit(cuda, family_db, seeds, aligns, num_hits):
         assert list(r["gapless_score"][a:b]) == [h.gapless_score for h in hits]
         assert list(r["gapless_length"][a:b]) == [h.gapless_length for h in hits]
         assert list(r["suffix_offset"][a:b]) == [h.suffix_offset for h in hits]
+        on = [i for i, h in enumerate(hits) if h.gapless_score >= 40]
+        for ours, name in (("sw_status", "status"), ("rawscore", "rawscore"), ("qend", "qend"), ("send", "send")):
+            assert [int(r[ours][a + i]) for i in on] == [getattr(hits[i], name) for i in on], (q, name)
         longest = max(longest, npops)
     if seeds == 300000:
         assert r["refill_elems"] > 0 and longest > 2000
