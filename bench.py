@@ -261,7 +261,7 @@ def extension_roofline(chain_elems, chain_ms, refill_elems, pops):
             "frac": round(ach / peak, 3) if ach and peak else None, "peak_source": src,
             "bytes_per_call": "8 B SA entry + up to 8 x 32 B text sectors",
             "computed_over_used": round((chain_elems + refill_elems) / max(pops, 1), 2),
-            "l2_hit_rate": "profiles/search_kernels_small.md (ncu)"}
+            "l2_hit_rate": "profiles/search_and_sw_kernels.md (ncu)"}
 
 
 _HBM_LIVE = []
@@ -409,9 +409,12 @@ def search_bench(args, dev):
     for t in th:
         t.join()
     torch.cuda.synchronize()
+    # seed and chain kernel times from a batch with the device to itself: the
+    # event intervals of overlapping batches hold other batches' kernels too
+    solo = ix.search(warm, mat, report=report)
     stage = np.zeros(4)
     nh = [0]
-    swc = [0, 0, 0.0, 0.0, 0, 0, 0]
+    swc = [0, 0]
     pops = []
     starts = list(range(0, len(q_aa), bsz))
     lock = threading.Lock()
@@ -431,11 +434,6 @@ def search_bench(args, dev):
                 nh[0] += len(r["protein"])
                 swc[0] += r["sw_pairs"]
                 swc[1] += r["sw_cells"]
-                swc[2] += r["seed_ms"]
-                swc[3] += r["chain_ms"]
-                swc[4] += r["positions"]
-                swc[5] += r["chain_elems"]
-                swc[6] += r["refill_elems"]
                 pops.extend(r["npops"].tolist())
 
     t0 = time.perf_counter()
@@ -461,8 +459,9 @@ def search_bench(args, dev):
            "reported_hits_per_query": round(nh / len(q_aa), 2),
            "sw_pairs_per_query": round(swc[0] / len(q_aa), 1),
            "sw_gcells": round(swc[1] / 1e9, 2),
-           "seed_lookup": seed_roofline(swc[4], swc[2], len(db.T)),
-           "extension": extension_roofline(swc[5], swc[3], swc[6], int(np.sum(pops))),
+           "seed_lookup": seed_roofline(solo["positions"], solo["seed_ms"], len(db.T)),
+           "extension": extension_roofline(solo["chain_elems"], solo["chain_ms"], solo["refill_elems"],
+                                           int(solo["npops"].sum())),
            "pops_per_query": {"mean": round(float(np.mean(pops)), 1),
                               "p50": int(np.percentile(pops, 50)), "p99": int(np.percentile(pops, 99)),
                               "max": int(np.max(pops))},
@@ -862,7 +861,7 @@ def native_arm(args, rank, local_rank, world):
                          "traffic": (round(traffic_per_cell * cells) if traffic_per_cell else None),
                          "traffic_source": ("not measured in this run: DRAM bytes per cell of the "
                                             "ncu capture in profiles/sw_microbench_traffic.txt "
-                                            "(100,000-pair case), scaled to this step's cells"
+                                            "(200,000-pair case), scaled to this step's cells"
                                             if traffic_per_cell else None)},
             "cpu_baseline": cpu,
             "per_pair_gpu": per_pair,

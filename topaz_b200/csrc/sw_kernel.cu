@@ -353,9 +353,10 @@ __device__ __forceinline__ void run_chunk_rows(const Args &a, const Chunk &ch, c
 }
 
 // One launch for the chunks of all row counts (the longest chunks first):
-// every R fits the 128 registers of two blocks per SM, so a chunk's end is
-// filled by whatever chunk comes next.  (A launch per R over 8 streams left
-// the SMs of a 1000-query batch half empty at each launch's end.)
+// two blocks per SM share the registers (128 a thread: with scores alone the
+// largest R spill nothing, 24 bytes in stripes, with ends 20 and 228), so a
+// chunk's end is filled by whatever chunk comes next.  (A launch per R over 8
+// streams left the SMs of a 1000-query batch half empty at each launch's end.)
 template <bool ENDS, bool STRIPED>
 __global__ void __launch_bounds__(kQmWarps * 32, 2) sw_query_kernel(const __grid_constant__ Args a,
                                                                     const QmArgs g) {
@@ -1525,7 +1526,7 @@ extern "C" int tpz_sw_batch_device_noalloc(int64_t n, const int8_t *q, const int
     // the stated matrix limit of this call
     int mx = 0;
     for (int i = 0; i < 625; ++i) mx = std::max<int>(mx, mat625_host[i]);
-    if ((int64_t)kNoAllocMaxQlen * mx >= std::min(32767 - 2 * std::max(mx, 1), kBig)) {
+    if ((int64_t)kNoAllocMaxQlen * mx >= kBig) {
         char buf[200];
         snprintf(buf, sizeof buf,
                  "tpz_sw_batch_device_noalloc: largest matrix entry %d is too large for exact "
